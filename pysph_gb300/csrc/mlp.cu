@@ -52,7 +52,8 @@ constexpr int OFF_W1 = SPH_MLP_OFF_W1, OFF_B1 = SPH_MLP_OFF_B1, OFF_W2 = SPH_MLP
 constexpr int TILE = 128;
 constexpr int THREADS = 256;   // two warps per tensor-memory lane quarter
 constexpr int L3_PART = NOUT * NH + NOUT;   // third-layer partial per block
-constexpr int L3_ROWS = 1024;               // rows per third-layer block
+constexpr int L3_ROWS = 64;                 // rows per third-layer tile
+constexpr int L3_THREADS = 256;
 constexpr int kMaxSpin = 1 << 22;           // bounded mbarrier wait
 // per-CTA partial gradients of the backward: rows of PART_STRIDE floats
 // (16-byte aligned)
@@ -1553,47 +1554,106 @@ __global__ void __launch_bounds__(R_THREADS, 1)
 }
 
 // third layer: dW3 [o][j] = sum_b dy[b][o] h2[b][j], db3 = sum_b dy
-__global__ void k_mlp_l3(const uint16_t *__restrict__ h2s, const float *__restrict__ dy,
-                         int64_t n, float *__restrict__ part) {
-    const int j = threadIdx.x;   // 128 threads
-    const int64_t r0 = (int64_t)blockIdx.x * L3_ROWS;
-    const int64_t r1 = min(n, r0 + L3_ROWS);
-    float a0 = 0.f, a1 = 0.f, s0 = 0.f, s1 = 0.f;
-    for (int64_t b = r0; b < r1; ++b) {
-        const float h = __uint_as_float((uint32_t)h2s[b * NH + j] << 16);
-        const float d0 = dy[b * 2], d1 = dy[b * 2 + 1];
-        a0 = fmaf(d0, h, a0);
-        a1 = fmaf(d1, h, a1);
-        s0 += d0;
-        s1 += d1;
+//
+// HBM-bound: 264 B per sample (h2 as BF16, dy), 4 FLOP per h2 value.  A
+// half-warp reads one row of h2 as sixteen 16-byte loads, so a block has
+// sixteen rows in flight per step (four steps unrolled), and every thread
+// keeps the 2 x 8 sums of its columns; the sixteen row groups are added in a
+// fixed order at the end.  Blocks take tiles of L3_ROWS rows round-robin, so
+// a minibatch of 8 192 spreads over 128 blocks.  (One thread per column and
+// 1 024 rows per block left a minibatch on 8 blocks, each a serial chain of
+// two-byte loads: 177 us against 5.4 us at 8 192 samples, cold cache.)
+// A caller's h2 off the 16-byte grid is read value by value (ALIGNED = false).
+template <bool ALIGNED>
+__global__ void __launch_bounds__(L3_THREADS)
+k_mlp_l3(const uint16_t *__restrict__ h2s, const float2 *__restrict__ dy, int64_t n,
+         float *__restrict__ part) {
+    constexpr int GROUPS = L3_THREADS / 16;      // rows per step
+    constexpr int STEPS = L3_ROWS / GROUPS;
+    __shared__ float s_a[GROUPS][NOUT * NH + 4];
+    __shared__ float2 s_d[GROUPS];
+    const int c = threadIdx.x & 15;              // columns 8 c .. 8 c + 7
+    const int r = threadIdx.x >> 4;
+    float a0[8], a1[8];
+    float2 sd = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) a0[i] = a1[i] = 0.f;
+    for (int64_t t = blockIdx.x; t * L3_ROWS < n; t += gridDim.x) {
+#pragma unroll
+        for (int st = 0; st < STEPS; ++st) {
+            const int64_t b = t * L3_ROWS + st * GROUPS + r;
+            if (b < n) {
+                const uint16_t *row = h2s + b * NH + 8 * c;
+                uint32_t w[4];
+                if (ALIGNED) {
+                    const uint4 h = __ldg(reinterpret_cast<const uint4 *>(row));
+                    w[0] = h.x; w[1] = h.y; w[2] = h.z; w[3] = h.w;
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        w[i] = (uint32_t)row[2 * i] | ((uint32_t)row[2 * i + 1] << 16);
+                }
+                const float2 d = __ldg(dy + b);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float lo = bf_lo(w[i]), hi = bf_hi(w[i]);
+                    a0[2 * i] = fmaf(d.x, lo, a0[2 * i]);
+                    a0[2 * i + 1] = fmaf(d.x, hi, a0[2 * i + 1]);
+                    a1[2 * i] = fmaf(d.y, lo, a1[2 * i]);
+                    a1[2 * i + 1] = fmaf(d.y, hi, a1[2 * i + 1]);
+                }
+                sd.x += d.x;
+                sd.y += d.y;
+            }
+        }
     }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        s_a[r][8 * c + i] = a0[i];
+        s_a[r][NH + 8 * c + i] = a1[i];
+    }
+    if (c == 0) s_d[r] = sd;
+    __syncthreads();
     float *P = part + (int64_t)blockIdx.x * L3_PART;
-    P[j] = a0;
-    P[NH + j] = a1;
-    if (j == 0) {
-        P[2 * NH] = s0;
-        P[2 * NH + 1] = s1;
+    for (int j = threadIdx.x; j < L3_PART; j += L3_THREADS) {
+        float v = 0.f;
+#pragma unroll
+        for (int q = 0; q < GROUPS; ++q)
+            v += j < NOUT * NH ? s_a[q][j] : (j == NOUT * NH ? s_d[q].x : s_d[q].y);
+        P[j] = v;
     }
 }
 
-// grad[p] = sum over CTAs (fixed order) of the partials
-__global__ void k_mlp_reduce(const float *__restrict__ part, int nparts,
-                             const float *__restrict__ l3, int nl3,
-                             const float *__restrict__ part_loss, float *__restrict__ grad,
-                             float *__restrict__ loss) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+// grad[p] = sum over CTAs (fixed order) of the partials: four threads per
+// parameter take every fourth partial (a chain of loads a quarter as long),
+// their sums added in a fixed order.
+constexpr int RED_PARAMS = 64;       // parameters per block of 256 threads
+__global__ void __launch_bounds__(4 * RED_PARAMS)
+k_mlp_reduce(const float *__restrict__ part, int nparts, const float *__restrict__ l3, int nl3,
+             const float *__restrict__ part_loss, float *__restrict__ grad,
+             float *__restrict__ loss) {
+    __shared__ float s_s[4][RED_PARAMS];
+    const int k = threadIdx.x % RED_PARAMS, q = threadIdx.x / RED_PARAMS;
+    const int p = blockIdx.x * RED_PARAMS + k;
+    const float *src = nullptr;
+    int64_t stride = 0;
+    int count = 0;
     if (p < OFF_W3) {
-        float s = 0.f;
-        for (int c = 0; c < nparts; ++c) s += part[(int64_t)c * PART_STRIDE + p];
-        grad[p] = s;
+        src = part + p; stride = PART_STRIDE; count = nparts;
     } else if (p < NPARAM) {
-        float s = 0.f;
-        for (int c = 0; c < nl3; ++c) s += l3[(int64_t)c * L3_PART + (p - OFF_W3)];
-        grad[p] = s;
-    } else if (p == NPARAM && loss) {
-        float s = 0.f;
-        for (int c = 0; c < nparts; ++c) s += part_loss[c];
-        *loss = s;
+        src = l3 + (p - OFF_W3); stride = L3_PART; count = nl3;
+    } else if (p == NPARAM) {
+        src = part_loss; stride = 1; count = nparts;
+    }
+    float s = 0.f;
+#pragma unroll 8
+    for (int c = q; c < count; c += 4) s += __ldg(src + c * stride);
+    s_s[q][k] = s;
+    __syncthreads();
+    if (q == 0) {
+        const float v = ((s_s[0][k] + s_s[1][k]) + s_s[2][k]) + s_s[3][k];
+        if (p < NPARAM) grad[p] = v;
+        else if (p == NPARAM && loss) *loss = v;
     }
 }
 
@@ -1772,10 +1832,17 @@ int mlp_grid(int64_t n) {
     return (int)std::max<int64_t>(1, std::min<int64_t>(tiles, g_num_sms));
 }
 
+// third-layer blocks: one per tile of rows, at most four per SM (a million
+// samples keep 32 warps of loads in flight per SM, and the partials that
+// k_mlp_reduce adds stay few)
+static int l3_blocks(int64_t n) {
+    const int64_t tiles = (n + L3_ROWS - 1) / L3_ROWS;
+    return (int)std::max<int64_t>(1, std::min<int64_t>(tiles, 4 * (int64_t)g_num_sms));
+}
+
 int64_t mlp_backward_scratch(int64_t n) {
     const int grid = mlp_grid(n);
-    const int64_t nl3 = (n + L3_ROWS - 1) / L3_ROWS;
-    return (int64_t)grid * PART_STRIDE + std::max<int64_t>(nl3, 1) * L3_PART + grid + 2 * n + 4;
+    return (int64_t)grid * PART_STRIDE + (int64_t)l3_blocks(n) * L3_PART + grid + 2 * n + 4;
 }
 
 int mlp_sync(const sph_mlp_model *M, cudaStream_t st) {
@@ -1820,7 +1887,7 @@ int mlp_backward(const sph_mlp_model *M, const uint16_t *x, const uint16_t *h1, 
         return set_error(SPH_ERR_ARG, "mlp backward: buffers must be 16-byte aligned");
     SPH_CUDA(init_attrs());
     const int grid = mlp_grid(n);
-    const int nl3 = (int)std::max<int64_t>(1, (n + L3_ROWS - 1) / L3_ROWS);
+    const int nl3 = l3_blocks(n);
     float *part = scratch;
     float *l3 = part + (int64_t)grid * PART_STRIDE;
     float *part_loss = l3 + (int64_t)nl3 * L3_PART;
@@ -1843,10 +1910,13 @@ int mlp_backward(const sph_mlp_model *M, const uint16_t *x, const uint16_t *h1, 
         count_launch();
         SPH_LAUNCH_CHECK("k_mlp_bwd_tma");
     }
-    k_mlp_l3<<<nl3, NH, 0, st>>>(h2, dy, n, l3);
+    if (aligned16(h2))
+        k_mlp_l3<true><<<nl3, L3_THREADS, 0, st>>>(h2, reinterpret_cast<const float2 *>(dy), n, l3);
+    else
+        k_mlp_l3<false><<<nl3, L3_THREADS, 0, st>>>(h2, reinterpret_cast<const float2 *>(dy), n, l3);
     count_launch();
     SPH_LAUNCH_CHECK("k_mlp_l3");
-    k_mlp_reduce<<<(NPARAM + 1 + 255) / 256, 256, 0, st>>>(part, grid, l3, nl3, part_loss, grad, loss);
+    k_mlp_reduce<<<(NPARAM + RED_PARAMS) / RED_PARAMS, 4 * RED_PARAMS, 0, st>>>(part, grid, l3, nl3, part_loss, grad, loss);
     count_launch();
     SPH_LAUNCH_CHECK("k_mlp_reduce");
     return SPH_OK;

@@ -86,6 +86,34 @@ def test_gradient_matches_oracle(n):
     assert abs(float(loss.item()) - lr) / lr < 1e-4
 
 
+@pytest.mark.parametrize("n,shift", [(1, 0), (63, 0), (64, 0), (65, 0), (1000, 0), (1000, 1),
+                                     (39000, 0), (39000, 3)])
+def test_third_layer_gradient(n, shift):
+    """dW3 = dy^T h2 and db3 = sum dy at the edges of the kernel's row tiles
+    (64 rows) and past one tile per block (38 912 rows at 608 blocks), with
+    h2 on and off the 16-byte grid.  Bound: a value passes at most 200 FP32
+    additions (tiles of a block, row groups, partials) and dy two roundings."""
+    _need_gpu()
+    model, _ = _model(3)
+    xg, _ = _x(n, 4)
+    tg = torch.tensor(np.random.default_rng(5).normal(0, 1, (n, M.NOUT)), dtype=torch.float32,
+                      device="cuda")
+    y, cache = model.forward(xg, save=True)
+    room = torch.empty(n * M.NH + 8, dtype=torch.bfloat16, device="cuda")
+    h2 = room[shift:shift + n * M.NH].view(n, M.NH)
+    h2.copy_(cache["h2"])
+    g, _ = model.backward(xg, dict(cache, h2=h2), y, tg)
+    g = g.double().cpu().numpy()
+    dy = ((y.double() - tg.double()) / n).cpu().numpy()
+    h = cache["h2"].double().cpu().numpy()
+    eps = 204 * 2.0 ** -24
+    w3, b3 = g[M.OFF_W3:M.OFF_B3].reshape(M.NOUT, M.NH), g[M.OFF_B3:M.NPARAM]
+    # y - t carries half an ulp of its operands' size
+    slack = 2.0 ** -23 * (np.abs(y.cpu().numpy()) + np.abs(tg.cpu().numpy())) / n
+    assert np.all(np.abs(w3 - dy.T @ h) <= eps * (np.abs(dy).T @ np.abs(h)) + slack.T @ np.abs(h))
+    assert np.all(np.abs(b3 - dy.sum(0)) <= eps * np.abs(dy).sum(0) + slack.sum(0))
+
+
 def test_gradient_deterministic():
     _need_gpu()
     model, _ = _model(6)
