@@ -24,6 +24,20 @@
 // (index T, just past the staged records): the pair loop needs no bounds
 // predicates.
 //
+// The tables of a block -- the slots and cells of its sources and of its
+// destinations -- are written once per full build (k_brick_count,
+// k_brick_fill), so a pass reads where its records are instead of deriving
+// it: the passes are bound by instruction issue, and finding the records from
+// the cell table in every block (a scan, a binary search and two divisions
+// per record) was nearly half of their instructions.  At 1 M particles (3D
+// lattice, 61 neighbours) density 151 -> 115 us, rates 255 -> 213 us.
+//
+// Small simulations do not fill the GPU with a thread per destination: there
+// S = 2 or 4 neighbouring threads (lanes) share a destination, lane s takes
+// the list's groups s, s + S, ..., and the groups' sums are folded in the
+// list's order (shuffles), so the result is the same bit for bit; the bricks
+// are divided into parts (blocks of their own, with the brick's origin).
+//
 // The neighbour relation is the reference's: strict r^2 < (radius_scale
 // h)^2, decided in FP32 outside a +-1e-5 relative band around the threshold
 // and by the FP64 test of base/nnps.pyx:337-353 inside it.  Neighbours are
@@ -49,27 +63,29 @@ namespace {
 // population rounded to warps); the kernels are compiled for at most this
 constexpr int kBrickMaxThreads = 512;
 
+// an array as the sources of a pass
 struct BrickSrcDev {
     const float4 *pm, *velh, *st;
     const float *scx;
     const int *cstart, *perm;
+    const int4 *bsrc;
+    const int2 *brow, *bstage;
     const double *x, *y, *z;
 };
 
+// an array as the destinations of a pass
 struct BrickDstDev {
     const float4 *pm, *velh, *st;
-    const float *scx;
-    const int *cstart, *perm;
-    const int *bdst;       // exclusive prefix of the destinations per brick
+    const int *perm;
+    const int2 *bdst, *bdest;
     const int64_t *tag;
-    const double *x, *y, *z, *h, *u, *v, *w, *p, *cs;
+    const double *x, *y, *z, *u, *v, *w, *p, *cs;
 };
 
 // shared-memory layout of a block (byte offsets into the dynamic array)
 struct BrickSmem {
-    int stage_cap;   // staged records (0: records are read from global memory)
-    int off_v, off_s;             // rates: velocity / state records
-    int off_rlo, off_roff, off_dlo, off_doff, off_scell;
+    int off_v, off_s;   // rates: velocity / state records
+    int off_scell;      // list build: cell table
 };
 
 // The neighbour radius of a uniform h, computed on the host with the
@@ -92,7 +108,6 @@ struct BrickDensityArgs {
     int *cnt;           // neighbour count per destination, brick order
     int *maxcnt;
     int cap;
-    int build;          // 1: traverse the stencil and write the list
     int write_out;      // 0: list build only
     int dim, tait;
     float co, ro, gamma;
@@ -110,6 +125,7 @@ struct BrickRatesArgs {
     BrickRadius rad;
     const uint16_t *nbr;
     const int *cnt;
+    const int *maxcnt;
     int cap;
     int dim;
     float alpha, beta, eta2, eps;
@@ -125,15 +141,29 @@ struct BrickRatesArgs {
     const unsigned *gate;
 };
 
-// The block's cells: brick [x0, x1) x [y0, y1) x [z0, z1), the staged
-// region [xs0, xs1) x ... (the brick grown by the stencil half-widths,
-// clipped to the grid) and the origin cell of the staged positions.
+// The block's cells: its part [x0, x1) x [y0, y1) x [z0, z1) of a brick, the
+// staged region [xs0, xs1) x ... (the part grown by the stencil half-widths,
+// clipped to the grid) and the origin cell of the staged positions (the
+// centre of the whole brick).
 struct BlockGeo {
     int x0, x1, y0, y1, z0, z1;
-    int xs0, xs1, ys0, ys1, zs0, zs1;
-    int lx, ry, nr, dry, ndr;
+    int xs0, ys0, zs0, xs1, ys1, zs1;
+    int lx, ry, nr;
     int cxc, cyc, czc;
 };
+
+// part i of the bricks of e cells (each in p parts) along an axis of n cells
+__device__ __forceinline__ void axis_part(int n, int e, int p, int i, int k, int &lo, int &hi,
+                                          int &slo, int &shi, int &centre) {
+    const int brick = i / p, part = i - brick * p;
+    const int b0 = brick * e;
+    const int q = e / p, rem = e - q * p;
+    lo = min(n, b0 + part * q + min(part, rem));
+    hi = min(n, lo + q + (part < rem ? 1 : 0));
+    slo = max(0, lo - k);
+    shi = min(n, hi + k);
+    centre = b0 + e / 2;
+}
 
 __device__ __forceinline__ BlockGeo block_geo(const Grid &g, const BrickGeom &bk, int b) {
     BlockGeo G;
@@ -141,136 +171,45 @@ __device__ __forceinline__ BlockGeo block_geo(const Grid &g, const BrickGeom &bk
     const int rest = b / bk.nbx;
     const int iby = rest % bk.nby;
     const int ibz = rest / bk.nby;
-    G.x0 = ibx * bk.bx; G.x1 = min(g.nx, G.x0 + bk.bx);
-    G.y0 = iby * bk.by; G.y1 = min(g.ny, G.y0 + bk.by);
-    G.z0 = ibz * bk.bz; G.z1 = min(g.nz, G.z0 + bk.bz);
-    G.xs0 = max(0, G.x0 - g.kx); G.xs1 = min(g.nx, G.x1 + g.kx);
-    G.ys0 = max(0, G.y0 - g.ky); G.ys1 = min(g.ny, G.y1 + g.ky);
-    G.zs0 = max(0, G.z0 - g.kz); G.zs1 = min(g.nz, G.z1 + g.kz);
+    axis_part(g.nx, bk.bx, bk.px, ibx, g.kx, G.x0, G.x1, G.xs0, G.xs1, G.cxc);
+    axis_part(g.ny, bk.by, bk.py, iby, g.ky, G.y0, G.y1, G.ys0, G.ys1, G.cyc);
+    axis_part(g.nz, bk.bz, bk.pz, ibz, g.kz, G.z0, G.z1, G.zs0, G.zs1, G.czc);
     G.lx = G.xs1 - G.xs0;
     G.ry = G.ys1 - G.ys0;
     G.nr = G.ry * (G.zs1 - G.zs0);
-    G.dry = G.y1 - G.y0;
-    G.ndr = G.dry * (G.z1 - G.z0);
-    G.cxc = G.x0 + bk.bx / 2;
-    G.cyc = G.y0 + bk.by / 2;
-    G.czc = G.z0 + bk.bz / 2;
     return G;
 }
 
-// In-place inclusive scan of a[1..n] by one warp (a[0] = 0 on return).
-__device__ __forceinline__ void warp_scan_inplace(int *a, int n) {
-    const int lane = threadIdx.x & 31;
-    int carry = 0;
-    for (int base = 1; base <= n; base += 32) {
-        const int i = base + lane;
-        int x = i <= n ? a[i] : 0;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, x, off);
-            if (lane >= off) x += y;
-        }
-        if (i <= n) a[i] = x + carry;
-        carry += __shfl_sync(0xffffffffu, x, 31);
-    }
-    if (lane == 0) a[0] = 0;
+// A brow entry: first sorted slot of the row's staged cells, staging offset
+// and length (both below 65 535 wherever the tables are used).
+__device__ __forceinline__ int row_off(const int2 &e) { return (int)((unsigned)e.y & 0xffffu); }
+__device__ __forceinline__ int row_len(const int2 &e) { return (int)((unsigned)e.y >> 16); }
+
+// A bstage or bdest entry: sorted slot and cell relative to the origin cell,
+// 128 added to each coordinate (a byte each; a brick spans at most 64 cells
+// and three more on either side).
+__device__ __forceinline__ int pack_cell(int cx, int cy, int cz) {
+    return (cx + 128) | ((cy + 128) << 8) | ((cz + 128) << 16);
+}
+template <int C>
+__device__ __forceinline__ int cell_int(int code) { return ((code >> (8 * C)) & 0xff) - 128; }
+// the same as a float: the byte OR-ed into the bits of 2^23, less 2^23 + 128
+template <int C>
+__device__ __forceinline__ float cell_float(int code) {
+    return __uint_as_float(__byte_perm((unsigned)code, 0x4B000000u, 0x7540u | C)) - 8388736.f;
 }
 
-// Largest r in [0, n) with off[r] <= t (off[n] > t): the row holding index t.
-__device__ __forceinline__ int row_of(const int *off, int n, int t) {
-    int lo = 0, hi = n;
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (off[mid] <= t) lo = mid; else hi = mid;
-    }
-    return lo;
-}
-
-// Position record (brick-relative x, y, z and the mass) of sorted slot j of
-// row (cy, cz): the same FP32 operations for destinations and sources.
-__device__ __forceinline__ float4 rel_pos(const float4 *pm, const float *scx, int j, int cy,
-                                          int cz, const BlockGeo &G, float csf) {
-    const float4 p = pm[j];
-    return make_float4(fmaf(scx[j] - (float)G.cxc, csf, p.x),
-                       fmaf((float)(cy - G.cyc), csf, p.y),
-                       fmaf((float)(cz - G.czc), csf, p.z), p.w);
-}
-
-// Tables of a block: source rows (slot of the row's first staged cell and
-// the staging offset of each row) and destination rows (the brick's rows of
-// the destination array).  Returns the staged count and the destinations.
-__device__ __forceinline__ void block_tables(const Grid &g, const BlockGeo &G, const int *scst,
-                                             const int *dcst, int *rlo, int *roff, int *dlo,
-                                             int *doff, int &T, int &D) {
-    const int nt = blockDim.x;
-    const int rowz = g.nx * g.ny;
-    for (int r = threadIdx.x; r < G.nr; r += nt) {
-        const int cy = G.ys0 + r % G.ry, cz = G.zs0 + r / G.ry;
-        const int c = cz * rowz + cy * g.nx + G.xs0;
-        const int lo = scst[c];
-        rlo[r] = lo;
-        roff[r + 1] = scst[c + G.lx] - lo;
-    }
-    for (int q = threadIdx.x; q < G.ndr; q += nt) {
-        const int cy = G.y0 + q % G.dry, cz = G.z0 + q / G.dry;
-        const int c = cz * rowz + cy * g.nx + G.x0;
-        const int lo = dcst[c];
-        dlo[q] = lo;
-        doff[q + 1] = dcst[c + (G.x1 - G.x0)] - lo;
-    }
-    __syncthreads();
-    const int wid = threadIdx.x >> 5;
-    if (wid == 0) warp_scan_inplace(roff, G.nr);
-    if (wid == (nt > 32 ? 1 : 0)) warp_scan_inplace(doff, G.ndr);
-    __syncthreads();
-    T = roff[G.nr];
-    D = doff[G.ndr];
-}
-
-// Staging offset of the first particle of every cell of every source row
-// (scell[r * (lx + 1) + i], i = 0 .. lx): the ranges a stencil traversal
-// visits.
-__device__ __forceinline__ void cell_table(const Grid &g, const BlockGeo &G, const int *scst,
-                                           const int *rlo, const int *roff, int *scell) {
-    const int w = G.lx + 1;
-    const int rowz = g.nx * g.ny;
-    for (int idx = threadIdx.x; idx < G.nr * w; idx += blockDim.x) {
-        const int r = idx / w, i = idx - r * w;
-        const int cy = G.ys0 + r % G.ry, cz = G.zs0 + r / G.ry;
-        scell[idx] = roff[r] + (scst[cz * rowz + cy * g.nx + G.xs0 + i] - rlo[r]);
-    }
-}
-
-// Sorted slot and row of staging index t (records read from global memory).
-__device__ __forceinline__ int staged_slot(const BlockGeo &G, const int *rlo, const int *roff,
-                                           int t, int &cy, int &cz) {
-    const int r = row_of(roff, G.nr, t);
-    cy = G.ys0 + r % G.ry;
-    cz = G.zs0 + r / G.ry;
-    return rlo[r] + (t - roff[r]);
+// Position record (brick-relative x, y, z and the mass) of record p in the
+// cell of a table entry: the same FP32 operations for destinations and
+// sources.
+__device__ __forceinline__ float4 rel_pos(const float4 &p, int code, float csf) {
+    return make_float4(fmaf(cell_float<0>(code), csf, p.x), fmaf(cell_float<1>(code), csf, p.y),
+                       fmaf(cell_float<2>(code), csf, p.z), p.w);
 }
 
 // The dynamic shared memory of the brick kernels: the staged records from
-// byte 0, then the block's tables.
+// byte 0, then the cell table of a list build.
 extern __shared__ __align__(16) unsigned char brick_smem[];
-
-// Table pointers and the state records' offset in the dynamic shared memory.
-struct SmemPtrs {
-    uint32_t voff, soff;
-    int *rlo, *roff, *dlo, *doff, *scell;
-};
-
-__device__ __forceinline__ SmemPtrs smem_ptrs(unsigned char *base, const BrickSmem &sm) {
-    SmemPtrs p;
-    p.voff = (uint32_t)sm.off_v;
-    p.soff = (uint32_t)sm.off_s;
-    p.rlo = reinterpret_cast<int *>(base + sm.off_rlo);
-    p.roff = reinterpret_cast<int *>(base + sm.off_roff);
-    p.dlo = reinterpret_cast<int *>(base + sm.off_dlo);
-    p.doff = reinterpret_cast<int *>(base + sm.off_doff);
-    p.scell = reinterpret_cast<int *>(base + sm.off_scell);
-    return p;
-}
 
 // The padding record (index T): far away, zero mass, at rest -- every pair
 // term with it is exactly 0.
@@ -284,7 +223,7 @@ __device__ __forceinline__ float2 pad_rstate() { return make_float2(0.f, 0.f); }
 // Source records: staged in shared memory, or (STAGED = false, a brick
 // more populous than the shared memory holds) recomputed from the sorted
 // arrays with the same operations.
-template <bool STAGED, int PSH>
+template <bool STAGED>
 struct SrcRecords;
 
 // Staged: the position record of source t at byte 16 t of the shared
@@ -297,8 +236,8 @@ struct SrcRecords;
 // A rates pass whose block has one source mass and whose cs follows Tait
 // (FAST) reads the first two only: the state record's 8-byte read was a
 // fifth of the shared-memory wavefronts of a pair.
-template <int PSH>
-struct SrcRecords<true, PSH> {
+template <>
+struct SrcRecords<true> {
     uint32_t voff, soff;
     __device__ __forceinline__ float4 pos(int t) const {
         return *reinterpret_cast<const float4 *>(brick_smem + ((uint32_t)t << 4));
@@ -322,19 +261,17 @@ struct SrcRecords<true, PSH> {
 };
 
 // recomputed from the sorted arrays with the staging's operations
-template <int PSH>
-struct SrcRecords<false, PSH> {
+template <>
+struct SrcRecords<false> {
     const BrickSrcDev *src;
-    BlockGeo G;
-    const int *rlo, *roff;
+    const int2 *tab;
     float csf;
     int T;
     float halpha;
     __device__ __forceinline__ float4 pos(int t) const {
         if (t >= T) return pad_pos();
-        int cy, cz;
-        const int j = staged_slot(G, rlo, roff, t, cy, cz);
-        return rel_pos(src->pm, src->scx, j, cy, cz, G, csf);
+        const int2 e = tab[t];
+        return rel_pos(src->pm[e.x], e.y, csf);
     }
     template <bool FAST>
     __device__ __forceinline__ void rates_rec(int t, float, float, float4 &p, float4 &v, float &mj,
@@ -346,9 +283,9 @@ struct SrcRecords<false, PSH> {
             hac = 0.f;
             return;
         }
-        int cy, cz;
-        const int j = staged_slot(G, rlo, roff, t, cy, cz);
-        p = rel_pos(src->pm, src->scx, j, cy, cz, G, csf);
+        const int2 e = tab[t];
+        const int j = e.x;
+        p = rel_pos(src->pm[j], e.y, csf);
         const float4 vh = src->velh[j], st = src->st[j];
         mj = p.w;
         p.w = 0.5f * st.x;
@@ -357,58 +294,114 @@ struct SrcRecords<false, PSH> {
     }
 };
 
-template <bool STAGED, int PSH>
-__device__ __forceinline__ SrcRecords<STAGED, PSH> make_records(const SmemPtrs &sp,
-                                                                const BrickSrcDev &S,
-                                                                const BlockGeo &G, float csf,
-                                                                int T, float halpha) {
+template <bool STAGED>
+__device__ __forceinline__ SrcRecords<STAGED> make_records(const BrickSmem &sm, const BrickSrcDev &S,
+                                                           float csf, const int2 *tab, int T,
+                                                           float halpha) {
     if constexpr (STAGED)
-        return SrcRecords<true, PSH>{sp.voff, sp.soff};
+        return SrcRecords<true>{(uint32_t)sm.off_v, (uint32_t)sm.off_s};
     else
-        return SrcRecords<false, PSH>{&S, G, sp.rlo, sp.roff, csf, T, halpha};
+        return SrcRecords<false>{&S, tab, csf, T, halpha};
+}
+
+// Asynchronous copies from global to shared memory (completed by the issuing
+// thread's cp_async_wait): 16 and 8 bytes.
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async8(uint32_t dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 // Copy the block's source records into shared memory (the layout of
-// SrcRecords<true, .>).  Rates records: (x, y, z, rho / 2), (u, v, w,
-// p / rho^2) and (m, alpha cs / 2), with the halves that the pair averages
-// of the artificial viscosity add.  Returns whether every record this
-// thread staged has mass mref.
+// SrcRecords<true>).  The raw records (position; rates: velocity, rho and
+// p / rho^2) are copied asynchronously, so that a thread has all its copies in
+// flight and holds none in registers; then every thread finishes the records
+// that it copied: the position from the block's origin cell, and in the rates
+// pass (x, y, z, rho / 2), (u, v, w, p / rho^2) and, with STATE, (m, alpha cs /
+// 2), with the halves that the pair averages of the artificial viscosity add.
+// Returns whether every record this thread staged has mass mref.
 template <bool RATES>
-__device__ __forceinline__ bool stage(const BrickSrcDev &S, const BlockGeo &G, const int *rlo,
-                                      const int *roff, int T, float csf, uint32_t voff,
-                                      uint32_t soff, float halpha = 0.f, float mref = 0.f) {
-    bool same = true;
-    // unrolled so that several records' loads are in flight at once
-#pragma unroll 4
-    for (int t = threadIdx.x; t <= T; t += blockDim.x) {
-        float4 *prec = reinterpret_cast<float4 *>(brick_smem + ((uint32_t)t << 4));
-        float4 *vrec = reinterpret_cast<float4 *>(brick_smem + voff + ((uint32_t)t << 4));
-        float2 *srec = reinterpret_cast<float2 *>(brick_smem + soff + ((uint32_t)t << 3));
-        if (t == T) {
-            // the padding record after the staged ones
-            if (RATES) {
-                *prec = pad_rpos();
-                *vrec = pad_vel();
-                *srec = pad_rstate();
-            } else {
-                *prec = pad_pos();
-            }
-            continue;
-        }
-        int cy, cz;
-        const int j = staged_slot(G, rlo, roff, t, cy, cz);
-        const float4 pr = rel_pos(S.pm, S.scx, j, cy, cz, G, csf);
+__device__ __forceinline__ bool stage(const BrickSrcDev &S, const int2 *tab, int T, float csf,
+                                      const BrickSmem &sm, bool state, float halpha, float mref) {
+    constexpr int U = 6;        // records of a thread in flight
+    const uint32_t base = (uint32_t)__cvta_generic_to_shared(brick_smem);
+    const uint32_t vb = base + sm.off_v, sb = base + sm.off_s;
+    const int nt = blockDim.x;
+    if (threadIdx.x == 0) {
+        // the padding record after the staged ones
+        *reinterpret_cast<float4 *>(brick_smem + ((uint32_t)T << 4)) = RATES ? pad_rpos() : pad_pos();
         if (RATES) {
-            const float4 vh = S.velh[j], st = S.st[j];
-            *prec = make_float4(pr.x, pr.y, pr.z, 0.5f * st.x);
-            *vrec = make_float4(vh.x, vh.y, vh.z, st.y);
-            *srec = make_float2(pr.w, halpha * st.z);
-            same = same && pr.w == mref;
-        } else {
-            *prec = pr;
+            *reinterpret_cast<float4 *>(brick_smem + sm.off_v + ((uint32_t)T << 4)) = pad_vel();
+            *reinterpret_cast<float2 *>(brick_smem + sm.off_s + ((uint32_t)T << 3)) = pad_rstate();
+        }
+    }
+    bool same = true;
+    for (int t0 = threadIdx.x; t0 < T; t0 += U * nt) {
+        int2 e[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (t0 + u * nt < T) e[u] = tab[t0 + u * nt];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint32_t t = (uint32_t)(t0 + u * nt);
+            if (t < (uint32_t)T) {
+                cp_async16(base + (t << 4), S.pm + e[u].x);
+                if (RATES) {
+                    cp_async16(vb + (t << 4), S.velh + e[u].x);
+                    cp_async8(sb + (t << 3), S.st + e[u].x);
+                }
+            }
+        }
+        cp_async_wait();
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const uint32_t t = (uint32_t)(t0 + u * nt);
+            if (t < (uint32_t)T) {
+                float4 *prec = reinterpret_cast<float4 *>(brick_smem + (t << 4));
+                float4 pr = rel_pos(*prec, e[u].y, csf);
+                if (RATES) {
+                    float2 *srec = reinterpret_cast<float2 *>(brick_smem + sm.off_s + (t << 3));
+                    const float2 rp = *srec;
+                    same = same && pr.w == mref;
+                    if (state) *srec = make_float2(pr.w, halpha * S.st[e[u].x].z);
+                    *reinterpret_cast<float *>(brick_smem + sm.off_v + (t << 4) + 12) = rp.y;
+                    pr.w = 0.5f * rp.x;
+                }
+                *prec = pr;
+            }
         }
     }
     return same;
+}
+
+// The state records (m, alpha cs / 2) of a block whose sources turned out not
+// to share one mass.
+__device__ __noinline__ void stage_state(const BrickSrcDev &S, const int2 *tab, int T, uint32_t soff,
+                                         float halpha) {
+    for (int t = threadIdx.x; t < T; t += blockDim.x) {
+        const int j = tab[t].x;
+        *reinterpret_cast<float2 *>(brick_smem + soff + ((uint32_t)t << 3)) =
+            make_float2(S.pm[j].w, halpha * S.st[j].z);
+    }
+}
+
+// Staging offset of the first particle of every cell of every staged row
+// (scell[r * (lx + 1) + i], i = 0 .. lx): the ranges a stencil traversal
+// visits.
+__device__ __forceinline__ void cell_table(const Grid &g, const BlockGeo &G, const int *scst,
+                                           const int2 *brow, int *scell) {
+    const int w = G.lx + 1;
+    const int rowz = g.nx * g.ny;
+    for (int idx = threadIdx.x; idx < G.nr * w; idx += blockDim.x) {
+        const int r = idx / w, i = idx - r * w;
+        const int cy = G.ys0 + r % G.ry, cz = G.zs0 + r / G.ry;
+        const int2 e = brow[r];
+        scell[idx] = row_off(e) + (scst[cz * rowz + cy * g.nx + G.xs0 + i] - e.x);
+    }
 }
 
 // The 16-bit entry i (0..7) of a group.
@@ -417,97 +410,110 @@ __device__ __forceinline__ int group_entry(const uint4 &q, int i) {
     return (int)((i & 1) ? (w >> 16) : (w & 0xffffu));
 }
 
-// One destination of the block.
+// One destination of the block: slot, original index, cell, the cell-local
+// offsets that prune the stencil and the brick-relative position and mass.
 struct BrickDest {
-    int s;          // sorted slot
-    int orig;       // original index
-    int cx, cy, cz; // build cell
-    float xi_x, xi_y, xi_z;     // cell-local offsets (stencil pruning)
-    float4 P;       // brick-relative position, mass
-    float r2lo, r2hi, r2list;
-    double radius2;
+    int s, orig;
+    int cx, cy, cz;
+    float4 xi, P;
 };
 
-__device__ __forceinline__ bool brick_dest(const Grid &g, const BrickDstDev &D, const BlockGeo &G,
-                                           const BrickRadius &rad, const int *dlo,
-                                           const int *doff, int d, BrickDest &q) {
-    const int r = row_of(doff, G.ndr, d);
-    q.s = dlo[r] + (d - doff[r]);
-    q.cy = G.y0 + r % G.dry;
-    q.cz = G.z0 + r / G.dry;
+__device__ __forceinline__ BrickDest brick_dest(const BrickDstDev &D, const BlockGeo &G, float csf,
+                                                const int2 &e) {
+    BrickDest q;
+    q.s = e.x;
+    q.cx = G.cxc + cell_int<0>(e.y);
+    q.cy = G.cyc + cell_int<1>(e.y);
+    q.cz = G.czc + cell_int<2>(e.y);
     q.orig = D.perm[q.s];
-    const float4 p = D.pm[q.s];
-    q.xi_x = p.x; q.xi_y = p.y; q.xi_z = p.z;
-    q.cx = (int)D.scx[q.s];
-    q.P = rel_pos(D.pm, D.scx, q.s, q.cy, q.cz, G, g.cs_f);
-    q.radius2 = rad.radius2;
-    q.r2lo = rad.r2lo;
-    q.r2hi = rad.r2hi;
-    q.r2list = rad.r2list;
-    return D.tag == nullptr || D.tag[q.orig] == SPH_TAG_LOCAL_REAL;
+    q.xi = D.pm[q.s];
+    q.P = rel_pos(q.xi, e.y, csf);
+    return q;
 }
 
-// Visit the listed sources of destination q in the staged records, in the
-// order of the list-streaming kernels: stencil rows in (dz, dy) order, each
-// clipped to the chord of the search sphere, ascending slot within a row.
-// fn(t, rx, ry, rz, hit): staging index, r = x_dest - x_src, neighbour or
-// (with a list skin) only within the list radius.  The ranges come from the
-// block's cell table (scell) or, without one, from the grid's cell table.
-template <int K, bool STAGED, int PSH, class Fn>
-__device__ __forceinline__ void brick_traverse(const Grid &g, const BlockGeo &G, const BrickSrcDev &S,
-                                               const BrickDstDev &D, const SrcRecords<STAGED, PSH> &R,
-                                               const int *rlo, const int *roff, const int *scell,
-                                               const BrickDest &q, Fn &&fn) {
+__device__ __forceinline__ bool is_real(const BrickDstDev &D, int orig) {
+    return D.tag == nullptr || D.tag[orig] == SPH_TAG_LOCAL_REAL;
+}
+
+// FP64 neighbour test of a source slot, inside the FP32 band
+__device__ __noinline__ bool exact_hit(const BrickSrcDev &S, const BrickDstDev &D, int slot, int orig,
+                                       double radius2) {
+    const int oj = S.perm[slot];
+    return exact_within(ld0(S.x, oj), ld0(S.y, oj), ld0(S.z, oj), ld0(D.x, orig), ld0(D.y, orig),
+                        ld0(D.z, orig), radius2);
+}
+
+// Visit the sources of destination q that its list holds, in the staged
+// records, in the order of the list-streaming kernels: stencil rows [r0, r1)
+// in (dz, dy) order, each clipped to the chord of the search sphere,
+// ascending slot within a row.  fn(t, r2): staging index and the FP32 squared
+// distance.  With a list skin every source within the list radius is listed,
+// without one the neighbours.  The ranges come from the block's cell table
+// (scell) or, without one, from the grid's cell table.
+template <bool SKIN, bool STAGED, class Fn>
+__device__ __forceinline__ void brick_rows(const Grid &g, const BlockGeo &G, const BrickSrcDev &S,
+                                               const BrickDstDev &D, const SrcRecords<STAGED> &R,
+                                               const BrickRadius &rad, const int2 *brow,
+                                               const int2 *tab, const int *scell,
+                                               const BrickDest &q, int r0, int r1,
+                                               Fn &&fn) {
     const float csf = g.cs_f;
     const float inv_cs = 1.f / csf;
-    const float R2 = fmaxf(q.r2hi, q.r2list) * 1.0002f;
+    const float R2 = fmaxf(rad.r2hi, rad.r2list) * 1.0002f;
+    // listed below rl, without a skin up to r2hi where the FP64 test says so
+    const float rl = SKIN ? rad.r2list : rad.r2lo;
     const int w = G.lx + 1;
+    const int K = g.kx, wy = 2 * g.ky + 1;
 #pragma unroll 1
-    for (int dz = -g.kz; dz <= g.kz; ++dz) {
-        const int czz = q.cz + dz;
-        if (czz < G.zs0 || czz >= G.zs1) continue;
-        const float ez = fmaxf(0.f, dz > 0 ? (float)dz * csf - q.xi_z
-                                           : (dz < 0 ? q.xi_z - (float)(dz + 1) * csf : 0.f));
-        const float ez2 = ez * ez;
-        if (ez2 > R2) continue;
-#pragma unroll 1
-        for (int dy = -g.ky; dy <= g.ky; ++dy) {
-            const int cyy = q.cy + dy;
-            if (cyy < G.ys0 || cyy >= G.ys1) continue;
-            const float ey = fmaxf(0.f, dy > 0 ? (float)dy * csf - q.xi_y
-                                               : (dy < 0 ? q.xi_y - (float)(dy + 1) * csf : 0.f));
-            const float rem = R2 - fmaf(ey, ey, ez2);
-            if (rem < 0.f) continue;
-            const float half = fmaf(rem * rsqrtf(fmaxf(rem, 1e-30f)), 1.0001f, 1e-5f * csf);
-            const int tlo = max(-K, __float2int_rd((q.xi_x - half) * inv_cs));
-            const int thi = min(K, __float2int_rd((q.xi_x + half) * inv_cs));
-            const int clo = max(q.cx + tlo, G.xs0);
-            const int chi = min(q.cx + thi, G.xs1 - 1);
-            if (clo > chi) continue;
-            const int rr = (cyy - G.ys0) + G.ry * (czz - G.zs0);
-            int ta, tb;
-            if (scell != nullptr) {
-                ta = scell[rr * w + (clo - G.xs0)];
-                tb = scell[rr * w + (chi + 1 - G.xs0)];
-            } else {
-                const int c = (czz * g.ny + cyy) * g.nx;
-                ta = roff[rr] + (__ldg(S.cstart + c + clo) - rlo[rr]);
-                tb = roff[rr] + (__ldg(S.cstart + c + chi + 1) - rlo[rr]);
-            }
-            for (int t = ta; t < tb; ++t) {
-                const float4 pj = R.pos(t);
-                const float rx = q.P.x - pj.x, ry = q.P.y - pj.y, rz = q.P.z - pj.z;
-                const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
-                bool hit = r2 < q.r2lo;
-                if (!hit && r2 <= q.r2hi) {
-                    const int oj = S.perm[rlo[rr] + (t - roff[rr])];
-                    hit = exact_within(ld0(S.x, oj), ld0(S.y, oj), ld0(S.z, oj), ld0(D.x, q.orig),
-                                       ld0(D.y, q.orig), ld0(D.z, q.orig), q.radius2);
-                }
-                if (hit || r2 < q.r2list) fn(t, rx, ry, rz, hit);
-            }
+    for (int rr = r0; rr < r1; ++rr) {
+        const int iz = rr / wy;
+        const int dz = iz - g.kz, dy = rr - iz * wy - g.ky;
+        const int czz = q.cz + dz, cyy = q.cy + dy;
+        if (czz < G.zs0 || czz >= G.zs1 || cyy < G.ys0 || cyy >= G.ys1) continue;
+        const float ez = fmaxf(0.f, dz > 0 ? (float)dz * csf - q.xi.z
+                                           : (dz < 0 ? q.xi.z - (float)(dz + 1) * csf : 0.f));
+        const float ey = fmaxf(0.f, dy > 0 ? (float)dy * csf - q.xi.y
+                                           : (dy < 0 ? q.xi.y - (float)(dy + 1) * csf : 0.f));
+        const float rem = R2 - fmaf(ey, ey, ez * ez);
+        if (rem < 0.f) continue;
+        const float half = fmaf(rem * rsqrtf(fmaxf(rem, 1e-30f)), 1.0001f, 1e-5f * csf);
+        const int tlo = max(-K, __float2int_rd((q.xi.x - half) * inv_cs));
+        const int thi = min(K, __float2int_rd((q.xi.x + half) * inv_cs));
+        const int clo = max(q.cx + tlo, G.xs0);
+        const int chi = min(q.cx + thi, G.xs1 - 1);
+        if (clo > chi) continue;
+        const int r = (cyy - G.ys0) + G.ry * (czz - G.zs0);
+        int ta, tb;
+        if (scell != nullptr) {
+            ta = scell[r * w + (clo - G.xs0)];
+            tb = scell[r * w + (chi + 1 - G.xs0)];
+        } else {
+            const int2 e = brow[r];
+            const int c = (czz * g.ny + cyy) * g.nx;
+            ta = row_off(e) + (__ldg(S.cstart + c + clo) - e.x);
+            tb = row_off(e) + (__ldg(S.cstart + c + chi + 1) - e.x);
+        }
+        for (int t = ta; t < tb; ++t) {
+            const float4 pj = R.pos(t);
+            const float rx = q.P.x - pj.x, ry = q.P.y - pj.y, rz = q.P.z - pj.z;
+            const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
+            bool listed = r2 < rl;
+            if (!SKIN && !listed && r2 <= rad.r2hi)
+                listed = exact_hit(S, D, tab[t].x, q.orig, rad.radius2);
+            if (listed) fn(t, r2);
         }
     }
+}
+
+template <bool STAGED, class Fn>
+__device__ __forceinline__ void brick_traverse(const Grid &g, const BlockGeo &G, const BrickSrcDev &S,
+                                               const BrickDstDev &D, const SrcRecords<STAGED> &R,
+                                               const BrickRadius &rad, const int2 *brow,
+                                               const int2 *tab, const int *scell,
+                                               const BrickDest &q, int r0, int r1,
+                                               Fn &&fn) {
+    if (rad.r2list > 0.f) brick_rows<true, STAGED>(g, G, S, D, R, rad, brow, tab, scell, q, r0, r1, fn);
+    else brick_rows<false, STAGED>(g, G, S, D, R, rad, brow, tab, scell, q, r0, r1, fn);
 }
 
 // Reciprocal square root and reciprocal, flushing subnormal inputs to zero
@@ -522,10 +528,6 @@ __device__ __forceinline__ float rcp_ftz(float x) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
-}
-
-__device__ __forceinline__ bool gate_off(const unsigned *gate) {
-    return gate != nullptr && __ldg(gate) != 0u;
 }
 
 // ---------------------------------------------------------------------------
@@ -545,9 +547,10 @@ __device__ __forceinline__ WCoef w_coef(float fac, float scale) {
 
 __device__ __forceinline__ float w_of(float q, const WCoef &c) {
     const float inner = fmaf(q * q, fmaf(c.i2, q, c.i1), c.i0);
-    const float t = 2.f - q;
+    // (2 - q) clamped at 0: the outer branch is 0 beyond q = 2
+    const float t = fmaxf(2.f - q, 0.f);
     const float outer = c.o * (t * t) * t;
-    return q > 2.f ? 0.f : (q > 1.f ? outer : inner);
+    return q > 1.f ? outer : inner;
 }
 
 __device__ __forceinline__ float density_term(const float4 &pi, const float4 &pj, float ih,
@@ -560,10 +563,12 @@ __device__ __forceinline__ float density_term(const float4 &pi, const float4 &pj
 
 // Density of one destination (the compensated sum hi + lo) and, with
 // Tait, its p and cs; the sorted state record when the pass writes the
-// destination's own properties.
+// destination's own properties.  FP64 values are made by integer operations
+// (f2d_exact): the FP64 pipe sees one addition per destination, not five
+// instructions (8 of the 155 us of this pass at 1 M particles).
 __device__ __forceinline__ void density_store(const BrickDensityArgs &A, int s, int orig, bool real,
-                                              float hi, float lo) {
-    const double r64 = (double)hi + (double)lo;
+                                              float mi, float hi, float lo) {
+    const double r64 = f2d_exact(hi) + f2d_exact(lo);
     if (A.rho_out) A.rho_out[orig] = r64;
     const float rf = hi + lo;
     float pf = 0.f, cf = 0.f;
@@ -577,206 +582,270 @@ __device__ __forceinline__ void density_store(const BrickDensityArgs &A, int s, 
             pf = Bt * expm1f(A.gamma * lr);
             cf = A.co * expf(0.5f * (A.gamma - 1.f) * lr);
         }
-        A.p_out[orig] = (double)pf;
-        A.cs_out[orig] = (double)cf;
+        A.p_out[orig] = f2d_exact(pf);
+        A.cs_out[orig] = f2d_exact(cf);
     }
     if (A.st_out) {
-        const float mi = A.d.pm[s].w;
         if (A.tait) {
             A.st_out[s] = make_float4(rf, pf / (rf * rf), cf, mi);
         } else {
-            const float pold = (float)ld0(A.d.p, orig);
-            A.st_out[s] = make_float4(rf, pold / (rf * rf), (float)ld0(A.d.cs, orig), mi);
+            const float pold = d2f_rn(ld0(A.d.p, orig));
+            A.st_out[s] = make_float4(rf, pold / (rf * rf), d2f_rn(ld0(A.d.cs, orig)), mi);
         }
     }
 }
 
-// What a destination's sums start from: its slot and records, its count
-// and the first two groups of its list.  The first destination of every
-// thread requests these before the block stages its sources, so their
-// latency overlaps the staging.
+// Fold the batches that the S lanes of a destination have just summed into
+// its compensated sum, in the order of the list: every lane adds all S of
+// them, so all hold the sum that one thread would have.
+template <int S>
+__device__ __forceinline__ void fold_lanes(CSum &c, float part) {
+    if (S == 1) {
+        c.add(part);
+    } else {
+        const unsigned mask = ((1u << S) - 1u) << (threadIdx.x & 31 & ~(S - 1));
+#pragma unroll
+        for (int s = 0; s < S; ++s) c.add(__shfl_sync(mask, part, s, S));
+    }
+}
+
+// What a column (a lane of a destination) starts from: the destination's
+// records, its count and the first two groups of the lane.  Every thread
+// requests those of its first column before the block stages its sources, so
+// their latency overlaps the staging.
 struct DestPre {
     int s, orig;    // sorted slot, original index
-    bool real;
     float4 P;       // brick-relative position, mass
     int c;
     uint4 b0, b1;
 };
 
-__device__ __forceinline__ void dest_prefetch(const BrickDstDev &Dd, const Grid &g,
-                                              const BlockGeo &G, const BrickRadius &rad,
-                                              const SmemPtrs &sp, const int *cnt,
-                                              const uint4 *lgrp, int cap, int D, int dbase,
-                                              int d, DestPre &p) {
-    BrickDest q;
-    p.real = brick_dest(g, Dd, G, rad, sp.dlo, sp.doff, d, q);
-    p.s = q.s;
-    p.orig = q.orig;
-    p.P = q.P;
-    p.c = cnt[dbase + d];
-    // every destination owns cap / 8 groups: the first two are read whatever
+template <int S>
+__device__ __forceinline__ void dest_prefetch(const BrickDstDev &Dd, float csf, const int2 &e,
+                                              const int *cnt, const uint4 *lgrp, int cap, int D,
+                                              int d, int lane, DestPre &p) {
+    p.s = e.x;
+    p.orig = Dd.perm[e.x];
+    p.P = rel_pos(Dd.pm[e.x], e.y, csf);
+    p.c = cnt[d];
+    // every destination owns cap / 8 groups: those inside are read whatever
     // the count (used only as far as it reaches)
+    const int ng = cap >> 3;
     const uint4 *lst = lgrp + d;
-    p.b0 = lst[0];
-    p.b1 = cap >= 16 ? lst[D] : make_uint4(0, 0, 0, 0);
+    p.b0 = lane < ng ? lst[(size_t)lane * D] : make_uint4(0, 0, 0, 0);
+    p.b1 = lane + S < ng ? lst[(size_t)(lane + S) * D] : make_uint4(0, 0, 0, 0);
 }
 
-// The density sum of one destination over its list: groups of 8 entries,
-// each requested two groups ahead into one of three rotating buffers.
-template <bool STAGED, int PSH>
-__device__ __forceinline__ void density_group(CSum &rho, const SrcRecords<STAGED, PSH> &R,
+// The density sum of a destination over its groups of 8 entries, every lane
+// taking every S-th group, each requested two ahead into one of three
+// rotating buffers (the loop is unrolled over the three, so no buffer is
+// copied).
+template <int S, bool STAGED>
+__device__ __forceinline__ void density_group(CSum &rho, const SrcRecords<STAGED> &R, bool mine,
                                               const uint4 &grp, const float4 &Pi, float ih,
                                               const WCoef &wc) {
     float part = 0.f;
+    if (S == 1 || mine) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        float4 pj[4];
+        for (int h = 0; h < 2; ++h) {
+            float4 pj[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) pj[i] = R.pos(group_entry(grp, 4 * h + i));
+            for (int i = 0; i < 4; ++i) pj[i] = R.pos(group_entry(grp, 4 * h + i));
 #pragma unroll
-        for (int i = 0; i < 4; ++i) part += density_term(Pi, pj[i], ih, wc);
+            for (int i = 0; i < 4; ++i) part += density_term(Pi, pj[i], ih, wc);
+        }
+    }
+    fold_lanes<S>(rho, part);
+}
+
+template <int S, bool STAGED>
+__device__ __forceinline__ void density_stream(CSum &rho, const SrcRecords<STAGED> &R,
+                                               const uint4 *lst, int D, int ng, int lane,
+                                               const float4 &Pi, float ih, const WCoef &wc, uint4 b0,
+                                               uint4 b1) {
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    const size_t step = (size_t)D;
+    uint4 b2;
+    // g0: the first group of the round, gi: this lane's
+    for (int g0 = 0, gi = lane;;) {
+        if (g0 >= ng) break;
+        b2 = gi + 2 * S < ng ? lst[(gi + 2 * S) * step] : zero;
+        density_group<S, STAGED>(rho, R, gi < ng, b0, Pi, ih, wc);
+        gi += S;
+        if ((g0 += S) >= ng) break;
+        b0 = gi + 2 * S < ng ? lst[(gi + 2 * S) * step] : zero;
+        density_group<S, STAGED>(rho, R, gi < ng, b1, Pi, ih, wc);
+        gi += S;
+        if ((g0 += S) >= ng) break;
+        b1 = gi + 2 * S < ng ? lst[(gi + 2 * S) * step] : zero;
+        density_group<S, STAGED>(rho, R, gi < ng, b2, Pi, ih, wc);
+        gi += S;
+        g0 += S;
+    }
+}
+
+// The list of one destination: its S lanes take consecutive shares of the
+// stencil rows.  One lane: entries are collected eight at a time in a 128-bit
+// shift register (the newest enters at the top) and written as one 16-byte
+// store per group.  Several: each counts its share, a scan over the lanes
+// gives its place in the list, and a second traversal writes the entries.
+// The last group is padded with the zero record.  Returns the list's count.
+template <int S, bool STAGED>
+__device__ __forceinline__ int build_list(const BrickDensityArgs &A, const BlockGeo &G,
+                                          const SrcRecords<STAGED> &R, const int2 *brow,
+                                          const int2 *tab, const int *scell, const BrickDest &q, bool active,
+                                          int lane, int T, uint4 *out, int D) {
+    const int cap = A.cap;
+    const int rows = (2 * A.g.ky + 1) * (2 * A.g.kz + 1);
+    int c = 0;
+    if (S == 1) {
+        if (!active) return 0;
+        uint4 grp = make_uint4(0, 0, 0, 0);
+        auto push = [&](unsigned t) {
+            grp.x = __funnelshift_r(grp.x, grp.y, 16);
+            grp.y = __funnelshift_r(grp.y, grp.z, 16);
+            grp.z = __funnelshift_r(grp.z, grp.w, 16);
+            grp.w = (grp.w >> 16) | (t << 16);
+        };
+        brick_traverse<STAGED>(A.g, G, A.s, A.d, R, A.rad, brow, tab, scell, q, 0, rows,
+            [&](int t, float) {
+                push((unsigned)t);
+                ++c;
+                if ((c & 7) == 0 && c <= cap) out[(size_t)((c >> 3) - 1) * D] = grp;
+            });
+        if (c < cap && (c & 7)) {
+            for (int k = c; k & 7; ++k) push((unsigned)T);
+            out[(size_t)(c >> 3) * D] = grp;
+        }
+        return c;
+    }
+    const int ra = rows * lane / S, rb = rows * (lane + 1) / S;
+    if (active)
+        brick_traverse<STAGED>(A.g, G, A.s, A.d, R, A.rad, brow, tab, scell, q, ra, rb,
+                               [&](int, float) { ++c; });
+    __syncwarp();
+    int end = c;
+#pragma unroll
+    for (int off = 1; off < S; off <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, end, off, S);
+        if (lane >= off) end += y;
+    }
+    const int total = __shfl_sync(0xffffffffu, end, S - 1, S);
+    if (active) {
+        int k = end - c;
+        uint16_t *o16 = reinterpret_cast<uint16_t *>(out);
+        auto write = [&](unsigned t) {
+            if (k < cap) o16[(size_t)(k >> 3) * D * 8 + (k & 7)] = (uint16_t)t;
+            ++k;
+        };
+        brick_traverse<STAGED>(A.g, G, A.s, A.d, R, A.rad, brow, tab, scell, q, ra, rb,
+                               [&](int t, float) { write((unsigned)t); });
+        if (lane == S - 1)
+            while (k & 7) write((unsigned)T);
+    }
+    // the lanes read each other's entries
+    __threadfence_block();
+    __syncwarp();
+    return total;
+}
+
+// The density sum of a list build: plain FP32 batches of 8 neighbours (the
+// listed sources that the skin adds do not count), each folded into the
+// compensated sum; past the list's capacity the traversal goes on.
+template <bool STAGED>
+__device__ __forceinline__ void build_sum(const BrickDensityArgs &A, const BlockGeo &G,
+                                          const SrcRecords<STAGED> &R, const int2 *brow,
+                                          const int2 *tab, const int *scell, const BrickDest &q, int c,
+                                          const uint4 *lst, int D, float ih, const WCoef &wc,
+                                          CSum &rho) {
+    const int cap = A.cap;
+    const float r2lo = A.rad.r2lo, r2hi = A.rad.r2hi;
+    float part = 0.f;
+    int nb = 0;
+    auto add = [&](float r2, float m) {
+        const float r = r2 * rsqrt_ftz(fmaxf(r2, 1e-30f));
+        part += w_of(r * ih, wc) * m;
+        if (++nb == 8) {
+            rho.add(part);
+            part = 0.f;
+            nb = 0;
+        }
+    };
+    auto dist2 = [&](const float4 &pj) {
+        const float rx = q.P.x - pj.x, ry = q.P.y - pj.y, rz = q.P.z - pj.z;
+        return fmaf(rx, rx, fmaf(ry, ry, rz * rz));
+    };
+    const int ng = (min(c, cap) + 7) >> 3;
+    uint4 next = ng > 0 ? lst[0] : make_uint4(0, 0, 0, 0);
+    for (int gi = 0; gi < ng; ++gi) {
+        const uint4 grp = next;
+        if (gi + 1 < ng) next = lst[(size_t)(gi + 1) * D];
+        float r2[8], m[8];
+        unsigned hit = 0, band = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float4 pj = R.pos(group_entry(grp, i));
+            r2[i] = dist2(pj);
+            m[i] = pj.w;
+            if (r2[i] <= r2hi) hit |= 1u << i;
+            if (!(r2[i] < r2lo) && r2[i] <= r2hi) band |= 1u << i;
+        }
+        if (band) {
+#pragma unroll 1
+            for (int i = 0; i < 8; ++i)
+                if ((band >> i) & 1u) {
+                    const unsigned w = i < 2 ? grp.x : (i < 4 ? grp.y : (i < 6 ? grp.z : grp.w));
+                    const int t = (int)((i & 1) ? (w >> 16) : (w & 0xffffu));
+                    if (!exact_hit(A.s, A.d, tab[t].x, q.orig, A.rad.radius2)) hit &= ~(1u << i);
+                }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if ((hit >> i) & 1u) add(r2[i], m[i]);
+    }
+    if (c > cap) {
+        int skip = cap;
+        const int rows = (2 * A.g.ky + 1) * (2 * A.g.kz + 1);
+        brick_traverse<STAGED>(A.g, G, A.s, A.d, R, A.rad, brow, tab, scell, q, 0, rows,
+            [&](int t, float) {
+                if (skip > 0) { --skip; return; }
+                const float4 pj = R.pos(t);
+                const float d2 = dist2(pj);
+                bool hit = d2 < r2lo;
+                if (!hit && d2 <= r2hi)
+                    hit = exact_hit(A.s, A.d, tab[t].x, q.orig, A.rad.radius2);
+                if (hit) add(d2, pj.w);
+            });
     }
     rho.add(part);
 }
 
-template <bool STAGED, int PSH>
-__device__ __forceinline__ void density_stream(CSum &rho, const SrcRecords<STAGED, PSH> &R,
-                                               const uint4 *lst, int D, int ng, const float4 &Pi,
-                                               float ih, const WCoef &wc, uint4 b0, uint4 b1) {
-    const uint4 zero = make_uint4(0, 0, 0, 0);
-    const size_t step = (size_t)D;
-    uint4 b2;
-    for (int gi = 0;;) {
-        if (gi >= ng) break;
-        b2 = gi + 2 < ng ? lst[(gi + 2) * step] : zero;
-        density_group<STAGED>(rho, R, b0, Pi, ih, wc);
-        if (++gi >= ng) break;
-        b0 = gi + 2 < ng ? lst[(gi + 2) * step] : zero;
-        density_group<STAGED>(rho, R, b1, Pi, ih, wc);
-        if (++gi >= ng) break;
-        b1 = gi + 2 < ng ? lst[(gi + 2) * step] : zero;
-        density_group<STAGED>(rho, R, b2, Pi, ih, wc);
-        ++gi;
-    }
-}
-
-template <int K, bool BUILD, bool STAGED>
-__global__ void __maxnreg__(64) k_bdensity(const __grid_constant__ BrickDensityArgs A) {
-    unsigned char *smem = brick_smem;
-    if (gate_off(A.gate)) return;
+// Destinations with more neighbours than their list holds: the rest come
+// from a traversal that skips the listed ones (in the order of the list
+// build), added to the stored partial density.  A call of its own, so that
+// the passes keep its registers out of their loops.
+template <bool STAGED>
+__device__ __noinline__ void density_rest(const BrickDensityArgs &A) {
     const int b = blockIdx.x;
-    const int nd = A.d.bdst[b + 1] - A.d.bdst[b];
-    if (nd == 0) return;
+    const int2 dh = A.d.bdst[b];
+    const int4 sh = A.s.bsrc[b];
     const Grid &g = A.g;
     const BlockGeo G = block_geo(g, A.bk, b);
-    SmemPtrs sp = smem_ptrs(smem, A.sm);
-    int T, D;
-    block_tables(g, G, A.s.cstart, A.d.cstart, sp.rlo, sp.roff, sp.dlo, sp.doff, T, D);
-    const int dbase = A.d.bdst[b];
-    const int cap = A.cap;            // a multiple of 8
-    const int ng_cap = cap >> 3;
-    // the stencil cell table of a list build (a destination whose neighbours
-    // outgrew the list reads the grid's table instead)
-    int *scell = BUILD ? sp.scell : nullptr;
-    const uint4 *lgrp = reinterpret_cast<const uint4 *>(A.nbr) + (size_t)dbase * ng_cap;
-    // the first destination of this thread, requested before the staging
-    DestPre pre;
-    if (!BUILD && (int)threadIdx.x < D)
-        dest_prefetch(A.d, g, G, A.rad, sp, A.cnt, lgrp, cap, D, dbase, threadIdx.x, pre);
-    if (BUILD) cell_table(g, G, A.s.cstart, sp.rlo, sp.roff, sp.scell);
-    if (STAGED) stage<false>(A.s, G, sp.rlo, sp.roff, T, g.cs_f, sp.voff, sp.soff);
-    __syncthreads();
-    const SrcRecords<STAGED, 4> R = make_records<STAGED, 4>(sp, A.s, G, g.cs_f, T, 0.f);
+    const int2 *brow = A.s.brow + (size_t)b * A.bk.nrmax, *tab = A.s.bstage + sh.y;
+    const SrcRecords<STAGED> R = make_records<STAGED>(A.sm, A.s, g.cs_f, tab, sh.x, 0.f);
     const float ih = __fdividef(1.f, g.h_uniform);
     const float fac = cubic_fac(A.dim, ih);
-    const WCoef wc = w_coef(fac, 1.f);
-    // destination d from its record p (for a list build, the traversal fills it)
-    auto one = [&](int d, DestPre &p) {
-        BrickDest q;
-        if (BUILD) {
-            p.real = brick_dest(g, A.d, G, A.rad, sp.dlo, sp.doff, d, q);
-            p.s = q.s;
-            p.orig = q.orig;
-        }
-        const bool real = p.real;
-        CSum rho;
-        int c = 0;
-        if (real) {
-            if (BUILD) {
-                // entries collected eight at a time in a 128-bit shift
-                // register (the newest enters at the top) and written as
-                // one 16-byte store per group
-                uint4 *out = reinterpret_cast<uint4 *>(A.nbr) + (size_t)dbase * ng_cap + d;
-                uint4 grp = make_uint4(0, 0, 0, 0);
-                auto push = [&](unsigned t) {
-                    grp.x = __funnelshift_r(grp.x, grp.y, 16);
-                    grp.y = __funnelshift_r(grp.y, grp.z, 16);
-                    grp.z = __funnelshift_r(grp.z, grp.w, 16);
-                    grp.w = (grp.w >> 16) | (t << 16);
-                };
-                // neighbours summed in plain FP32 batches of 8 hits, each
-                // batch folded into the compensated sum
-                float part = 0.f;
-                int nb = 0;
-                brick_traverse<K, STAGED>(g, G, A.s, A.d, R, sp.rlo, sp.roff, scell, q,
-                    [&](int t, float rx, float ry, float rz, bool hit) {
-                        if (c < cap) {
-                            push((unsigned)t);
-                            if ((c & 7) == 7) out[(size_t)(c >> 3) * D] = grp;
-                        }
-                        ++c;
-                        if (!hit) return;
-                        const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
-                        const float r = r2 * rsqrt_ftz(fmaxf(r2, 1e-30f));
-                        part += w_of(r * ih, wc) * R.pos(t).w;
-                        if (++nb == 8) {
-                            rho.add(part);
-                            part = 0.f;
-                            nb = 0;
-                        }
-                    });
-                rho.add(part);
-                // pad the last group with the zero record
-                if (c < cap && (c & 7)) {
-                    for (int k = c; k & 7; ++k) push((unsigned)T);
-                    out[(size_t)(c >> 3) * D] = grp;
-                }
-            } else {
-                c = p.c;
-                density_stream<STAGED>(rho, R, lgrp + d, D, (min(c, cap) + 7) >> 3, p.P, ih, wc,
-                                       p.b0, p.b1);
-            }
-        }
-        if (BUILD) {
-            A.cnt[dbase + d] = c;
-            const unsigned act = __activemask();
-            const int wmax = __reduce_max_sync(act, c);
-            if ((threadIdx.x & 31) == (__ffs(act) - 1)) atomicMax(A.maxcnt, wmax);
-        }
-        if (A.write_out)
-            density_store(A, p.s, p.orig, real, real ? rho.hi : 0.f, real ? rho.lo : 0.f);
-    };
-    for (int d = threadIdx.x; d < D; d += blockDim.x) {
-        if (!BUILD && d != (int)threadIdx.x)
-            dest_prefetch(A.d, g, G, A.rad, sp, A.cnt, lgrp, cap, D, dbase, d, pre);
-        one(d, pre);
-    }
-    if constexpr (BUILD) return;
-    if (!A.write_out || A.rho_out == nullptr) return;
-    // destinations with more neighbours than their list holds: the rest
-    // come from a traversal that skips the listed ones (in the order of
-    // the list build), added to the stored partial density
-    for (int d = threadIdx.x; d < D; d += blockDim.x) {
-        if (A.cnt[dbase + d] <= cap) continue;
-        BrickDest q;
-        if (!brick_dest(g, A.d, G, A.rad, sp.dlo, sp.doff, d, q)) continue;
+    const int rows = (2 * g.ky + 1) * (2 * g.kz + 1);
+    __syncthreads();    // the partial densities, another thread's with several lanes
+    for (int d = threadIdx.x; d < dh.x; d += blockDim.x) {
+        if (A.cnt[dh.y + d] <= A.cap) continue;
+        const BrickDest q = brick_dest(A.d, G, g.cs_f, A.d.bdest[dh.y + d]);
+        if (!is_real(A.d, q.orig)) continue;
         CSum rest;
-        int skip = cap;
-        brick_traverse<K, STAGED>(g, G, A.s, A.d, R, sp.rlo, sp.roff, nullptr, q,
-            [&](int t, float rx, float ry, float rz, bool hit) {
+        int skip = A.cap;
+        brick_traverse<STAGED>(g, G, A.s, A.d, R, A.rad, brow, tab, nullptr, q, 0, rows,
+            [&](int t, float r2) {
                 if (skip > 0) { --skip; return; }
-                if (!hit) return;
-                const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
                 const float r = r2 > 0.f ? r2 * rsqrtf(r2) : 0.f;
                 rest.add(cubic_w(r * ih) * fac * R.pos(t).w);
             });
@@ -786,7 +855,122 @@ __global__ void __maxnreg__(64) k_bdensity(const __grid_constant__ BrickDensityA
         const double part = A.rho_out[q.orig];
         const float phi = (float)part;
         tot.merge(phi, (float)(part - (double)phi));
-        density_store(A, q.s, q.orig, true, tot.hi, tot.lo);
+        density_store(A, q.s, q.orig, true, q.P.w, tot.hi, tot.lo);
+    }
+}
+
+// The density of destination d of the block (its prefetched records p).
+template <int S, bool STAGED>
+__device__ __forceinline__ void density_dest(const BrickDensityArgs &A, const SrcRecords<STAGED> &R,
+                                             const uint4 *lst, int D, int lane, const DestPre &p) {
+    const float ih = __fdividef(1.f, A.g.h_uniform);
+    const WCoef wc = w_coef(cubic_fac(A.dim, ih), 1.f);
+    CSum rho;
+    density_stream<S, STAGED>(rho, R, lst, D, (min(p.c, A.cap) + 7) >> 3, lane, p.P, ih, wc, p.b0,
+                              p.b1);
+    if (lane == 0) {
+        const bool real = is_real(A.d, p.orig);
+        density_store(A, p.s, p.orig, real, p.P.w, real ? rho.hi : 0.f, real ? rho.lo : 0.f);
+    }
+}
+
+// Destinations past one per column of the block (few: blocks are launched
+// with the threads of an ordinary brick), shared by four lanes each.  A call
+// of its own, so that the passes keep its registers out of their loops.
+template <bool STAGED>
+__device__ __noinline__ void density_more(const BrickDensityArgs &A, int first) {
+    constexpr int S = 4;
+    const int b = blockIdx.x;
+    const int2 dh = A.d.bdst[b];
+    const int4 sh = A.s.bsrc[b];
+    const SrcRecords<STAGED> R =
+        make_records<STAGED>(A.sm, A.s, A.g.cs_f, A.s.bstage + sh.y, sh.x, 0.f);
+    const uint4 *lgrp = reinterpret_cast<const uint4 *>(A.nbr) + (size_t)dh.y * (A.cap >> 3);
+    const int lane = threadIdx.x % S;
+    for (int d = first + threadIdx.x / S; d < dh.x; d += blockDim.x / S) {
+        DestPre p;
+        dest_prefetch<S>(A.d, A.g.cs_f, A.d.bdest[dh.y + d], A.cnt + dh.y, lgrp, A.cap, dh.x, d,
+                         lane, p);
+        density_dest<S, STAGED>(A, R, lgrp + d, dh.x, lane, p);
+    }
+}
+
+template <int S, bool STAGED>
+__global__ void __maxnreg__(64) k_bdensity(const __grid_constant__ BrickDensityArgs A) {
+    const int b = blockIdx.x;
+    const int2 dh = A.d.bdst[b];        // destinations, first destination
+    const int4 sh = A.s.bsrc[b];        // staged records, their table
+    if (dh.x == 0) return;
+    // read now, tested after the staging: everything up to there only reads
+    // tables and lists of the last build and positions
+    const unsigned off = A.gate != nullptr ? *A.gate : 0u;
+    const int T = sh.x, D = dh.x;
+    const int2 *tab = A.s.bstage + sh.y;
+    const uint4 *lgrp = reinterpret_cast<const uint4 *>(A.nbr) + (size_t)dh.y * (A.cap >> 3);
+    const int lane = threadIdx.x % S, d = threadIdx.x / S;
+    // the destination of this thread, requested before the staging
+    DestPre pre;
+    if (d < D)
+        dest_prefetch<S>(A.d, A.g.cs_f, A.d.bdest[dh.y + d], A.cnt + dh.y, lgrp, A.cap, D, d, lane,
+                         pre);
+    if (STAGED) stage<false>(A.s, tab, T, A.g.cs_f, A.sm, false, 0.f, 0.f);
+    __syncthreads();
+    if (off != 0u) return;
+    const SrcRecords<STAGED> R = make_records<STAGED>(A.sm, A.s, A.g.cs_f, tab, T, 0.f);
+    if (d < D) density_dest<S, STAGED>(A, R, lgrp + d, D, lane, pre);
+    if (D > (int)blockDim.x / S) density_more<STAGED>(A, blockDim.x / S);
+    if (*A.maxcnt > A.cap && A.rho_out != nullptr) density_rest<STAGED>(A);
+}
+
+// List build: every destination's list from a traversal, and (write_out) its
+// density from the list just written.  Bound by issue, half the lanes idle in
+// the traversal (the chords of a warp's destinations differ in length), so
+// that loop only tests and lists; summing in it, under the same divergence,
+// took 790 us at 1 M particles against 626.
+template <int S, bool STAGED>
+__global__ void __maxnreg__(64) k_bbuild(const __grid_constant__ BrickDensityArgs A) {
+    const int b = blockIdx.x;
+    const int2 dh = A.d.bdst[b];
+    const int4 sh = A.s.bsrc[b];
+    if (dh.x == 0) return;
+    const unsigned off = A.gate != nullptr ? *A.gate : 0u;
+    const Grid &g = A.g;
+    const BlockGeo G = block_geo(g, A.bk, b);
+    const int2 *brow = A.s.brow + (size_t)b * A.bk.nrmax, *tab = A.s.bstage + sh.y;
+    const int T = sh.x, D = dh.x;
+    const int cap = A.cap;              // a multiple of 8
+    uint4 *lgrp = reinterpret_cast<uint4 *>(A.nbr) + (size_t)dh.y * (cap >> 3);
+    int *cnt = A.cnt + dh.y;
+    const int2 *bdest = A.d.bdest + dh.y;
+    int *scell = reinterpret_cast<int *>(brick_smem + A.sm.off_scell);
+    const int lane = threadIdx.x % S, d0 = threadIdx.x / S, step = blockDim.x / S;
+    cell_table(g, G, A.s.cstart, brow, scell);
+    if (STAGED) stage<false>(A.s, tab, T, g.cs_f, A.sm, false, 0.f, 0.f);
+    __syncthreads();
+    if (off != 0u) return;
+    const SrcRecords<STAGED> R = make_records<STAGED>(A.sm, A.s, g.cs_f, tab, T, 0.f);
+    // every thread of a warp runs every round (build_list shuffles)
+    for (int r0 = 0; r0 < D; r0 += step) {
+        const int d = r0 + d0;
+        const bool active = d < D;
+        BrickDest q;
+        bool real = false;
+        if (active) {
+            q = brick_dest(A.d, G, g.cs_f, bdest[d]);
+            real = is_real(A.d, q.orig);
+        }
+        const int c = build_list<S, STAGED>(A, G, R, brow, tab, scell, q, real, lane, T, lgrp + d, D);
+        if (!active) continue;
+        if (lane == 0) cnt[d] = c;
+        const unsigned act = __activemask();
+        const int wmax = __reduce_max_sync(act, c);
+        if ((threadIdx.x & 31) == (__ffs(act) - 1)) atomicMax(A.maxcnt, wmax);
+        if (!A.write_out || lane != 0) continue;
+        const float ih = __fdividef(1.f, g.h_uniform);
+        const WCoef wc = w_coef(cubic_fac(A.dim, ih), 1.f);
+        CSum rho;
+        if (real) build_sum<STAGED>(A, G, R, brow, tab, scell, q, c, lgrp + d, D, ih, wc, rho);
+        density_store(A, q.s, q.orig, real, q.P.w, real ? rho.hi : 0.f, real ? rho.lo : 0.f);
     }
 }
 
@@ -866,82 +1050,63 @@ __device__ __forceinline__ void rates_pair(RatesAcc &a, const RatesConst &k, flo
     }
 }
 
-template <bool XSPH>
+template <int S, bool XSPH>
 __device__ __forceinline__ void rates_flush(RatesAcc &a) {
-    a.ax.add(a.pax); a.ay.add(a.pay); a.az.add(a.paz);
+    fold_lanes<S>(a.ax, a.pax); fold_lanes<S>(a.ay, a.pay); fold_lanes<S>(a.az, a.paz);
     a.pax = a.pay = a.paz = 0.f;
     if (XSPH) {
-        a.xx.add(a.pxx); a.xy.add(a.pxy); a.xz.add(a.pxz);
+        fold_lanes<S>(a.xx, a.pxx); fold_lanes<S>(a.xy, a.pxy); fold_lanes<S>(a.xz, a.pxz);
         a.pxx = a.pxy = a.pxz = 0.f;
     }
 }
 
 // The pairs of one group of 8 list entries, records two at a time, then
 // the batch's partial sums folded into the compensated ones.
-template <bool XSPH, bool ETA0, bool FAST, bool STAGED, int PSH>
+template <int S, bool XSPH, bool ETA0, bool FAST, bool STAGED>
 __device__ __forceinline__ void rates_group(RatesAcc &acc, const RatesConst &kc,
-                                            const SrcRecords<STAGED, PSH> &R, const uint4 &grp,
+                                            const SrcRecords<STAGED> &R, bool mine, const uint4 &grp,
                                             const float4 &Pi) {
+    if (S == 1 || mine) {
 #pragma unroll
-    for (int h = 0; h < 4; ++h) {
-        float4 pj[2], vj[2];
-        float mj[2], hac[2];
+        for (int h = 0; h < 4; ++h) {
+            float4 pj[2], vj[2];
+            float mj[2], hac[2];
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
-            R.template rates_rec<FAST>(group_entry(grp, 2 * h + i), kc.mb, kc.tkc, pj[i], vj[i],
-                                       mj[i], hac[i]);
+            for (int i = 0; i < 2; ++i)
+                R.template rates_rec<FAST>(group_entry(grp, 2 * h + i), kc.mb, kc.tkc, pj[i], vj[i],
+                                           mj[i], hac[i]);
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
-            rates_pair<XSPH, ETA0>(acc, kc, Pi.x - pj[i].x, Pi.y - pj[i].y, Pi.z - pj[i].z,
-                                   pj[i], vj[i], mj[i], hac[i]);
+            for (int i = 0; i < 2; ++i)
+                rates_pair<XSPH, ETA0>(acc, kc, Pi.x - pj[i].x, Pi.y - pj[i].y, Pi.z - pj[i].z,
+                                       pj[i], vj[i], mj[i], hac[i]);
+        }
     }
-    rates_flush<XSPH>(acc);
+    rates_flush<S, XSPH>(acc);
 }
 
-// The sums of one destination: its list streamed in groups of 8 entries,
-// each group requested two groups ahead into one of three rotating
-// buffers (the loop body is unrolled over the three, so no buffer is
-// copied).
-template <bool XSPH, bool ETA0, bool FAST, bool STAGED, int PSH>
+// The sums of a destination, its list streamed as in density_stream.
+template <int S, bool XSPH, bool ETA0, bool FAST, bool STAGED>
 __device__ __forceinline__ void rates_stream(RatesAcc &acc, const RatesConst &kc,
-                                             const SrcRecords<STAGED, PSH> &R, const uint4 *lst, int D,
-                                             int ng, const float4 &Pi, uint4 b0, uint4 b1) {
+                                             const SrcRecords<STAGED> &R, const uint4 *lst, int D,
+                                             int ng, int lane, const float4 &Pi, uint4 b0, uint4 b1) {
     const uint4 zero = make_uint4(0, 0, 0, 0);
-    uint4 b2;
     const size_t step = (size_t)D;
-    for (int gi = 0;;) {
-        if (gi >= ng) break;
-        b2 = gi + 2 < ng ? lst[(gi + 2) * step] : zero;
-        rates_group<XSPH, ETA0, FAST, STAGED>(acc, kc, R, b0, Pi);
-        if (++gi >= ng) break;
-        b0 = gi + 2 < ng ? lst[(gi + 2) * step] : zero;
-        rates_group<XSPH, ETA0, FAST, STAGED>(acc, kc, R, b1, Pi);
-        if (++gi >= ng) break;
-        b1 = gi + 2 < ng ? lst[(gi + 2) * step] : zero;
-        rates_group<XSPH, ETA0, FAST, STAGED>(acc, kc, R, b2, Pi);
-        ++gi;
+    uint4 b2;
+    for (int g0 = 0, gi = lane;;) {
+        if (g0 >= ng) break;
+        b2 = gi + 2 * S < ng ? lst[(gi + 2 * S) * step] : zero;
+        rates_group<S, XSPH, ETA0, FAST, STAGED>(acc, kc, R, gi < ng, b0, Pi);
+        gi += S;
+        if ((g0 += S) >= ng) break;
+        b0 = gi + 2 * S < ng ? lst[(gi + 2 * S) * step] : zero;
+        rates_group<S, XSPH, ETA0, FAST, STAGED>(acc, kc, R, gi < ng, b1, Pi);
+        gi += S;
+        if ((g0 += S) >= ng) break;
+        b1 = gi + 2 * S < ng ? lst[(gi + 2 * S) * step] : zero;
+        rates_group<S, XSPH, ETA0, FAST, STAGED>(acc, kc, R, gi < ng, b2, Pi);
+        gi += S;
+        g0 += S;
     }
-}
-
-// Neighbours of destination q past its list's capacity: a traversal that
-// skips the listed ones (in the order of the list build).
-template <int K, bool XSPH, bool ETA0, bool STAGED, int PSH>
-__device__ __forceinline__ void rates_rest(RatesAcc &acc, const RatesConst &kc, const Grid &g,
-                                           const BlockGeo &G, const BrickSrcDev &S,
-                                           const BrickDstDev &D, const SrcRecords<STAGED, PSH> &R,
-                                           const int *rlo, const int *roff, const BrickDest &q,
-                                           int cap) {
-    int skip = cap;
-    brick_traverse<K, STAGED>(g, G, S, D, R, rlo, roff, nullptr, q,
-        [&](int t, float rx, float ry, float rz, bool hit) {
-            if (skip > 0) { --skip; return; }
-            if (!hit) return;
-            float4 pj, vj;
-            float mj, hac;
-            R.template rates_rec<false>(t, 0.f, 0.f, pj, vj, mj, hac);
-            rates_pair<XSPH, ETA0>(acc, kc, rx, ry, rz, pj, vj, mj, hac);
-            rates_flush<XSPH>(acc);
-        });
 }
 
 __device__ __forceinline__ void rates_acc_init(RatesAcc &acc, const float4 &vi, const float4 &st,
@@ -953,70 +1118,72 @@ __device__ __forceinline__ void rates_acc_init(RatesAcc &acc, const float4 &vi, 
     acc.haci = halpha * st.z;
 }
 
-// The sums of destination d (listed part) and their store.
-template <bool XSPH, bool ETA0, bool FAST, bool STAGED, int PSH>
-__device__ __forceinline__ void rates_dest(const BrickRatesArgs &A, const SrcRecords<STAGED, PSH> &R,
-                                           const RatesConst &kc, const uint4 *lgrp, int D, int d,
-                                           const DestPre &pre) {
-    const int cap = A.cap;
-    const bool real = pre.real;
-    RatesAcc acc;
-    rates_acc_init(acc, A.d.velh[pre.s], A.d.st[pre.s], 0.5f * A.alpha);
-    if (real)
-        rates_stream<XSPH, ETA0, FAST, STAGED>(acc, kc, R, lgrp + d, D, (min(pre.c, cap) + 7) >> 3,
-                                         pre.P, pre.b0, pre.b1);
-    const int orig = pre.orig;
-    double a3[3] = {0.0, 0.0, 0.0}, p3[3] = {0.0, 0.0, 0.0};
-    if (real) {
-        // the compensated sums rounded once to FP32 (far below the pair
-        // terms' own FP32 error), one conversion each
-        a3[0] = (double)acc.ax.fvalue(); a3[1] = (double)acc.ay.fvalue();
-        a3[2] = (double)acc.az.fvalue();
-        if (XSPH) {
-            p3[0] = (double)acc.xx.fvalue(); p3[1] = (double)acc.xy.fvalue();
-            p3[2] = (double)acc.xz.fvalue();
+// Store the destination's rates, the six components dealt out to its lanes.
+template <int S, bool XSPH>
+__device__ __forceinline__ void rates_store(const BrickRatesArgs &A, const RatesAcc &acc, int orig,
+                                            int lane) {
+    const bool real = is_real(A.d, orig);
+    auto put = [&](int k, float sum, float shift, const double *vel, double grav) {
+        if (A.acc[k] && (S == 1 || lane == (2 * k) % S)) {
+            // the compensated sum rounded once to FP32 (far below the pair
+            // terms' own FP32 error), then to FP64 by integer operations
+            double v = real ? f2d_exact(sum) : 0.0;
+            if (A.add_gravity && real) v += grav;
+            A.acc[k][orig] = A.accumulate ? A.acc[k][orig] + v : v;
         }
-        if (A.add_gravity) { a3[0] += A.gx; a3[1] += A.gy; a3[2] += A.gz; }
-        if (A.add_velocity) {
-            // exact FP64 velocity of the destination (position_funcs.pyx:47-50)
-            p3[0] += ld0(A.d.u, orig);
-            p3[1] += ld0(A.d.v, orig);
-            p3[2] += ld0(A.d.w, orig);
+        if (A.pos[k] && (S == 1 || lane == (2 * k + 1) % S)) {
+            double v = 0.0;
+            if (real) {
+                if (XSPH) v = f2d_exact(shift);
+                // exact FP64 velocity of the destination (position_funcs.pyx:47-50)
+                if (A.add_velocity) v = XSPH ? v + ld0(vel, orig) : ld0(vel, orig);
+            }
+            A.pos[k][orig] = A.accumulate ? A.pos[k][orig] + v : v;
         }
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        if (A.acc[k]) A.acc[k][orig] = (A.accumulate ? A.acc[k][orig] : 0.0) + a3[k];
-        if (A.pos[k]) A.pos[k][orig] = (A.accumulate ? A.pos[k][orig] : 0.0) + p3[k];
-    }
+    };
+    put(0, acc.ax.fvalue(), acc.xx.fvalue(), A.d.u, A.gx);
+    put(1, acc.ay.fvalue(), acc.xy.fvalue(), A.d.v, A.gy);
+    put(2, acc.az.fvalue(), acc.xz.fvalue(), A.d.w, A.gz);
 }
 
-template <int K, bool XSPH, bool ETA0, bool FAST, bool STAGED, int PSH>
-__device__ __forceinline__ void rates_block(const BrickRatesArgs &A, const Grid &g,
-                                            const BlockGeo &G, const SmemPtrs &sp,
-                                            const SrcRecords<STAGED, PSH> &R, const RatesConst &kc,
-                                            int D, int dbase, const DestPre &first) {
-    const int cap = A.cap;
+// Destinations with more neighbours than their list holds, as density_rest:
+// the rest added to the stored sums.
+template <bool XSPH, bool ETA0, bool STAGED>
+__device__ __noinline__ void rates_rest(const BrickRatesArgs &A) {
+    const int b = blockIdx.x;
+    const int2 dh = A.d.bdst[b];
+    const int4 sh = A.s.bsrc[b];
+    const Grid &g = A.g;
+    const BlockGeo G = block_geo(g, A.bk, b);
+    const int2 *brow = A.s.brow + (size_t)b * A.bk.nrmax, *tab = A.s.bstage + sh.y;
     const float halpha = 0.5f * A.alpha;
-    const uint4 *lgrp = reinterpret_cast<const uint4 *>(A.nbr) + (size_t)dbase * (cap >> 3);
-    // the first destination of the thread from its prefetched record, the
-    // others (bricks with more destinations than threads) as they come
-    if ((int)threadIdx.x < D)
-        rates_dest<XSPH, ETA0, FAST, STAGED>(A, R, kc, lgrp, D, threadIdx.x, first);
-    for (int d = threadIdx.x + blockDim.x; d < D; d += blockDim.x) {
-        DestPre pre;
-        dest_prefetch(A.d, g, G, A.rad, sp, A.cnt, lgrp, cap, D, dbase, d, pre);
-        rates_dest<XSPH, ETA0, FAST, STAGED>(A, R, kc, lgrp, D, d, pre);
+    const SrcRecords<STAGED> R = make_records<STAGED>(A.sm, A.s, g.cs_f, tab, sh.x, halpha);
+    const float ih = __fdividef(1.f, g.h_uniform);
+    const RatesConst kc = rates_const(g.h_uniform, cubic_fac(A.dim, ih), A.beta, A.eta2, A.eps);
+    const int rows = (2 * g.ky + 1) * (2 * g.kz + 1);
+    // a two-record block has staged no state records
+    if (STAGED) {
+        __syncthreads();
+        stage_state(A.s, tab, sh.x, A.sm.off_s, halpha);
     }
-    // destinations with more neighbours than their list holds: the rest
-    // added to the stored sums
-    for (int d = threadIdx.x; d < D; d += blockDim.x) {
-        if (A.cnt[dbase + d] <= cap) continue;
-        BrickDest q;
-        if (!brick_dest(g, A.d, G, A.rad, sp.dlo, sp.doff, d, q)) continue;
+    __syncthreads();
+    for (int d = threadIdx.x; d < dh.x; d += blockDim.x) {
+        if (A.cnt[dh.y + d] <= A.cap) continue;
+        const BrickDest q = brick_dest(A.d, G, g.cs_f, A.d.bdest[dh.y + d]);
+        if (!is_real(A.d, q.orig)) continue;
         RatesAcc acc;
         rates_acc_init(acc, A.d.velh[q.s], A.d.st[q.s], halpha);
-        rates_rest<K, XSPH, ETA0, STAGED>(acc, kc, g, G, A.s, A.d, R, sp.rlo, sp.roff, q, cap);
+        int skip = A.cap;
+        brick_traverse<STAGED>(g, G, A.s, A.d, R, A.rad, brow, tab, nullptr, q, 0, rows,
+            [&](int t, float) {
+                if (skip > 0) { --skip; return; }
+                float4 pj, vj;
+                float mj, hac;
+                R.template rates_rec<false>(t, 0.f, 0.f, pj, vj, mj, hac);
+                rates_pair<XSPH, ETA0>(acc, kc, q.P.x - pj.x, q.P.y - pj.y, q.P.z - pj.z, pj, vj,
+                                       mj, hac);
+                rates_flush<1, XSPH>(acc);
+            });
         const double a3[3] = {(double)acc.ax.fvalue(), (double)acc.ay.fvalue(),
                               (double)acc.az.fvalue()};
         const double p3[3] = {(double)acc.xx.fvalue(), (double)acc.xy.fvalue(),
@@ -1029,89 +1196,201 @@ __device__ __forceinline__ void rates_block(const BrickRatesArgs &A, const Grid 
     }
 }
 
-template <int K, bool XSPH, bool STAGED>
-__global__ void __maxnreg__(XSPH ? 80 : 64) k_brates(const __grid_constant__ BrickRatesArgs A) {
-    unsigned char *smem = brick_smem;
-    if (gate_off(A.gate)) return;
+// The rates of a destination (its prefetched records p, velocity, state).
+template <int S, bool XSPH, bool ETA0, bool FAST, bool STAGED>
+__device__ __forceinline__ void rates_dest(const BrickRatesArgs &A, const SrcRecords<STAGED> &R,
+                                           float mb, const uint4 *lst, int D, int lane,
+                                           const DestPre &p, const float4 &vi, const float4 &st) {
+    const float ih = __fdividef(1.f, A.g.h_uniform);
+    RatesConst kc = rates_const(A.g.h_uniform, cubic_fac(A.dim, ih), A.beta, A.eta2, A.eps);
+    kc.mb = mb;
+    kc.tkc = A.tait_kc;
+    RatesAcc acc;
+    rates_acc_init(acc, vi, st, 0.5f * A.alpha);
+    rates_stream<S, XSPH, ETA0, FAST, STAGED>(acc, kc, R, lst, D, (min(p.c, A.cap) + 7) >> 3, lane,
+                                              p.P, p.b0, p.b1);
+    rates_store<S, XSPH>(A, acc, p.orig, lane);
+}
+
+// Destinations past one per column of the block, as density_more.
+template <bool XSPH, bool ETA0, bool FAST, bool STAGED>
+__device__ __noinline__ void rates_more(const BrickRatesArgs &A, float mb, int first) {
+    constexpr int S = 4;
     const int b = blockIdx.x;
-    const int nd = A.d.bdst[b + 1] - A.d.bdst[b];
-    if (nd == 0) return;
-    const Grid &g = A.g;
-    const BlockGeo G = block_geo(g, A.bk, b);
-    SmemPtrs sp = smem_ptrs(smem, A.sm);
-    int T, D;
-    block_tables(g, G, A.s.cstart, A.d.cstart, sp.rlo, sp.roff, sp.dlo, sp.doff, T, D);
-    const int dbase = A.d.bdst[b];
+    const int2 dh = A.d.bdst[b];
+    const int4 sh = A.s.bsrc[b];
+    const SrcRecords<STAGED> R = make_records<STAGED>(A.sm, A.s, A.g.cs_f, A.s.bstage + sh.y, sh.x,
+                                                      0.5f * A.alpha);
+    const uint4 *lgrp = reinterpret_cast<const uint4 *>(A.nbr) + (size_t)dh.y * (A.cap >> 3);
+    const int lane = threadIdx.x % S;
+    for (int d = first + threadIdx.x / S; d < dh.x; d += blockDim.x / S) {
+        DestPre p;
+        dest_prefetch<S>(A.d, A.g.cs_f, A.d.bdest[dh.y + d], A.cnt + dh.y, lgrp, A.cap, dh.x, d,
+                         lane, p);
+        rates_dest<S, XSPH, ETA0, FAST, STAGED>(A, R, mb, lgrp + d, dh.x, lane, p, A.d.velh[p.s],
+                                                A.d.st[p.s]);
+    }
+}
+
+template <int S, bool XSPH, bool ETA0, bool FAST, bool STAGED>
+__device__ __forceinline__ void rates_block(const BrickRatesArgs &A, const SrcRecords<STAGED> &R,
+                                            float mb, const uint4 *lgrp, int D, int d, int lane,
+                                            const DestPre &pre, const float4 &vi, const float4 &st) {
+    if (d < D)
+        rates_dest<S, XSPH, ETA0, FAST, STAGED>(A, R, mb, lgrp + d, D, lane, pre, vi, st);
+    if (D > (int)blockDim.x / S) rates_more<XSPH, ETA0, FAST, STAGED>(A, mb, blockDim.x / S);
+    if (*A.maxcnt > A.cap) rates_rest<XSPH, ETA0, STAGED>(A);
+}
+
+template <int S, bool XSPH, bool STAGED>
+__global__ void __maxnreg__(XSPH ? 80 : 64) k_brates(const __grid_constant__ BrickRatesArgs A) {
+    const int b = blockIdx.x;
+    const int2 dh = A.d.bdst[b];        // destinations, first destination
+    const int4 sh = A.s.bsrc[b];        // staged records, their table, the first's slot
+    if (dh.x == 0) return;
+    const unsigned off = A.gate != nullptr ? *A.gate : 0u;   // tested after the staging
+    const int T = sh.x, D = dh.x;
+    const int2 *tab = A.s.bstage + sh.y;
+    const uint4 *lgrp = reinterpret_cast<const uint4 *>(A.nbr) + (size_t)dh.y * (A.cap >> 3);
+    const int lane = threadIdx.x % S, d = threadIdx.x / S;
     DestPre pre;
-    if ((int)threadIdx.x < D) {
-        const uint4 *lgrp = reinterpret_cast<const uint4 *>(A.nbr) + (size_t)dbase * (A.cap >> 3);
-        dest_prefetch(A.d, g, G, A.rad, sp, A.cnt, lgrp, A.cap, D, dbase, threadIdx.x, pre);
+    float4 vi = pad_vel(), st = pad_vel();
+    if (d < D) {
+        dest_prefetch<S>(A.d, A.g.cs_f, A.d.bdest[dh.y + d], A.cnt + dh.y, lgrp, A.cap, D, d, lane,
+                         pre);
+        vi = A.d.velh[pre.s];
+        st = A.d.st[pre.s];
     }
     const float halpha = 0.5f * A.alpha;
     // two-record blocks: staged sources of one mass (that of the first) whose
     // cs follows Tait
     const bool try_fast = STAGED && A.tait_state != 0 && A.eta2 == 0.f && T > 0;
-    float mref = 0.f;
-    if (try_fast) {
-        int cy, cz;
-        mref = A.s.pm[staged_slot(G, sp.rlo, sp.roff, 0, cy, cz)].w;
-    }
+    const float mref = try_fast ? A.s.pm[sh.z].w : 0.f;
     bool same = true;
-    if (STAGED) same = stage<true>(A.s, G, sp.rlo, sp.roff, T, g.cs_f, sp.voff, sp.soff, halpha, mref);
+    if (STAGED) same = stage<true>(A.s, tab, T, A.g.cs_f, A.sm, !try_fast, halpha, mref);
     const bool fast = __syncthreads_and(try_fast && same) != 0;
-    const SrcRecords<STAGED, 5> R = make_records<STAGED, 5>(sp, A.s, G, g.cs_f, T, halpha);
-    const float ih = __fdividef(1.f, g.h_uniform);
-    RatesConst kc = rates_const(g.h_uniform, cubic_fac(A.dim, ih), A.beta, A.eta2, A.eps);
+    if (STAGED && try_fast && !fast) {
+        stage_state(A.s, tab, T, A.sm.off_s, halpha);
+        __syncthreads();
+    }
+    if (off != 0u) return;
+    const SrcRecords<STAGED> R = make_records<STAGED>(A.sm, A.s, A.g.cs_f, tab, T, halpha);
     if (A.eta2 == 0.f) {
         if constexpr (STAGED) {
             if (fast) {
-                kc.mb = mref;
-                kc.tkc = A.tait_kc;
-                rates_block<K, XSPH, true, true, STAGED>(A, g, G, sp, R, kc, D, dbase, pre);
+                rates_block<S, XSPH, true, true, STAGED>(A, R, mref, lgrp, D, d, lane, pre, vi, st);
                 return;
             }
         }
-        rates_block<K, XSPH, true, false, STAGED>(A, g, G, sp, R, kc, D, dbase, pre);
+        rates_block<S, XSPH, true, false, STAGED>(A, R, 0.f, lgrp, D, d, lane, pre, vi, st);
     } else {
-        rates_block<K, XSPH, false, false, STAGED>(A, g, G, sp, R, kc, D, dbase, pre);
+        rates_block<S, XSPH, false, false, STAGED>(A, R, 0.f, lgrp, D, d, lane, pre, vi, st);
     }
 }
 
 // ---------------------------------------------------------------------------
-// per-brick tables of one array: destinations per brick (then scanned into
-// bdst) and the largest count of source particles a brick stages
+// tables of the blocks of one array (ArraySnap): first, a warp per block, the
+// staged rows, the counts, and the places of its entries (one atomic per
+// table; they differ from build to build, the results do not depend on
+// them), then, the tables allocated, the entries, four warps per block (42 us
+// at 1 M particles, once per full build; a warp per block took 20 us more at
+// 275 000)
 // ---------------------------------------------------------------------------
-__global__ void k_brick_tables(Grid g, BrickGeom bk, const int *cstart, int *dcount,
-                               unsigned *stats) {
-    const int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    unsigned tmax = 0, dmax = 0;
-    if (b < bk.nbricks) {
-        const BlockGeo G = block_geo(g, bk, (int)b);
-        const int rowz = g.nx * g.ny;
-        int D = 0;
-        for (int cz = G.z0; cz < G.z1; ++cz)
-            for (int cy = G.y0; cy < G.y1; ++cy) {
-                const int c = cz * rowz + cy * g.nx;
-                D += cstart[c + G.x1] - cstart[c + G.x0];
-            }
-        // every brick: as a source this array is staged by the bricks that
-        // hold destinations of any array
-        int T = 0;
-        for (int cz = G.zs0; cz < G.zs1; ++cz)
-            for (int cy = G.ys0; cy < G.ys1; ++cy) {
-                const int c = cz * rowz + cy * g.nx;
-                T += cstart[c + G.xs1] - cstart[c + G.xs0];
-            }
-        dcount[b] = D;
-        tmax = (unsigned)T;
-        dmax = (unsigned)D;
+__device__ __forceinline__ int warp_scan(int v) {     // inclusive
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += y;
     }
-    if (b == bk.nbricks) dcount[b] = 0;
-    tmax = __reduce_max_sync(0xffffffffu, tmax);
-    dmax = __reduce_max_sync(0xffffffffu, dmax);
-    if ((threadIdx.x & 31) == 0) {
-        atomicMax(stats, tmax);
-        atomicMax(stats + 1, dmax);
+    return v;
+}
+
+// first slot and length of destination row r of a block (0 past the last)
+__device__ __forceinline__ int dest_row(const Grid &g, const BlockGeo &G, const int *cstart, int r,
+                                        int &lo) {
+    const int dry = G.y1 - G.y0, ndr = dry * (G.z1 - G.z0);
+    lo = 0;
+    if (r >= ndr) return 0;
+    const int c = ((G.z0 + r / dry) * g.ny + G.y0 + r % dry) * g.nx;
+    lo = cstart[c + G.x0];
+    return cstart[c + G.x1] - lo;
+}
+
+__global__ void __launch_bounds__(128) k_brick_count(Grid g, BrickGeom bk, const int *cstart,
+                                                     int4 *bsrc, int2 *brow, int2 *bdst,
+                                                     unsigned *stats) {
+    const int lane = threadIdx.x & 31;
+    const int64_t b = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (b >= bk.nbricks) return;
+    const BlockGeo G = block_geo(g, bk, (int)b);
+    int T = 0, first = 0;
+    int2 *rows = brow + b * bk.nrmax;
+    for (int r0 = 0; r0 < G.nr; r0 += 32) {
+        const int r = r0 + lane;
+        int lo = 0, len = 0;
+        if (r < G.nr) {
+            const int c = ((G.zs0 + r / G.ry) * g.ny + G.ys0 + r % G.ry) * g.nx + G.xs0;
+            lo = cstart[c];
+            len = cstart[c + G.lx] - lo;
+        }
+        const int inc = warp_scan(len);
+        if (r < G.nr) rows[r] = make_int2(lo, (int)((unsigned)(T + inc - len) | ((unsigned)len << 16)));
+        const unsigned some = __ballot_sync(0xffffffffu, len > 0);
+        if (T == 0 && some) first = __shfl_sync(0xffffffffu, lo, __ffs(some) - 1);
+        T += __shfl_sync(0xffffffffu, inc, 31);
+    }
+    const int ndr = (G.y1 - G.y0) * (G.z1 - G.z0);
+    int D = 0, lo;
+    for (int r0 = 0; r0 < ndr; r0 += 32)
+        D += __reduce_add_sync(0xffffffffu, dest_row(g, G, cstart, r0 + lane, lo));
+    if (lane == 0) {
+        // every block: as a source this array is staged by the blocks that
+        // hold destinations of any array
+        const int tb = T > 0 ? (int)atomicAdd(stats + 3, (unsigned)T) : 0;
+        const int db = D > 0 ? (int)atomicAdd(stats + 2, (unsigned)D) : 0;
+        atomicMax(stats, (unsigned)T);
+        atomicMax(stats + 1, (unsigned)D);
+        bsrc[b] = make_int4(T, tb, first, 0);
+        bdst[b] = make_int2(D, db);
+    }
+}
+
+__global__ void __launch_bounds__(128) k_brick_fill(Grid g, BrickGeom bk, const int *cstart,
+                                                    const float *scx, const int4 *bsrc,
+                                                    const int2 *brow, const int2 *bdst,
+                                                    int2 *bstage, int2 *bdest) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int b = blockIdx.x;
+    const int D = bdst[b].x;
+    const BlockGeo G = block_geo(g, bk, b);
+    const int2 *rows = brow + (int64_t)b * bk.nrmax;
+    int2 *stab = bstage + bsrc[b].y;
+    // a warp takes a row of cells at a time, its slots over the lanes
+#pragma unroll 4
+    for (int r = wid; r < G.nr; r += nw) {
+        const int2 e = rows[r];
+        const int c = pack_cell(-128, G.ys0 + r % G.ry - G.cyc, G.zs0 + r / G.ry - G.czc) -
+                      G.cxc + 128;
+        for (int i = lane; i < row_len(e); i += 32)
+            stab[row_off(e) + i] = make_int2(e.x + i, c + (int)scx[e.x + i]);
+    }
+    if (D == 0) return;
+    const int dry = G.y1 - G.y0, ndr = dry * (G.z1 - G.z0);
+    int2 *dtab = bdest + bdst[b].y;
+    for (int r0 = 0; r0 < ndr; r0 += 32) {
+        int lo;
+        const int len = dest_row(g, G, cstart, r0 + lane, lo);
+        const int inc = warp_scan(len);
+        const int cnt = min(32, ndr - r0);
+        for (int k = wid; k < cnt; k += nw) {
+            const int l = __shfl_sync(0xffffffffu, lo, k), n = __shfl_sync(0xffffffffu, len, k);
+            const int at = __shfl_sync(0xffffffffu, inc - len, k);
+            const int cy = G.y0 + (r0 + k) % dry - G.cyc, cz = G.z0 + (r0 + k) / dry - G.czc;
+            for (int i = lane; i < n; i += 32)
+                dtab[at + i] = make_int2(l + i, pack_cell((int)scx[l + i] - G.cxc, cy, cz));
+        }
+        dtab += __shfl_sync(0xffffffffu, inc, 31);
     }
 }
 
@@ -1119,18 +1398,11 @@ __global__ void k_brick_tables(Grid g, BrickGeom bk, const int *cstart, int *dco
 // staged-record capacity, if it fits the shared memory of a block
 constexpr int kBrickSmemLimit = 200 * 1024;
 
-// Shared-memory layout of a pass over destination array D from source S.
+// Shared-memory layout of a pass over the sources S.
 int brick_layout(const sph_ctx *ctx, const ArraySnap &S, bool rates, bool cells, BrickSmem *sm,
                  size_t *bytes) {
     const BrickGeom &bk = ctx->bricks;
-    const Grid &g = ctx->grid;
-    const int lx = bk.bx + 2 * g.kx, ry = bk.by + 2 * g.ky, rz = bk.bz + 2 * g.kz;
-    const int nr = ry * rz;
-    const int ndr = bk.by * bk.bz;
-    // tables (ints): rlo[nr], roff[nr + 1], dlo[ndr], doff[ndr + 1], and for
-    // a list build scell[nr (lx + 1)]
-    const size_t ncell = cells ? (size_t)nr * (lx + 1) : 0;
-    const size_t tables = sizeof(int) * ((size_t)nr + nr + 1 + ndr + ndr + 1 + ncell);
+    const size_t ncell = cells ? (size_t)bk.nrmax * (bk.rowmax + 1) : 0;
     const size_t rec = rates ? (16 + 16 + 8) : 16;
     // the staged records and the padding record after them
     size_t cap = (size_t)std::max(S.b_tmax, 0) + 1;
@@ -1142,10 +1414,9 @@ int brick_layout(const sph_ctx *ctx, const ArraySnap &S, bool rates, bool cells,
         const char *e = getenv("SPH_BRICK_UNSTAGED");
         unstaged = (e && atoi(e) > 0) ? 1 : 0;
     }
-    bool staged = !unstaged && tables + cap * rec + 64 <= (size_t)kBrickSmemLimit;
+    const bool staged = !unstaged && sizeof(int) * ncell + cap * rec + 64 <= (size_t)kBrickSmemLimit;
     if (!staged) cap = 0;
     size_t off = 0;
-    sm->stage_cap = (int)cap;
     // position records, then (rates) velocity and state records
     off += cap * 16;
     sm->off_v = (int)off;
@@ -1153,10 +1424,6 @@ int brick_layout(const sph_ctx *ctx, const ArraySnap &S, bool rates, bool cells,
     sm->off_s = (int)off;
     if (rates) off += cap * 8;
     off = (off + 15) & ~(size_t)15;
-    sm->off_rlo = (int)off; off += sizeof(int) * nr;
-    sm->off_roff = (int)off; off += sizeof(int) * (nr + 1);
-    sm->off_dlo = (int)off; off += sizeof(int) * ndr;
-    sm->off_doff = (int)off; off += sizeof(int) * (ndr + 1);
     sm->off_scell = (int)off; off += sizeof(int) * ncell;
     *bytes = off;
     return staged ? 1 : 0;
@@ -1182,35 +1449,39 @@ BrickSrcDev make_bsrc(const ArraySnap &S) {
     BrickSrcDev s;
     s.pm = S.pm; s.velh = S.velh; s.st = S.st; s.scx = S.scx;
     s.cstart = S.cstart; s.perm = S.perm;
+    s.bsrc = S.bsrc; s.brow = S.brow; s.bstage = S.bstage;
     s.x = S.view.x; s.y = S.view.y; s.z = S.view.z;
     return s;
 }
 
 BrickDstDev make_bdst(const ArraySnap &D) {
     BrickDstDev d;
-    d.pm = D.pm; d.velh = D.velh; d.st = D.st; d.scx = D.scx;
-    d.cstart = D.cstart; d.perm = D.perm; d.bdst = D.bdst;
+    d.pm = D.pm; d.velh = D.velh; d.st = D.st;
+    d.perm = D.perm; d.bdst = D.bdst; d.bdest = D.bdest;
     d.tag = D.view.tag;
-    d.x = D.view.x; d.y = D.view.y; d.z = D.view.z; d.h = D.view.h;
+    d.x = D.view.x; d.y = D.view.y; d.z = D.view.z;
     d.u = D.view.u; d.v = D.view.v; d.w = D.view.w;
     d.p = D.view.p; d.cs = D.view.cs;
     return d;
 }
 
-// Threads per block: the largest brick population rounded to warps, at
-// most 320 (three blocks of 64-register threads per SM); a brick with more
-// destinations takes them in rounds.
-int brick_threads(const ArraySnap &D) {
+// Threads per block: the columns (destinations times lanes) of the most
+// populous block rounded to warps, at most 320 with one lane (three blocks of
+// 64-register threads per SM) and 512 with more; a block with more columns
+// takes them in rounds.
+int brick_threads(const sph_ctx *ctx, const ArraySnap &D) {
     // environment SPH_BRICK_MAX_THREADS: another ceiling (a multiple of 32
     // up to 512), to measure it
     static int ceiling = -1;
     if (ceiling < 0) {
         const char *e = getenv("SPH_BRICK_MAX_THREADS");
         const int v = e ? atoi(e) : 0;
-        ceiling = (v >= 64 && v <= kBrickMaxThreads && v % 32 == 0) ? v : 320;
+        ceiling = (v >= 64 && v <= kBrickMaxThreads && v % 32 == 0) ? v : 0;
     }
-    const int want = (std::max(D.b_dmax, 1) + 31) / 32 * 32;
-    return std::min(std::max(want, 64), ceiling);
+    const int lanes = ctx->bricks.lanes;
+    const int top = ceiling > 0 ? ceiling : (lanes == 1 ? 320 : kBrickMaxThreads);
+    const int want = (std::max(D.b_dmax, 1) * lanes + 31) / 32 * 32;
+    return std::min(std::max(want, 64), top);
 }
 
 template <class Kern>
@@ -1273,30 +1544,90 @@ void brick_geometry(sph_ctx *ctx) {
         bk.bx = 64;
         bk.by = bk.bz = 1;
     }
-    bk.nbx = (g.nx + bk.bx - 1) / bk.bx;
-    bk.nby = (g.ny + bk.by - 1) / bk.by;
-    bk.nbz = (g.nz + bk.bz - 1) / bk.bz;
+    // Lanes per destination and parts of a brick: a small simulation has fewer
+    // bricks than there are SMs and each thread a long chain, so its
+    // destinations get 2 or 4 lanes and its bricks as many parts; a larger one
+    // pays for the parts' wider staging and the second traversal of a list
+    // build.  Measured, rates + density in us at 1 / 2 / 4 lanes -- 3D: 4 096
+    // particles 26.3 / 22.4 / 19.1, 8 000 28.9 / 23.8 / 22.3, 21 952 29.0 /
+    // 26.6 / 35.6, 64 000 50.3 / 49.6 / 68.2; 2D: 5 025 18.2 / 17.8 / 15.9,
+    // 10 300 17.8 / 16.9 / 15.6, 20 106 17.9 / 18.4 / 22.4.  Environment SPH_BRICK_LANES forces the lanes (to measure them, and
+    // to test them at any size).
+    static int force_lanes = -1;
+    if (force_lanes < 0) {
+        const char *l = getenv("SPH_BRICK_LANES");
+        const int v = l ? atoi(l) : 0;
+        force_lanes = (v == 1 || v == 2 || v == 4) ? v : 0;
+    }
+    int64_t n = 0;
+    for (const ArraySnap &A : ctx->arrays) n = std::max(n, A.n);
+    bk.lanes = force_lanes ? force_lanes
+                           : (n < 12000 ? 4 : (g.kz > 0 && n < 40000 ? 2 : 1));
+    bk.px = bk.lanes > 1 && bk.bx > 1 ? 2 : 1;
+    bk.py = bk.lanes > 2 && bk.by > 1 ? 2 : 1;
+    bk.pz = 1;
+    bk.nbx = (g.nx + bk.bx - 1) / bk.bx * bk.px;
+    bk.nby = (g.ny + bk.by - 1) / bk.by * bk.py;
+    bk.nbz = (g.nz + bk.bz - 1) / bk.bz * bk.pz;
+    const int sx = (bk.bx + bk.px - 1) / bk.px, sy = (bk.by + bk.py - 1) / bk.py,
+              sz = (bk.bz + bk.pz - 1) / bk.pz;
+    bk.nrmax = (sy + 2 * g.ky) * (sz + 2 * g.kz);
+    bk.rowmax = sx + 2 * g.kx;
     bk.nbricks = (int64_t)bk.nbx * bk.nby * bk.nbz;
 }
 
 // Per-array brick tables for the current build (queued on the context's
-// stream); the statistics land in stats[2 a], stats[2 a + 1].
-int brick_tables(sph_ctx *ctx, int a, unsigned *stats) {
+// stream): the counts, whose statistics land in stats[0 .. kBrickStats), then,
+// when those are known on the host, the entries.
+int brick_count(sph_ctx *ctx, int a, unsigned *stats) {
     ArraySnap &A = ctx->arrays[a];
     const BrickGeom &bk = ctx->bricks;
-    const int64_t need = bk.nbricks + 1;
-    if (need > A.bdst_cap || !A.bdst) {
+    if (bk.nbricks > A.brick_cap || !A.bsrc) {
+        cudaFree(A.bsrc);
         cudaFree(A.bdst);
+        A.bsrc = nullptr;
         A.bdst = nullptr;
-        SPH_CUDA(cudaMalloc(&A.bdst, sizeof(int) * need));
-        A.bdst_cap = need;
+        SPH_CUDA(cudaMalloc(&A.bsrc, sizeof(int4) * bk.nbricks));
+        SPH_CUDA(cudaMalloc(&A.bdst, sizeof(int2) * bk.nbricks));
+        A.brick_cap = bk.nbricks;
     }
-    const int th = 128;
-    const int blocks = (int)((need + th - 1) / th);
-    k_brick_tables<<<blocks, th, 0, ctx->stream>>>(ctx->grid, bk, A.cstart, A.bdst, stats);
+    const int64_t nrow = bk.nbricks * bk.nrmax;
+    if (nrow > A.brow_cap || !A.brow) {
+        cudaFree(A.brow);
+        A.brow = nullptr;
+        SPH_CUDA(cudaMalloc(&A.brow, sizeof(int2) * nrow));
+        A.brow_cap = nrow;
+    }
+    const int th = 128, per = th / 32;
+    const int blocks = (int)((bk.nbricks + per - 1) / per);
+    k_brick_count<<<blocks, th, 0, ctx->stream>>>(ctx->grid, bk, A.cstart, A.bsrc, A.brow, A.bdst,
+                                                  stats);
     count_launch();
-    SPH_LAUNCH_CHECK("k_brick_tables");
-    return scan_exclusive(ctx, A.bdst, need);
+    SPH_LAUNCH_CHECK("k_brick_count");
+    return SPH_OK;
+}
+
+int brick_fill(sph_ctx *ctx, int a) {
+    ArraySnap &A = ctx->arrays[a];
+    const BrickGeom &bk = ctx->bricks;
+    if (A.n > A.bdest_cap || !A.bdest) {
+        cudaFree(A.bdest);
+        A.bdest = nullptr;
+        SPH_CUDA(cudaMalloc(&A.bdest, sizeof(int2) * A.n));
+        A.bdest_cap = A.n;
+    }
+    if (A.b_staged > A.bstage_cap || !A.bstage) {
+        cudaFree(A.bstage);
+        A.bstage = nullptr;
+        const int64_t want = A.b_staged + A.b_staged / 8;   // the next builds' too
+        SPH_CUDA(cudaMalloc(&A.bstage, sizeof(int2) * std::max<int64_t>(want, 1)));
+        A.bstage_cap = want;
+    }
+    k_brick_fill<<<(unsigned)bk.nbricks, 128, 0, ctx->stream>>>(ctx->grid, bk, A.cstart, A.scx, A.bsrc, A.brow,
+                                                 A.bdst, A.bstage, A.bdest);
+    count_launch();
+    SPH_LAUNCH_CHECK("k_brick_fill");
+    return SPH_OK;
 }
 
 bool brick_density_eligible(const sph_ctx *ctx, int dst, const int *srcs, int nsrc,
@@ -1343,7 +1674,6 @@ int brick_density(sph_ctx *ctx, int dst, int src, NbrList &L, bool build, bool w
     a.cnt = L.cnt;
     a.maxcnt = L.maxcnt;
     a.cap = L.cap;
-    a.build = build ? 1 : 0;
     a.write_out = write_out ? 1 : 0;
     if (prm) {
         a.dim = prm->dim;
@@ -1356,20 +1686,20 @@ int brick_density(sph_ctx *ctx, int dst, int src, NbrList &L, bool build, bool w
     a.st_out = st_out;
     a.gate = ctx->gate;
     if (D.n == 0) return SPH_OK;
-    const int nt = brick_threads(D);
+    const int nt = brick_threads(ctx, D);
     const int blocks = (int)ctx->bricks.nbricks;
-    const int K = ctx->grid.kx;
-#define BDL2(K_, B_, S_)                                                                  \
+    const int lanes = ctx->bricks.lanes;
+#define BDL2(K_, L_, S_)                                                                  \
     do {                                                                                  \
-        int rc_ = allow_smem(k_bdensity<K_, B_, S_>, bytes);                              \
+        int rc_ = allow_smem(K_<L_, S_>, bytes);                                          \
         if (rc_) return rc_;                                                              \
-        k_bdensity<K_, B_, S_><<<blocks, nt, bytes, ctx->stream>>>(a);                    \
+        K_<L_, S_><<<blocks, nt, bytes, ctx->stream>>>(a);                                \
     } while (0)
-#define BDL1(K_, B_) do { if (staged) BDL2(K_, B_, true); else BDL2(K_, B_, false); } while (0)
-#define BDL(K_) do { if (build) BDL1(K_, true); else BDL1(K_, false); } while (0)
-    if (K == 1) BDL(1);
-    else if (K == 2) BDL(2);
-    else BDL(3);
+#define BDL1(K_, L_) do { if (staged) BDL2(K_, L_, true); else BDL2(K_, L_, false); } while (0)
+#define BDL(L_) do { if (build) BDL1(k_bbuild, L_); else BDL1(k_bdensity, L_); } while (0)
+    if (lanes == 1) BDL(1);
+    else if (lanes == 2) BDL(2);
+    else BDL(4);
 #undef BDL
 #undef BDL1
 #undef BDL2
@@ -1393,6 +1723,7 @@ int brick_rates(sph_ctx *ctx, int dst, const sph_source_term &term, NbrList &L,
     const bool staged = brick_layout(ctx, S, true, false, &a.sm, &bytes) != 0;
     a.nbr = L.nbr16;
     a.cnt = L.cnt;
+    a.maxcnt = L.maxcnt;
     a.cap = L.cap;
     a.dim = prm->dim;
     a.alpha = (float)term.alpha;
@@ -1419,25 +1750,25 @@ int brick_rates(sph_ctx *ctx, int dst, const sph_source_term &term, NbrList &L,
     a.gate = ctx->gate;
     if (D.n == 0) return SPH_OK;
     const bool xsph = (term.flags & SPH_TERM_XSPH) != 0;
-    const int nt = brick_threads(D);
+    const int nt = brick_threads(ctx, D);
     const int blocks = (int)ctx->bricks.nbricks;
-    const int K = ctx->grid.kx;
-#define BRL2(K_, X_)                                                                      \
+    const int lanes = ctx->bricks.lanes;
+#define BRL2(L_, X_)                                                                      \
     do {                                                                                  \
         if (staged) {                                                                     \
-            int rc_ = allow_smem(k_brates<K_, X_, true>, bytes);                          \
+            int rc_ = allow_smem(k_brates<L_, X_, true>, bytes);                          \
             if (rc_) return rc_;                                                          \
-            k_brates<K_, X_, true><<<blocks, nt, bytes, ctx->stream>>>(a);                \
+            k_brates<L_, X_, true><<<blocks, nt, bytes, ctx->stream>>>(a);                \
         } else {                                                                          \
-            int rc_ = allow_smem(k_brates<K_, X_, false>, bytes);                         \
+            int rc_ = allow_smem(k_brates<L_, X_, false>, bytes);                         \
             if (rc_) return rc_;                                                          \
-            k_brates<K_, X_, false><<<blocks, nt, bytes, ctx->stream>>>(a);               \
+            k_brates<L_, X_, false><<<blocks, nt, bytes, ctx->stream>>>(a);               \
         }                                                                                 \
     } while (0)
-#define BRL(K_) do { if (xsph) BRL2(K_, true); else BRL2(K_, false); } while (0)
-    if (K == 1) BRL(1);
-    else if (K == 2) BRL(2);
-    else BRL(3);
+#define BRL(L_) do { if (xsph) BRL2(L_, true); else BRL2(L_, false); } while (0)
+    if (lanes == 1) BRL(1);
+    else if (lanes == 2) BRL(2);
+    else BRL(4);
 #undef BRL
 #undef BRL2
     count_launch();

@@ -85,8 +85,8 @@ int sph_ctx_create(int dim, sph_ctx **out) {
             cudaSuccess ||
         (e = cudaHostGetDevicePointer((void **)&c->hd_box, c->h_box, 0)) != cudaSuccess ||
         (e = cudaHostGetDevicePointer((void **)&c->hd_status, c->h_status, 0)) != cudaSuccess ||
-        (e = cudaMalloc(&c->d_bstats, 2 * kMaxBrickArrays * sizeof(unsigned))) != cudaSuccess ||
-        (e = cudaHostAlloc(&c->h_bstats, 2 * kMaxBrickArrays * sizeof(unsigned),
+        (e = cudaMalloc(&c->d_bstats, kBrickStats * kMaxBrickArrays * sizeof(unsigned))) != cudaSuccess ||
+        (e = cudaHostAlloc(&c->h_bstats, kBrickStats * kMaxBrickArrays * sizeof(unsigned),
                            cudaHostAllocMapped)) != cudaSuccess ||
         (e = cudaHostGetDevicePointer((void **)&c->hd_bstats, c->h_bstats, 0)) != cudaSuccess ||
         (e = cudaEventCreateWithFlags(&c->pending_event, cudaEventDisableTiming)) != cudaSuccess) {
@@ -108,7 +108,11 @@ int sph_ctx_destroy(sph_ctx *c) {
         cudaFree(A.scx); cudaFree(A.pm); cudaFree(A.velh); cudaFree(A.st);
         cudaFree(A.nrm); cudaFree(A.tan);
         cudaFree(A.cstart); cudaFree(A.cursor); cudaFree(A.refcell); cudaFree(A.pm0); cudaFree(A.inv);
+        cudaFree(A.bsrc);
         cudaFree(A.bdst);
+        cudaFree(A.brow);
+        cudaFree(A.bstage);
+        cudaFree(A.bdest);
     }
     cudaFree(c->d_box); cudaFree(c->d_hmax); cudaFree(c->d_status);
     cudaFree(c->scan_tmp); cudaFree(c->d_part); cudaFree(c->d_cnt);

@@ -819,19 +819,29 @@ int nnps_build(sph_ctx *ctx, const sph_array_view *arrays, int narrays, double c
     if (ctx->bricks_on && g.uniform_h && !g.periodic && !g.symmetric &&
         narrays <= kMaxBrickArrays) {
         brick_geometry(ctx);
-        SPH_CUDA(cudaMemsetAsync(ctx->d_bstats, 0, 2 * narrays * sizeof(unsigned), st));
+        SPH_CUDA(cudaMemsetAsync(ctx->d_bstats, 0, kBrickStats * narrays * sizeof(unsigned), st));
         for (int a = 0; a < narrays; ++a) {
             if (arrays[a].n == 0) continue;
-            const int rc = brick_tables(ctx, a, ctx->d_bstats + 2 * a);
+            const int rc = brick_count(ctx, a, ctx->d_bstats + kBrickStats * a);
             if (rc) return rc;
         }
-        const int rp = publish_words(ctx, ctx->d_bstats, ctx->hd_bstats, 2 * narrays);
+        const int rp = publish_words(ctx, ctx->d_bstats, ctx->hd_bstats, kBrickStats * narrays);
         if (rp) return rp;
         SPH_CUDA(cudaStreamSynchronize(st));
         for (int a = 0; a < narrays; ++a) {
             ArraySnap &A = ctx->arrays[a];
-            A.b_tmax = arrays[a].n > 0 ? (int)ctx->h_bstats[2 * a] : 0;
-            A.b_dmax = arrays[a].n > 0 ? (int)ctx->h_bstats[2 * a + 1] : 0;
+            const unsigned *q = ctx->h_bstats + kBrickStats * a;
+            const bool any = arrays[a].n > 0;
+            A.b_tmax = any ? (int)q[0] : 0;
+            A.b_dmax = any ? (int)q[1] : 0;
+            A.b_staged = any ? (int64_t)q[3] : 0;
+            // (tables of 32-bit indices; a block too populous for them, or for
+            // 16-bit list entries, leaves the array to the list-streaming passes)
+            if (A.b_staged >= INT32_MAX) A.b_tmax = INT32_MAX;
+            if (any && A.b_tmax < 65535) {
+                const int rc = brick_fill(ctx, a);
+                if (rc) return rc;
+            }
         }
         ctx->bricks_ready = true;
     }

@@ -171,12 +171,31 @@ __device__ __forceinline__ double image_x(const Grid &g, double xj, double xi, f
     return s == 0.0 ? xj : __dadd_rn(xj, s * g.plen);
 }
 
+// FP32 -> FP64 (exact) by integer operations, as d2f_rn: the pattern's
+// exponent moved to FP64's bias, its mantissa to the top 23 bits.  Zeros,
+// infinities and NaN keep their meaning; a subnormal takes the hardware
+// conversion in a separate call.
+static __device__ __noinline__ double f2d_subnormal(float x) { return (double)x; }
+__device__ __forceinline__ double f2d_exact(float x) {
+    const unsigned u = __float_as_uint(x);
+    const unsigned a = u & 0x7fffffffu;
+    if (a - 1u < 0x7fffffu) return f2d_subnormal(x);
+    unsigned hi = (a >> 3) + (a >= 0x7f800000u ? 0x70000000u : 0x38000000u);
+    if (a == 0u) hi = 0u;
+    hi |= u & 0x80000000u;
+    return __hiloint2double((int)hi, (int)(u << 29));
+}
+
 // Bricks of grid cells, the unit of work of the brick-staged pair passes:
-// bx * by * bz cells per brick, nbx * nby * nbz bricks over the grid.
+// bx * by * bz cells per brick, each brick in px * py * pz parts, a block per
+// part (nbx * nby * nbz of them over the grid).
 struct BrickGeom {
     int bx = 1, by = 1, bz = 1;
+    int px = 1, py = 1, pz = 1;
     int nbx = 1, nby = 1, nbz = 1;
-    int64_t nbricks = 0;
+    int lanes = 1;                 // threads that share a destination
+    int nrmax = 1, rowmax = 1;     // staged rows of a block, cells of a row
+    int64_t nbricks = 0;           // blocks
 };
 
 struct ArraySnap {
@@ -205,12 +224,19 @@ struct ArraySnap {
     float4 *pm0 = nullptr; // pm at the last full build, in original order (skin lists)
     int *inv = nullptr;      // original -> sorted slot of the last full build
     int64_t pm0_cap = 0;
-    // brick tables of the last full build: exclusive prefix of the
-    // destinations per brick (nbricks + 1), the largest count of source
-    // particles a brick stages and of destinations in one brick
-    int *bdst = nullptr;
-    int64_t bdst_cap = 0;
+    // tables of the brick blocks of the last full build.  As sources: per
+    // block the staged count, the index of its first bstage entry and the
+    // first staged slot (bsrc), per staged row of cells its first slot and
+    // staging offset | length << 16 (brow), per staged particle its slot and
+    // cell (bstage).  As destinations: per block their count and the index of
+    // the first bdest entry (bdst), per destination its slot and cell (bdest).
+    int4 *bsrc = nullptr;
+    int2 *bdst = nullptr, *brow = nullptr, *bstage = nullptr, *bdest = nullptr;
+    int64_t brick_cap = 0, brow_cap = 0, bstage_cap = 0, bdest_cap = 0;
+    // largest staged count and largest count of destinations of a block,
+    // staged particles of all blocks
     int b_tmax = 0, b_dmax = 0;
+    int64_t b_staged = 0;
 };
 
 // Neighbour list of one (destination, source) pair of arrays: entry k of
@@ -219,9 +245,10 @@ struct ArraySnap {
 // cap neighbours keep the first cap and are completed by a re-traversal.
 struct NbrList {
     uint32_t *nbr = nullptr;
-    // brick-staged list: entry k of destination d of brick b at
-    // nbr16[bdst[b] * cap + k * D_b + d] (an index into the brick's staged
-    // sources), count in cnt[bdst[b] + d]
+    // brick-staged list: 8-entry group g of destination d of block b (D_b
+    // destinations, the first of them destination d0_b) at uint4
+    // d0_b * cap / 8 + g * D_b + d, entries are indices into the block's
+    // staged sources; count in cnt[d0_b + d]
     uint16_t *nbr16 = nullptr;
     bool brick = false;
     int *cnt = nullptr;
@@ -295,7 +322,7 @@ struct sph_ctx {
     int bricks_on = 1;
     bool bricks_ready = false;
     sphgb::BrickGeom bricks;
-    unsigned *d_bstats = nullptr;       // 2 words per array: staged max, destinations max
+    unsigned *d_bstats = nullptr;       // kBrickStats words per array
     unsigned *h_bstats = nullptr;       // mapped mirror
     unsigned *hd_bstats = nullptr;
     long long n_brick_passes = 0;       // pair passes run by the brick kernels
@@ -435,8 +462,12 @@ int record_integrate(sph_ctx *ctx, int64_t n, const sph_axpy_line *lines, int nl
 int record_refresh(sph_ctx *ctx, int array, const sph_array_view *view);
 // brick-staged pair passes (bricks.cu)
 constexpr int kMaxBrickArrays = 16;
+// statistics of an array's brick tables: largest staged count and largest
+// count of destinations of a block, destinations and staged particles in all
+constexpr int kBrickStats = 4;
 void brick_geometry(sph_ctx *ctx);
-int brick_tables(sph_ctx *ctx, int a, unsigned *stats);
+int brick_count(sph_ctx *ctx, int a, unsigned *stats);
+int brick_fill(sph_ctx *ctx, int a);
 bool brick_density_eligible(const sph_ctx *ctx, int dst, const int *srcs, int nsrc,
                             const sph_density_params *prm);
 bool brick_rates_eligible(const sph_ctx *ctx, int dst, const sph_source_term *terms, int nterms,

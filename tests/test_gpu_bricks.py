@@ -199,3 +199,46 @@ def test_brick_fallback_paths_match_oracle(env):
     r = subprocess.run([sys.executable, "-c", _SUB], cwd=ROOT, env=e, capture_output=True,
                        text=True, timeout=600)
     assert r.returncode == 0 and "ok" in r.stdout, r.stderr[-3000:]
+
+
+_HASH = r'''
+import sys, hashlib
+sys.path.insert(0, ".")
+import pysph_gb300
+from pysph_gb300 import workloads as W
+api = pysph_gb300.api()
+h = hashlib.sha256()
+def add(particles, names):
+    for a in particles.arrays:
+        for f in names:
+            h.update(a.get(f).tobytes())
+for n in (343, 4096, 32768):
+    s, particles = W.setup_cube(api, W.cube_lattice(n, seed=31))
+    for _ in range(3):
+        s.integrator.integrate(1e-4)
+    assert particles.cell_manager.brick_pass_count() > 0
+    add(particles, ("x", "y", "z", "u", "v", "w", "rho", "p", "cs"))
+for dx in (0.2, 0.03):
+    s, particles = W.setup_drop(api, W.elliptical_drop(dx=dx, c0=100.0), c0=100.0)
+    for _ in range(4):
+        s.integrator.integrate(1e-5)
+    add(particles, ("x", "y", "u", "v", "rho", "p", "cs"))
+print(h.hexdigest())
+'''
+
+
+@pytest.mark.parametrize("subdiv", [1, 2, 3])
+def test_lanes_and_rounds_give_the_same_bits(subdiv):
+    """One, two or four threads per destination, and destinations past a
+    block's threads (64 threads per block), fold the same batches in the same
+    order: the steps agree bit for bit."""
+    _need_gpu()
+    seen = set()
+    for env in ({"SPH_BRICK_LANES": "1"}, {"SPH_BRICK_LANES": "2"}, {"SPH_BRICK_LANES": "4"},
+                {"SPH_BRICK_LANES": "1", "SPH_BRICK_MAX_THREADS": "64"}):
+        e = dict(os.environ, PYSPH_GB300_BRICKS="1", PYSPH_GB300_SUBDIV=str(subdiv), **env)
+        r = subprocess.run([sys.executable, "-c", _HASH], cwd=ROOT, env=e, capture_output=True,
+                           text=True, timeout=600)
+        assert r.returncode == 0, r.stderr[-3000:]
+        seen.add(r.stdout.split()[-1])
+    assert len(seen) == 1
