@@ -168,12 +168,17 @@ struct NoExtra {
 // if the list overflowed, the remaining neighbours come from a re-traversal.
 // fn(ok, j, rx, ry, rz, mj, x) is called for every slot of a batch (x =
 // extra(j)); ok is false for the padding of the last batch (its data are
-// those of a valid neighbour, its contribution must be dropped).  done() is
+// those of a valid neighbour, its contribution must be dropped).  done(.) is
 // called after every batch.  With a list skin, filter keeps only the
 // neighbours (ok false for the others); without it a skin entry reaches fn
 // with ok true -- right for terms that vanish beyond the radius (W and
 // grad W of the uniform-h cubic spline are exactly 0 for q >= 2 in FP32).
-template <int KX, int B, bool EXT, class Extra, class Fn, class Done>
+// S > 1: S neighbouring threads (lanes) share the destination; lane l takes
+// the batches l, l + S, ... of the list, fn is called for them, and done(true)
+// after every round of S batches, by all lanes (those past the end of the
+// list have called fn with ok false or not at all); the re-traversal is run by
+// every lane, with done(false) after each neighbour.
+template <int KX, int B, bool EXT, int S_ = 1, class Extra, class Fn, class Done>
 __device__ __forceinline__ void for_listed(const Grid &g, const SrcDev &S, int cap, int64_t stride,
                                            int s, const DestPos &d, const DestDev &D, bool filter,
                                            Extra &&extra, Fn &&fn, Done &&done) {
@@ -189,12 +194,14 @@ __device__ __forceinline__ void for_listed(const Grid &g, const SrcDev &S, int c
         for (int b = 1; b < B; ++b) e[b] = (k + b < m) ? lst[(int64_t)(k + b) * stride] : e[0];
     };
     uint32_t e[B];
-    if (m > 0) entries(e, 0);
+    const int k0 = S_ > 1 ? (int)(threadIdx.x % S_) * B : 0;
+    if (k0 < m) entries(e, k0);
     const float csf = g.cs_f;
-    for (int k = 0; k < m; k += B) {
+    for (int r = 0, k = k0; r < m; r += S_ * B, k += S_ * B) {
         uint32_t en[B];
-        const bool more = k + B < m;
-        if (more) entries(en, k + B);
+        const bool more = k + S_ * B < m;
+        if (more) entries(en, k + S_ * B);
+        if (S_ == 1 || k < m) {
         float4 p[B];
         X x[B];
 #pragma unroll
@@ -213,7 +220,8 @@ __device__ __forceinline__ void for_listed(const Grid &g, const SrcDev &S, int c
             fn(k + b < m && (!filter || listed_exact_test<EXT>(g, S, D, d, j, rx, ry, rz)), j, rx, ry, rz,
                p[b].w, x[b]);
         }
-        done();
+        }
+        done(true);     // (one call for all lanes: it shuffles)
         if (more) {
 #pragma unroll
             for (int b = 0; b < B; ++b) e[b] = en[b];
@@ -230,8 +238,39 @@ __device__ __forceinline__ void for_listed(const Grid &g, const SrcDev &S, int c
                                }
                                if (!exact) return;
                                fn(true, j, rx, ry, rz, S.pm[j].w, extra(j));
-                               done();
+                               done(false);
                            });
+    }
+}
+
+// ---------------------------------------------------------------------------
+// lanes: in small simulations S = 2 or 8 neighbouring threads share a
+// destination of the rates pass (a thread per destination leaves most of the
+// GPU idle there, each thread a serial chain over all its neighbours).  Sums
+// stay the same bit for bit: the batches are those of the list, folded in its
+// order.
+// ---------------------------------------------------------------------------
+template <int S>
+__device__ __forceinline__ unsigned lane_mask() {
+    return ((1u << S) - 1u) << (threadIdx.x & 31 & ~(S - 1));
+}
+
+// v[S q + t] of lane l becomes v[S q + l] of lane t (transposes over the lanes)
+template <int S>
+__device__ __forceinline__ void lane_transpose(float (&v)[8]) {
+    const unsigned mask = lane_mask<S>();
+    const int lane = threadIdx.x % S;
+#pragma unroll
+    for (int b = 1; b < S; b <<= 1) {
+        const bool up = (lane & b) != 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (i & b) continue;
+            const int j = i | b;
+            const float got = __shfl_xor_sync(mask, up ? v[i] : v[j], b);
+            if (up) v[i] = got;
+            else v[j] = got;
+        }
     }
 }
 
@@ -334,7 +373,7 @@ __global__ void __launch_bounds__(kPairBlock, (UH && MODE != 2) ? 8 : 1) k_densi
                     const float w = cubic_w(r * ih) * fac * mj;
                     part += ok ? w : 0.f;
                 },
-                [&]() {
+                [&](bool) {
                     rho.add(part);
                     part = 0.f;
                 });
@@ -383,19 +422,21 @@ struct VelState {
 
 // SPEC 0: any terms, runtime flags; 1: PGrad + AV, uniform h, one source;
 // 2: PGrad + AV + XSPH, uniform h, one source.
-template <int KX, int SPEC, int MODE>
+template <int KX, int SPEC, int MODE, int S_ = 1>
 __global__ void __launch_bounds__(kPairBlock) k_rates(const __grid_constant__ RatesArgs A) {
     constexpr uint32_t SF = SPEC == 1 ? (SPH_TERM_PGRAD | SPH_TERM_AVISC)
                           : (SPEC == 2 ? (SPH_TERM_PGRAD | SPH_TERM_AVISC | SPH_TERM_XSPH) : 0u);
     constexpr bool MAY_XSPH = SPEC != 1;
     constexpr bool MAY_BF = SPEC == 0;
     constexpr bool MAY_DRHO = SPEC == 0;
-    const int64_t s = (MODE == 1 ? A.d.s0 : 0) + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t s = (MODE == 1 ? A.d.s0 : 0) + (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / S_;
     if (s >= A.d.n || gated_off(A.gate)) return;
     const Grid &g = grid_of<MODE == 1>(A.g, A.d, (int)s);
     DestPos d;
     const bool real = load_dest(g, A.d, (int)s, d);
     CSum ax, ay, az, xx, xy, xz, dr;
+    // lanes: lane l keeps the sums l, l + S, ... of (ax, ay, az, dr, xx, xy, xz)
+    CSum mine[S_ > 1 ? 8 / S_ : 1];
     if (real) {
         const float4 vi = A.d.velh[s];
         const float4 sti = A.d.st[s];
@@ -411,7 +452,7 @@ __global__ void __launch_bounds__(kPairBlock) k_rates(const __grid_constant__ Ra
             const uint32_t fl = SPEC != 0 ? SF : S.flags;
             // the boundary force has its own support (normal distance, delp)
             const bool filt = !uh || (fl & SPH_TERM_BFORCE) != 0;
-            for_listed<KX, (SPEC != 0 ? 3 : 2), MODE == 2>(g, S, A.cap[si], A.stride[si], (int)s, d, A.d, filt,
+            for_listed<KX, (SPEC != 0 ? 3 : 2), MODE == 2, S_>(g, S, A.cap[si], A.stride[si], (int)s, d, A.d, filt,
                 [&](int j) { return VelState{S.velh[j], S.st[j]}; },
                 [&](bool ok, int j, float rx, float ry, float rz, float mj, const VelState &vs) {
                 const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
@@ -486,7 +527,28 @@ __global__ void __launch_bounds__(kPairBlock) k_rates(const __grid_constant__ Ra
                     }
                 }
             },
-            [&]() {
+            [&](bool round) {
+                if constexpr (S_ > 1) {
+                    float v[8] = {pax, pay, paz, pdr, pxx, pxy, pxz, 0.f};
+                    if (round) {
+                        lane_transpose<S_>(v);
+#pragma unroll
+                        for (int q = 0; q < 8 / S_; ++q)
+#pragma unroll
+                            for (int t = 0; t < S_; ++t) mine[q].add(v[S_ * q + t]);
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < 8 / S_; ++q) {
+                            float x = 0.f;
+#pragma unroll
+                            for (int t = 0; t < S_; ++t)
+                                if ((int)(threadIdx.x % S_) == t) x = v[S_ * q + t];
+                            mine[q].add(x);
+                        }
+                    }
+                    pax = pay = paz = pdr = pxx = pxy = pxz = 0.f;
+                    return;
+                }
                 ax.add(pax); ay.add(pay); az.add(paz);
                 pax = pay = paz = 0.f;
                 if (MAY_DRHO) {
@@ -501,6 +563,27 @@ __global__ void __launch_bounds__(kPairBlock) k_rates(const __grid_constant__ Ra
         }
     }
     const int orig = d.orig;
+    if constexpr (S_ > 1) {
+        // each lane stores its sums
+#pragma unroll
+        for (int q = 0; q < 8 / S_; ++q) {
+            const int l = S_ * q + threadIdx.x % S_;
+            double v = real ? f2d_exact(mine[q].hi) + f2d_exact(mine[q].lo) : 0.0;
+            double *out = nullptr;
+            if (l < 3) {
+                out = l == 0 ? A.acc[0] : (l == 1 ? A.acc[1] : A.acc[2]);
+                if (real && A.add_gravity) v += l == 0 ? A.gx : (l == 1 ? A.gy : A.gz);
+            } else if (l == 3) {
+                out = A.drho;
+                if (A.drho && A.vdiv && real) v = -v / A.d.rho[orig];
+            } else if (l < 7) {
+                out = l == 4 ? A.pos[0] : (l == 5 ? A.pos[1] : A.pos[2]);
+                if (real && A.add_velocity) v += ld0(l == 4 ? A.d.u : (l == 5 ? A.d.v : A.d.w), orig);
+            }
+            if (out) out[orig] = (A.accumulate ? out[orig] : 0.0) + v;
+        }
+        return;
+    }
     double a3[3] = {0.0, 0.0, 0.0}, p3[3] = {0.0, 0.0, 0.0};
     if (real) {
         a3[0] = ax.value(); a3[1] = ay.value(); a3[2] = az.value();
@@ -820,6 +903,23 @@ SrcDev make_src(const ArraySnap &S) {
 
 int blocks_for(int64_t n) {
     return (int)std::max<int64_t>(1, (n + kPairBlock - 1) / kPairBlock);
+}
+
+// Threads that share a destination of the rates pass.  Measured (us per pass
+// with 1 / 2 / 4 / 8): variable-h drop of 5 025 particles 44 / 27 / 18 / 14,
+// 31 400 46 / 29 / 34 / 46, 100 000 91 / 80 / 93 / 122; fluid-solver patch
+// of 5 025 52 / 31 / 20 / 15, 20 106 52 / 32 / 36 / 37, 87 000 103 / 92 / 91 /
+// 116; dam break of 5 000 34 / 24 / 16 / 14, 20 000 33 / 22 / 25 / 29, 80 000
+// 54 / 50 / 54 / 79.
+int pair_lanes(int64_t n) {
+    // environment SPH_PAIR_LANES = 1, 2, 8: forced, to measure and test
+    static int force = -1;
+    if (force < 0) {
+        const char *e = getenv("SPH_PAIR_LANES");
+        const int v = e ? atoi(e) : 0;
+        force = (v == 1 || v == 2 || v == 8) ? v : 0;
+    }
+    return force ? force : (n < 10000 ? 8 : (n < 120000 ? 2 : 1));
 }
 
 // List capacity override (environment SPH_LIST_CAP, >= 1): forces the
@@ -1213,7 +1313,6 @@ int rates_pass(sph_ctx *ctx, int dst, const sph_source_term *terms, int nterms,
         a.vdiv = vdiv ? 1 : 0;
     }
     if (D.n == 0) return SPH_OK;
-    const int b = blocks_for(D.n);
     int spec = 0;
     if (nterms == 1 && a.g.uniform_h) {
         if (terms[0].flags == (SPH_TERM_PGRAD | SPH_TERM_AVISC)) spec = 1;
@@ -1222,16 +1321,31 @@ int rates_pass(sph_ctx *ctx, int dst, const sph_source_term *terms, int nterms,
     // the extended search (periodic x, variable-h lists) has its own
     // instantiation of the general kernel; the specialised ones need neither
     if (a.g.periodic || a.g.symmetric) spec = 3;
+    // the specialised kernels keep a thread per destination (one source of
+    // uniform h runs in the brick passes)
+    const int v = code_variant(ctx);
+    const int lanes = v == 4 || spec == 1 || spec == 2 ? 1 : pair_lanes(D.n);
+    const int b = blocks_for(D.n * lanes);
+#define RLAUNCH1(K, L) (spec == 3 ? k_rates<K, 0, 2, L><<<b, kPairBlock, 0, ctx->stream>>>(a) \
+                                  : k_rates<K, 0, 0, L><<<b, kPairBlock, 0, ctx->stream>>>(a))
 #define RLAUNCH(K) (spec == 1 ? k_rates<K, 1, 0><<<b, kPairBlock, 0, ctx->stream>>>(a) \
                     : spec == 2 ? k_rates<K, 2, 0><<<b, kPairBlock, 0, ctx->stream>>>(a) \
-                    : spec == 3 ? k_rates<K, 0, 2><<<b, kPairBlock, 0, ctx->stream>>>(a) \
-                                : k_rates<K, 0, 0><<<b, kPairBlock, 0, ctx->stream>>>(a))
-    switch (code_variant(ctx)) {
-        case 1: RLAUNCH(1); break;
-        case 2: RLAUNCH(2); break;
-        case 4: RLAUNCH(4); break;
-        default: RLAUNCH(3); break;
+                                : RLAUNCH1(K, 1))
+#define RLAUNCH8(K) (lanes == 8 ? RLAUNCH1(K, 8) : RLAUNCH1(K, 2))
+    if (lanes > 1) {
+        if (v == 1) RLAUNCH8(1);
+        else if (v == 2) RLAUNCH8(2);
+        else RLAUNCH8(3);
+    } else {
+        switch (v) {
+            case 1: RLAUNCH(1); break;
+            case 2: RLAUNCH(2); break;
+            case 4: RLAUNCH(4); break;
+            default: RLAUNCH(3); break;
+        }
     }
+#undef RLAUNCH1
+#undef RLAUNCH8
 #undef RLAUNCH
     count_launch();
     SPH_LAUNCH_CHECK("k_rates");

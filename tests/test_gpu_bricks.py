@@ -242,3 +242,51 @@ def test_lanes_and_rounds_give_the_same_bits(subdiv):
         assert r.returncode == 0, r.stderr[-3000:]
         seen.add(r.stdout.split()[-1])
     assert len(seen) == 1
+
+
+_HASH_LISTS = r'''
+import sys, hashlib
+sys.path.insert(0, ".")
+import numpy as np, pysph_gb300
+from pysph_gb300 import workloads as W
+api = pysph_gb300.api()
+h = hashlib.sha256()
+def run(s, particles, dt, names, steps=3):
+    for _ in range(steps):
+        s.integrator.integrate(dt)
+    for a in particles.arrays:
+        for f in names:
+            h.update((a.get(f) + 0.0).tobytes())
+names = ("x", "y", "u", "v", "w", "rho", "p", "cs")
+for dx in (0.5, 0.04):
+    drop = W.elliptical_drop(dx=dx, c0=100.0)
+    run(*W.setup_drop(api, W.jitter_h(drop), c0=100.0, variable_h=True), 1e-5, names)
+    run(*W.setup_fluid_solver(api, W.circular_patch(dx=dx)), 1e-5, names)
+strip = W.periodic_strip(dx=0.05, nx=31, ny=7, jitter=0.1)
+run(*W.setup_drop(api, strip, c0=10.0, periodic_domain=api.base.PeriodicDomain(0.0, 1.55)), 1e-4,
+    names)
+fluid, wall = W.dam_break(dx=0.04)
+rng = np.random.default_rng(3)
+fluid["u"], fluid["v"] = rng.normal(0, 1, (2, fluid["x"].size))
+run(*W.setup_dam_break(api, fluid, wall, 0.04, W.dam_break_c0()), 2.5e-5, names)
+print(h.hexdigest())
+'''
+
+
+@pytest.mark.parametrize("cap", ["", "9"], ids=["lists", "over-full-lists"])
+def test_list_rates_lanes_give_the_same_bits(cap):
+    """One, two or eight threads per destination of the list-streaming rates
+    pass fold the same batches in the same order: variable-h, periodic,
+    continuity and boundary-force steps agree bit for bit, also where lists
+    overflow and the rest comes from a traversal."""
+    _need_gpu()
+    seen = set()
+    for lanes in ("1", "2", "8"):
+        e = dict(os.environ, SPH_PAIR_LANES=lanes)
+        if cap:
+            e["SPH_LIST_CAP"] = cap
+        r = subprocess.run([sys.executable, "-c", _HASH_LISTS], cwd=ROOT, env=e,
+                           capture_output=True, text=True, timeout=600)
+        assert r.returncode == 0, r.stderr[-3000:]
+        seen.add(r.stdout.split()[-1])
+    assert len(seen) == 1
