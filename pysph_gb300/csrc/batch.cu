@@ -35,7 +35,8 @@ __global__ void k_inst_fill(int *inst_of, int64_t offset, int64_t n, int k) {
 // keys on the per-instance grids (+ jump check against the instance's
 // reference cell, base/cell.pyx:1422-1437)
 __global__ void k_bkeys(sph_array_view a, const Grid *grids, const double *inv_cs_ref,
-                        const int *inst_of, int *key, int *count, int *refcell, int check_jump,
+                        const int *inst_of, int *key, int *place, int *count, int *refcell,
+                        int check_jump,
                         unsigned *err) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.n;
          i += (int64_t)gridDim.x * blockDim.x) {
@@ -60,7 +61,7 @@ __global__ void k_bkeys(sph_array_view a, const Grid *grids, const double *inv_c
         if (out) atomicOr(err, SPH_EFLAG_BOX);
         const int kc = (int)g.cell_base + c[0] + g.nx * (c[1] + g.ny * c[2]);
         key[i] = kc;
-        atomicAdd(&count[kc], 1);
+        place[i] = atomicAdd(&count[kc], 1);
         const double ir = inv_cs_ref[k];
         bool jump = false;
 #pragma unroll
@@ -74,11 +75,14 @@ __global__ void k_bkeys(sph_array_view a, const Grid *grids, const double *inv_c
 }
 
 __global__ void k_breorder(sph_array_view a, const Grid *grids, const int *inst_of,
-                           const int *perm, const int *key, int *skey, int *sinst, float *scx,
-                           float4 *velh, float4 *st, float4 *pm) {
-    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < a.n;
-         s += (int64_t)gridDim.x * blockDim.x) {
-        const int i = perm[s];
+                           const int *order, const int *cstart, int *perm, const int *key,
+                           int *skey, int *sinst, float *scx, float4 *velh, float4 *st,
+                           float4 *pm) {
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < a.n;
+         e += (int64_t)gridDim.x * blockDim.x) {
+        const int i = order[e];
+        const int s = sorted_slot(order, cstart, key[i], i);
+        perm[s] = i;
         const int k = inst_of[i];
         const Grid &g = grids[k];
         const int kl = key[i] - (int)g.cell_base;
@@ -197,14 +201,12 @@ int batch_place(sph_batch *b, const double *lo, const double *hi) {
     ArraySnap &A = b->snap;
     if (cells + 1 > b->cell_cap) {
         cudaFree(A.cstart);
-        cudaFree(A.cursor);
-        A.cstart = A.cursor = nullptr;
+        A.cstart = nullptr;
         const int64_t cap = cells + 1 + (cells + 1) / 4;
         SPH_CUDA(cudaMalloc(&A.cstart, sizeof(int) * cap));
-        SPH_CUDA(cudaMalloc(&A.cursor, sizeof(int) * cap));
         b->cell_cap = cap;
         // scan scratch (sized now: nothing is allocated while a step is captured)
-        const int64_t ntiles = (cap + 2047) / 2048 + 1;
+        const int64_t ntiles = (cap + 8191) / 8192 + 1;
         if (ntiles > b->ctx->scan_tmp_cap) {
             cudaFree(b->ctx->scan_tmp);
             b->ctx->scan_tmp = nullptr;
@@ -257,17 +259,16 @@ int batch_build(sph_batch *b, int check_jump) {
     SPH_CUDA(cudaMemsetAsync(A.cstart, 0, sizeof(int) * (b->total_cells + 1), st));
     const int nb = grid_blocks(n, kThreads);
     k_bkeys<<<nb, kThreads, 0, st>>>(b->view, b->d_grids, b->d_inv_ref, b->inst_of, A.key,
-                                     A.cstart, A.refcell, check_jump && b->steps_built > 0,
+                                     A.skey, A.cstart, A.refcell, check_jump && b->steps_built > 0,
                                      b->d_err);
     count_launch();
     SPH_LAUNCH_CHECK("k_bkeys");
     int rc = scan_exclusive(b->ctx, A.cstart, b->total_cells + 1);
     if (rc) return rc;
-    SPH_CUDA(cudaMemcpyAsync(A.cursor, A.cstart, sizeof(int) * b->total_cells,
-                             cudaMemcpyDeviceToDevice, st));
-    launch_counting_sort(st, n, b->total_cells, A.key, A.cursor, A.cstart, A.perm);
-    k_breorder<<<nb, kThreads, 0, st>>>(b->view, b->d_grids, b->inst_of, A.perm, A.key, A.skey,
-                                        b->sinst, A.scx, A.velh, A.st, A.pm);
+    launch_scatter(st, n, A.key, A.skey, A.cstart, A.order);
+    k_breorder<<<grid_blocks(n, kThreads, 64), kThreads, 0, st>>>(
+        b->view, b->d_grids, b->inst_of, A.order, A.cstart, A.perm, A.key, A.skey, b->sinst, A.scx,
+        A.velh, A.st, A.pm);
     count_launch();
     SPH_LAUNCH_CHECK("k_breorder");
     b->steps_built += 1;
@@ -347,6 +348,7 @@ int batch_setup(sph_batch *b, const sph_array_view *all, const sph_batch_instanc
     ArraySnap &A = b->snap;
     A.n = n;
     SPH_CUDA(cudaMalloc(&A.key, sizeof(int) * n));
+    SPH_CUDA(cudaMalloc(&A.order, sizeof(int) * n));
     SPH_CUDA(cudaMalloc(&A.perm, sizeof(int) * n));
     SPH_CUDA(cudaMalloc(&A.skey, sizeof(int) * n));
     SPH_CUDA(cudaMalloc(&A.scx, sizeof(float) * n));
@@ -566,7 +568,7 @@ void batch_free(sph_batch *b) {
     if (b->graph_exec) cudaGraphExecDestroy(b->graph_exec);
     ArraySnap &A = b->snap;
     cudaFree(A.key); cudaFree(A.perm); cudaFree(A.skey); cudaFree(A.scx); cudaFree(A.pm); cudaFree(A.velh);
-    cudaFree(A.st); cudaFree(A.cstart); cudaFree(A.cursor); cudaFree(A.refcell);
+    cudaFree(A.st); cudaFree(A.cstart); cudaFree(A.order); cudaFree(A.refcell);
     cudaFree(b->d_grids); cudaFree(b->d_inv_ref); cudaFree(b->inst_of); cudaFree(b->sinst);
     cudaFree(b->list.nbr); cudaFree(b->list.cnt); cudaFree(b->list.maxcnt);
     for (int c = 0; c < 6; ++c) {

@@ -107,7 +107,7 @@ int sph_ctx_destroy(sph_ctx *c) {
         cudaFree(A.key); cudaFree(A.perm); cudaFree(A.skey);
         cudaFree(A.scx); cudaFree(A.pm); cudaFree(A.velh); cudaFree(A.st);
         cudaFree(A.nrm); cudaFree(A.tan);
-        cudaFree(A.cstart); cudaFree(A.cursor); cudaFree(A.refcell); cudaFree(A.pm0); cudaFree(A.inv);
+        cudaFree(A.cstart); cudaFree(A.order); cudaFree(A.refcell); cudaFree(A.pm0); cudaFree(A.inv);
         cudaFree(A.bsrc);
         cudaFree(A.bdst);
         cudaFree(A.brow);

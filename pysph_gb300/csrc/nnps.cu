@@ -7,11 +7,12 @@
 //
 //   k_box       bounding box of all arrays in internal cells, max h, and the
 //               reference's jump-tolerance check (cell.pyx:1422-1437)
-//   k_keys      dense cell index per particle + per-cell counts (atomics)
+//   k_keys      dense cell index per particle, per-cell counts (atomics) and
+//               the particle's place among its cell's arrivals
 //   scan        exclusive prefix of the counts -> cstart
-//   k_scatter   counting-sort scatter (order within a cell arbitrary)
-//   k_cellsort  per-cell insertion sort by original index (deterministic)
-//   k_reorder   gather of the sorted FP32 snapshot (cell-local offsets)
+//   k_scatter   particles by cell (order within a cell arbitrary)
+//   k_reorder   gather of the sorted FP32 snapshot (cell-local offsets), the
+//               order within a cell by original index (deterministic)
 //
 // No per-destination neighbour list is stored: the pair kernels walk the
 // stencil rows of the sorted arrays directly.
@@ -40,26 +41,33 @@ __device__ __forceinline__ int floor_cell(double x, double inv_cs) {
 __global__ void k_box(sph_array_view a, double inv_cs, double inv_cs_ref, int *refcell,
                       int check_jump, int *box, unsigned long long *hmax, unsigned *err,
                       Grid pg) {
+    // cells screened in FP32, h compared by its bits (as signed integers,
+    // ordered like the non-negative doubles; a NaN does not count): the FP64
+    // pipe bound this kernel, 37 -> 19 us at 1 M particles
     int mn[3] = {INT_MAX, INT_MAX, INT_MAX};
     int mx[3] = {INT_MIN, INT_MIN, INT_MIN};
-    double hm = 0.0, hn = 1.0e308;
+    long long hm = 0, hn = __double_as_longlong(1.0e308);
     bool jump = false;
+    const float inv_f = (float)inv_cs, inv_ref_f = (float)inv_cs_ref;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.n;
          i += (int64_t)gridDim.x * blockDim.x) {
         double p[3] = {ld0(a.x, i), ld0(a.y, i), ld0(a.z, i)};
         const double pb[3] = {bin_x(pg, p[0]), p[1], p[2]};
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            int c = floor_cell(pb[d], inv_cs);
+            int c = floor_cell_screened(pb[d], inv_cs, inv_f);
             mn[d] = min(mn[d], c);
             mx[d] = max(mx[d], c);
         }
-        hm = fmax(hm, a.h[i]);
-        hn = fmin(hn, a.h[i]);
+        const long long hb = __double_as_longlong(a.h[i]);
+        if ((hb & 0x7fffffffffffffffll) <= 0x7ff0000000000000ll) {
+            hm = max(hm, hb);
+            hn = min(hn, hb);
+        }
         if (refcell) {
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
-                int c = floor_cell(p[d], inv_cs_ref);
+                int c = floor_cell_screened(p[d], inv_cs_ref, inv_ref_f);
                 if (check_jump && abs(c - refcell[3 * i + d]) > 1) jump = true;
                 refcell[3 * i + d] = c;
             }
@@ -67,7 +75,7 @@ __global__ void k_box(sph_array_view a, double inv_cs, double inv_cs_ref, int *r
     }
     // warp, then block, then one set of atomics per block
     __shared__ int s_mn[3][32], s_mx[3][32];
-    __shared__ double s_h[32], s_hn[32];
+    __shared__ long long s_h[32], s_hn[32];
     __shared__ int s_j[32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
@@ -76,8 +84,8 @@ __global__ void k_box(sph_array_view a, double inv_cs, double inv_cs_ref, int *r
         mx[d] = __reduce_max_sync(0xffffffffu, mx[d]);
     }
     for (int off = 16; off > 0; off >>= 1) {
-        hm = fmax(hm, __shfl_xor_sync(0xffffffffu, hm, off));
-        hn = fmin(hn, __shfl_xor_sync(0xffffffffu, hn, off));
+        hm = max(hm, __shfl_xor_sync(0xffffffffu, hm, off));
+        hn = min(hn, __shfl_xor_sync(0xffffffffu, hn, off));
     }
     int anyjump = __any_sync(0xffffffffu, jump) ? 1 : 0;
     if (lane == 0) {
@@ -97,11 +105,11 @@ __global__ void k_box(sph_array_view a, double inv_cs, double inv_cs_ref, int *r
             a[d] = __reduce_min_sync(0xffffffffu, a[d]);
             b[d] = __reduce_max_sync(0xffffffffu, b[d]);
         }
-        double hh = lane < nw ? s_h[lane] : 0.0;
-        double hl = lane < nw ? s_hn[lane] : 1.0e308;
+        long long hh = lane < nw ? s_h[lane] : 0;
+        long long hl = lane < nw ? s_hn[lane] : __double_as_longlong(1.0e308);
         for (int off = 16; off > 0; off >>= 1) {
-            hh = fmax(hh, __shfl_xor_sync(0xffffffffu, hh, off));
-            hl = fmin(hl, __shfl_xor_sync(0xffffffffu, hl, off));
+            hh = max(hh, __shfl_xor_sync(0xffffffffu, hh, off));
+            hl = min(hl, __shfl_xor_sync(0xffffffffu, hl, off));
         }
         int jj = __any_sync(0xffffffffu, lane < nw && s_j[lane]);
         if (lane == 0) {
@@ -110,8 +118,8 @@ __global__ void k_box(sph_array_view a, double inv_cs, double inv_cs_ref, int *r
                 atomicMin(&box[d], a[d]);
                 atomicMax(&box[3 + d], b[d]);
             }
-            atomicMax(hmax, (unsigned long long)__double_as_longlong(hh));
-            atomicMin(hmax + 1, (unsigned long long)__double_as_longlong(hl));
+            atomicMax(hmax, (unsigned long long)hh);
+            atomicMin(hmax + 1, (unsigned long long)hl);
             if (jj) atomicOr(err, SPH_EFLAG_JUMP);
         }
     }
@@ -122,7 +130,17 @@ __global__ void k_publish(const unsigned *src, unsigned *dst, int n) {
     __threadfence_system();
 }
 
-__global__ void k_box_init(int *box, unsigned long long *hmax) {
+// the results of k_box and the status block, in one launch
+__global__ void k_publish_box(const int *box, const unsigned *hrange, int *hbox,
+                              const unsigned *status, unsigned *hstatus, int n) {
+    const int i = threadIdx.x;
+    if (i < 6) hbox[i] = box[i];
+    else if (i < 10) hbox[i] = (int)hrange[i - 6];
+    for (int k = i; k < n; k += blockDim.x) hstatus[k] = status[k];
+    __threadfence_system();
+}
+
+__global__ void k_box_init(int *box, unsigned long long *hmax, unsigned *err) {
     if (threadIdx.x < 3) {
         box[threadIdx.x] = INT_MAX;
         box[3 + threadIdx.x] = INT_MIN;
@@ -130,13 +148,14 @@ __global__ void k_box_init(int *box, unsigned long long *hmax) {
     if (threadIdx.x == 0) {
         hmax[0] = 0ull;
         hmax[1] = (unsigned long long)__double_as_longlong(1.0e308);
+        *err = 0u;
     }
 }
 
 // -------------------------------------------------------------------------
 // keys, counting sort
 // -------------------------------------------------------------------------
-__global__ void k_keys(sph_array_view a, Grid g, int *key, int *count) {
+__global__ void k_keys(sph_array_view a, Grid g, int *key, int *place, int *count) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.n;
          i += (int64_t)gridDim.x * blockDim.x) {
         int cx = bin_cell_x(g, bin_x(g, ld0(a.x, i)));
@@ -144,17 +163,19 @@ __global__ void k_keys(sph_array_view a, Grid g, int *key, int *count) {
         int cz = floor_cell(ld0(a.z, i), g.inv_cs) - g.bz0;
         int k = cx + g.nx * (cy + g.ny * cz);
         key[i] = k;
-        atomicAdd(&count[k], 1);
+        place[i] = atomicAdd(&count[k], 1);
     }
 }
 
-// exclusive scan, 3 phases over tiles of kScanTile counts: tile totals
-// (read only), exclusive scan of the totals, then each tile re-read, scanned
-// and written with its offset.  Every thread moves one int4 per step, so a
-// warp's accesses are 512 contiguous bytes.
-constexpr int kScanV = 4;                                   // counts per thread per step
+// exclusive scan over tiles of kScanTile counts: tile totals (read only), then
+// each tile re-read, scanned and written with its offset.  The offset is the
+// sum of the totals before the tile, which every block adds up itself, or,
+// past kScanTotals tiles, their exclusive scan by a launch between the two.
+// One tile is scanned by the second launch alone.
+constexpr int kScanV = 4;                                   // counts per load
 constexpr int kScanSteps = 8;
 constexpr int kScanTile = kThreads * kScanV * kScanSteps;   // 8192 counts
+constexpr int64_t kScanTotals = 4096;
 
 __device__ __forceinline__ int block_exclusive_scan(int v, int *smem, int &total) {
     // warp inclusive scan
@@ -221,16 +242,34 @@ __global__ void k_scan_totals(int *tot, int64_t ntiles) {
     }
 }
 
-__global__ void k_scan_apply(int *data, int64_t n, const int *tile_off) {
+// Every thread scans kScanSteps * kScanV consecutive counts (one 128-byte
+// line), so a tile takes one block scan.  totals: tile_off holds totals to be
+// summed, else offsets.
+__global__ void k_scan_apply(int *data, int64_t n, const int *tile_off, int totals) {
     __shared__ int smem[32];
-    const int64_t base = blockIdx.x * (int64_t)kScanTile;
-    int carry = tile_off[blockIdx.x];
+    int carry = 0, total;
+    if (totals) {
+        int s = 0;
+        for (int64_t t = threadIdx.x; t < blockIdx.x; t += kThreads) s += tile_off[t];
+        block_exclusive_scan(s, smem, carry);
+    } else {
+        carry = tile_off[blockIdx.x];
+    }
+    const int64_t base = blockIdx.x * (int64_t)kScanTile +
+                         (int64_t)threadIdx.x * (kScanSteps * kScanV);
+    int4 v[kScanSteps];
+    int s = 0;
+#pragma unroll
     for (int st = 0; st < kScanSteps; ++st) {
-        const int64_t i = base + ((int64_t)st * kThreads + threadIdx.x) * kScanV;
-        const int4 v = scan_load(data, n, i);
-        int total;
-        const int pre = carry + block_exclusive_scan(v.x + v.y + v.z + v.w, smem, total);
-        const int4 o = make_int4(pre, pre + v.x, pre + v.x + v.y, pre + v.x + v.y + v.z);
+        v[st] = scan_load(data, n, base + st * kScanV);
+        s += v[st].x + v[st].y + v[st].z + v[st].w;
+    }
+    int pre = carry + block_exclusive_scan(s, smem, total);
+#pragma unroll
+    for (int st = 0; st < kScanSteps; ++st) {
+        const int64_t i = base + st * kScanV;
+        const int4 o = make_int4(pre, pre + v[st].x, pre + v[st].x + v[st].y,
+                                 pre + v[st].x + v[st].y + v[st].z);
         if (i + kScanV <= n) {
             *reinterpret_cast<int4 *>(data + i) = o;
         } else {
@@ -238,44 +277,40 @@ __global__ void k_scan_apply(int *data, int64_t n, const int *tile_off) {
             if (i + 1 < n) data[i + 1] = o.y;
             if (i + 2 < n) data[i + 2] = o.z;
         }
-        carry += total;
+        pre = o.w + v[st].w;
     }
 }
 
-__global__ void k_scatter(int64_t n, const int *key, int *cursor, int *perm) {
+__global__ void k_scatter(int64_t n, const int *key, const int *place, const int *cstart,
+                          int *order) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        int slot = atomicAdd(&cursor[key[i]], 1);
-        perm[slot] = (int)i;
-    }
-}
-
-__global__ void k_cellsort(int64_t ncells, const int *cstart, int *perm) {
-    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < ncells;
-         c += (int64_t)gridDim.x * blockDim.x) {
-        int s = cstart[c], e = cstart[c + 1];
-        for (int a = s + 1; a < e; ++a) {
-            int v = perm[a];
-            int b = a - 1;
-            while (b >= s && perm[b] > v) {
-                perm[b + 1] = perm[b];
-                --b;
-            }
-            perm[b + 1] = v;
-        }
-    }
+         i += (int64_t)gridDim.x * blockDim.x)
+        order[cstart[key[i]] + place[i]] = (int)i;
 }
 
 // -------------------------------------------------------------------------
 // sorted snapshot
 // -------------------------------------------------------------------------
-__global__ void k_reorder(sph_array_view a, Grid g, const int *perm, const int *key, int *skey,
-                          float *scx, float4 *velh, float4 *st, float4 *nrm, float4 *tan,
-                          float4 *pm) {
-    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < a.n;
-         s += (int64_t)gridDim.x * blockDim.x) {
-        int i = perm[s];
-        int k = key[i];
+// Snapshot of the particles in cell order.  SORT (a full build): entry s of
+// the scatter's order gives the particle, its rank by original index among its
+// cell's entries the slot (a pass that sorted the cells one by one first took
+// 17 us at 1 M particles, in the batches 25), perm, the inverse permutation
+// and the build's position records in original order (so that a light refresh
+// reads them with its other per-particle loads, not through the slot it has
+// yet to load) are written too.  Otherwise perm is the order.
+template <bool SORT>
+__global__ void k_reorder(sph_array_view a, Grid g, const int *order, const int *cstart, int *perm,
+                          const int *key, int *skey, float *scx, float4 *velh, float4 *st,
+                          float4 *nrm, float4 *tan, float4 *pm, int *inv, float4 *pm0) {
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < a.n;
+         e += (int64_t)gridDim.x * blockDim.x) {
+        const int i = SORT ? order[e] : perm[e];
+        const int k = key[i];
+        int64_t s = e;
+        if (SORT) {
+            s = sorted_slot(order, cstart, k, i);
+            perm[s] = i;
+        }
         skey[s] = k;
         int cx, cy, cz;
         decode_cell(g, k, cx, cy, cz);
@@ -289,6 +324,10 @@ __global__ void k_reorder(sph_array_view a, Grid g, const int *perm, const int *
         float rho = (float)ld0(a.rho, i), p = (float)ld0(a.p, i), m = (float)a.m[i];
         st[s] = make_float4(rho, p / (rho * rho), (float)ld0(a.cs, i), m);
         pm[s] = make_float4(xi, yi, zi, m);
+        if (SORT && inv) {
+            inv[i] = (int)s;
+            pm0[i] = make_float4(xi, yi, zi, m);
+        }
         if (nrm) {
             nrm[s] = make_float4((float)ld0(a.nx, i), (float)ld0(a.ny, i), (float)ld0(a.nz, i), 0.f);
             tan[s] = make_float4((float)ld0(a.tx, i), (float)ld0(a.ty, i), (float)ld0(a.tz, i), 0.f);
@@ -347,18 +386,6 @@ __global__ void k_selftest_conversions(long long n, unsigned long long *bad) {
         if (floor_cell_screened(pos, inv, (float)inv) != (int)floor(pos * inv)) ++miss;
     }
     if (miss) atomicAdd(bad, miss);
-}
-
-// original -> sorted slot, and the build's position records in original
-// order (so that a light refresh reads them with its other per-particle
-// loads, not through the slot it has yet to load)
-__global__ void k_invperm(int64_t n, const int *perm, const float4 *pm, int *inv, float4 *pm0) {
-    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < n;
-         s += (int64_t)gridDim.x * blockDim.x) {
-        const int i = perm[s];
-        inv[i] = (int)s;
-        pm0[i] = pm[s];
-    }
 }
 
 __global__ void __launch_bounds__(256, 5) k_light(sph_array_view a, Grid g, double inv_cs_ref, const int *inv,
@@ -540,14 +567,15 @@ int ensure(T **p, int64_t &cap, int64_t need) {
 
 int alloc_array(ArraySnap &A, int64_t n, bool nrm) {
     if (n <= A.cap && A.perm && (!nrm || A.nrm)) return SPH_OK;
-    cudaFree(A.key); cudaFree(A.perm); cudaFree(A.skey);
+    cudaFree(A.key); cudaFree(A.order); cudaFree(A.perm); cudaFree(A.skey);
     cudaFree(A.scx); cudaFree(A.pm); cudaFree(A.velh); cudaFree(A.st); cudaFree(A.nrm);
     cudaFree(A.tan);
-    A.key = A.perm = A.skey = nullptr;
+    A.key = A.order = A.perm = A.skey = nullptr;
     A.scx = nullptr;
     A.pm = A.velh = A.st = A.nrm = A.tan = nullptr;
     int64_t c = std::max<int64_t>(n, 1);
     SPH_CUDA(cudaMalloc(&A.key, sizeof(int) * c));
+    SPH_CUDA(cudaMalloc(&A.order, sizeof(int) * c));
     SPH_CUDA(cudaMalloc(&A.perm, sizeof(int) * c));
     SPH_CUDA(cudaMalloc(&A.skey, sizeof(int) * c));
     SPH_CUDA(cudaMalloc(&A.scx, sizeof(float) * c));
@@ -576,19 +604,25 @@ int scan_exclusive(sph_ctx *ctx, int *data, int64_t n) {
     int64_t ntiles = (n + kScanTile - 1) / kScanTile;
     int rc = ensure(&ctx->scan_tmp, ctx->scan_tmp_cap, ntiles);
     if (rc) return rc;
-    k_scan_reduce<<<(unsigned)ntiles, kThreads, 0, ctx->stream>>>(data, n, ctx->scan_tmp);
-    k_scan_totals<<<1, 1024, 0, ctx->stream>>>(ctx->scan_tmp, ntiles);
-    k_scan_apply<<<(unsigned)ntiles, kThreads, 0, ctx->stream>>>(data, n, ctx->scan_tmp);
-    count_launch(3);
+    const bool totals = ntiles <= kScanTotals;
+    if (ntiles > 1) {
+        k_scan_reduce<<<(unsigned)ntiles, kThreads, 0, ctx->stream>>>(data, n, ctx->scan_tmp);
+        count_launch();
+    }
+    if (!totals) {
+        k_scan_totals<<<1, 1024, 0, ctx->stream>>>(ctx->scan_tmp, ntiles);
+        count_launch();
+    }
+    k_scan_apply<<<(unsigned)ntiles, kThreads, 0, ctx->stream>>>(data, n, ctx->scan_tmp, totals);
+    count_launch();
     SPH_LAUNCH_CHECK("scan");
     return SPH_OK;
 }
 
-void launch_counting_sort(cudaStream_t st, int64_t n, int64_t ncells, const int *key, int *cursor,
-                          const int *cstart, int *perm) {
-    k_scatter<<<grid_blocks(n, kThreads), kThreads, 0, st>>>(n, key, cursor, perm);
-    k_cellsort<<<grid_blocks(ncells, kThreads), kThreads, 0, st>>>(ncells, cstart, perm);
-    count_launch(2);
+void launch_scatter(cudaStream_t st, int64_t n, const int *key, const int *place, const int *cstart,
+                    int *order) {
+    k_scatter<<<grid_blocks(n, kThreads), kThreads, 0, st>>>(n, key, place, cstart, order);
+    count_launch();
 }
 
 int grid_blocks(int64_t n, int threads, int per_sm) {
@@ -640,9 +674,8 @@ int nnps_build(sph_ctx *ctx, const sph_array_view *arrays, int narrays, double c
     const double inv_cs = 1.0 / cs;
     const double inv_cs_ref = 1.0 / cell_size;
 
-    k_box_init<<<1, 32, 0, st>>>(ctx->d_box, ctx->d_hmax);
+    k_box_init<<<1, 32, 0, st>>>(ctx->d_box, ctx->d_hmax, ctx->d_err);
     count_launch();
-    SPH_CUDA(cudaMemsetAsync(ctx->d_err, 0, sizeof(unsigned), st));
     for (int a = 0; a < narrays; ++a) {
         ArraySnap &A = ctx->arrays[a];
         const sph_array_view &v = arrays[a];
@@ -664,15 +697,12 @@ int nnps_build(sph_ctx *ctx, const sph_array_view *arrays, int narrays, double c
         count_launch();
         SPH_LAUNCH_CHECK("k_box");
     }
-    {
-        int rcp = publish_words(ctx, ctx->d_box, ctx->hd_box, 6);
-        if (!rcp) rcp = publish_words(ctx, ctx->d_hmax, ctx->hd_box + 6, 4);   // hmax, hmin
-        if (rcp) return rcp;
-    }
-    {
-        const int rcm = list_maxima_async(ctx);   // with the error word
-        if (rcm) return rcm;
-    }
+    // box, h range (hmax, hmin) and the status block (error word, list maxima)
+    k_publish_box<<<1, 128, 0, st>>>(ctx->d_box, (const unsigned *)ctx->d_hmax, ctx->hd_box,
+                                     ctx->d_status, ctx->hd_status,
+                                     kListWord0 + std::min((int)ctx->lists.size(), kMaxListSlots));
+    count_launch();
+    SPH_LAUNCH_CHECK("k_publish_box");
     SPH_CUDA(cudaStreamSynchronize(st));
     list_maxima_collect(ctx);
     unsigned err = ctx->h_status[0];
@@ -760,50 +790,40 @@ int nnps_build(sph_ctx *ctx, const sph_array_view *arrays, int narrays, double c
         if (rc) return rc;
         if (g.ncells + 1 > A.cell_cap || !A.cstart) {
             cudaFree(A.cstart);
-            cudaFree(A.cursor);
-            A.cstart = A.cursor = nullptr;
+            A.cstart = nullptr;
             int64_t c = g.ncells + 1 + (g.ncells + 1) / 4;
             SPH_CUDA(cudaMalloc(&A.cstart, sizeof(int) * c));
-            SPH_CUDA(cudaMalloc(&A.cursor, sizeof(int) * c));
             A.cell_cap = c;
         }
         SPH_CUDA(cudaMemsetAsync(A.cstart, 0, sizeof(int) * (g.ncells + 1), st));
         if (v.n > 0) {
             int nb = grid_blocks(v.n, kThreads);
-            k_keys<<<nb, kThreads, 0, st>>>(v, g, A.key, A.cstart);
+            // (the place among a cell's arrivals: in skey, which k_reorder writes later)
+            k_keys<<<nb, kThreads, 0, st>>>(v, g, A.key, A.skey, A.cstart);
             count_launch();
             SPH_LAUNCH_CHECK("k_keys");
         }
         rc = scan_exclusive(ctx, A.cstart, g.ncells + 1);
         if (rc) return rc;
         if (v.n > 0) {
-            SPH_CUDA(cudaMemcpyAsync(A.cursor, A.cstart, sizeof(int) * g.ncells,
-                                     cudaMemcpyDeviceToDevice, st));
-            int nb = grid_blocks(v.n, kThreads);
-            k_scatter<<<nb, kThreads, 0, st>>>(v.n, A.key, A.cursor, A.perm);
-            k_cellsort<<<grid_blocks(g.ncells, kThreads), kThreads, 0, st>>>(g.ncells, A.cstart, A.perm);
-            k_reorder<<<nb, kThreads, 0, st>>>(v, g, A.perm, A.key, A.skey, A.scx, A.velh, A.st,
-                                               A.has_nrm ? A.nrm : nullptr,
-                                               A.has_nrm ? A.tan : nullptr, A.pm);
-            count_launch(3);
+            if (g.skin > 0.f && A.pm0_cap < v.n) {
+                cudaFree(A.pm0);
+                cudaFree(A.inv);
+                A.pm0 = nullptr;
+                A.inv = nullptr;
+                SPH_CUDA(cudaMalloc(&A.pm0, sizeof(float4) * v.n));
+                SPH_CUDA(cudaMalloc(&A.inv, sizeof(int) * v.n));
+                A.pm0_cap = v.n;
+            }
+            launch_scatter(st, v.n, A.key, A.skey, A.cstart, A.order);
+            k_reorder<true><<<grid_blocks(v.n, kThreads, 64), kThreads, 0, st>>>(
+                v, g, A.order, A.cstart, A.perm, A.key, A.skey, A.scx, A.velh, A.st,
+                A.has_nrm ? A.nrm : nullptr, A.has_nrm ? A.tan : nullptr, A.pm,
+                g.skin > 0.f ? A.inv : nullptr, A.pm0);
+            count_launch();
             SPH_LAUNCH_CHECK("nnps sort/reorder");
             A.st_fresh = true;
             A.st_tait_f = 0.0;
-            if (g.skin > 0.f) {
-                if (A.pm0_cap < v.n) {
-                    cudaFree(A.pm0);
-                    cudaFree(A.inv);
-                    A.pm0 = nullptr;
-                    A.inv = nullptr;
-                    SPH_CUDA(cudaMalloc(&A.pm0, sizeof(float4) * v.n));
-                    SPH_CUDA(cudaMalloc(&A.inv, sizeof(int) * v.n));
-                    A.pm0_cap = v.n;
-                }
-                k_invperm<<<grid_blocks(v.n, kThreads), kThreads, 0, st>>>(v.n, A.perm, A.pm, A.inv,
-                                                                           A.pm0);
-                count_launch();
-                SPH_LAUNCH_CHECK("k_invperm");
-            }
         }
     }
     ctx->built = true;
@@ -1023,9 +1043,9 @@ int refresh_state(sph_ctx *ctx, int a, const sph_array_view *view) {
     A.st_fresh = true;
     A.st_tait_f = 0.0;
     if (A.n == 0) return SPH_OK;
-    k_reorder<<<grid_blocks(A.n, kThreads), kThreads, 0, ctx->stream>>>(
-        A.view, ctx->grid, A.perm, A.key, A.skey, A.scx, A.velh, A.st, nrm ? A.nrm : nullptr,
-        nrm ? A.tan : nullptr, A.pm);
+    k_reorder<false><<<grid_blocks(A.n, kThreads, 64), kThreads, 0, ctx->stream>>>(
+        A.view, ctx->grid, nullptr, nullptr, A.perm, A.key, A.skey, A.scx, A.velh, A.st,
+        nrm ? A.nrm : nullptr, nrm ? A.tan : nullptr, A.pm, nullptr, nullptr);
     count_launch();
     SPH_LAUNCH_CHECK("k_reorder (refresh)");
     return SPH_OK;

@@ -134,8 +134,10 @@ static __device__ __noinline__ int floor_cell_fp64(double x, double inv) {
 // floor(x * inv) with the product rounded in FP64 (the reference's cell
 // index), screened in FP32: the FP32 product is within |t| 2^-22 of it, so
 // its floor is the same unless a cell boundary lies that close; only then
-// the FP64 product.
+// the FP64 product.  (A coordinate of exactly 0, every z of a 2D set, is on
+// such a boundary: its cell is 0.)
 __device__ __forceinline__ int floor_cell_screened(double x, double inv, float invf) {
+    if (((unsigned long long)__double_as_longlong(x) << 1) == 0ull) return 0;
     const float tf = d2f_rn(x) * invf;
     const float at = fabsf(tf);
     int c = __float2int_rd(tf);
@@ -211,13 +213,13 @@ struct ArraySnap {
     // cs = st_tait_f rho^3 (co / ro^3); 0 when st came from anything else
     double st_tait_f = 0.0;
     int *key = nullptr;   // original order, dense cell index
+    int *order = nullptr; // particles by cell, in arrival order within a cell
     int *perm = nullptr;  // sorted -> original
     int *skey = nullptr;  // sorted: cell
     float4 *velh = nullptr, *st = nullptr, *nrm = nullptr, *tan = nullptr;
     float4 *pm = nullptr;
     float *scx = nullptr;   // sorted: dense x cell
     int *cstart = nullptr; // ncells + 1
-    int *cursor = nullptr; // ncells
     int64_t cell_cap = 0;
     int *refcell = nullptr; // original order, 3 ints per particle (jump check)
     int64_t ref_n = -1;     // particle count the refcell entries belong to
@@ -479,8 +481,8 @@ int brick_rates(sph_ctx *ctx, int dst, const sph_source_term &term, NbrList &L,
                 const sph_rates_params *prm, double *const *acc, double *const *pos,
                 int accumulate);
 int scan_exclusive(sph_ctx *ctx, int *data, int64_t n);
-void launch_counting_sort(cudaStream_t st, int64_t n, int64_t ncells, const int *key, int *cursor,
-                          const int *cstart, int *perm);
+void launch_scatter(cudaStream_t st, int64_t n, const int *key, const int *place, const int *cstart,
+                    int *order);
 int batch_setup(sph_batch *b, const sph_array_view *all, const sph_batch_instance *inst,
                 int ninst, const sph_batch_recipe *rec);
 int batch_build(sph_batch *b, int check_jump);
@@ -773,6 +775,15 @@ __device__ __forceinline__ void for_neighbours(const Grid &g, const SrcDev &S, c
             }
         }
     }
+}
+
+// Sorted slot of particle i of cell k: its rank by original index among the
+// entries of the cell.
+__device__ __forceinline__ int sorted_slot(const int *order, const int *cstart, int k, int i) {
+    const int lo = cstart[k], hi = cstart[k + 1];
+    int s = lo;
+    for (int e = lo; e < hi; ++e) s += order[e] < i;
+    return s;
 }
 
 // Dense-grid coordinates of a cell key.

@@ -110,3 +110,39 @@ def test_extent_beyond_the_grid_limit_raises():
     pa = base.get_particle_array(name="fluid", type=Fluid, **props)
     with pytest.raises(RuntimeError, match="grid cells"):
         base.Particles(arrays=[pa])
+
+
+@pytest.mark.parametrize("ncells", [8190, 8191, 8192, 8193, 24576, 1 << 24, 1 << 26])
+def test_counting_sort_over_tiles_of_cells(ncells, monkeypatch):
+    """The prefix sum of the cell counts (ncells + 1 of them) in one tile of
+    8192, at its edge, in several, and in more than 4096, with a crowded cell
+    whose particles arrive in any order: exact neighbour sets, and the same
+    bits of the sums (in the order of the sort) from every build."""
+    _need_gpu()
+    monkeypatch.setenv("PYSPH_GB300_SUBDIV", "1")
+    rng = np.random.default_rng(ncells)
+    h = 0.1
+    cs = 2.0 * h                            # cell size: the search radius
+    rows = 1 if ncells <= 24576 else 16     # grid of nx by rows cells (stencil borders included)
+    ny = rows - 2 if rows > 1 else 1
+    nx = ncells // rows - 2
+    n = 600
+    x = cs * (0.5 + rng.integers(0, nx, n) + rng.uniform(-0.4, 0.4, n))
+    y = cs * (0.5 + rng.integers(0, ny, n) + rng.uniform(-0.4, 0.4, n))
+    x[:2], y[:2] = [0.5 * cs, (nx - 0.5) * cs], [0.5 * cs, (ny - 0.5) * cs]
+    x[300:] = cs * (nx // 2 + 0.5 + rng.uniform(-0.4, 0.4, 300))
+    y[300:] = cs * (ny // 2 + 0.5 + rng.uniform(-0.4, 0.4, 300))
+    perm = rng.permutation(n)
+    props = _props(x[perm], y[perm], h=h)
+    pa = base.get_particle_array(name="fluid", type=Fluid, **props)
+    particles = base.Particles(arrays=[pa], update_particles=False)
+    particles.cell_manager.set_skin(0.0)
+    particles.update()
+    loc = particles.nnps_manager.get_neighbor_particle_locator(pa, pa, 2.0)
+    off, idx = loc.neighbour_csr()
+    ro, ri = oracle.neighbors(props, props, 2.0 * h, same=True)
+    assert csr_sets(off, idx) == csr_sets(ro, ri)
+    first = _rho_and_pgrad(props)
+    again = _rho_and_pgrad(props)
+    for f in ("rho", "ax", "ay"):
+        np.testing.assert_array_equal(first.get(f), again.get(f))
