@@ -628,6 +628,7 @@ struct FeatureArgs {
     float *out_f;       // [n][192] FP32 by original index (or null)
     const int *s_skey;  // sorted: cell of each source slot
     const unsigned *gate;
+    int per;            // destinations per warp (k_features_warp)
 };
 
 template <int KX, bool EXT>
@@ -727,7 +728,11 @@ __global__ void __launch_bounds__(kPairBlock) k_features(const __grid_constant__
 }
 
 // The same features with one warp per destination (no periodic axis or
-// symmetry plane): lane k takes list entry k of every chunk of 32, the warp
+// symmetry plane).  A list of up to 32 entries, the ordinary case: lane k
+// takes entry k with its whole record, counts the smaller squared distances
+// of the warp's entries (four to a shared-memory load; of equal ones the
+// earlier entry, whose slot is the smaller, comes first) and writes that row.
+// A longer list: lane k takes entry k of every chunk of 32, the warp
 // sorts the chunk's 64-bit keys (FP32 squared distance bits, sorted slot:
 // the order of the thread-per-destination kernel) with a bitonic network
 // of shuffles and merges them into the 32 nearest so far; lane k then
@@ -759,28 +764,49 @@ __device__ __forceinline__ void feat_sort32(uint64_t &key, int lane) {
     for (int k = 2; k <= 32; k <<= 1) feat_stages(key, lane, k, k >> 1);
 }
 
-// (six blocks per SM, 40 registers: 49 us at 80 000 destinations in 2D;
-// four and eight blocks per SM measured slower)
+// the row of rank r: neighbour at (rx, ry), velocities and states, or zeros
+struct FeatRow {
+    static constexpr int NC = SPH_MLP_NCH;
+    float f[NC];
+    __device__ __forceinline__ FeatRow(const FeatureArgs &A, bool have, float rx, float ry, float vx,
+                                       float vy, float ih, const float4 &vj, const float4 &st) {
+        // (products rounded by themselves, as in the other kernel)
+        const float raw[NC] = {__fmul_rn(rx, ih), __fmul_rn(ry, ih),
+                               __fmul_rn(vj.x - vx, A.inv_c0), __fmul_rn(vj.y - vy, A.inv_c0),
+                               st.x, __fmul_rn(__fmul_rn(st.y, st.x), st.x)};
+#pragma unroll
+        for (int q = 0; q < NC; ++q) f[q] = have ? (raw[q] - A.mean[q]) * A.inv_std[q] : 0.f;
+    }
+    __device__ __forceinline__ uint32_t pair(int i) const {
+        __nv_bfloat162 h = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
+        return *reinterpret_cast<uint32_t *>(&h);
+    }
+    __device__ __forceinline__ void store_f(float *out) const {
+        float2 *o = reinterpret_cast<float2 *>(out);
+#pragma unroll
+        for (int i = 0; i < NC / 2; ++i) o[i] = make_float2(f[2 * i], f[2 * i + 1]);
+    }
+};
+
+// a destination by the sort of its chunks (all lanes, the same s)
 template <int KX>
-__global__ void __launch_bounds__(256, 6) k_features_warp(const __grid_constant__ FeatureArgs A) {
+__device__ __noinline__ void features_sorted(const FeatureArgs &A, int64_t s) {
     constexpr int NN = SPH_MLP_NNBR, NC = SPH_MLP_NCH;
     static_assert(NN == 32, "one lane per kept neighbour");
     const int lane = threadIdx.x & 31;
-    const int64_t s = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    if (s >= A.d.n || gated_off(A.gate)) return;
     DestPos d;
-    const bool real = load_dest(A.g, A.d, (int)s, d);
+    if (!load_dest(A.g, A.d, (int)s, d)) return;
     const SrcDev &S = A.s;
     const float csf = A.g.cs_f;
+    const int listed = S.ncnt[s];
     constexpr uint64_t none = ~0ull;
     uint64_t best = none;
     // offsets carried by neighbours found by the traversal (flag set)
     float crx = 0.f, cry = 0.f;
     bool carried = false;
-    if (real) {
+    {
         using C = Code<KX>;
-        const int c = S.ncnt[s];
-        const int m = min(c, A.cap);
+        const int m = min(listed, A.cap);
         auto candidate = [&](int k) {
             uint64_t key = none;
             if (k < m) {
@@ -809,7 +835,7 @@ __global__ void __launch_bounds__(256, 6) k_features_warp(const __grid_constant_
             if (k0 == 0) best = c0;
             else merge(c0);
         }
-        if (c > A.cap) {
+        if (listed > A.cap) {
             // the rest, in the order of the list build, every lane alike
             int skip = A.cap;
             for_neighbours<KX, false>(A.g, S, d, A.d.x, A.d.y, A.d.z,
@@ -833,12 +859,12 @@ __global__ void __launch_bounds__(256, 6) k_features_warp(const __grid_constant_
         }
     }
     const bool have = best != none;
-    float raw[NC] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    float rx = crx, ry = cry;
     // (loaded here, beside the neighbour's records, not live through the sort)
     const float4 vi = A.d.velh[s];
+    float4 vj = make_float4(0.f, 0.f, 0.f, 0.f), st = vj;
     if (have) {
         const int j = (int)(uint32_t)best;
-        float rx = crx, ry = cry;
         if (!carried) {
             // the list pass's offsets: cell offset from the source's cell
             int cxj, cyj, czj;
@@ -847,33 +873,130 @@ __global__ void __launch_bounds__(256, 6) k_features_warp(const __grid_constant_
             rx = fmaf((float)(d.cx - cxj), csf, d.xi_x - p.x);
             ry = fmaf((float)(d.cy - cyj), csf, d.xi_y - p.y);
         }
-        const float ih = 1.f / vi.w;
-        const float4 vj = S.velh[j];
-        const float4 st = S.st[j];
-        raw[0] = rx * ih;
-        raw[1] = ry * ih;
-        raw[2] = (vj.x - vi.x) * A.inv_c0;
-        raw[3] = (vj.y - vi.y) * A.inv_c0;
-        raw[4] = st.x;
-        raw[5] = st.y * st.x * st.x;
+        vj = S.velh[j];
+        st = S.st[j];
     }
-    float f[NC];
-#pragma unroll
-    for (int q = 0; q < NC; ++q) f[q] = have ? (raw[q] - A.mean[q]) * A.inv_std[q] : 0.f;
-    const int64_t row = (int64_t)d.orig * (NN * NC) + lane * NC;
+    const FeatRow row(A, have, rx, ry, vi.x, vi.y, 1.f / vi.w, vj, st);
+    const int64_t at = (int64_t)d.orig * (NN * NC) + lane * NC;
     if (A.out_bf) {
-        uint32_t *o = reinterpret_cast<uint32_t *>(A.out_bf + row);
+        uint32_t *o = reinterpret_cast<uint32_t *>(A.out_bf + at);
 #pragma unroll
-        for (int i = 0; i < NC / 2; ++i) {
-            __nv_bfloat162 h = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
-            o[i] = *reinterpret_cast<uint32_t *>(&h);
+        for (int i = 0; i < NC / 2; ++i) o[i] = row.pair(i);
+    }
+    if (A.out_f) row.store_f(A.out_f + at);
+}
+
+// Up to kFeatDests destinations per warp: lane i reads and decodes
+// destination i (once, not in every lane), then the warp takes them one after
+// the other, the next one's list entries on their way meanwhile.  Bound by
+// issue and by the latency of the dependent gathers: 60 us at 80 000
+// destinations in 2D with every list sorted and every lane decoding, 33 so.
+// As many per warp as fill the chip, so that a small simulation's chain stays
+// short.  With 1 / 2 / 4 / 8: 10 200 destinations 11.3 / 8.4 / 9.1 / 12.1 us,
+// 20 000 16.7 / 14.0 / 12.5 / 15.0, 41 000 28 / 22 / 19 / 21, 80 000 52 / 40 /
+// 34 / 33.
+constexpr int kFeatDests = 8;
+constexpr int64_t kFeatWarps = 152 * 40;     // resident on the chip
+
+template <int KX>
+__global__ void __launch_bounds__(256, 5) k_features_warp(const __grid_constant__ FeatureArgs A) {
+    constexpr int NN = SPH_MLP_NNBR, NC = SPH_MLP_NCH;
+    struct Dest {
+        float4 pos;         // offset in the cell, r2lo
+        float4 vel;         // u, v, 1 / h, r2hi
+        double radius2;
+        int orig, listed;
+    };
+    __shared__ Dest s_dest[8][kFeatDests];
+    __shared__ uint4 s_key[8][8];
+    __shared__ uint4 s_row[8][NN * NC / 8];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int64_t s0 = (blockIdx.x * (int64_t)8 + wid) * A.per;
+    if (s0 >= A.d.n || gated_off(A.gate)) return;
+    const SrcDev &S = A.s;
+    const float csf = A.g.cs_f;
+    const int nd = (int)min((int64_t)A.per, A.d.n - s0);
+    const int limit = min(32, A.cap);
+    if (lane < nd) {
+        DestPos d;
+        Dest t;
+        const int s = (int)s0 + lane;
+        const bool real = load_dest(A.g, A.d, s, d);
+        const float4 v = A.d.velh[s];
+        t.pos = real ? make_float4(d.xi_x, d.xi_y, d.xi_z, d.r2lo) : make_float4(0.f, 0.f, 0.f, 0.f);
+        t.vel = make_float4(v.x, v.y, 1.f / v.w, real ? d.r2hi : 0.f);
+        t.radius2 = real ? d.radius2 : 0.0;
+        t.orig = d.orig;
+        t.listed = real ? S.ncnt[s] : 0;
+        s_dest[wid][lane] = t;
+    }
+    __syncwarp();
+    uint4 *keys = s_key[wid];
+    uint32_t *row = reinterpret_cast<uint32_t *>(s_row[wid]);
+    const uint32_t *lst = S.nbr + s0 + (int64_t)lane * A.stride;
+    uint32_t e = lane < min(s_dest[wid][0].listed, limit) ? lst[0] : 0u;
+    unsigned longer = 0;
+#pragma unroll 1
+    for (int i = 0; i < nd; ++i) {
+        const Dest &t = s_dest[wid][i];
+        const int listed = t.listed;
+        const uint32_t ec = e;
+        if (i + 1 < nd && lane < min(s_dest[wid][i + 1].listed, limit)) e = lst[i + 1];
+        if (listed > limit) {
+            longer |= 1u << i;
+            continue;
         }
-    }
-    if (A.out_f) {
-        float2 *o = reinterpret_cast<float2 *>(A.out_f + row);
+        const float4 pos = t.pos, vel = t.vel;
+        float4 vj = make_float4(0.f, 0.f, 0.f, 0.f), st = vj;
+        float rx = 0.f, ry = 0.f;
+        // (past the entries: above every squared distance, NaN too)
+        uint32_t key = 0x80000000u | lane;
+        bool have = false;
+        if (lane < listed) {
+            const int j = (int)(ec & Code<KX>::JMASK);
+            const float3 sh = neg_cell_offset<KX>(ec);
+            const float4 p = S.pm[j];
+            vj = S.velh[j];
+            st = S.st[j];
+            rx = fmaf(sh.x, csf, pos.x - p.x);
+            ry = fmaf(sh.y, csf, pos.y - p.y);
+            const float rz = fmaf(sh.z, csf, pos.z - p.z);
+            const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
+            // (listed_exact_test)
+            have = A.g.skin <= 0.f || r2 < pos.w;
+            if (!have && r2 <= vel.w) {
+                const int oj = S.perm[j];
+                have = exact_within(ld0(S.x, oj), ld0(S.y, oj), ld0(S.z, oj), ld0(A.d.x, t.orig),
+                                    ld0(A.d.y, t.orig), ld0(A.d.z, t.orig), t.radius2);
+            }
+            if (have) key = __float_as_uint(r2);
+        }
+        reinterpret_cast<uint32_t *>(keys)[lane] = key;
+        __syncwarp();
+        // rank: smaller keys, and equal ones of earlier entries
+        int rank = lane;
+        if (lane < listed) {
+            const uint4 own = keys[lane >> 2];
+            rank = ((lane & 3) > 0 && own.x == key) + ((lane & 3) > 1 && own.y == key) +
+                   ((lane & 3) > 2 && own.z == key);
+            for (int k = 0; 4 * k < listed; ++k) {
+                const uint4 o = keys[k];
+                const uint32_t lim = key + (k < (lane >> 2) ? 1u : 0u);
+                rank += (o.x < lim) + (o.y < lim) + (o.z < lim) + (o.w < lim);
+            }
+        }
+        const FeatRow r(A, have, rx, ry, vel.x, vel.y, vel.z, vj, st);
+        const int64_t at = (int64_t)t.orig * (NN * NC);
+        if (A.out_f) r.store_f(A.out_f + at + rank * NC);
+        if (A.out_bf) {
 #pragma unroll
-        for (int i = 0; i < NC / 2; ++i) o[i] = make_float2(f[2 * i], f[2 * i + 1]);
+            for (int q = 0; q < NC / 2; ++q) row[rank * (NC / 2) + q] = r.pair(q);
+        }
+        __syncwarp();
+        if (A.out_bf && lane < NN * NC / 8)
+            reinterpret_cast<uint4 *>(A.out_bf + at)[lane] = s_row[wid][lane];
     }
+    for (; longer; longer &= longer - 1) features_sorted<KX>(A, s0 + (__ffs(longer) - 1));
 }
 
 DestDev make_dest(const ArraySnap &D) {
@@ -1390,7 +1513,8 @@ int features_pass(sph_ctx *ctx, int dst, int src, const sph_mlp_feature_params *
     // every call: one thread per destination)
     const char *env_thread = getenv("SPH_FEATURES_THREAD");
     const bool per_thread = env_thread && atoi(env_thread) > 0;
-    const int bw = (int)((D.n * 32 + 255) / 256);
+    a.per = (int)std::min<int64_t>(kFeatDests, 1 + D.n / kFeatWarps);
+    const int bw = (int)((D.n + 8 * a.per - 1) / (8 * a.per));
 #define FLAUNCH(K) (ext ? k_features<K, true><<<b, kPairBlock, 0, ctx->stream>>>(a) \
                     : per_thread ? k_features<K, false><<<b, kPairBlock, 0, ctx->stream>>>(a) \
                                  : k_features_warp<K><<<bw, 256, 0, ctx->stream>>>(a))

@@ -257,6 +257,32 @@ def test_feature_kernels_agree(monkeypatch):
     assert float((out["0"][0] != 0).any(dim=1).float().mean()) > 0.5
 
 
+@pytest.mark.parametrize("hfac", [0.4, 0.9, 1.3, 1.5, 1.62, 2.2])
+@pytest.mark.parametrize("jitter,side", [(0.0, 24), (0.2, 24), (0.2, 111), (0.0, 231)])
+def test_feature_rows_over_list_lengths(hfac, jitter, side, monkeypatch):
+    """Lists of the particle alone, of up to 32 entries (ranked), of both
+    kinds and longer ones (sorted), on a lattice (equal distances, ordered
+    by slot) and a jittered one, with one, three and eight destinations per
+    warp: the rows of one thread per destination."""
+    _need_gpu()
+    dx = 0.05
+    g = dx * np.arange(side)
+    x, y = (c.ravel() for c in np.meshgrid(g, g[:-1]))
+    rng = np.random.default_rng(11)
+    n = x.size
+    props = {"x": x + jitter * dx * rng.uniform(-1, 1, n), "y": y + jitter * dx * rng.uniform(-1, 1, n),
+             "h": np.full(n, hfac * dx), "m": np.full(n, dx * dx), "rho": np.ones(n),
+             "p": rng.uniform(0, 1, n), "cs": np.full(n, 100.0),
+             "u": rng.normal(0, 1, n), "v": rng.normal(0, 1, n)}
+    pa = API.base.get_particle_array(name="fluid", type=API.base.ParticleType.Fluid, **props)
+    cm = API.base.Particles(arrays=[pa]).cell_manager
+    rows = {}
+    for thread in ("1", "0"):
+        monkeypatch.setenv("SPH_FEATURES_THREAD", thread)
+        rows[thread] = L.features(cm, pa, L.Normalisation(100.0), raw=True).clone()
+    assert torch.equal(rows["1"], rows["0"])
+
+
 _FEAT_OVERFULL = r"""
 import sys
 sys.path.insert(0, ".")
