@@ -51,7 +51,14 @@ __global__ void k_box(sph_array_view a, double inv_cs, double inv_cs_ref, int *r
     const float inv_f = (float)inv_cs, inv_ref_f = (float)inv_cs_ref;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.n;
          i += (int64_t)gridDim.x * blockDim.x) {
+        // (every load before the first cell, whose FP64 case is a call)
         double p[3] = {ld0(a.x, i), ld0(a.y, i), ld0(a.z, i)};
+        const long long hb = __double_as_longlong(a.h[i]);
+        int was[3] = {0, 0, 0};
+        if (check_jump && refcell) {
+#pragma unroll
+            for (int d = 0; d < 3; ++d) was[d] = refcell[3 * i + d];
+        }
         const double pb[3] = {bin_x(pg, p[0]), p[1], p[2]};
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
@@ -59,7 +66,6 @@ __global__ void k_box(sph_array_view a, double inv_cs, double inv_cs_ref, int *r
             mn[d] = min(mn[d], c);
             mx[d] = max(mx[d], c);
         }
-        const long long hb = __double_as_longlong(a.h[i]);
         if ((hb & 0x7fffffffffffffffll) <= 0x7ff0000000000000ll) {
             hm = max(hm, hb);
             hn = min(hn, hb);
@@ -68,7 +74,7 @@ __global__ void k_box(sph_array_view a, double inv_cs, double inv_cs_ref, int *r
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
                 int c = floor_cell_screened(p[d], inv_cs_ref, inv_ref_f);
-                if (check_jump && abs(c - refcell[3 * i + d]) > 1) jump = true;
+                if (check_jump && abs(c - was[d]) > 1) jump = true;
                 refcell[3 * i + d] = c;
             }
         }

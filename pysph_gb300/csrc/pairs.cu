@@ -181,7 +181,8 @@ struct NoExtra {
 template <int KX, int B, bool EXT, int S_ = 1, class Extra, class Fn, class Done>
 __device__ __forceinline__ void for_listed(const Grid &g, const SrcDev &S, int cap, int64_t stride,
                                            int s, const DestPos &d, const DestDev &D, bool filter,
-                                           Extra &&extra, Fn &&fn, Done &&done) {
+                                           Extra &&extra, Fn &&fn, Done &&done,
+                                           unsigned mask = 0xffffffffu) {
     filter = filter && g.skin > 0.f;
     using C = Code<KX>;
     using X = decltype(extra(0));
@@ -197,7 +198,8 @@ __device__ __forceinline__ void for_listed(const Grid &g, const SrcDev &S, int c
     const int k0 = S_ > 1 ? (int)(threadIdx.x % S_) * B : 0;
     if (k0 < m) entries(e, k0);
     const float csf = g.cs_f;
-    for (int r = 0, k = k0; r < m; r += S_ * B, k += S_ * B) {
+    const int mw = S_ > 1 ? __reduce_max_sync(mask, m) : m;
+    for (int r = 0, k = k0; r < mw; r += S_ * B, k += S_ * B) {
         uint32_t en[B];
         const bool more = k + S_ * B < m;
         if (more) entries(en, k + S_ * B);
@@ -244,11 +246,14 @@ __device__ __forceinline__ void for_listed(const Grid &g, const SrcDev &S, int c
 }
 
 // ---------------------------------------------------------------------------
-// lanes: in small simulations S = 2 or 8 neighbouring threads share a
-// destination of the rates pass (a thread per destination leaves most of the
-// GPU idle there, each thread a serial chain over all its neighbours).  Sums
-// stay the same bit for bit: the batches are those of the list, folded in its
-// order.
+// lanes: in small simulations several neighbouring threads share a
+// destination of the rates pass and of the list build (a thread per
+// destination leaves most of the GPU idle there, each thread a serial chain
+// over all its neighbours).  Sums stay the same bit for bit: the terms, or
+// batches of the list, are folded in its order.  The lanes of a warp run every
+// loop to its longest trip count under one mask: with a mask per destination
+// the warp ran each destination's shuffles by themselves (density of 31 400
+// variable-h particles with four lanes 54 us against 42).
 // ---------------------------------------------------------------------------
 template <int S>
 __device__ __forceinline__ unsigned lane_mask() {
@@ -257,8 +262,7 @@ __device__ __forceinline__ unsigned lane_mask() {
 
 // v[S q + t] of lane l becomes v[S q + l] of lane t (transposes over the lanes)
 template <int S>
-__device__ __forceinline__ void lane_transpose(float (&v)[8]) {
-    const unsigned mask = lane_mask<S>();
+__device__ __forceinline__ void lane_transpose(unsigned mask, float (&v)[8]) {
     const int lane = threadIdx.x % S;
 #pragma unroll
     for (int b = 1; b < S; b <<= 1) {
@@ -277,24 +281,44 @@ __device__ __forceinline__ void lane_transpose(float (&v)[8]) {
 // ---------------------------------------------------------------------------
 // neighbour list (base/nnps.pyx:525-620 FixedDestNbrParticleLocator cache)
 // ---------------------------------------------------------------------------
-template <int KX, int MODE>
+// Place of the next hit of this lane among the lanes' hits, in order (c: the
+// hits so far, the same on the lanes of a destination).
+template <int S_>
+__device__ __forceinline__ int lane_place(unsigned mask, bool hit, int &c) {
+    const unsigned hits = __ballot_sync(mask, hit) & lane_mask<S_>();
+    const int at = c + __popc(hits & ((1u << (threadIdx.x & 31)) - 1u));
+    c += __popc(hits);
+    return at;
+}
+
+template <int KX, int MODE, int S_ = 1>
 __global__ void __launch_bounds__(kPairBlock) k_nbrlist(const __grid_constant__ ListArgs A) {
     using C = Code<KX>;
     if (gated_off(A.gate)) return;
-    const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t s = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / S_;
     int c = 0;
-    if (s < A.d.n) {
-        const Grid &g = grid_of<MODE == 1>(A.g, A.d, (int)s);
-        DestPos d;
-        if (load_dest(g, A.d, (int)s, d)) {
+    const bool in = s < A.d.n;
+    const Grid &g = grid_of<MODE == 1>(A.g, A.d, (int)s);
+    DestPos d;
+    const bool real = in && load_dest(g, A.d, (int)s, d);
+    const unsigned mask = __ballot_sync(0xffffffffu, real);
+    if (in) {
+        if (real) {
             uint32_t *out = A.nbr + s;
             const int cap = A.cap;
             const int64_t stride = A.stride;
-            for_neighbours<KX, MODE == 2>(g, A.s, d, A.d.x, A.d.y, A.d.z,
-                               [&](int j, float, float, float, int code, bool) {
-                                   if (c < cap) out[(int64_t)c * stride] = (uint32_t)j | ((uint32_t)code << C::SHIFT);
-                                   ++c;
-                               });
+            auto put = [&](int at, int j, int code) {
+                if (at < cap) out[(int64_t)at * stride] = (uint32_t)j | ((uint32_t)code << C::SHIFT);
+            };
+            if constexpr (S_ > 1)
+                for_neighbours<KX, MODE == 2, S_>(g, A.s, d, A.d.x, A.d.y, A.d.z,
+                    [&](bool listed, int j, float, float, float, int code, bool) {
+                        const int at = lane_place<S_>(mask, listed, c);
+                        if (listed) put(at, j, code);
+                    }, mask);
+            else
+                for_neighbours<KX, MODE == 2>(g, A.s, d, A.d.x, A.d.y, A.d.z,
+                    [&](int j, float, float, float, int code, bool) { put(c++, j, code); });
         }
         A.cnt[s] = c;
     }
@@ -308,13 +332,17 @@ __global__ void __launch_bounds__(kPairBlock) k_nbrlist(const __grid_constant__ 
 // MODE 0: one simulation; 1: a batch of simulations (per-instance grids);
 // 2: one simulation with the extended search (periodic x or variable-h
 // symmetric lists), kept apart so the other modes carry none of its state.
-template <int KX, bool UH, int MODE>
-__global__ void __launch_bounds__(kPairBlock, (UH && MODE != 2) ? 8 : 1) k_density(const __grid_constant__ DensityArgs A) {
-    const int64_t s = (MODE == 1 ? A.d.s0 : 0) + blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (s >= A.d.n || gated_off(A.gate)) return;
+// S_: lanes per destination, where every source's list is built by the pass.
+template <int KX, bool UH, int MODE, int S_ = 1>
+__global__ void __launch_bounds__(kPairBlock, (UH && MODE != 2 && S_ == 1) ? 8 : 1) k_density(const __grid_constant__ DensityArgs A) {
+    const int64_t s = (MODE == 1 ? A.d.s0 : 0) + (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / S_;
+    if ((S_ == 1 && s >= A.d.n) || gated_off(A.gate)) return;
+    const bool in = S_ == 1 || s < A.d.n;
     const Grid &g = grid_of<MODE == 1>(A.g, A.d, (int)s);
     DestPos d;
-    const bool real = load_dest(g, A.d, (int)s, d);
+    const bool real = in && load_dest(g, A.d, (int)s, d);
+    const unsigned mask = S_ > 1 ? __ballot_sync(0xffffffffu, real) : 0xffffffffu;
+    if (!in) return;
     CSum rho;
     if (!real) {
         for (int si = 0; si < A.nsrc; ++si)
@@ -339,21 +367,39 @@ __global__ void __launch_bounds__(kPairBlock, (UH && MODE != 2) ? 8 : 1) k_densi
                 const int cap = A.cap[si];
                 const int64_t stride = A.stride[si];
                 int c = 0;
-                for_neighbours<KX, MODE == 2>(g, S, d, A.d.x, A.d.y, A.d.z,
-                    [&](int j, float rx, float ry, float rz, int code, bool exact) {
-                        if (c < cap) out[(int64_t)c * stride] = (uint32_t)j | ((uint32_t)code << C::SHIFT);
-                        ++c;
-                        if (!exact) return;
-                        const float mj = S.pm[j].w;
-                        float ih = ihi, fac = faci;
-                        if (!uh && !fixed) {
-                            ih = __fdividef(1.f, 0.5f * (hi + S.velh[j].w));
-                            fac = cubic_fac(dim, ih);
-                        }
-                        const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
-                        const float r = r2 > 0.f ? r2 * rsqrtf(r2) : 0.f;
-                        rho.add(cubic_w(r * ih) * fac * mj);
-                    });
+                auto put = [&](int at, int j, int code) {
+                    if (at < cap) out[(int64_t)at * stride] = (uint32_t)j | ((uint32_t)code << C::SHIFT);
+                };
+                auto term = [&](int j, float rx, float ry, float rz) {
+                    const float mj = S.pm[j].w;
+                    float ih = ihi, fac = faci;
+                    if (!uh && !fixed) {
+                        ih = __fdividef(1.f, 0.5f * (hi + S.velh[j].w));
+                        fac = cubic_fac(dim, ih);
+                    }
+                    const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
+                    const float r = r2 > 0.f ? r2 * rsqrtf(r2) : 0.f;
+                    return cubic_w(r * ih) * fac * mj;
+                };
+                if constexpr (S_ > 1) {
+                    for_neighbours<KX, MODE == 2, S_>(g, S, d, A.d.x, A.d.y, A.d.z,
+                        [&](bool listed, int j, float rx, float ry, float rz, int code, bool exact) {
+                            const int at = lane_place<S_>(mask, listed, c);
+                            if (listed) put(at, j, code);
+                            // the lanes' terms, folded in order by each (adding
+                            // the 0 of a source that is none changes nothing)
+                            float w = 0.f;
+                            if (exact) w = term(j, rx, ry, rz);
+#pragma unroll
+                            for (int t = 0; t < S_; ++t) rho.add(__shfl_sync(mask, w, t, S_));
+                        }, mask);
+                } else {
+                    for_neighbours<KX, MODE == 2>(g, S, d, A.d.x, A.d.y, A.d.z,
+                        [&](int j, float rx, float ry, float rz, int code, bool exact) {
+                            put(c++, j, code);
+                            if (exact) rho.add(term(j, rx, ry, rz));
+                        });
+                }
                 A.lcnt[si][s] = c;
                 const unsigned act = __activemask();
                 const int wmax = __reduce_max_sync(act, c);
@@ -361,6 +407,7 @@ __global__ void __launch_bounds__(kPairBlock, (UH && MODE != 2) ? 8 : 1) k_densi
                 continue;
             }
             // with variable h (or a fixed h), W can reach past the radius of h_i
+            if constexpr (S_ == 1)
             for_listed<KX, (UH && MODE == 0) ? 6 : 4, MODE == 2>(g, S, A.cap[si], A.stride[si], (int)s, d, A.d, !uh, NoExtra(),
                 [&](bool ok, int j, float rx, float ry, float rz, float mj, int) {
                     float ih = ihi, fac = faci;
@@ -379,6 +426,7 @@ __global__ void __launch_bounds__(kPairBlock, (UH && MODE != 2) ? 8 : 1) k_densi
                 });
         }
     }
+    if (S_ > 1 && threadIdx.x % S_ != 0) return;
     const int orig = d.orig;
     const double r64 = real ? rho.value() : 0.0;
     if (A.rho_out) A.rho_out[orig] = r64;
@@ -430,10 +478,15 @@ __global__ void __launch_bounds__(kPairBlock) k_rates(const __grid_constant__ Ra
     constexpr bool MAY_BF = SPEC == 0;
     constexpr bool MAY_DRHO = SPEC == 0;
     const int64_t s = (MODE == 1 ? A.d.s0 : 0) + (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / S_;
-    if (s >= A.d.n || gated_off(A.gate)) return;
+    if ((S_ == 1 && s >= A.d.n) || gated_off(A.gate)) return;
+    const bool in = S_ == 1 || s < A.d.n;
     const Grid &g = grid_of<MODE == 1>(A.g, A.d, (int)s);
     DestPos d;
-    const bool real = load_dest(g, A.d, (int)s, d);
+    const bool real = in && load_dest(g, A.d, (int)s, d);
+    // the lanes that shuffle: one mask for the warp (a mask per destination
+    // makes it run each destination's shuffles by themselves)
+    const unsigned mask = S_ > 1 ? __ballot_sync(0xffffffffu, real) : 0xffffffffu;
+    if (!in) return;
     CSum ax, ay, az, xx, xy, xz, dr;
     // lanes: lane l keeps the sums l, l + S, ... of (ax, ay, az, dr, xx, xy, xz)
     CSum mine[S_ > 1 ? 8 / S_ : 1];
@@ -531,7 +584,7 @@ __global__ void __launch_bounds__(kPairBlock) k_rates(const __grid_constant__ Ra
                 if constexpr (S_ > 1) {
                     float v[8] = {pax, pay, paz, pdr, pxx, pxy, pxz, 0.f};
                     if (round) {
-                        lane_transpose<S_>(v);
+                        lane_transpose<S_>(mask, v);
 #pragma unroll
                         for (int q = 0; q < 8 / S_; ++q)
 #pragma unroll
@@ -559,7 +612,7 @@ __global__ void __launch_bounds__(kPairBlock) k_rates(const __grid_constant__ Ra
                     xx.add(pxx); xy.add(pxy); xz.add(pxz);
                     pxx = pxy = pxz = 0.f;
                 }
-            });
+            }, mask);
         }
     }
     const int orig = d.orig;
@@ -1028,22 +1081,34 @@ int blocks_for(int64_t n) {
     return (int)std::max<int64_t>(1, (n + kPairBlock - 1) / kPairBlock);
 }
 
-// Threads that share a destination of the rates pass.  Measured (us per pass
-// with 1 / 2 / 4 / 8): variable-h drop of 5 025 particles 44 / 27 / 18 / 14,
-// 31 400 46 / 29 / 34 / 46, 100 000 91 / 80 / 93 / 122; fluid-solver patch
-// of 5 025 52 / 31 / 20 / 15, 20 106 52 / 32 / 36 / 37, 87 000 103 / 92 / 91 /
-// 116; dam break of 5 000 34 / 24 / 16 / 14, 20 000 33 / 22 / 25 / 29, 80 000
-// 54 / 50 / 54 / 79.
-int pair_lanes(int64_t n) {
-    // environment SPH_PAIR_LANES = 1, 2, 8: forced, to measure and test
+// Threads that share a destination of a list build or a list-streaming rates
+// pass of n destinations: as many of 8 and 4 as run in one wave (blocks: the
+// resident blocks per SM), else two while the pass is short, where a chain of
+// half the length still counts more than the instructions that are added.
+// Measured (us per pass with 1 / 2 / 4 / 8):
+//   rates (4 blocks), variable h: 5 025 particles 44 / 26 / 17 / 13, 16 000
+//   44 / 27 / 18 / 25, 31 400 45 / 28 / 33 / 45, 100 000 89 / 76 / 89 / 119,
+//   196 000 135 / 143 / 160 / 221; fluid-solver patch of 20 106 52 / 31 / 34 /
+//   38, 87 000 107 / 86 / 87 / 116;
+//   density with the lists (4 blocks), variable h: 5 025 51 / 33 / 22 / 16,
+//   16 000 52 / 34 / 24 / 31, 31 400 54 / 35 / 42 / 54, 100 000 94 / 92 / 113 /
+//   146, 196 000 142 / 172 / 205 / 274;
+//   lists alone (8 blocks), patch: 20 106 31 / 23 / 15 / 13, 87 000 35 / 31 /
+//   34 / 43, 196 000 64 / 64 / 68 / 87.
+int pair_lanes(int64_t n, int blocks) {
+    // environment SPH_PAIR_LANES = 1, 2, 4, 8: forced, to measure and test
     static int force = -1;
     if (force < 0) {
         const char *e = getenv("SPH_PAIR_LANES");
         const int v = e ? atoi(e) : 0;
-        force = (v == 1 || v == 2 || v == 8) ? v : 0;
+        force = (v == 1 || v == 2 || v == 4 || v == 8) ? v : 0;
     }
-    return force ? force : (n < 10000 ? 8 : (n < 120000 ? 2 : 1));
+    if (force) return force;
+    const int64_t wave = 152ll * blocks * kPairBlock;
+    return n * 8 <= wave ? 8 : (n * 4 <= wave ? 4 : (n < 120000 ? 2 : 1));
 }
+constexpr int kPairResident = 4;    // blocks of up to 128 registers a thread
+constexpr int kListResident = 8;    // blocks of up to 64
 
 // List capacity override (environment SPH_LIST_CAP, >= 1): forces the
 // re-traversal path of destinations with more neighbours than the capacity.
@@ -1164,17 +1229,22 @@ int ensure_list(sph_ctx *ctx, int dst, int src, NbrList **out) {
         a.stride = L.stride;
         a.cap = L.cap;
         a.gate = ctx->gate;
-        const int b = blocks_for(D.n);
+        // (base-5 codes are for the largest sets)
+        const int v = code_variant(ctx);
+        const int lanes = v == 4 ? 1 : pair_lanes(D.n, kListResident);
+        const int b = blocks_for(D.n * lanes);
         const bool ext = g.periodic || g.symmetric;
-#define LLAUNCH(K) (ext ? k_nbrlist<K, 2><<<b, kPairBlock, 0, ctx->stream>>>(a) \
-                        : k_nbrlist<K, 0><<<b, kPairBlock, 0, ctx->stream>>>(a))
-        switch (code_variant(ctx)) {
+#define LLAUNCH1(K, L) (ext ? k_nbrlist<K, 2, L><<<b, kPairBlock, 0, ctx->stream>>>(a) \
+                            : k_nbrlist<K, 0, L><<<b, kPairBlock, 0, ctx->stream>>>(a))
+#define LLAUNCH(K) (lanes == 1 ? LLAUNCH1(K, 1) : lanes == 2 ? LLAUNCH1(K, 2) : lanes == 4 ? LLAUNCH1(K, 4) : LLAUNCH1(K, 8))
+        switch (v) {
             case 1: LLAUNCH(1); break;
             case 2: LLAUNCH(2); break;
-            case 4: LLAUNCH(4); break;
+            case 4: LLAUNCH1(4, 1); break;
             default: LLAUNCH(3); break;
         }
 #undef LLAUNCH
+#undef LLAUNCH1
         count_launch();
         SPH_LAUNCH_CHECK("k_nbrlist");
     }
@@ -1324,21 +1394,27 @@ int density_pass(sph_ctx *ctx, int dst, const int *srcs, int nsrc, const sph_den
     if (prm->h0 < 0.0) return set_error(SPH_ERR_ARG, "density: h0 must be >= 0");
     a.ih0 = prm->h0 > 0.0 ? (float)(1.0 / prm->h0) : 0.f;
     if (D.n == 0) return SPH_OK;
-    const int b = blocks_for(D.n);
+    bool building = true;
+    for (int i = 0; i < nsrc; ++i) building = building && a.lnbr[i] != nullptr;
+    const int v = code_variant(ctx);
+    const int lanes = building && v != 4 ? pair_lanes(D.n, kPairResident) : 1;
+    const int b = blocks_for(D.n * lanes);
     // a fixed h (pilot density) runs in the variable-h kernels
     const bool uh = a.g.uniform_h != 0 && a.ih0 == 0.f;
     const bool ext = a.g.periodic || a.g.symmetric;
-#define DLAUNCH(K) (ext ? (uh ? k_density<K, true, 2><<<b, kPairBlock, 0, ctx->stream>>>(a) \
-                              : k_density<K, false, 2><<<b, kPairBlock, 0, ctx->stream>>>(a)) \
-                        : (uh ? k_density<K, true, 0><<<b, kPairBlock, 0, ctx->stream>>>(a) \
-                              : k_density<K, false, 0><<<b, kPairBlock, 0, ctx->stream>>>(a)))
-    switch (code_variant(ctx)) {
+#define DLAUNCH2(K, U, L) (ext ? k_density<K, U, 2, L><<<b, kPairBlock, 0, ctx->stream>>>(a) \
+                               : k_density<K, U, 0, L><<<b, kPairBlock, 0, ctx->stream>>>(a))
+#define DLAUNCH1(K, L) (uh ? DLAUNCH2(K, true, L) : DLAUNCH2(K, false, L))
+#define DLAUNCH(K) (lanes == 1 ? DLAUNCH1(K, 1) : lanes == 2 ? DLAUNCH1(K, 2) : lanes == 4 ? DLAUNCH1(K, 4) : DLAUNCH1(K, 8))
+    switch (v) {
         case 1: DLAUNCH(1); break;
         case 2: DLAUNCH(2); break;
-        case 4: DLAUNCH(4); break;
+        case 4: DLAUNCH1(4, 1); break;
         default: DLAUNCH(3); break;
     }
 #undef DLAUNCH
+#undef DLAUNCH1
+#undef DLAUNCH2
     count_launch();
     SPH_LAUNCH_CHECK("k_density");
     if (a.st_out) {
@@ -1447,14 +1523,14 @@ int rates_pass(sph_ctx *ctx, int dst, const sph_source_term *terms, int nterms,
     // the specialised kernels keep a thread per destination (one source of
     // uniform h runs in the brick passes)
     const int v = code_variant(ctx);
-    const int lanes = v == 4 || spec == 1 || spec == 2 ? 1 : pair_lanes(D.n);
+    const int lanes = v == 4 || spec == 1 || spec == 2 ? 1 : pair_lanes(D.n, kPairResident);
     const int b = blocks_for(D.n * lanes);
 #define RLAUNCH1(K, L) (spec == 3 ? k_rates<K, 0, 2, L><<<b, kPairBlock, 0, ctx->stream>>>(a) \
                                   : k_rates<K, 0, 0, L><<<b, kPairBlock, 0, ctx->stream>>>(a))
 #define RLAUNCH(K) (spec == 1 ? k_rates<K, 1, 0><<<b, kPairBlock, 0, ctx->stream>>>(a) \
                     : spec == 2 ? k_rates<K, 2, 0><<<b, kPairBlock, 0, ctx->stream>>>(a) \
                                 : RLAUNCH1(K, 1))
-#define RLAUNCH8(K) (lanes == 8 ? RLAUNCH1(K, 8) : RLAUNCH1(K, 2))
+#define RLAUNCH8(K) (lanes == 8 ? RLAUNCH1(K, 8) : lanes == 4 ? RLAUNCH1(K, 4) : RLAUNCH1(K, 2))
     if (lanes > 1) {
         if (v == 1) RLAUNCH8(1);
         else if (v == 2) RLAUNCH8(2);

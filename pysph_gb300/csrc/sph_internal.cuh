@@ -702,10 +702,15 @@ struct DestPos {
 // (d.r2list > 0) the sources within the list radius that are not neighbours
 // are visited too, with exact = false.  scx[j] holds the source's
 // dense-grid x cell.
-template <int KX, bool EXT, class Fn>
+// With S_ > 1 the S_ lanes of a destination (consecutive, all with its d) take
+// consecutive sources of a row, and fn(listed, j, rx, ry, rz, code, exact) is
+// called for each step by all lanes of mask (the warp's lanes that came here):
+// every loop has the warp's longest trip count, so that they stay together.
+template <int KX, bool EXT, int S_ = 1, class Fn>
 __device__ __forceinline__ void for_neighbours(const Grid &g, const SrcDev &S, const DestPos &d,
                                                const double *dx64, const double *dy64,
-                                               const double *dz64, Fn &&fn) {
+                                               const double *dz64, Fn &&fn,
+                                               unsigned mask = 0xffffffffu) {
     constexpr int K = stencil_k<KX>();
     const float csf = g.cs_f;
     const float inv_cs = 1.f / csf;
@@ -719,14 +724,15 @@ __device__ __forceinline__ void for_neighbours(const Grid &g, const SrcDev &S, c
         const float ez = fmaxf(0.f, dz > 0 ? (float)dz * csf - d.xi_z
                                            : (dz < 0 ? d.xi_z - (float)(dz + 1) * csf : 0.f));
         const float ez2 = ez * ez;
-        if (ez2 > R2) continue;
+        if (S_ == 1 && ez2 > R2) continue;
         const int zbase = (d.cz + dz) * rowstride_z + d.cx;
         const float bz = d.xi_z - (float)dz * csf;
         for (int dy = -g.ky; dy <= g.ky; ++dy) {
             const float ey = fmaxf(0.f, dy > 0 ? (float)dy * csf - d.xi_y
                                                : (dy < 0 ? d.xi_y - (float)(dy + 1) * csf : 0.f));
             const float rem = R2 - fmaf(ey, ey, ez2);
-            if (rem < 0.f) continue;
+            if (S_ == 1 && rem < 0.f) continue;
+            const bool row = rem >= 0.f;
             // chord half-width with a relative margin (covers the rsqrt error)
             const float half = fmaf(rem * rsqrtf(fmaxf(rem, 1e-30f)), 1.0001f, 1e-5f * csf);
             const int tlo = max(-K, __float2int_rd((d.xi_x - half) * inv_cs));
@@ -738,40 +744,48 @@ __device__ __forceinline__ void for_neighbours(const Grid &g, const SrcDev &S, c
             // range, or on a periodic axis up to three -- the cells past the
             // low / high end wrap to the other end, where the sources' cell
             // index is nx more / less than the unwrapped one (wrap -1 / +1)
-            auto visit = [&](int rlo, int rhi, int wrap) {
-            const int lo = __ldg(cst + c0 + rlo);
-            const int hi = __ldg(cst + c0 + rhi + 1);
+            auto visit = [&](bool some, int rlo, int rhi, int wrap) {
+            const int lo = some ? __ldg(cst + c0 + rlo) : 0;
+            const int hi = some ? __ldg(cst + c0 + rhi + 1) : 0;
             const float wshift = (float)(wrap * g.nx);
-            for (int j = lo; j < hi; ++j) {
+            const int len = S_ > 1 ? __reduce_max_sync(mask, hi - lo) : hi - lo;
+            for (int t = 0; t < len; t += S_) {
+                // (a lane past its row takes some source, not listed)
+                const int jt = lo + t + (S_ > 1 ? (int)(threadIdx.x % S_) : 0);
+                const bool in = S_ == 1 || jt < hi;
+                const int j = in ? jt : 0;
                 const float4 pj = __ldg(S.pm + j);
                 const float dxc = (__ldg(S.scx + j) + wshift) - cxf;  // exact: small integers in FP32
                 const float rx = fmaf(-dxc, csf, d.xi_x - pj.x);
                 const float ry = by - pj.y, rz = bz - pj.z;
                 const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
-                bool hit = r2 < d.r2lo;
-                if (!hit && r2 <= d.r2hi) {
+                bool hit = in && r2 < d.r2lo;
+                if (in && !hit && r2 <= d.r2hi) {
                     const int oj = S.perm[j];
                     const double xi = ld0(dx64, d.orig);
                     hit = exact_within(EXT ? image_x(g, ld0(S.x, oj), xi, rx) : ld0(S.x, oj),
                                        ld0(S.y, oj), ld0(S.z, oj), xi, ld0(dy64, d.orig),
                                        ld0(dz64, d.orig), d.radius2);
                 }
-                bool listed = hit || r2 < d.r2list;
-                if (EXT && g.symmetric && !hit && r2 <= g.reach2) {
+                bool listed = hit || (in && r2 < d.r2list);
+                if (EXT && g.symmetric && in && !hit && r2 <= g.reach2) {
                     bool in_list;
                     hit = reverse_within(g, S, j, r2, rx, dx64, dy64, dz64, d.orig, in_list);
                     listed = listed || hit || in_list;
                 }
-                if (listed) fn(j, rx, ry, rz, code_yz + (int)dxc, hit);
+                if constexpr (S_ > 1) fn(listed, j, rx, ry, rz, code_yz + (int)dxc, hit);
+                else if (listed) fn(j, rx, ry, rz, code_yz + (int)dxc, hit);
             }
             };
             if (!EXT || !g.periodic) {
-                visit(tlo, thi, 0);
+                visit(row, tlo, thi, 0);
             } else {
                 const int a0 = d.cx + tlo, a1 = d.cx + thi;
-                if (a0 < 0) visit(a0 + g.nx - d.cx, min(a1, -1) + g.nx - d.cx, -1);
-                visit(max(a0, 0) - d.cx, min(a1, g.nx - 1) - d.cx, 0);
-                if (a1 >= g.nx) visit(max(a0, g.nx) - g.nx - d.cx, a1 - g.nx - d.cx, 1);
+                if (S_ > 1 || a0 < 0)
+                    visit(row && a0 < 0, a0 + g.nx - d.cx, min(a1, -1) + g.nx - d.cx, -1);
+                visit(row, max(a0, 0) - d.cx, min(a1, g.nx - 1) - d.cx, 0);
+                if (S_ > 1 || a1 >= g.nx)
+                    visit(row && a1 >= g.nx, max(a0, g.nx) - g.nx - d.cx, a1 - g.nx - d.cx, 1);
             }
         }
     }

@@ -290,3 +290,19 @@ def test_list_rates_lanes_give_the_same_bits(cap):
         assert r.returncode == 0, r.stderr[-3000:]
         seen.add(r.stdout.split()[-1])
     assert len(seen) == 1
+
+@pytest.mark.parametrize("cap", ["", "9"], ids=["lists", "over-full-lists"])
+def test_four_list_lanes_give_the_same_bits(cap):
+    """Four threads per destination of the list builds and the rates pass:
+    the bits of one."""
+    _need_gpu()
+    seen = set()
+    for lanes in ("1", "4"):
+        e = dict(os.environ, SPH_PAIR_LANES=lanes)
+        if cap:
+            e["SPH_LIST_CAP"] = cap
+        r = subprocess.run([sys.executable, "-c", _HASH_LISTS], cwd=ROOT, env=e,
+                           capture_output=True, text=True, timeout=600)
+        assert r.returncode == 0, r.stderr[-3000:]
+        seen.add(r.stdout.split()[-1])
+    assert len(seen) == 1
