@@ -83,6 +83,10 @@ struct BrickDstDev {
 };
 
 // shared-memory layout of a block (byte offsets into the dynamic array)
+// position records behind the padding record that a traversal may read (it
+// takes eight at a time)
+constexpr int kSlack = 6;
+
 struct BrickSmem {
     int off_v, off_s;   // rates: velocity / state records
     int off_scell;      // list build: cell table
@@ -446,8 +450,11 @@ __device__ __noinline__ bool exact_hit(const BrickSrcDev &S, const BrickDstDev &
 // Visit the sources of destination q that its list holds, in the staged
 // records, in the order of the list-streaming kernels: stencil rows [r0, r1)
 // in (dz, dy) order, each clipped to the chord of the search sphere,
-// ascending slot within a row.  fn(t, r2): staging index and the FP32 squared
-// distance.  With a list skin every source within the list radius is listed,
+// ascending slot within a row.  fn(t0, m): the listed ones among staging
+// indices t0 .. t0 + 31, as bits.  (A listed source costs several times a
+// candidate, one in four or five is listed, and a warp that handled each as it
+// came paid for it at nearly every candidate: list build of 275 K particles
+// 218 us, 195 by masks.)  With a list skin every source within the list radius is listed,
 // without one the neighbours.  The ranges come from the block's cell table
 // (scell) or, without one, from the grid's cell table.
 template <bool SKIN, bool STAGED, class Fn>
@@ -464,10 +471,10 @@ __device__ __forceinline__ void brick_rows(const Grid &g, const BlockGeo &G, con
     const float rl = SKIN ? rad.r2list : rad.r2lo;
     const int w = G.lx + 1;
     const int K = g.kx, wy = 2 * g.ky + 1;
+    int dz = r0 / wy, dy = r0 - dz * wy - g.ky;
+    dz -= g.kz;
 #pragma unroll 1
-    for (int rr = r0; rr < r1; ++rr) {
-        const int iz = rr / wy;
-        const int dz = iz - g.kz, dy = rr - iz * wy - g.ky;
+    for (int rr = r0; rr < r1; ++rr, dz += dy == g.ky ? 1 : 0, dy = dy == g.ky ? -g.ky : dy + 1) {
         const int czz = q.cz + dz, cyy = q.cy + dy;
         if (czz < G.zs0 || czz >= G.zs1 || cyy < G.ys0 || cyy >= G.ys1) continue;
         const float ez = fmaxf(0.f, dz > 0 ? (float)dz * csf - q.xi.z
@@ -493,14 +500,33 @@ __device__ __forceinline__ void brick_rows(const Grid &g, const BlockGeo &G, con
             ta = row_off(e) + (__ldg(S.cstart + c + clo) - e.x);
             tb = row_off(e) + (__ldg(S.cstart + c + chi + 1) - e.x);
         }
-        for (int t = ta; t < tb; ++t) {
-            const float4 pj = R.pos(t);
-            const float rx = q.P.x - pj.x, ry = q.P.y - pj.y, rz = q.P.z - pj.z;
-            const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
-            bool listed = r2 < rl;
-            if (!SKIN && !listed && r2 <= rad.r2hi)
-                listed = exact_hit(S, D, tab[t].x, q.orig, rad.radius2);
-            if (listed) fn(t, r2);
+        for (int t0 = ta; t0 < tb; t0 += 32) {
+            const int e = min(32, tb - t0);
+            unsigned m = 0, band = 0;
+            for (int u0 = 0; u0 < e; u0 += 8) {
+                unsigned mm = 0, bb = 0;
+                // (records past the row are read, not used: kSlack of them follow
+                // the last)
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const float4 pj = R.pos(t0 + u0 + u);
+                    const float rx = q.P.x - pj.x, ry = q.P.y - pj.y, rz = q.P.z - pj.z;
+                    const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
+                    if (r2 < rl) mm |= 1u << u;
+                    else if (!SKIN && r2 <= rad.r2hi) bb |= 1u << u;
+                }
+                m |= mm << u0;
+                if (!SKIN) band |= bb << u0;
+            }
+            const unsigned row = 0xffffffffu >> (32 - e);
+            m &= row;
+            if (!SKIN) {
+                for (band &= row; band; band &= band - 1) {
+                    const int u = __ffs(band) - 1;
+                    if (exact_hit(S, D, tab[t0 + u].x, q.orig, rad.radius2)) m |= 1u << u;
+                }
+            }
+            fn(t0, m);
         }
     }
 }
@@ -598,12 +624,13 @@ __device__ __forceinline__ void density_store(const BrickDensityArgs &A, int s, 
 // Fold the batches that the S lanes of a destination have just summed into
 // its compensated sum, in the order of the list: every lane adds all S of
 // them, so all hold the sum that one thread would have.
+// mask: the warp's lanes that fold together (a mask per destination would make
+// the warp run each destination's shuffles by themselves).
 template <int S>
-__device__ __forceinline__ void fold_lanes(CSum &c, float part) {
+__device__ __forceinline__ void fold_lanes(CSum &c, float part, unsigned mask) {
     if (S == 1) {
         c.add(part);
     } else {
-        const unsigned mask = ((1u << S) - 1u) << (threadIdx.x & 31 & ~(S - 1));
 #pragma unroll
         for (int s = 0; s < S; ++s) c.add(__shfl_sync(mask, part, s, S));
     }
@@ -643,7 +670,7 @@ __device__ __forceinline__ void dest_prefetch(const BrickDstDev &Dd, float csf, 
 template <int S, bool STAGED>
 __device__ __forceinline__ void density_group(CSum &rho, const SrcRecords<STAGED> &R, bool mine,
                                               const uint4 &grp, const float4 &Pi, float ih,
-                                              const WCoef &wc) {
+                                              const WCoef &wc, unsigned mask) {
     float part = 0.f;
     if (S == 1 || mine) {
 #pragma unroll
@@ -655,30 +682,32 @@ __device__ __forceinline__ void density_group(CSum &rho, const SrcRecords<STAGED
             for (int i = 0; i < 4; ++i) part += density_term(Pi, pj[i], ih, wc);
         }
     }
-    fold_lanes<S>(rho, part);
+    fold_lanes<S>(rho, part, mask);
 }
 
 template <int S, bool STAGED>
 __device__ __forceinline__ void density_stream(CSum &rho, const SrcRecords<STAGED> &R,
                                                const uint4 *lst, int D, int ng, int lane,
                                                const float4 &Pi, float ih, const WCoef &wc, uint4 b0,
-                                               uint4 b1) {
+                                               uint4 b1, unsigned mask) {
     const uint4 zero = make_uint4(0, 0, 0, 0);
+    // the rounds of the warp's longest list (a batch of none adds 0)
+    const int nr = S > 1 ? __reduce_max_sync(mask, ng) : ng;
     const size_t step = (size_t)D;
     uint4 b2;
     // g0: the first group of the round, gi: this lane's
     for (int g0 = 0, gi = lane;;) {
-        if (g0 >= ng) break;
+        if (g0 >= nr) break;
         b2 = gi + 2 * S < ng ? lst[(gi + 2 * S) * step] : zero;
-        density_group<S, STAGED>(rho, R, gi < ng, b0, Pi, ih, wc);
+        density_group<S, STAGED>(rho, R, gi < ng, b0, Pi, ih, wc, mask);
         gi += S;
-        if ((g0 += S) >= ng) break;
+        if ((g0 += S) >= nr) break;
         b0 = gi + 2 * S < ng ? lst[(gi + 2 * S) * step] : zero;
-        density_group<S, STAGED>(rho, R, gi < ng, b1, Pi, ih, wc);
+        density_group<S, STAGED>(rho, R, gi < ng, b1, Pi, ih, wc, mask);
         gi += S;
-        if ((g0 += S) >= ng) break;
+        if ((g0 += S) >= nr) break;
         b1 = gi + 2 * S < ng ? lst[(gi + 2 * S) * step] : zero;
-        density_group<S, STAGED>(rho, R, gi < ng, b2, Pi, ih, wc);
+        density_group<S, STAGED>(rho, R, gi < ng, b2, Pi, ih, wc, mask);
         gi += S;
         g0 += S;
     }
@@ -708,10 +737,12 @@ __device__ __forceinline__ int build_list(const BrickDensityArgs &A, const Block
             grp.w = (grp.w >> 16) | (t << 16);
         };
         brick_traverse<STAGED>(A.g, G, A.s, A.d, R, A.rad, brow, tab, scell, q, 0, rows,
-            [&](int t, float) {
-                push((unsigned)t);
-                ++c;
-                if ((c & 7) == 0 && c <= cap) out[(size_t)((c >> 3) - 1) * D] = grp;
+            [&](int t0, unsigned m) {
+                for (; m; m &= m - 1) {
+                    push((unsigned)(t0 + __ffs(m) - 1));
+                    ++c;
+                    if ((c & 7) == 0 && c <= cap) out[(size_t)((c >> 3) - 1) * D] = grp;
+                }
             });
         if (c < cap && (c & 7)) {
             for (int k = c; k & 7; ++k) push((unsigned)T);
@@ -722,7 +753,7 @@ __device__ __forceinline__ int build_list(const BrickDensityArgs &A, const Block
     const int ra = rows * lane / S, rb = rows * (lane + 1) / S;
     if (active)
         brick_traverse<STAGED>(A.g, G, A.s, A.d, R, A.rad, brow, tab, scell, q, ra, rb,
-                               [&](int, float) { ++c; });
+                               [&](int, unsigned m) { c += __popc(m); });
     __syncwarp();
     int end = c;
 #pragma unroll
@@ -739,7 +770,9 @@ __device__ __forceinline__ int build_list(const BrickDensityArgs &A, const Block
             ++k;
         };
         brick_traverse<STAGED>(A.g, G, A.s, A.d, R, A.rad, brow, tab, scell, q, ra, rb,
-                               [&](int t, float) { write((unsigned)t); });
+                               [&](int t0, unsigned m) {
+                                   for (; m; m &= m - 1) write((unsigned)(t0 + __ffs(m) - 1));
+                               });
         if (lane == S - 1)
             while (k & 7) write((unsigned)T);
     }
@@ -807,14 +840,17 @@ __device__ __forceinline__ void build_sum(const BrickDensityArgs &A, const Block
         int skip = cap;
         const int rows = (2 * A.g.ky + 1) * (2 * A.g.kz + 1);
         brick_traverse<STAGED>(A.g, G, A.s, A.d, R, A.rad, brow, tab, scell, q, 0, rows,
-            [&](int t, float) {
-                if (skip > 0) { --skip; return; }
-                const float4 pj = R.pos(t);
-                const float d2 = dist2(pj);
-                bool hit = d2 < r2lo;
-                if (!hit && d2 <= r2hi)
-                    hit = exact_hit(A.s, A.d, tab[t].x, q.orig, A.rad.radius2);
-                if (hit) add(d2, pj.w);
+            [&](int t0, unsigned bits) {
+                for (; bits; bits &= bits - 1) {
+                    if (skip > 0) { --skip; continue; }
+                    const int t = t0 + __ffs(bits) - 1;
+                    const float4 pj = R.pos(t);
+                    const float d2 = dist2(pj);
+                    bool hit = d2 < r2lo;
+                    if (!hit && d2 <= r2hi)
+                        hit = exact_hit(A.s, A.d, tab[t].x, q.orig, A.rad.radius2);
+                    if (hit) add(d2, pj.w);
+                }
             });
     }
     rho.add(part);
@@ -844,10 +880,15 @@ __device__ __noinline__ void density_rest(const BrickDensityArgs &A) {
         CSum rest;
         int skip = A.cap;
         brick_traverse<STAGED>(g, G, A.s, A.d, R, A.rad, brow, tab, nullptr, q, 0, rows,
-            [&](int t, float r2) {
-                if (skip > 0) { --skip; return; }
-                const float r = r2 > 0.f ? r2 * rsqrtf(r2) : 0.f;
-                rest.add(cubic_w(r * ih) * fac * R.pos(t).w);
+            [&](int t0, unsigned m) {
+                for (; m; m &= m - 1) {
+                    if (skip > 0) { --skip; continue; }
+                    const float4 pj = R.pos(t0 + __ffs(m) - 1);
+                    const float rx = q.P.x - pj.x, ry = q.P.y - pj.y, rz = q.P.z - pj.z;
+                    const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
+                    const float r = r2 > 0.f ? r2 * rsqrtf(r2) : 0.f;
+                    rest.add(cubic_w(r * ih) * fac * pj.w);
+                }
             });
         // the stored partial density (hi + lo of the listed part, in FP64)
         // plus the rest, as a compensated FP32 pair
@@ -862,12 +903,13 @@ __device__ __noinline__ void density_rest(const BrickDensityArgs &A) {
 // The density of destination d of the block (its prefetched records p).
 template <int S, bool STAGED>
 __device__ __forceinline__ void density_dest(const BrickDensityArgs &A, const SrcRecords<STAGED> &R,
-                                             const uint4 *lst, int D, int lane, const DestPre &p) {
+                                             const uint4 *lst, int D, int lane, const DestPre &p,
+                                             unsigned mask) {
     const float ih = __fdividef(1.f, A.g.h_uniform);
     const WCoef wc = w_coef(cubic_fac(A.dim, ih), 1.f);
     CSum rho;
     density_stream<S, STAGED>(rho, R, lst, D, (min(p.c, A.cap) + 7) >> 3, lane, p.P, ih, wc, p.b0,
-                              p.b1);
+                              p.b1, mask);
     if (lane == 0) {
         const bool real = is_real(A.d, p.orig);
         density_store(A, p.s, p.orig, real, p.P.w, real ? rho.hi : 0.f, real ? rho.lo : 0.f);
@@ -887,11 +929,14 @@ __device__ __noinline__ void density_more(const BrickDensityArgs &A, int first) 
         make_records<STAGED>(A.sm, A.s, A.g.cs_f, A.s.bstage + sh.y, sh.x, 0.f);
     const uint4 *lgrp = reinterpret_cast<const uint4 *>(A.nbr) + (size_t)dh.y * (A.cap >> 3);
     const int lane = threadIdx.x % S;
-    for (int d = first + threadIdx.x / S; d < dh.x; d += blockDim.x / S) {
+    for (int r0 = first; r0 < dh.x; r0 += blockDim.x / S) {
+        const int d = r0 + threadIdx.x / S;
+        const unsigned mask = __ballot_sync(0xffffffffu, d < dh.x);
+        if (d >= dh.x) continue;
         DestPre p;
         dest_prefetch<S>(A.d, A.g.cs_f, A.d.bdest[dh.y + d], A.cnt + dh.y, lgrp, A.cap, dh.x, d,
                          lane, p);
-        density_dest<S, STAGED>(A, R, lgrp + d, dh.x, lane, p);
+        density_dest<S, STAGED>(A, R, lgrp + d, dh.x, lane, p, mask);
     }
 }
 
@@ -917,7 +962,8 @@ __global__ void __maxnreg__(64) k_bdensity(const __grid_constant__ BrickDensityA
     __syncthreads();
     if (off != 0u) return;
     const SrcRecords<STAGED> R = make_records<STAGED>(A.sm, A.s, A.g.cs_f, tab, T, 0.f);
-    if (d < D) density_dest<S, STAGED>(A, R, lgrp + d, D, lane, pre);
+    const unsigned mask = S > 1 ? __ballot_sync(0xffffffffu, d < D) : 0xffffffffu;
+    if (d < D) density_dest<S, STAGED>(A, R, lgrp + d, D, lane, pre, mask);
     if (D > (int)blockDim.x / S) density_more<STAGED>(A, blockDim.x / S);
     if (*A.maxcnt > A.cap && A.rho_out != nullptr) density_rest<STAGED>(A);
 }
@@ -1051,11 +1097,11 @@ __device__ __forceinline__ void rates_pair(RatesAcc &a, const RatesConst &k, flo
 }
 
 template <int S, bool XSPH>
-__device__ __forceinline__ void rates_flush(RatesAcc &a) {
-    fold_lanes<S>(a.ax, a.pax); fold_lanes<S>(a.ay, a.pay); fold_lanes<S>(a.az, a.paz);
+__device__ __forceinline__ void rates_flush(RatesAcc &a, unsigned mask) {
+    fold_lanes<S>(a.ax, a.pax, mask); fold_lanes<S>(a.ay, a.pay, mask); fold_lanes<S>(a.az, a.paz, mask);
     a.pax = a.pay = a.paz = 0.f;
     if (XSPH) {
-        fold_lanes<S>(a.xx, a.pxx); fold_lanes<S>(a.xy, a.pxy); fold_lanes<S>(a.xz, a.pxz);
+        fold_lanes<S>(a.xx, a.pxx, mask); fold_lanes<S>(a.xy, a.pxy, mask); fold_lanes<S>(a.xz, a.pxz, mask);
         a.pxx = a.pxy = a.pxz = 0.f;
     }
 }
@@ -1065,7 +1111,7 @@ __device__ __forceinline__ void rates_flush(RatesAcc &a) {
 template <int S, bool XSPH, bool ETA0, bool FAST, bool STAGED>
 __device__ __forceinline__ void rates_group(RatesAcc &acc, const RatesConst &kc,
                                             const SrcRecords<STAGED> &R, bool mine, const uint4 &grp,
-                                            const float4 &Pi) {
+                                            const float4 &Pi, unsigned mask) {
     if (S == 1 || mine) {
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
@@ -1081,29 +1127,31 @@ __device__ __forceinline__ void rates_group(RatesAcc &acc, const RatesConst &kc,
                                        pj[i], vj[i], mj[i], hac[i]);
         }
     }
-    rates_flush<S, XSPH>(acc);
+    rates_flush<S, XSPH>(acc, mask);
 }
 
 // The sums of a destination, its list streamed as in density_stream.
 template <int S, bool XSPH, bool ETA0, bool FAST, bool STAGED>
 __device__ __forceinline__ void rates_stream(RatesAcc &acc, const RatesConst &kc,
                                              const SrcRecords<STAGED> &R, const uint4 *lst, int D,
-                                             int ng, int lane, const float4 &Pi, uint4 b0, uint4 b1) {
+                                             int ng, int lane, const float4 &Pi, uint4 b0, uint4 b1,
+                                             unsigned mask) {
     const uint4 zero = make_uint4(0, 0, 0, 0);
+    const int nr = S > 1 ? __reduce_max_sync(mask, ng) : ng;
     const size_t step = (size_t)D;
     uint4 b2;
     for (int g0 = 0, gi = lane;;) {
-        if (g0 >= ng) break;
+        if (g0 >= nr) break;
         b2 = gi + 2 * S < ng ? lst[(gi + 2 * S) * step] : zero;
-        rates_group<S, XSPH, ETA0, FAST, STAGED>(acc, kc, R, gi < ng, b0, Pi);
+        rates_group<S, XSPH, ETA0, FAST, STAGED>(acc, kc, R, gi < ng, b0, Pi, mask);
         gi += S;
-        if ((g0 += S) >= ng) break;
+        if ((g0 += S) >= nr) break;
         b0 = gi + 2 * S < ng ? lst[(gi + 2 * S) * step] : zero;
-        rates_group<S, XSPH, ETA0, FAST, STAGED>(acc, kc, R, gi < ng, b1, Pi);
+        rates_group<S, XSPH, ETA0, FAST, STAGED>(acc, kc, R, gi < ng, b1, Pi, mask);
         gi += S;
-        if ((g0 += S) >= ng) break;
+        if ((g0 += S) >= nr) break;
         b1 = gi + 2 * S < ng ? lst[(gi + 2 * S) * step] : zero;
-        rates_group<S, XSPH, ETA0, FAST, STAGED>(acc, kc, R, gi < ng, b2, Pi);
+        rates_group<S, XSPH, ETA0, FAST, STAGED>(acc, kc, R, gi < ng, b2, Pi, mask);
         gi += S;
         g0 += S;
     }
@@ -1175,14 +1223,16 @@ __device__ __noinline__ void rates_rest(const BrickRatesArgs &A) {
         rates_acc_init(acc, A.d.velh[q.s], A.d.st[q.s], halpha);
         int skip = A.cap;
         brick_traverse<STAGED>(g, G, A.s, A.d, R, A.rad, brow, tab, nullptr, q, 0, rows,
-            [&](int t, float) {
-                if (skip > 0) { --skip; return; }
-                float4 pj, vj;
-                float mj, hac;
-                R.template rates_rec<false>(t, 0.f, 0.f, pj, vj, mj, hac);
-                rates_pair<XSPH, ETA0>(acc, kc, q.P.x - pj.x, q.P.y - pj.y, q.P.z - pj.z, pj, vj,
-                                       mj, hac);
-                rates_flush<1, XSPH>(acc);
+            [&](int t0, unsigned m) {
+                for (; m; m &= m - 1) {
+                    if (skip > 0) { --skip; continue; }
+                    float4 pj, vj;
+                    float mj, hac;
+                    R.template rates_rec<false>(t0 + __ffs(m) - 1, 0.f, 0.f, pj, vj, mj, hac);
+                    rates_pair<XSPH, ETA0>(acc, kc, q.P.x - pj.x, q.P.y - pj.y, q.P.z - pj.z, pj, vj,
+                                           mj, hac);
+                    rates_flush<1, XSPH>(acc, 0u);
+                }
             });
         const double a3[3] = {(double)acc.ax.fvalue(), (double)acc.ay.fvalue(),
                               (double)acc.az.fvalue()};
@@ -1200,7 +1250,8 @@ __device__ __noinline__ void rates_rest(const BrickRatesArgs &A) {
 template <int S, bool XSPH, bool ETA0, bool FAST, bool STAGED>
 __device__ __forceinline__ void rates_dest(const BrickRatesArgs &A, const SrcRecords<STAGED> &R,
                                            float mb, const uint4 *lst, int D, int lane,
-                                           const DestPre &p, const float4 &vi, const float4 &st) {
+                                           const DestPre &p, const float4 &vi, const float4 &st,
+                                           unsigned mask) {
     const float ih = __fdividef(1.f, A.g.h_uniform);
     RatesConst kc = rates_const(A.g.h_uniform, cubic_fac(A.dim, ih), A.beta, A.eta2, A.eps);
     kc.mb = mb;
@@ -1208,7 +1259,7 @@ __device__ __forceinline__ void rates_dest(const BrickRatesArgs &A, const SrcRec
     RatesAcc acc;
     rates_acc_init(acc, vi, st, 0.5f * A.alpha);
     rates_stream<S, XSPH, ETA0, FAST, STAGED>(acc, kc, R, lst, D, (min(p.c, A.cap) + 7) >> 3, lane,
-                                              p.P, p.b0, p.b1);
+                                              p.P, p.b0, p.b1, mask);
     rates_store<S, XSPH>(A, acc, p.orig, lane);
 }
 
@@ -1223,12 +1274,15 @@ __device__ __noinline__ void rates_more(const BrickRatesArgs &A, float mb, int f
                                                       0.5f * A.alpha);
     const uint4 *lgrp = reinterpret_cast<const uint4 *>(A.nbr) + (size_t)dh.y * (A.cap >> 3);
     const int lane = threadIdx.x % S;
-    for (int d = first + threadIdx.x / S; d < dh.x; d += blockDim.x / S) {
+    for (int r0 = first; r0 < dh.x; r0 += blockDim.x / S) {
+        const int d = r0 + threadIdx.x / S;
+        const unsigned mask = __ballot_sync(0xffffffffu, d < dh.x);
+        if (d >= dh.x) continue;
         DestPre p;
         dest_prefetch<S>(A.d, A.g.cs_f, A.d.bdest[dh.y + d], A.cnt + dh.y, lgrp, A.cap, dh.x, d,
                          lane, p);
         rates_dest<S, XSPH, ETA0, FAST, STAGED>(A, R, mb, lgrp + d, dh.x, lane, p, A.d.velh[p.s],
-                                                A.d.st[p.s]);
+                                                A.d.st[p.s], mask);
     }
 }
 
@@ -1236,8 +1290,9 @@ template <int S, bool XSPH, bool ETA0, bool FAST, bool STAGED>
 __device__ __forceinline__ void rates_block(const BrickRatesArgs &A, const SrcRecords<STAGED> &R,
                                             float mb, const uint4 *lgrp, int D, int d, int lane,
                                             const DestPre &pre, const float4 &vi, const float4 &st) {
+    const unsigned mask = S > 1 ? __ballot_sync(0xffffffffu, d < D) : 0xffffffffu;
     if (d < D)
-        rates_dest<S, XSPH, ETA0, FAST, STAGED>(A, R, mb, lgrp + d, D, lane, pre, vi, st);
+        rates_dest<S, XSPH, ETA0, FAST, STAGED>(A, R, mb, lgrp + d, D, lane, pre, vi, st, mask);
     if (D > (int)blockDim.x / S) rates_more<XSPH, ETA0, FAST, STAGED>(A, mb, blockDim.x / S);
     if (*A.maxcnt > A.cap) rates_rest<XSPH, ETA0, STAGED>(A);
 }
@@ -1414,11 +1469,12 @@ int brick_layout(const sph_ctx *ctx, const ArraySnap &S, bool rates, bool cells,
         const char *e = getenv("SPH_BRICK_UNSTAGED");
         unstaged = (e && atoi(e) > 0) ? 1 : 0;
     }
-    const bool staged = !unstaged && sizeof(int) * ncell + cap * rec + 64 <= (size_t)kBrickSmemLimit;
+    const bool staged = !unstaged && sizeof(int) * ncell + cap * rec + kSlack * 16 + 64 <=
+                                         (size_t)kBrickSmemLimit;
     if (!staged) cap = 0;
     size_t off = 0;
     // position records, then (rates) velocity and state records
-    off += cap * 16;
+    off += staged ? (cap + kSlack) * 16 : 0;
     sm->off_v = (int)off;
     if (rates) off += cap * 16;
     sm->off_s = (int)off;
