@@ -354,6 +354,20 @@ __global__ void k_reorder(sph_array_view a, Grid g, const int *order, const int 
 // every neighbour), or when a list of this build holds more neighbours than
 // its capacity (the re-traversal that completes it needs the build's
 // positions).
+// What a light refresh reads and writes of an array.
+struct LightArray {
+    sph_array_view a;
+    const int *inv, *key;
+    const float4 *pm0;
+    float4 *velh, *nrm, *tan, *pm;
+    int *refcell;
+};
+constexpr int kLightArrays = 4;     // in one launch
+template <int NA>
+struct LightArgs {
+    LightArray l[NA];
+};
+
 struct ListCaps {
     int n;                      // lists to check (0: none)
     int cap[kMaxListSlots];     // capacity, INT_MAX for a list of an older build
@@ -394,21 +408,28 @@ __global__ void k_selftest_conversions(long long n, unsigned long long *bad) {
     if (miss) atomicAdd(bad, miss);
 }
 
-__global__ void __launch_bounds__(256, 5) k_light(sph_array_view a, Grid g, double inv_cs_ref, const int *inv,
-                        const int *key, const float4 *pm0, float4 *velh,
-                        float4 *nrm, float4 *tan, float4 *pm, int *refcell,
-                        int check_jump,
+// NA arrays in one launch, one per grid row.
+template <int NA>
+__global__ void __launch_bounds__(256, 5) k_light(const __grid_constant__ LightArgs<NA> args, Grid g,
+                        double inv_cs_ref, int check_jump,
                         double build_h, float stale_thr, const __grid_constant__ ListCaps caps,
                         unsigned *status, unsigned stale_bit) {
+    const LightArray &L = args.l[NA > 1 ? blockIdx.y : 0];
+    const sph_array_view &a = L.a;
+    const int *inv = L.inv, *key = L.key;
+    const float4 *pm0 = L.pm0;
+    float4 *velh = L.velh, *nrm = L.nrm, *tan = L.tan, *pm = L.pm;
+    int *refcell = L.refcell;
     float dm = 0.f;
     bool jump = false, hch = false;
     const float inv_ref_f = (float)inv_cs_ref;
     // list maxima: written by the passes before this launch
-    if (blockIdx.x == 0 && threadIdx.x < caps.n &&
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < caps.n &&
         (int)status[kListWord0 + threadIdx.x] > caps.cap[threadIdx.x]) {
         atomicOr(status + kStaleWord, kStaleLists);
         if (stale_bit) atomicOr(status + kStaleBitsWord, stale_bit);
     }
+    if (NA > 1 && blockIdx.x * (int64_t)blockDim.x >= a.n) return;   // (a shorter array's row)
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < a.n;
          i += (int64_t)gridDim.x * blockDim.x) {
         const int s = inv[i];
@@ -970,18 +991,36 @@ int nnps_update(sph_ctx *ctx, const sph_array_view *arrays, int narrays, double 
         const NbrList &L = ctx->lists[i];
         caps.cap[i] = (L.maxcnt && L.build == ctx->build_id) ? L.cap : INT_MAX;
     }
+    LightArgs<kLightArrays> la;
+    int na = 0;
+    int64_t nmax = 0;
     for (int a = 0; a < narrays; ++a) {
         ArraySnap &A = ctx->arrays[a];
         const sph_array_view &v = arrays[a];
-        if (v.n == 0) continue;
+        if (v.n > 0) {
+            la.l[na++] = {v, A.inv, A.key, A.pm0, A.velh, A.has_nrm ? A.nrm : nullptr,
+                          A.has_nrm ? A.tan : nullptr, A.pm, A.refcell};
+            nmax = std::max<int64_t>(nmax, v.n);
+            A.st_fresh = false;
+        }
+        if (na == 0 || (na < kLightArrays && a + 1 < narrays)) continue;
         // one thread per particle (more loads in flight than a grid-stride
         // loop over a resident grid: 55 against 61 us at 1 M particles)
-        k_light<<<grid_blocks(v.n, kThreads, 64), kThreads, 0, st>>>(
-            v, ctx->grid, inv_cs_ref, A.inv, A.key, A.pm0, A.velh,
-            A.has_nrm ? A.nrm : nullptr, A.has_nrm ? A.tan : nullptr, A.pm, A.refcell, check_jump,
-            ctx->build_h, stale_thr, caps, ctx->d_status, ctx->capture_stale_bit);
+        const unsigned nb = (unsigned)grid_blocks(nmax, kThreads, 64);
+        if (na == 1) {
+            LightArgs<1> one;
+            one.l[0] = la.l[0];
+            k_light<1><<<nb, kThreads, 0, st>>>(one, ctx->grid, inv_cs_ref, check_jump, ctx->build_h,
+                                                stale_thr, caps, ctx->d_status,
+                                                ctx->capture_stale_bit);
+        } else {
+            k_light<kLightArrays><<<dim3(nb, (unsigned)na), kThreads, 0, st>>>(
+                la, ctx->grid, inv_cs_ref, check_jump, ctx->build_h, stale_thr, caps, ctx->d_status,
+                ctx->capture_stale_bit);
+        }
         caps.n = 0;   // checked once
-        A.st_fresh = false;
+        na = 0;
+        nmax = 0;
         count_launch();
         SPH_LAUNCH_CHECK("k_light");
     }

@@ -72,3 +72,44 @@ def test_skin_drop_matches_oracle(monkeypatch):
     for p in ("x", "y", "u", "v"):
         assert normwise(a[p] - props[p], ref[p] - props[p]) < 1e-4, p
     assert normwise(a["rho"], ref["rho"]) < 1e-5
+
+
+@pytest.mark.parametrize("sizes", [(600,), (600, 150), (40, 0, 600), (300, 20, 1, 270),
+                                   (90, 0, 300, 20, 70, 110)])
+def test_light_refresh_of_several_arrays(sizes, monkeypatch):
+    """One launch refreshes up to four arrays, of any lengths (none included):
+    after a move inside the skin every array's density over all arrays is the
+    oracle's at the new positions."""
+    _need_gpu()
+    monkeypatch.setenv("PYSPH_GB300_SKIN", "0.05")
+    rng = np.random.default_rng(len(sizes))
+    base, sph = API.base, API.sph
+    h = 0.05
+    props = [{"x": rng.uniform(0, 1, n), "y": rng.uniform(0, 1, n), "h": np.full(n, h),
+              "m": rng.uniform(0.5, 1.5, n), "rho": np.ones(n)} for n in sizes]
+    arrays = [base.get_particle_array(name="a%d" % k, type=base.ParticleType.Fluid, **p)
+              for k, p in enumerate(props)]
+    particles = base.Particles(arrays=arrays)
+    kern = base.CubicSplineKernel(dim=2)
+    for step in range(2):
+        if step:
+            for pa, p in zip(arrays, props):
+                for c in "xy":
+                    p[c] = p[c] + 0.001 * rng.uniform(-1, 1, len(p[c]))
+                pa.set(x=p["x"], y=p["y"])
+            particles.update()
+        for pa, p in zip(arrays, props):
+            if len(p["x"]) == 0:
+                continue
+            calc = sph.SPHCalc(particles, arrays, pa, kern,
+                               [sph.SPHRho.get_func(s, pa) for s in arrays], ["rho"])
+            calc.sph("rho")
+            want = np.zeros(len(p["x"]))
+            for q in props:
+                if len(q["x"]) == 0:
+                    continue
+                off, idx = oracle.neighbors(p, q, 2.0 * h, same=q is p)
+                want += oracle.pair_sum("rho", p, q, off, idx, 2, nout=1)[0]
+            assert normwise(pa.get("rho"), want) < 1e-5
+    full, light = particles.cell_manager.build_stats()
+    assert light >= 1, (full, light)
