@@ -267,11 +267,13 @@ __device__ __forceinline__ float tanh_approx(float x) {
     return y;
 }
 constexpr float kGeluU1 = kGeluC * 0.044715f;             // u = z (C + U1 z^2)
-__device__ __forceinline__ uint64_t gelu2(uint64_t z) {
-    const uint64_t u = mul2(z, fma2(mul2(z, z), f2(kGeluU1, kGeluU1), f2(kGeluC, kGeluC)));
+// From z / 2, which the bias step leaves (a power of two: the same bits as from
+// z, with one operation less in an epilogue that instruction issue bounds).
+__device__ __forceinline__ uint64_t gelu2_half(uint64_t hz) {
+    const uint64_t u = mul2(hz, fma2(mul2(hz, hz), f2(8.f * kGeluU1, 8.f * kGeluU1),
+                                     f2(2.f * kGeluC, 2.f * kGeluC)));
     float u0, u1;
     f2_split(u, u0, u1);
-    const uint64_t hz = mul2(z, f2(0.5f, 0.5f));
     return fma2(hz, f2(tanh_approx(u0), tanh_approx(u1)), hz);
 }
 
@@ -612,8 +614,8 @@ __global__ void __launch_bounds__(G_THREADS, 1)
     auto bar = [&](int i) { return sbase + G_BAR + 8u * (uint32_t)i; };
 
     for (int i = t; i < NH; i += G_THREADS) {
-        b1f[i] = params[OFF_B1 + i];
-        b2f[i] = params[OFF_B2 + i];
+        b1f[i] = 0.5f * params[OFF_B1 + i];     // (the epilogues work with z / 2)
+        b2f[i] = 0.5f * params[OFF_B2 + i];
     }
     for (int i = t; i < NOUT * NH; i += G_THREADS) w3f[i] = __uint_as_float((uint32_t)w3b[i] << 16);
     if (t < NOUT) b3f[t] = params[OFF_B3 + t];
@@ -713,6 +715,7 @@ __global__ void __launch_bounds__(G_THREADS, 1)
         auto wwait = [&](int k, int parity) {
             return __all_sync(0xffffffffu, gwait(bar(k), (uint32_t)parity & 1u, abort)) != 0;
         };
+        const uint64_t half = f2(0.5f, 0.5f);
         // layer 1 of tile i: acc1[i % 2] + b1, GELU -> H1 (and the saved values)
         auto layer1 = [&](int i) -> bool {
             const int s = i & 1;
@@ -734,27 +737,27 @@ __global__ void __launch_bounds__(G_THREADS, 1)
 #pragma unroll
                 for (int e = 0; e < 16; ++e) v[e] = __uint_as_float(rr[c][e]);
                 // + b1 and GELU, two columns per packed instruction
-                uint64_t z[8];
+                uint64_t hz[8];
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const float4 bb = *reinterpret_cast<const float4 *>(b1f + cb + 16 * c + 4 * e);
-                    z[2 * e] = add2(f2(v[4 * e], v[4 * e + 1]), f2(bb.x, bb.y));
-                    z[2 * e + 1] = add2(f2(v[4 * e + 2], v[4 * e + 3]), f2(bb.z, bb.w));
+                    hz[2 * e] = fma2(f2(v[4 * e], v[4 * e + 1]), half, f2(bb.x, bb.y));
+                    hz[2 * e + 1] = fma2(f2(v[4 * e + 2], v[4 * e + 3]), half, f2(bb.z, bb.w));
                 }
                 if (valid && z1s) {
                     float4 *zp = reinterpret_cast<float4 *>(z1s + grow * NH + cb + 16 * c);
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
                         float a0, a1, a2, a3;
-                        f2_split(z[2 * e], a0, a1);
-                        f2_split(z[2 * e + 1], a2, a3);
+                        f2_split(add2(hz[2 * e], hz[2 * e]), a0, a1);
+                        f2_split(add2(hz[2 * e + 1], hz[2 * e + 1]), a2, a3);
                         zp[e] = make_float4(a0, a1, a2, a3);
                     }
                 }
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
                     float g0, g1;
-                    f2_split(gelu2(z[e]), g0, g1);
+                    f2_split(gelu2_half(hz[e]), g0, g1);
                     hw[8 * c + e] = pack2(g0, g1);
                 }
             }
@@ -802,17 +805,17 @@ __global__ void __launch_bounds__(G_THREADS, 1)
 #pragma unroll
                 for (int e = 0; e < 16; ++e) v[e] = __uint_as_float(rr2[c][e]);
                 uint32_t w2w[8];
-                uint64_t z[8];
+                uint64_t hz[8];
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const float4 bb = *reinterpret_cast<const float4 *>(b2f + cb + 16 * c + 4 * e);
-                    z[2 * e] = add2(f2(v[4 * e], v[4 * e + 1]), f2(bb.x, bb.y));
-                    z[2 * e + 1] = add2(f2(v[4 * e + 2], v[4 * e + 3]), f2(bb.z, bb.w));
+                    hz[2 * e] = fma2(f2(v[4 * e], v[4 * e + 1]), half, f2(bb.x, bb.y));
+                    hz[2 * e + 1] = fma2(f2(v[4 * e + 2], v[4 * e + 3]), half, f2(bb.z, bb.w));
                 }
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
                     float g0, g1;
-                    f2_split(gelu2(z[e]), g0, g1);
+                    f2_split(gelu2_half(hz[e]), g0, g1);
                     w2w[e] = pack2(g0, g1);
                     const int j = cb + 16 * c + 2 * e;
                     const uint64_t h = f2(bf_lo(w2w[e]), bf_hi(w2w[e]));
@@ -824,8 +827,8 @@ __global__ void __launch_bounds__(G_THREADS, 1)
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
                         float a0, a1, a2, a3;
-                        f2_split(z[2 * e], a0, a1);
-                        f2_split(z[2 * e + 1], a2, a3);
+                        f2_split(add2(hz[2 * e], hz[2 * e]), a0, a1);
+                        f2_split(add2(hz[2 * e + 1], hz[2 * e + 1]), a2, a3);
                         zp[e] = make_float4(a0, a1, a2, a3);
                     }
                 }
