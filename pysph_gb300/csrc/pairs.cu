@@ -470,7 +470,9 @@ struct VelState {
 
 // SPEC 0: any terms, runtime flags; 1: PGrad + AV, uniform h, one source;
 // 2: PGrad + AV + XSPH, uniform h, one source.
-template <int KX, int SPEC, int MODE, int S_ = 1>
+// Z false: nobody asked for the third components (2D batches), which are then
+// not summed either.
+template <int KX, int SPEC, int MODE, int S_ = 1, bool Z = true>
 __global__ void __launch_bounds__(kPairBlock) k_rates(const __grid_constant__ RatesArgs A) {
     constexpr uint32_t SF = SPEC == 1 ? (SPH_TERM_PGRAD | SPH_TERM_AVISC)
                           : (SPEC == 2 ? (SPH_TERM_PGRAD | SPH_TERM_AVISC | SPH_TERM_XSPH) : 0u);
@@ -537,7 +539,7 @@ __global__ void __launch_bounds__(kPairBlock) k_rates(const __grid_constant__ Ra
                     const float gf = cubic_gfac(q, ih, rinv) * fac * t * okf;
                     pax = fmaf(gf, rx, pax);
                     pay = fmaf(gf, ry, pay);
-                    paz = fmaf(gf, rz, paz);
+                    if (Z) paz = fmaf(gf, rz, paz);
                 }
                 if (MAY_DRHO && (fl & (SPH_TERM_DRHO | SPH_TERM_VDIV))) {
                     // drho_i += m_j (v_i - v_j) . grad W(hab)  (density_funcs.pyx:117-158);
@@ -550,7 +552,7 @@ __global__ void __launch_bounds__(kPairBlock) k_rates(const __grid_constant__ Ra
                     const float temp = __fdividef(mj * (cubic_w(q) * fac), rhoab) * S.eps * okf;
                     pxx = fmaf(temp, vj.x - vi.x, pxx);
                     pxy = fmaf(temp, vj.y - vi.y, pxy);
-                    pxz = fmaf(temp, vj.z - vi.z, pxz);
+                    if (Z) pxz = fmaf(temp, vj.z - vi.z, pxz);
                 }
                 if (MAY_BF && (fl & SPH_TERM_BFORCE)) {
                     const float4 nj = S.nrm[j], tj = S.tan[j];
@@ -602,14 +604,16 @@ __global__ void __launch_bounds__(kPairBlock) k_rates(const __grid_constant__ Ra
                     pax = pay = paz = pdr = pxx = pxy = pxz = 0.f;
                     return;
                 }
-                ax.add(pax); ay.add(pay); az.add(paz);
+                ax.add(pax); ay.add(pay);
+                if (Z) az.add(paz);
                 pax = pay = paz = 0.f;
                 if (MAY_DRHO) {
                     dr.add(pdr);
                     pdr = 0.f;
                 }
                 if (MAY_XSPH) {
-                    xx.add(pxx); xy.add(pxy); xz.add(pxz);
+                    xx.add(pxx); xy.add(pxy);
+                    if (Z) xz.add(pxz);
                     pxx = pxy = pxz = 0.f;
                 }
             }, mask);
@@ -639,18 +643,18 @@ __global__ void __launch_bounds__(kPairBlock) k_rates(const __grid_constant__ Ra
     }
     double a3[3] = {0.0, 0.0, 0.0}, p3[3] = {0.0, 0.0, 0.0};
     if (real) {
-        a3[0] = ax.value(); a3[1] = ay.value(); a3[2] = az.value();
-        p3[0] = xx.value(); p3[1] = xy.value(); p3[2] = xz.value();
+        a3[0] = ax.value(); a3[1] = ay.value(); a3[2] = Z ? az.value() : 0.0;
+        p3[0] = xx.value(); p3[1] = xy.value(); p3[2] = Z ? xz.value() : 0.0;
         if (A.add_gravity) { a3[0] += A.gx; a3[1] += A.gy; a3[2] += A.gz; }
         if (A.add_velocity) {
             // exact FP64 velocity of the destination (position_funcs.pyx:47-50)
             p3[0] += ld0(A.d.u, orig);
             p3[1] += ld0(A.d.v, orig);
-            p3[2] += ld0(A.d.w, orig);
+            if (Z) p3[2] += ld0(A.d.w, orig);
         }
     }
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
+    for (int c = 0; c < (Z ? 3 : 2); ++c) {
         if (A.acc[c]) A.acc[c][orig] = (A.accumulate ? A.acc[c][orig] : 0.0) + a3[c];
         if (A.pos[c]) A.pos[c][orig] = (A.accumulate ? A.pos[c][orig] : 0.0) + p3[c];
     }
@@ -1713,17 +1717,20 @@ int batch_rates(sph_batch *b, double *const *acc, double *const *pos) {
         if (r.term.flags == (SPH_TERM_PGRAD | SPH_TERM_AVISC)) spec = 1;
         else if (r.term.flags == (SPH_TERM_PGRAD | SPH_TERM_AVISC | SPH_TERM_XSPH)) spec = 2;
     }
+    const bool z = acc[2] != nullptr || pos[2] != nullptr;
     for (const BatchGroup &grp : b->groups) {
         a.d.s0 = grp.s0;
         a.d.n = grp.s1;
         const int blocks = blocks_for(grp.s1 - grp.s0);
-#define BRL(K_) (spec == 1 ? k_rates<K_, 1, 1><<<blocks, kPairBlock, 0, b->stream>>>(a) \
-                 : spec == 2 ? k_rates<K_, 2, 1><<<blocks, kPairBlock, 0, b->stream>>>(a) \
-                             : k_rates<K_, 0, 1><<<blocks, kPairBlock, 0, b->stream>>>(a))
+#define BRL2(K_, Z_) (spec == 1 ? k_rates<K_, 1, 1, 1, Z_><<<blocks, kPairBlock, 0, b->stream>>>(a) \
+                      : k_rates<K_, 2, 1, 1, Z_><<<blocks, kPairBlock, 0, b->stream>>>(a))
+#define BRL(K_) (spec == 0 ? k_rates<K_, 0, 1><<<blocks, kPairBlock, 0, b->stream>>>(a) \
+                 : z ? BRL2(K_, true) : BRL2(K_, false))
         if (grp.K == 1) BRL(1);
         else if (grp.K == 2) BRL(2);
         else BRL(3);
 #undef BRL
+#undef BRL2
         count_launch();
         SPH_LAUNCH_CHECK("k_rates (batch)");
     }

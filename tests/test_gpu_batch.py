@@ -59,6 +59,28 @@ def test_batch_instances_vs_oracle():
         assert normwise(batch.get(k, "rho"), ref["rho"]) < TOL
 
 
+@pytest.mark.parametrize("xsph", [False, True])
+def test_batch_of_3d_instances_vs_oracle(xsph):
+    """The rates pass with its third components (a 2D batch's leaves them
+    out), with and without XSPH, over two Euler steps."""
+    _need_gpu()
+    cubes = [W.cube_lattice(n, seed=n, vel_std=0.1) for n in (1000, 2197)]
+    terms = ("pgrad", "avisc") + (("xsph",) if xsph else ())
+    batch = SimulationBatch(cubes, dim=3, dt=1e-4, co=1.0, terms=terms, alpha=0.1, eps=0.5)
+    batch.step(2)
+    ops = oracle.cube_ops()
+    if xsph:
+        ops.append(oracle.Op("xsph", "fluid", ["x", "y", "z"], ["fluid"], integrates=True, eps=0.5))
+    for k, props in enumerate(cubes):
+        prob = oracle.Problem({"fluid": props}, ops, dim=3)
+        for _ in range(2):
+            prob.integrate_euler(1e-4)
+        ref = prob.arrays["fluid"]
+        for p in ("x", "y", "z", "u", "v", "w"):
+            assert normwise(batch.get(k, p) - props[p], ref[p] - props[p]) < TOL, (k, p)
+        assert normwise(batch.get(k, "rho"), ref["rho"]) < TOL
+
+
 def test_batch_rk2_from_solvers():
     _need_gpu()
     drops = _drops(4, seed=3)
