@@ -56,20 +56,19 @@ STEP_ALG_BYTES = 694.0
 # FLOPs per neighbour pair: density 24, momentum 72 (FMA = 2)
 PAIR_FLOPS = {"RatesStage": 72.0, "DensityStage": 24.0, "ListStage": 12.0}
 FP32_NOMINAL_TFLOPS = 152 * 128 * 2 * 2.07e9 / 1e12
-# DRAM bytes per particle per launch (dram__bytes_read.sum + dram__bytes_write.sum
-# of one ncu capture of the 1M-particle lattice, brick-staged passes at cell
+# DRAM bytes per particle per launch (from the DRAM throughput and duration of
+# one ncu capture of the 1M-particle lattice, brick-staged passes at cell
 # subdivision 2); the traffic grows with the particle count, so it is scaled
 # by n
-NCU_TRAFFIC_PER_PARTICLE = {"DensityStage": 222.3, "RatesStage": 286.1}
+NCU_TRAFFIC_PER_PARTICLE = {"DensityStage": 270.0, "RatesStage": 335.0}
 # The unit that bounds each pair kernel in the same capture, as a fraction of
-# that unit's peak: the rates pass is bound by the L1 / shared-memory pipe
-# that serves its staged-record reads (and their latency), the density pass
-# by instruction issue
+# that unit's peak: the L1 / shared-memory pipe that serves the staged-record
+# reads, with instruction issue behind it
 NCU_LIMITER = {
-    "RatesStage": {"kernel": "k_brates", "unit": "L1 / shared-memory pipe", "frac": 0.702,
-                   "issue_frac": 0.618, "dram_frac": 0.141},
-    "DensityStage": {"kernel": "k_bdensity", "unit": "instruction issue", "frac": 0.646,
-                     "l1_frac": 0.603, "dram_frac": 0.179},
+    "RatesStage": {"kernel": "k_brates", "unit": "L1 / shared-memory pipe", "frac": 0.783,
+                   "issue_frac": 0.601, "dram_frac": 0.197},
+    "DensityStage": {"kernel": "k_bdensity", "unit": "L1 / shared-memory pipe", "frac": 0.702,
+                     "issue_frac": 0.590, "dram_frac": 0.283},
 }
 
 
@@ -557,8 +556,8 @@ def run_gpu(args):
                      "traffic_source": "ncu capture at 1M particles, scaled by n",
                      "peak_kind": peak_kind,
                      "alg_bytes_per_particle": ALG_BYTES[dom],
-                     "note": "brick-staged pair kernels bound by issue (density) and the "
-                             "L1 / shared-memory pipe (rates: staged-record reads), not HBM; "
+                     "note": "brick-staged pair kernels bound by the L1 / shared-memory "
+                             "pipe (staged-record reads) and by issue, not HBM; "
                              "fp32 context in fp32_context",
                      "limiter": dict(NCU_LIMITER.get(dom, {}),
                                      source="ncu --set full capture at 1M particles")},
