@@ -52,7 +52,7 @@ constexpr int OFF_W1 = SPH_MLP_OFF_W1, OFF_B1 = SPH_MLP_OFF_B1, OFF_W2 = SPH_MLP
 constexpr int TILE = 128;
 constexpr int THREADS = 256;   // two warps per tensor-memory lane quarter
 constexpr int L3_PART = NOUT * NH + NOUT;   // third-layer partial per block
-constexpr int L3_ROWS = 64;                 // rows per third-layer tile
+constexpr int L3_ROWS = 1024;               // rows per third-layer block
 constexpr int L3_THREADS = 256;
 constexpr int kMaxSpin = 1 << 22;           // bounded mbarrier wait
 // per-CTA partial gradients of the backward: rows of PART_STRIDE floats
@@ -1558,106 +1558,99 @@ __global__ void __launch_bounds__(R_THREADS, 1)
 
 // third layer: dW3 [o][j] = sum_b dy[b][o] h2[b][j], db3 = sum_b dy
 //
-// HBM-bound: 264 B per sample (h2 as BF16, dy), 4 FLOP per h2 value.  A
-// half-warp reads one row of h2 as sixteen 16-byte loads, so a block has
-// sixteen rows in flight per step (four steps unrolled), and every thread
-// keeps the 2 x 8 sums of its columns; the sixteen row groups are added in a
-// fixed order at the end.  Blocks take tiles of L3_ROWS rows round-robin, so
-// a minibatch of 8 192 spreads over 128 blocks.  (One thread per column and
-// 1 024 rows per block left a minibatch on 8 blocks, each a serial chain of
-// two-byte loads: 177 us against 5.4 us at 8 192 samples, cold cache.)
-// A caller's h2 off the 16-byte grid is read value by value (ALIGNED = false).
+// A thread adds one (o, j) over the rows of its block in their order (one FMA
+// chain: the order is part of the result, a training run feels its last bits
+// through the BF16 weights).  The block brings the rows in tiles of L3_TILE as
+// 16-byte loads, the next tile's on their way while this one is added.  (The
+// same chain on two-byte loads from global memory, 128 threads: 177 us at
+// 8 192 samples, cold cache, against 17; row groups added separately took 5.4,
+// in another order.)  A caller's h2 off the 16-byte grid is read value
+// by value (ALIGNED = false).
+constexpr int L3_TILE = 64;
 template <bool ALIGNED>
 __global__ void __launch_bounds__(L3_THREADS)
 k_mlp_l3(const uint16_t *__restrict__ h2s, const float2 *__restrict__ dy, int64_t n,
          float *__restrict__ part) {
-    constexpr int GROUPS = L3_THREADS / 16;      // rows per step
-    constexpr int STEPS = L3_ROWS / GROUPS;
-    __shared__ float s_a[GROUPS][NOUT * NH + 4];
-    __shared__ float2 s_d[GROUPS];
-    const int c = threadIdx.x & 15;              // columns 8 c .. 8 c + 7
-    const int r = threadIdx.x >> 4;
-    float a0[8], a1[8];
-    float2 sd = make_float2(0.f, 0.f);
+    constexpr int CH = L3_TILE * (NH / 8) / L3_THREADS;     // 16-byte pieces per thread
+    __shared__ uint4 s_h[2][L3_TILE * NH / 8];
+    __shared__ float2 s_d[2][L3_TILE];
+    const int t = threadIdx.x, j = t % NH, o = t / NH;
+    const int64_t r0 = (int64_t)blockIdx.x * L3_ROWS;
+    const int rows = (int)min((int64_t)L3_ROWS, n - r0);
+    uint4 h[CH];
+    float2 d = make_float2(0.f, 0.f);
+    auto fetch = [&](int first) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) a0[i] = a1[i] = 0.f;
-    for (int64_t t = blockIdx.x; t * L3_ROWS < n; t += gridDim.x) {
-#pragma unroll
-        for (int st = 0; st < STEPS; ++st) {
-            const int64_t b = t * L3_ROWS + st * GROUPS + r;
-            if (b < n) {
-                const uint16_t *row = h2s + b * NH + 8 * c;
+        for (int k = 0; k < CH; ++k) {
+            const int piece = t + k * L3_THREADS, r = first + piece / (NH / 8);
+            h[k] = make_uint4(0, 0, 0, 0);
+            if (r >= rows) continue;
+            const uint16_t *src = h2s + (r0 + r) * NH + 8 * (piece % (NH / 8));
+            if (ALIGNED) {
+                h[k] = __ldg(reinterpret_cast<const uint4 *>(src));
+            } else {
                 uint32_t w[4];
-                if (ALIGNED) {
-                    const uint4 h = __ldg(reinterpret_cast<const uint4 *>(row));
-                    w[0] = h.x; w[1] = h.y; w[2] = h.z; w[3] = h.w;
-                } else {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        w[i] = (uint32_t)row[2 * i] | ((uint32_t)row[2 * i + 1] << 16);
-                }
-                const float2 d = __ldg(dy + b);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float lo = bf_lo(w[i]), hi = bf_hi(w[i]);
-                    a0[2 * i] = fmaf(d.x, lo, a0[2 * i]);
-                    a0[2 * i + 1] = fmaf(d.x, hi, a0[2 * i + 1]);
-                    a1[2 * i] = fmaf(d.y, lo, a1[2 * i]);
-                    a1[2 * i + 1] = fmaf(d.y, hi, a1[2 * i + 1]);
-                }
-                sd.x += d.x;
-                sd.y += d.y;
+                for (int i = 0; i < 4; ++i)
+                    w[i] = (uint32_t)src[2 * i] | ((uint32_t)src[2 * i + 1] << 16);
+                h[k] = make_uint4(w[0], w[1], w[2], w[3]);
             }
         }
-    }
+        if (t < L3_TILE && first + t < rows) d = __ldg(dy + r0 + first + t);
+    };
+    float a = 0.f, sum = 0.f;
+    fetch(0);
+    for (int first = 0, p = 0; first < rows; first += L3_TILE, p ^= 1) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        s_a[r][8 * c + i] = a0[i];
-        s_a[r][NH + 8 * c + i] = a1[i];
+        for (int k = 0; k < CH; ++k) s_h[p][t + k * L3_THREADS] = h[k];
+        if (t < L3_TILE) s_d[p][t] = d;
+        __syncthreads();    // (the other buffer is free: all passed the last one)
+        if (first + L3_TILE < rows) fetch(first + L3_TILE);
+        const uint16_t *col = reinterpret_cast<const uint16_t *>(s_h[p]) + j;
+        const float *dv = reinterpret_cast<const float *>(s_d[p]) + o;
+        const int m = min(L3_TILE, rows - first);
+#pragma unroll 16
+        for (int r = 0; r < m; ++r) {
+            const float w = dv[2 * r];
+            a = fmaf(w, __uint_as_float((uint32_t)col[r * NH] << 16), a);
+            sum += w;
+        }
     }
-    if (c == 0) s_d[r] = sd;
-    __syncthreads();
     float *P = part + (int64_t)blockIdx.x * L3_PART;
-    for (int j = threadIdx.x; j < L3_PART; j += L3_THREADS) {
-        float v = 0.f;
-#pragma unroll
-        for (int q = 0; q < GROUPS; ++q)
-            v += j < NOUT * NH ? s_a[q][j] : (j == NOUT * NH ? s_d[q].x : s_d[q].y);
-        P[j] = v;
-    }
+    P[o * NH + j] = a;
+    if (j == 0) P[NOUT * NH + o] = sum;
 }
 
-// grad[p] = sum over CTAs (fixed order) of the partials: four threads per
-// parameter take every fourth partial (a chain of loads a quarter as long),
-// their sums added in a fixed order.
-constexpr int RED_PARAMS = 64;       // parameters per block of 256 threads
-__global__ void __launch_bounds__(4 * RED_PARAMS)
+// grad[p] = sum over CTAs of the partials in their order (sixteen loads on
+// their way at a time)
+__global__ void __launch_bounds__(128)
 k_mlp_reduce(const float *__restrict__ part, int nparts, const float *__restrict__ l3, int nl3,
              const float *__restrict__ part_loss, float *__restrict__ grad,
              float *__restrict__ loss) {
-    __shared__ float s_s[4][RED_PARAMS];
-    const int k = threadIdx.x % RED_PARAMS, q = threadIdx.x / RED_PARAMS;
-    const int p = blockIdx.x * RED_PARAMS + k;
-    const float *src = nullptr;
-    int64_t stride = 0;
-    int count = 0;
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    const float *src;
+    int64_t stride;
+    int count;
     if (p < OFF_W3) {
         src = part + p; stride = PART_STRIDE; count = nparts;
     } else if (p < NPARAM) {
         src = l3 + (p - OFF_W3); stride = L3_PART; count = nl3;
-    } else if (p == NPARAM) {
+    } else if (p == NPARAM && loss) {
         src = part_loss; stride = 1; count = nparts;
+    } else {
+        return;
     }
     float s = 0.f;
-#pragma unroll 8
-    for (int c = q; c < count; c += 4) s += __ldg(src + c * stride);
-    s_s[q][k] = s;
-    __syncthreads();
-    if (q == 0) {
-        const float v = ((s_s[0][k] + s_s[1][k]) + s_s[2][k]) + s_s[3][k];
-        if (p < NPARAM) grad[p] = v;
-        else if (p == NPARAM && loss) *loss = v;
+    for (int c0 = 0; c0 < count; c0 += 16) {
+        float v[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v[k] = c0 + k < count ? __ldg(src + (c0 + k) * stride) : 0.f;
+#pragma unroll
+        for (int k = 0; k < 16; ++k)
+            if (c0 + k < count) s += v[k];
     }
+    if (p < NPARAM) grad[p] = s;
+    else *loss = s;
 }
 
 __device__ __forceinline__ void write_copies(const MlpDev &W, uint16_t *w1, uint16_t *w2,
@@ -1835,12 +1828,9 @@ int mlp_grid(int64_t n) {
     return (int)std::max<int64_t>(1, std::min<int64_t>(tiles, g_num_sms));
 }
 
-// third-layer blocks: one per tile of rows, at most four per SM (a million
-// samples keep 32 warps of loads in flight per SM, and the partials that
-// k_mlp_reduce adds stay few)
+// third-layer blocks
 static int l3_blocks(int64_t n) {
-    const int64_t tiles = (n + L3_ROWS - 1) / L3_ROWS;
-    return (int)std::max<int64_t>(1, std::min<int64_t>(tiles, 4 * (int64_t)g_num_sms));
+    return (int)std::max<int64_t>(1, (n + L3_ROWS - 1) / L3_ROWS);
 }
 
 int64_t mlp_backward_scratch(int64_t n) {
@@ -1919,7 +1909,7 @@ int mlp_backward(const sph_mlp_model *M, const uint16_t *x, const uint16_t *h1, 
         k_mlp_l3<false><<<nl3, L3_THREADS, 0, st>>>(h2, reinterpret_cast<const float2 *>(dy), n, l3);
     count_launch();
     SPH_LAUNCH_CHECK("k_mlp_l3");
-    k_mlp_reduce<<<(NPARAM + RED_PARAMS) / RED_PARAMS, 4 * RED_PARAMS, 0, st>>>(part, grid, l3, nl3, part_loss, grad, loss);
+    k_mlp_reduce<<<(NPARAM + 128) / 128, 128, 0, st>>>(part, grid, l3, nl3, part_loss, grad, loss);
     count_launch();
     SPH_LAUNCH_CHECK("k_mlp_reduce");
     return SPH_OK;
