@@ -1411,6 +1411,7 @@ __global__ void __launch_bounds__(128) k_brick_count(Grid g, BrickGeom bk, const
     }
 }
 
+// bstage null: an array that no pass stages (brick_fill) gets its destinations only
 __global__ void __launch_bounds__(128) k_brick_fill(Grid g, BrickGeom bk, const int *cstart,
                                                     const float *scx, const int4 *bsrc,
                                                     const int2 *brow, const int2 *bdst,
@@ -1421,9 +1422,10 @@ __global__ void __launch_bounds__(128) k_brick_fill(Grid g, BrickGeom bk, const 
     const BlockGeo G = block_geo(g, bk, b);
     const int2 *rows = brow + (int64_t)b * bk.nrmax;
     int2 *stab = bstage + bsrc[b].y;
+    const int nr = bstage != nullptr ? G.nr : 0;
     // a warp takes a row of cells at a time, its slots over the lanes
 #pragma unroll 4
-    for (int r = wid; r < G.nr; r += nw) {
+    for (int r = wid; r < nr; r += nw) {
         const int2 e = rows[r];
         const int c = pack_cell(-128, G.ys0 + r % G.ry - G.cyc, G.zs0 + r / G.ry - G.czc) -
                       G.cxc + 128;
@@ -1663,24 +1665,29 @@ int brick_count(sph_ctx *ctx, int a, unsigned *stats) {
     return SPH_OK;
 }
 
+// The destinations are filled for every array: a pass over another, sparser
+// source takes this array's blocks however populous they are.  The sources
+// only where the array can be staged (the fields of brow hold 16 bits each).
 int brick_fill(sph_ctx *ctx, int a) {
     ArraySnap &A = ctx->arrays[a];
     const BrickGeom &bk = ctx->bricks;
+    const bool source = A.b_tmax < 65535;
     if (A.n > A.bdest_cap || !A.bdest) {
         cudaFree(A.bdest);
         A.bdest = nullptr;
         SPH_CUDA(cudaMalloc(&A.bdest, sizeof(int2) * A.n));
         A.bdest_cap = A.n;
     }
-    if (A.b_staged > A.bstage_cap || !A.bstage) {
+    if (source && (A.b_staged > A.bstage_cap || !A.bstage)) {
         cudaFree(A.bstage);
         A.bstage = nullptr;
         const int64_t want = A.b_staged + A.b_staged / 8;   // the next builds' too
         SPH_CUDA(cudaMalloc(&A.bstage, sizeof(int2) * std::max<int64_t>(want, 1)));
         A.bstage_cap = want;
     }
-    k_brick_fill<<<(unsigned)bk.nbricks, 128, 0, ctx->stream>>>(ctx->grid, bk, A.cstart, A.scx, A.bsrc, A.brow,
-                                                 A.bdst, A.bstage, A.bdest);
+    k_brick_fill<<<(unsigned)bk.nbricks, 128, 0, ctx->stream>>>(
+        ctx->grid, bk, A.cstart, A.scx, A.bsrc, A.brow, A.bdst, source ? A.bstage : nullptr,
+        A.bdest);
     count_launch();
     SPH_LAUNCH_CHECK("k_brick_fill");
     return SPH_OK;

@@ -306,3 +306,47 @@ def test_four_list_lanes_give_the_same_bits(cap):
         assert r.returncode == 0, r.stderr[-3000:]
         seen.add(r.stdout.split()[-1])
     assert len(seen) == 1
+
+
+@pytest.mark.parametrize("n", [65534, 65535, 70001])
+def test_crowded_destination_with_a_sparse_source(n, monkeypatch):
+    """Sample points so many that no block could stage them (65 535 and more
+    around one brick) among the particles of another, sparse array: their
+    blocks' destinations are those of the build, first and after a move that
+    crowds them.  Density and momentum rates against the oracle."""
+    _need_gpu()
+    monkeypatch.setenv("PYSPH_GB300_BRICKS", "1")
+    base, sph = API.base, API.sph
+    rng = np.random.default_rng(n)
+    h, m = 0.05, 400
+
+    def state(k, x, y):
+        return dict(x=x, y=y, u=rng.normal(0, 1, k), v=rng.normal(0, 1, k),
+                    m=rng.uniform(0.5, 1.5, k), h=np.full(k, h), rho=rng.uniform(1.0, 2.0, k),
+                    p=rng.uniform(1.0, 2.0, k), cs=rng.uniform(1.0, 2.0, k), ax=np.zeros(k),
+                    ay=np.zeros(k))
+
+    sp = state(m, rng.uniform(0, 0.3, m), rng.uniform(0, 0.3, m))
+    dp = state(n, rng.uniform(0, 4.0, n), rng.uniform(0, 4.0, n))
+    src = base.get_particle_array(name="fluid", **sp)
+    dst = base.get_particle_array(name="samples", **dp)
+    particles = base.Particles(arrays=[src, dst])
+    cm = particles.cell_manager
+    kern = base.CubicSplineKernel(dim=2)
+    for crowded in (False, True):
+        if crowded:
+            dp["x"], dp["y"] = 0.075 * dp["x"], 0.075 * dp["y"]
+            dst.set(x=dp["x"], y=dp["y"])
+            cm.rebuild(check_jump=False)
+        passes = cm.brick_pass_count()
+        sph.SPHCalc(particles, [src], dst, kern, [sph.SPHRho.get_func(src, dst)], ["rho"]).sph("rho")
+        got = dst.get("rho")
+        dst.set(rho=dp["rho"])
+        mom = sph.MomentumEquation.withargs(alpha=0.5, beta=0.5, dim=2)
+        sph.SPHCalc(particles, [src], dst, kern, [mom.get_func(src, dst)], ["ax", "ay"]).sph("ax", "ay")
+        assert cm.brick_pass_count() == passes + 2
+        off, idx = oracle.neighbors(dp, sp, 2.0 * h)
+        assert normwise(got, oracle.pair_sum("rho", dp, sp, off, idx, 2, nout=1)[0]) < TOL
+        ax, ay = oracle.pair_sum("momentum", dp, sp, off, idx, 2,
+                                 dict(alpha=0.5, beta=0.5, eta=0.1), nout=2)[:2]
+        assert normwise(dst.get("ax"), ax) < TOL and normwise(dst.get("ay"), ay) < TOL
