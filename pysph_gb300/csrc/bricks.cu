@@ -36,7 +36,10 @@
 // S = 2 or 4 neighbouring threads (lanes) share a destination, lane s takes
 // the list's groups s, s + S, ..., and the groups' sums are folded in the
 // list's order (shuffles), so the result is the same bit for bit; the bricks
-// are divided into parts (blocks of their own, with the brick's origin).
+// are divided into parts (blocks of their own, with the brick's origin).  (Two
+// source masses: whether a block reads two records per pair or three is its
+// own matter, and a part may hold one mass where its brick holds two; the last
+// bit of the viscosity's sound speed then differs.)
 //
 // The neighbour relation is the reference's: strict r^2 < (radius_scale
 // h)^2, decided in FP32 outside a +-1e-5 relative band around the threshold
@@ -203,6 +206,48 @@ __device__ __forceinline__ float cell_float(int code) {
     return __uint_as_float(__byte_perm((unsigned)code, 0x4B000000u, 0x7540u | C)) - 8388736.f;
 }
 
+// bstage entry t of the calling block, from its rows
+__device__ __noinline__ int2 row_entry(const Grid &g, const BrickGeom &bk, const BrickSrcDev &S,
+                                       int t) {
+    const BlockGeo G = block_geo(g, bk, blockIdx.x);
+    const int2 *rows = S.brow + (size_t)blockIdx.x * bk.nrmax;
+    int r = 0;      // the last row that starts at or before t: the one that holds it
+    for (int hi = G.nr - 1; r < hi;) {
+        const int mid = (r + hi + 1) >> 1;
+        if (row_off(rows[mid]) <= t) r = mid;
+        else hi = mid - 1;
+    }
+    const int j = rows[r].x + (t - row_off(rows[r]));
+    return make_int2(j, pack_cell((int)S.scx[j] - G.cxc, G.ys0 + r % G.ry - G.cyc,
+                                  G.zs0 + r / G.ry - G.czc));
+}
+
+// The entries of the calling block's staged records: its part of bstage, or
+// (TABLE = false: a build without that table, see brick_fill) found from the
+// rows of cells that they come from.
+template <bool TABLE>
+struct StageTab;
+
+template <>
+struct StageTab<true> {
+    const int2 *tab;
+    __device__ __forceinline__ const int2 &operator[](int t) const { return tab[t]; }
+};
+
+template <>
+struct StageTab<false> {
+    const Grid *g;
+    const BrickGeom *bk;
+    const BrickSrcDev *S;
+    __device__ __forceinline__ int2 operator[](int t) const { return row_entry(*g, *bk, *S, t); }
+};
+
+template <bool TABLE, class Args>
+__device__ __forceinline__ StageTab<TABLE> stage_tab(const Args &A, const int4 &sh) {
+    if constexpr (TABLE) return StageTab<true>{A.s.bstage + sh.y};
+    else return StageTab<false>{&A.g, &A.bk, &A.s};
+}
+
 // Position record (brick-relative x, y, z and the mass) of record p in the
 // cell of a table entry: the same FP32 operations for destinations and
 // sources.
@@ -227,7 +272,7 @@ __device__ __forceinline__ float2 pad_rstate() { return make_float2(0.f, 0.f); }
 // Source records: staged in shared memory, or (STAGED = false, a brick
 // more populous than the shared memory holds) recomputed from the sorted
 // arrays with the same operations.
-template <bool STAGED>
+template <bool STAGED, bool TABLE>
 struct SrcRecords;
 
 // Staged: the position record of source t at byte 16 t of the shared
@@ -240,8 +285,8 @@ struct SrcRecords;
 // A rates pass whose block has one source mass and whose cs follows Tait
 // (FAST) reads the first two only: the state record's 8-byte read was a
 // fifth of the shared-memory wavefronts of a pair.
-template <>
-struct SrcRecords<true> {
+template <bool TABLE>
+struct SrcRecords<true, TABLE> {
     uint32_t voff, soff;
     __device__ __forceinline__ float4 pos(int t) const {
         return *reinterpret_cast<const float4 *>(brick_smem + ((uint32_t)t << 4));
@@ -265,10 +310,10 @@ struct SrcRecords<true> {
 };
 
 // recomputed from the sorted arrays with the staging's operations
-template <>
-struct SrcRecords<false> {
+template <bool TABLE>
+struct SrcRecords<false, TABLE> {
     const BrickSrcDev *src;
-    const int2 *tab;
+    StageTab<TABLE> tab;
     float csf;
     int T;
     float halpha;
@@ -298,14 +343,15 @@ struct SrcRecords<false> {
     }
 };
 
-template <bool STAGED>
-__device__ __forceinline__ SrcRecords<STAGED> make_records(const BrickSmem &sm, const BrickSrcDev &S,
-                                                           float csf, const int2 *tab, int T,
-                                                           float halpha) {
+template <bool STAGED, bool TABLE>
+__device__ __forceinline__ SrcRecords<STAGED, TABLE> make_records(const BrickSmem &sm,
+                                                                  const BrickSrcDev &S, float csf,
+                                                                  const StageTab<TABLE> &tab, int T,
+                                                                  float halpha) {
     if constexpr (STAGED)
-        return SrcRecords<true>{(uint32_t)sm.off_v, (uint32_t)sm.off_s};
+        return SrcRecords<true, TABLE>{(uint32_t)sm.off_v, (uint32_t)sm.off_s};
     else
-        return SrcRecords<false>{&S, tab, csf, T, halpha};
+        return SrcRecords<false, TABLE>{&S, tab, csf, T, halpha};
 }
 
 // Asynchronous copies from global to shared memory (completed by the issuing
@@ -320,6 +366,39 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
+// The records of stage, row by row (a build without the table of entries).
+template <bool RATES>
+__device__ __forceinline__ bool stage_rows(const StageTab<false> &tab, float csf,
+                                           const BrickSmem &sm, bool state, float halpha,
+                                           float mref) {
+    const BrickSrcDev &S = *tab.S;
+    const BlockGeo G = block_geo(*tab.g, *tab.bk, blockIdx.x);
+    const int2 *rows = S.brow + (size_t)blockIdx.x * tab.bk->nrmax;
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    bool same = true;
+    for (int r = threadIdx.x >> 5; r < G.nr; r += nw) {
+        const int2 e = rows[r];
+        const int cy = G.ys0 + r % G.ry - G.cyc, cz = G.zs0 + r / G.ry - G.czc;
+        for (int i = lane; i < row_len(e); i += 32) {
+            const int j = e.x + i;
+            const uint32_t t = (uint32_t)(row_off(e) + i);
+            float4 pr = rel_pos(S.pm[j], pack_cell((int)S.scx[j] - G.cxc, cy, cz), csf);
+            if (RATES) {
+                const float4 vh = S.velh[j], st = S.st[j];
+                same = same && pr.w == mref;
+                *reinterpret_cast<float4 *>(brick_smem + sm.off_v + (t << 4)) =
+                    make_float4(vh.x, vh.y, vh.z, st.y);
+                if (state)
+                    *reinterpret_cast<float2 *>(brick_smem + sm.off_s + (t << 3)) =
+                        make_float2(pr.w, halpha * st.z);
+                pr.w = 0.5f * st.x;
+            }
+            *reinterpret_cast<float4 *>(brick_smem + (t << 4)) = pr;
+        }
+    }
+    return same;
+}
+
 // Copy the block's source records into shared memory (the layout of
 // SrcRecords<true>).  The raw records (position; rates: velocity, rho and
 // p / rho^2) are copied asynchronously, so that a thread has all its copies in
@@ -328,9 +407,10 @@ __device__ __forceinline__ void cp_async_wait() {
 // pass (x, y, z, rho / 2), (u, v, w, p / rho^2) and, with STATE, (m, alpha cs /
 // 2), with the halves that the pair averages of the artificial viscosity add.
 // Returns whether every record this thread staged has mass mref.
-template <bool RATES>
-__device__ __forceinline__ bool stage(const BrickSrcDev &S, const int2 *tab, int T, float csf,
-                                      const BrickSmem &sm, bool state, float halpha, float mref) {
+template <bool RATES, bool TABLE>
+__device__ __forceinline__ bool stage(const BrickSrcDev &S, const StageTab<TABLE> &tab, int T,
+                                      float csf, const BrickSmem &sm, bool state, float halpha,
+                                      float mref) {
     constexpr int U = 6;        // records of a thread in flight
     const uint32_t base = (uint32_t)__cvta_generic_to_shared(brick_smem);
     const uint32_t vb = base + sm.off_v, sb = base + sm.off_s;
@@ -343,6 +423,7 @@ __device__ __forceinline__ bool stage(const BrickSrcDev &S, const int2 *tab, int
             *reinterpret_cast<float2 *>(brick_smem + sm.off_s + ((uint32_t)T << 3)) = pad_rstate();
         }
     }
+    if constexpr (!TABLE) return stage_rows<RATES>(tab, csf, sm, state, halpha, mref);
     bool same = true;
     for (int t0 = threadIdx.x; t0 < T; t0 += U * nt) {
         int2 e[U];
@@ -384,8 +465,9 @@ __device__ __forceinline__ bool stage(const BrickSrcDev &S, const int2 *tab, int
 
 // The state records (m, alpha cs / 2) of a block whose sources turned out not
 // to share one mass.
-__device__ __noinline__ void stage_state(const BrickSrcDev &S, const int2 *tab, int T, uint32_t soff,
-                                         float halpha) {
+template <bool TABLE>
+__device__ __noinline__ void stage_state(const BrickSrcDev &S, StageTab<TABLE> tab, int T,
+                                         uint32_t soff, float halpha) {
     for (int t = threadIdx.x; t < T; t += blockDim.x) {
         const int j = tab[t].x;
         *reinterpret_cast<float2 *>(brick_smem + soff + ((uint32_t)t << 3)) =
@@ -457,11 +539,11 @@ __device__ __noinline__ bool exact_hit(const BrickSrcDev &S, const BrickDstDev &
 // 218 us, 195 by masks.)  With a list skin every source within the list radius is listed,
 // without one the neighbours.  The ranges come from the block's cell table
 // (scell) or, without one, from the grid's cell table.
-template <bool SKIN, bool STAGED, class Fn>
+template <bool SKIN, bool STAGED, bool TABLE, class Fn>
 __device__ __forceinline__ void brick_rows(const Grid &g, const BlockGeo &G, const BrickSrcDev &S,
-                                               const BrickDstDev &D, const SrcRecords<STAGED> &R,
+                                               const BrickDstDev &D, const SrcRecords<STAGED, TABLE> &R,
                                                const BrickRadius &rad, const int2 *brow,
-                                               const int2 *tab, const int *scell,
+                                               const StageTab<TABLE> &tab, const int *scell,
                                                const BrickDest &q, int r0, int r1,
                                                Fn &&fn) {
     const float csf = g.cs_f;
@@ -531,15 +613,15 @@ __device__ __forceinline__ void brick_rows(const Grid &g, const BlockGeo &G, con
     }
 }
 
-template <bool STAGED, class Fn>
+template <bool STAGED, bool TABLE, class Fn>
 __device__ __forceinline__ void brick_traverse(const Grid &g, const BlockGeo &G, const BrickSrcDev &S,
-                                               const BrickDstDev &D, const SrcRecords<STAGED> &R,
+                                               const BrickDstDev &D, const SrcRecords<STAGED, TABLE> &R,
                                                const BrickRadius &rad, const int2 *brow,
-                                               const int2 *tab, const int *scell,
+                                               const StageTab<TABLE> &tab, const int *scell,
                                                const BrickDest &q, int r0, int r1,
                                                Fn &&fn) {
-    if (rad.r2list > 0.f) brick_rows<true, STAGED>(g, G, S, D, R, rad, brow, tab, scell, q, r0, r1, fn);
-    else brick_rows<false, STAGED>(g, G, S, D, R, rad, brow, tab, scell, q, r0, r1, fn);
+    if (rad.r2list > 0.f) brick_rows<true, STAGED, TABLE>(g, G, S, D, R, rad, brow, tab, scell, q, r0, r1, fn);
+    else brick_rows<false, STAGED, TABLE>(g, G, S, D, R, rad, brow, tab, scell, q, r0, r1, fn);
 }
 
 // Reciprocal square root and reciprocal, flushing subnormal inputs to zero
@@ -667,8 +749,8 @@ __device__ __forceinline__ void dest_prefetch(const BrickDstDev &Dd, float csf, 
 // taking every S-th group, each requested two ahead into one of three
 // rotating buffers (the loop is unrolled over the three, so no buffer is
 // copied).
-template <int S, bool STAGED>
-__device__ __forceinline__ void density_group(CSum &rho, const SrcRecords<STAGED> &R, bool mine,
+template <int S, bool STAGED, bool TABLE>
+__device__ __forceinline__ void density_group(CSum &rho, const SrcRecords<STAGED, TABLE> &R, bool mine,
                                               const uint4 &grp, const float4 &Pi, float ih,
                                               const WCoef &wc, unsigned mask) {
     float part = 0.f;
@@ -685,8 +767,8 @@ __device__ __forceinline__ void density_group(CSum &rho, const SrcRecords<STAGED
     fold_lanes<S>(rho, part, mask);
 }
 
-template <int S, bool STAGED>
-__device__ __forceinline__ void density_stream(CSum &rho, const SrcRecords<STAGED> &R,
+template <int S, bool STAGED, bool TABLE>
+__device__ __forceinline__ void density_stream(CSum &rho, const SrcRecords<STAGED, TABLE> &R,
                                                const uint4 *lst, int D, int ng, int lane,
                                                const float4 &Pi, float ih, const WCoef &wc, uint4 b0,
                                                uint4 b1, unsigned mask) {
@@ -699,15 +781,15 @@ __device__ __forceinline__ void density_stream(CSum &rho, const SrcRecords<STAGE
     for (int g0 = 0, gi = lane;;) {
         if (g0 >= nr) break;
         b2 = gi + 2 * S < ng ? lst[(gi + 2 * S) * step] : zero;
-        density_group<S, STAGED>(rho, R, gi < ng, b0, Pi, ih, wc, mask);
+        density_group<S, STAGED, TABLE>(rho, R, gi < ng, b0, Pi, ih, wc, mask);
         gi += S;
         if ((g0 += S) >= nr) break;
         b0 = gi + 2 * S < ng ? lst[(gi + 2 * S) * step] : zero;
-        density_group<S, STAGED>(rho, R, gi < ng, b1, Pi, ih, wc, mask);
+        density_group<S, STAGED, TABLE>(rho, R, gi < ng, b1, Pi, ih, wc, mask);
         gi += S;
         if ((g0 += S) >= nr) break;
         b1 = gi + 2 * S < ng ? lst[(gi + 2 * S) * step] : zero;
-        density_group<S, STAGED>(rho, R, gi < ng, b2, Pi, ih, wc, mask);
+        density_group<S, STAGED, TABLE>(rho, R, gi < ng, b2, Pi, ih, wc, mask);
         gi += S;
         g0 += S;
     }
@@ -719,10 +801,11 @@ __device__ __forceinline__ void density_stream(CSum &rho, const SrcRecords<STAGE
 // store per group.  Several: each counts its share, a scan over the lanes
 // gives its place in the list, and a second traversal writes the entries.
 // The last group is padded with the zero record.  Returns the list's count.
-template <int S, bool STAGED>
+template <int S, bool STAGED, bool TABLE>
 __device__ __forceinline__ int build_list(const BrickDensityArgs &A, const BlockGeo &G,
-                                          const SrcRecords<STAGED> &R, const int2 *brow,
-                                          const int2 *tab, const int *scell, const BrickDest &q, bool active,
+                                          const SrcRecords<STAGED, TABLE> &R, const int2 *brow,
+                                          const StageTab<TABLE> &tab, const int *scell,
+                                          const BrickDest &q, bool active,
                                           int lane, int T, uint4 *out, int D) {
     const int cap = A.cap;
     const int rows = (2 * A.g.ky + 1) * (2 * A.g.kz + 1);
@@ -736,7 +819,7 @@ __device__ __forceinline__ int build_list(const BrickDensityArgs &A, const Block
             grp.z = __funnelshift_r(grp.z, grp.w, 16);
             grp.w = (grp.w >> 16) | (t << 16);
         };
-        brick_traverse<STAGED>(A.g, G, A.s, A.d, R, A.rad, brow, tab, scell, q, 0, rows,
+        brick_traverse<STAGED, TABLE>(A.g, G, A.s, A.d, R, A.rad, brow, tab, scell, q, 0, rows,
             [&](int t0, unsigned m) {
                 for (; m; m &= m - 1) {
                     push((unsigned)(t0 + __ffs(m) - 1));
@@ -752,7 +835,7 @@ __device__ __forceinline__ int build_list(const BrickDensityArgs &A, const Block
     }
     const int ra = rows * lane / S, rb = rows * (lane + 1) / S;
     if (active)
-        brick_traverse<STAGED>(A.g, G, A.s, A.d, R, A.rad, brow, tab, scell, q, ra, rb,
+        brick_traverse<STAGED, TABLE>(A.g, G, A.s, A.d, R, A.rad, brow, tab, scell, q, ra, rb,
                                [&](int, unsigned m) { c += __popc(m); });
     __syncwarp();
     int end = c;
@@ -769,7 +852,7 @@ __device__ __forceinline__ int build_list(const BrickDensityArgs &A, const Block
             if (k < cap) o16[(size_t)(k >> 3) * D * 8 + (k & 7)] = (uint16_t)t;
             ++k;
         };
-        brick_traverse<STAGED>(A.g, G, A.s, A.d, R, A.rad, brow, tab, scell, q, ra, rb,
+        brick_traverse<STAGED, TABLE>(A.g, G, A.s, A.d, R, A.rad, brow, tab, scell, q, ra, rb,
                                [&](int t0, unsigned m) {
                                    for (; m; m &= m - 1) write((unsigned)(t0 + __ffs(m) - 1));
                                });
@@ -785,10 +868,11 @@ __device__ __forceinline__ int build_list(const BrickDensityArgs &A, const Block
 // The density sum of a list build: plain FP32 batches of 8 neighbours (the
 // listed sources that the skin adds do not count), each folded into the
 // compensated sum; past the list's capacity the traversal goes on.
-template <bool STAGED>
+template <bool STAGED, bool TABLE>
 __device__ __forceinline__ void build_sum(const BrickDensityArgs &A, const BlockGeo &G,
-                                          const SrcRecords<STAGED> &R, const int2 *brow,
-                                          const int2 *tab, const int *scell, const BrickDest &q, int c,
+                                          const SrcRecords<STAGED, TABLE> &R, const int2 *brow,
+                                          const StageTab<TABLE> &tab, const int *scell,
+                                          const BrickDest &q, int c,
                                           const uint4 *lst, int D, float ih, const WCoef &wc,
                                           CSum &rho) {
     const int cap = A.cap;
@@ -839,7 +923,7 @@ __device__ __forceinline__ void build_sum(const BrickDensityArgs &A, const Block
     if (c > cap) {
         int skip = cap;
         const int rows = (2 * A.g.ky + 1) * (2 * A.g.kz + 1);
-        brick_traverse<STAGED>(A.g, G, A.s, A.d, R, A.rad, brow, tab, scell, q, 0, rows,
+        brick_traverse<STAGED, TABLE>(A.g, G, A.s, A.d, R, A.rad, brow, tab, scell, q, 0, rows,
             [&](int t0, unsigned bits) {
                 for (; bits; bits &= bits - 1) {
                     if (skip > 0) { --skip; continue; }
@@ -860,15 +944,16 @@ __device__ __forceinline__ void build_sum(const BrickDensityArgs &A, const Block
 // from a traversal that skips the listed ones (in the order of the list
 // build), added to the stored partial density.  A call of its own, so that
 // the passes keep its registers out of their loops.
-template <bool STAGED>
+template <bool STAGED, bool TABLE>
 __device__ __noinline__ void density_rest(const BrickDensityArgs &A) {
     const int b = blockIdx.x;
     const int2 dh = A.d.bdst[b];
     const int4 sh = A.s.bsrc[b];
     const Grid &g = A.g;
     const BlockGeo G = block_geo(g, A.bk, b);
-    const int2 *brow = A.s.brow + (size_t)b * A.bk.nrmax, *tab = A.s.bstage + sh.y;
-    const SrcRecords<STAGED> R = make_records<STAGED>(A.sm, A.s, g.cs_f, tab, sh.x, 0.f);
+    const int2 *brow = A.s.brow + (size_t)b * A.bk.nrmax;
+    const StageTab<TABLE> tab = stage_tab<TABLE>(A, sh);
+    const SrcRecords<STAGED, TABLE> R = make_records<STAGED, TABLE>(A.sm, A.s, g.cs_f, tab, sh.x, 0.f);
     const float ih = __fdividef(1.f, g.h_uniform);
     const float fac = cubic_fac(A.dim, ih);
     const int rows = (2 * g.ky + 1) * (2 * g.kz + 1);
@@ -879,7 +964,7 @@ __device__ __noinline__ void density_rest(const BrickDensityArgs &A) {
         if (!is_real(A.d, q.orig)) continue;
         CSum rest;
         int skip = A.cap;
-        brick_traverse<STAGED>(g, G, A.s, A.d, R, A.rad, brow, tab, nullptr, q, 0, rows,
+        brick_traverse<STAGED, TABLE>(g, G, A.s, A.d, R, A.rad, brow, tab, nullptr, q, 0, rows,
             [&](int t0, unsigned m) {
                 for (; m; m &= m - 1) {
                     if (skip > 0) { --skip; continue; }
@@ -901,14 +986,14 @@ __device__ __noinline__ void density_rest(const BrickDensityArgs &A) {
 }
 
 // The density of destination d of the block (its prefetched records p).
-template <int S, bool STAGED>
-__device__ __forceinline__ void density_dest(const BrickDensityArgs &A, const SrcRecords<STAGED> &R,
+template <int S, bool STAGED, bool TABLE>
+__device__ __forceinline__ void density_dest(const BrickDensityArgs &A, const SrcRecords<STAGED, TABLE> &R,
                                              const uint4 *lst, int D, int lane, const DestPre &p,
                                              unsigned mask) {
     const float ih = __fdividef(1.f, A.g.h_uniform);
     const WCoef wc = w_coef(cubic_fac(A.dim, ih), 1.f);
     CSum rho;
-    density_stream<S, STAGED>(rho, R, lst, D, (min(p.c, A.cap) + 7) >> 3, lane, p.P, ih, wc, p.b0,
+    density_stream<S, STAGED, TABLE>(rho, R, lst, D, (min(p.c, A.cap) + 7) >> 3, lane, p.P, ih, wc, p.b0,
                               p.b1, mask);
     if (lane == 0) {
         const bool real = is_real(A.d, p.orig);
@@ -919,14 +1004,14 @@ __device__ __forceinline__ void density_dest(const BrickDensityArgs &A, const Sr
 // Destinations past one per column of the block (few: blocks are launched
 // with the threads of an ordinary brick), shared by four lanes each.  A call
 // of its own, so that the passes keep its registers out of their loops.
-template <bool STAGED>
+template <bool STAGED, bool TABLE>
 __device__ __noinline__ void density_more(const BrickDensityArgs &A, int first) {
     constexpr int S = 4;
     const int b = blockIdx.x;
     const int2 dh = A.d.bdst[b];
     const int4 sh = A.s.bsrc[b];
-    const SrcRecords<STAGED> R =
-        make_records<STAGED>(A.sm, A.s, A.g.cs_f, A.s.bstage + sh.y, sh.x, 0.f);
+    const SrcRecords<STAGED, TABLE> R =
+        make_records<STAGED, TABLE>(A.sm, A.s, A.g.cs_f, stage_tab<TABLE>(A, sh), sh.x, 0.f);
     const uint4 *lgrp = reinterpret_cast<const uint4 *>(A.nbr) + (size_t)dh.y * (A.cap >> 3);
     const int lane = threadIdx.x % S;
     for (int r0 = first; r0 < dh.x; r0 += blockDim.x / S) {
@@ -936,11 +1021,11 @@ __device__ __noinline__ void density_more(const BrickDensityArgs &A, int first) 
         DestPre p;
         dest_prefetch<S>(A.d, A.g.cs_f, A.d.bdest[dh.y + d], A.cnt + dh.y, lgrp, A.cap, dh.x, d,
                          lane, p);
-        density_dest<S, STAGED>(A, R, lgrp + d, dh.x, lane, p, mask);
+        density_dest<S, STAGED, TABLE>(A, R, lgrp + d, dh.x, lane, p, mask);
     }
 }
 
-template <int S, bool STAGED>
+template <int S, bool STAGED, bool TABLE>
 __global__ void __maxnreg__(64) k_bdensity(const __grid_constant__ BrickDensityArgs A) {
     const int b = blockIdx.x;
     const int2 dh = A.d.bdst[b];        // destinations, first destination
@@ -950,7 +1035,7 @@ __global__ void __maxnreg__(64) k_bdensity(const __grid_constant__ BrickDensityA
     // tables and lists of the last build and positions
     const unsigned off = A.gate != nullptr ? *A.gate : 0u;
     const int T = sh.x, D = dh.x;
-    const int2 *tab = A.s.bstage + sh.y;
+    const StageTab<TABLE> tab = stage_tab<TABLE>(A, sh);
     const uint4 *lgrp = reinterpret_cast<const uint4 *>(A.nbr) + (size_t)dh.y * (A.cap >> 3);
     const int lane = threadIdx.x % S, d = threadIdx.x / S;
     // the destination of this thread, requested before the staging
@@ -958,14 +1043,14 @@ __global__ void __maxnreg__(64) k_bdensity(const __grid_constant__ BrickDensityA
     if (d < D)
         dest_prefetch<S>(A.d, A.g.cs_f, A.d.bdest[dh.y + d], A.cnt + dh.y, lgrp, A.cap, D, d, lane,
                          pre);
-    if (STAGED) stage<false>(A.s, tab, T, A.g.cs_f, A.sm, false, 0.f, 0.f);
+    if (STAGED) stage<false, TABLE>(A.s, tab, T, A.g.cs_f, A.sm, false, 0.f, 0.f);
     __syncthreads();
     if (off != 0u) return;
-    const SrcRecords<STAGED> R = make_records<STAGED>(A.sm, A.s, A.g.cs_f, tab, T, 0.f);
+    const SrcRecords<STAGED, TABLE> R = make_records<STAGED, TABLE>(A.sm, A.s, A.g.cs_f, tab, T, 0.f);
     const unsigned mask = S > 1 ? __ballot_sync(0xffffffffu, d < D) : 0xffffffffu;
-    if (d < D) density_dest<S, STAGED>(A, R, lgrp + d, D, lane, pre, mask);
-    if (D > (int)blockDim.x / S) density_more<STAGED>(A, blockDim.x / S);
-    if (*A.maxcnt > A.cap && A.rho_out != nullptr) density_rest<STAGED>(A);
+    if (d < D) density_dest<S, STAGED, TABLE>(A, R, lgrp + d, D, lane, pre, mask);
+    if (D > (int)blockDim.x / S) density_more<STAGED, TABLE>(A, blockDim.x / S);
+    if (*A.maxcnt > A.cap && A.rho_out != nullptr) density_rest<STAGED, TABLE>(A);
 }
 
 // List build: every destination's list from a traversal, and (write_out) its
@@ -973,7 +1058,7 @@ __global__ void __maxnreg__(64) k_bdensity(const __grid_constant__ BrickDensityA
 // the traversal (the chords of a warp's destinations differ in length), so
 // that loop only tests and lists; summing in it, under the same divergence,
 // took 790 us at 1 M particles against 626 (both before the masks).
-template <int S, bool STAGED>
+template <int S, bool STAGED, bool TABLE>
 __global__ void __maxnreg__(64) k_bbuild(const __grid_constant__ BrickDensityArgs A) {
     const int b = blockIdx.x;
     const int2 dh = A.d.bdst[b];
@@ -982,7 +1067,8 @@ __global__ void __maxnreg__(64) k_bbuild(const __grid_constant__ BrickDensityArg
     const unsigned off = A.gate != nullptr ? *A.gate : 0u;
     const Grid &g = A.g;
     const BlockGeo G = block_geo(g, A.bk, b);
-    const int2 *brow = A.s.brow + (size_t)b * A.bk.nrmax, *tab = A.s.bstage + sh.y;
+    const int2 *brow = A.s.brow + (size_t)b * A.bk.nrmax;
+    const StageTab<TABLE> tab = stage_tab<TABLE>(A, sh);
     const int T = sh.x, D = dh.x;
     const int cap = A.cap;              // a multiple of 8
     uint4 *lgrp = reinterpret_cast<uint4 *>(A.nbr) + (size_t)dh.y * (cap >> 3);
@@ -991,10 +1077,10 @@ __global__ void __maxnreg__(64) k_bbuild(const __grid_constant__ BrickDensityArg
     int *scell = reinterpret_cast<int *>(brick_smem + A.sm.off_scell);
     const int lane = threadIdx.x % S, d0 = threadIdx.x / S, step = blockDim.x / S;
     cell_table(g, G, A.s.cstart, brow, scell);
-    if (STAGED) stage<false>(A.s, tab, T, g.cs_f, A.sm, false, 0.f, 0.f);
+    if (STAGED) stage<false, TABLE>(A.s, tab, T, g.cs_f, A.sm, false, 0.f, 0.f);
     __syncthreads();
     if (off != 0u) return;
-    const SrcRecords<STAGED> R = make_records<STAGED>(A.sm, A.s, g.cs_f, tab, T, 0.f);
+    const SrcRecords<STAGED, TABLE> R = make_records<STAGED, TABLE>(A.sm, A.s, g.cs_f, tab, T, 0.f);
     // every thread of a warp runs every round (build_list shuffles)
     for (int r0 = 0; r0 < D; r0 += step) {
         const int d = r0 + d0;
@@ -1005,7 +1091,7 @@ __global__ void __maxnreg__(64) k_bbuild(const __grid_constant__ BrickDensityArg
             q = brick_dest(A.d, G, g.cs_f, bdest[d]);
             real = is_real(A.d, q.orig);
         }
-        const int c = build_list<S, STAGED>(A, G, R, brow, tab, scell, q, real, lane, T, lgrp + d, D);
+        const int c = build_list<S, STAGED, TABLE>(A, G, R, brow, tab, scell, q, real, lane, T, lgrp + d, D);
         if (!active) continue;
         if (lane == 0) cnt[d] = c;
         const unsigned act = __activemask();
@@ -1015,7 +1101,7 @@ __global__ void __maxnreg__(64) k_bbuild(const __grid_constant__ BrickDensityArg
         const float ih = __fdividef(1.f, g.h_uniform);
         const WCoef wc = w_coef(cubic_fac(A.dim, ih), 1.f);
         CSum rho;
-        if (real) build_sum<STAGED>(A, G, R, brow, tab, scell, q, c, lgrp + d, D, ih, wc, rho);
+        if (real) build_sum<STAGED, TABLE>(A, G, R, brow, tab, scell, q, c, lgrp + d, D, ih, wc, rho);
         density_store(A, q.s, q.orig, real, q.P.w, real ? rho.hi : 0.f, real ? rho.lo : 0.f);
     }
 }
@@ -1108,9 +1194,9 @@ __device__ __forceinline__ void rates_flush(RatesAcc &a, unsigned mask) {
 
 // The pairs of one group of 8 list entries, records two at a time, then
 // the batch's partial sums folded into the compensated ones.
-template <int S, bool XSPH, bool ETA0, bool FAST, bool STAGED>
+template <int S, bool XSPH, bool ETA0, bool FAST, bool STAGED, bool TABLE>
 __device__ __forceinline__ void rates_group(RatesAcc &acc, const RatesConst &kc,
-                                            const SrcRecords<STAGED> &R, bool mine, const uint4 &grp,
+                                            const SrcRecords<STAGED, TABLE> &R, bool mine, const uint4 &grp,
                                             const float4 &Pi, unsigned mask) {
     if (S == 1 || mine) {
 #pragma unroll
@@ -1131,9 +1217,9 @@ __device__ __forceinline__ void rates_group(RatesAcc &acc, const RatesConst &kc,
 }
 
 // The sums of a destination, its list streamed as in density_stream.
-template <int S, bool XSPH, bool ETA0, bool FAST, bool STAGED>
+template <int S, bool XSPH, bool ETA0, bool FAST, bool STAGED, bool TABLE>
 __device__ __forceinline__ void rates_stream(RatesAcc &acc, const RatesConst &kc,
-                                             const SrcRecords<STAGED> &R, const uint4 *lst, int D,
+                                             const SrcRecords<STAGED, TABLE> &R, const uint4 *lst, int D,
                                              int ng, int lane, const float4 &Pi, uint4 b0, uint4 b1,
                                              unsigned mask) {
     const uint4 zero = make_uint4(0, 0, 0, 0);
@@ -1143,15 +1229,15 @@ __device__ __forceinline__ void rates_stream(RatesAcc &acc, const RatesConst &kc
     for (int g0 = 0, gi = lane;;) {
         if (g0 >= nr) break;
         b2 = gi + 2 * S < ng ? lst[(gi + 2 * S) * step] : zero;
-        rates_group<S, XSPH, ETA0, FAST, STAGED>(acc, kc, R, gi < ng, b0, Pi, mask);
+        rates_group<S, XSPH, ETA0, FAST, STAGED, TABLE>(acc, kc, R, gi < ng, b0, Pi, mask);
         gi += S;
         if ((g0 += S) >= nr) break;
         b0 = gi + 2 * S < ng ? lst[(gi + 2 * S) * step] : zero;
-        rates_group<S, XSPH, ETA0, FAST, STAGED>(acc, kc, R, gi < ng, b1, Pi, mask);
+        rates_group<S, XSPH, ETA0, FAST, STAGED, TABLE>(acc, kc, R, gi < ng, b1, Pi, mask);
         gi += S;
         if ((g0 += S) >= nr) break;
         b1 = gi + 2 * S < ng ? lst[(gi + 2 * S) * step] : zero;
-        rates_group<S, XSPH, ETA0, FAST, STAGED>(acc, kc, R, gi < ng, b2, Pi, mask);
+        rates_group<S, XSPH, ETA0, FAST, STAGED, TABLE>(acc, kc, R, gi < ng, b2, Pi, mask);
         gi += S;
         g0 += S;
     }
@@ -1196,23 +1282,24 @@ __device__ __forceinline__ void rates_store(const BrickRatesArgs &A, const Rates
 
 // Destinations with more neighbours than their list holds, as density_rest:
 // the rest added to the stored sums.
-template <bool XSPH, bool ETA0, bool STAGED>
+template <bool XSPH, bool ETA0, bool STAGED, bool TABLE>
 __device__ __noinline__ void rates_rest(const BrickRatesArgs &A) {
     const int b = blockIdx.x;
     const int2 dh = A.d.bdst[b];
     const int4 sh = A.s.bsrc[b];
     const Grid &g = A.g;
     const BlockGeo G = block_geo(g, A.bk, b);
-    const int2 *brow = A.s.brow + (size_t)b * A.bk.nrmax, *tab = A.s.bstage + sh.y;
+    const int2 *brow = A.s.brow + (size_t)b * A.bk.nrmax;
+    const StageTab<TABLE> tab = stage_tab<TABLE>(A, sh);
     const float halpha = 0.5f * A.alpha;
-    const SrcRecords<STAGED> R = make_records<STAGED>(A.sm, A.s, g.cs_f, tab, sh.x, halpha);
+    const SrcRecords<STAGED, TABLE> R = make_records<STAGED, TABLE>(A.sm, A.s, g.cs_f, tab, sh.x, halpha);
     const float ih = __fdividef(1.f, g.h_uniform);
     const RatesConst kc = rates_const(g.h_uniform, cubic_fac(A.dim, ih), A.beta, A.eta2, A.eps);
     const int rows = (2 * g.ky + 1) * (2 * g.kz + 1);
     // a two-record block has staged no state records
     if (STAGED) {
         __syncthreads();
-        stage_state(A.s, tab, sh.x, A.sm.off_s, halpha);
+        stage_state<TABLE>(A.s, tab, sh.x, A.sm.off_s, halpha);
     }
     __syncthreads();
     for (int d = threadIdx.x; d < dh.x; d += blockDim.x) {
@@ -1222,7 +1309,7 @@ __device__ __noinline__ void rates_rest(const BrickRatesArgs &A) {
         RatesAcc acc;
         rates_acc_init(acc, A.d.velh[q.s], A.d.st[q.s], halpha);
         int skip = A.cap;
-        brick_traverse<STAGED>(g, G, A.s, A.d, R, A.rad, brow, tab, nullptr, q, 0, rows,
+        brick_traverse<STAGED, TABLE>(g, G, A.s, A.d, R, A.rad, brow, tab, nullptr, q, 0, rows,
             [&](int t0, unsigned m) {
                 for (; m; m &= m - 1) {
                     if (skip > 0) { --skip; continue; }
@@ -1247,8 +1334,8 @@ __device__ __noinline__ void rates_rest(const BrickRatesArgs &A) {
 }
 
 // The rates of a destination (its prefetched records p, velocity, state).
-template <int S, bool XSPH, bool ETA0, bool FAST, bool STAGED>
-__device__ __forceinline__ void rates_dest(const BrickRatesArgs &A, const SrcRecords<STAGED> &R,
+template <int S, bool XSPH, bool ETA0, bool FAST, bool STAGED, bool TABLE>
+__device__ __forceinline__ void rates_dest(const BrickRatesArgs &A, const SrcRecords<STAGED, TABLE> &R,
                                            float mb, const uint4 *lst, int D, int lane,
                                            const DestPre &p, const float4 &vi, const float4 &st,
                                            unsigned mask) {
@@ -1258,19 +1345,19 @@ __device__ __forceinline__ void rates_dest(const BrickRatesArgs &A, const SrcRec
     kc.tkc = A.tait_kc;
     RatesAcc acc;
     rates_acc_init(acc, vi, st, 0.5f * A.alpha);
-    rates_stream<S, XSPH, ETA0, FAST, STAGED>(acc, kc, R, lst, D, (min(p.c, A.cap) + 7) >> 3, lane,
+    rates_stream<S, XSPH, ETA0, FAST, STAGED, TABLE>(acc, kc, R, lst, D, (min(p.c, A.cap) + 7) >> 3, lane,
                                               p.P, p.b0, p.b1, mask);
     rates_store<S, XSPH>(A, acc, p.orig, lane);
 }
 
 // Destinations past one per column of the block, as density_more.
-template <bool XSPH, bool ETA0, bool FAST, bool STAGED>
+template <bool XSPH, bool ETA0, bool FAST, bool STAGED, bool TABLE>
 __device__ __noinline__ void rates_more(const BrickRatesArgs &A, float mb, int first) {
     constexpr int S = 4;
     const int b = blockIdx.x;
     const int2 dh = A.d.bdst[b];
     const int4 sh = A.s.bsrc[b];
-    const SrcRecords<STAGED> R = make_records<STAGED>(A.sm, A.s, A.g.cs_f, A.s.bstage + sh.y, sh.x,
+    const SrcRecords<STAGED, TABLE> R = make_records<STAGED, TABLE>(A.sm, A.s, A.g.cs_f, stage_tab<TABLE>(A, sh), sh.x,
                                                       0.5f * A.alpha);
     const uint4 *lgrp = reinterpret_cast<const uint4 *>(A.nbr) + (size_t)dh.y * (A.cap >> 3);
     const int lane = threadIdx.x % S;
@@ -1281,23 +1368,23 @@ __device__ __noinline__ void rates_more(const BrickRatesArgs &A, float mb, int f
         DestPre p;
         dest_prefetch<S>(A.d, A.g.cs_f, A.d.bdest[dh.y + d], A.cnt + dh.y, lgrp, A.cap, dh.x, d,
                          lane, p);
-        rates_dest<S, XSPH, ETA0, FAST, STAGED>(A, R, mb, lgrp + d, dh.x, lane, p, A.d.velh[p.s],
+        rates_dest<S, XSPH, ETA0, FAST, STAGED, TABLE>(A, R, mb, lgrp + d, dh.x, lane, p, A.d.velh[p.s],
                                                 A.d.st[p.s], mask);
     }
 }
 
-template <int S, bool XSPH, bool ETA0, bool FAST, bool STAGED>
-__device__ __forceinline__ void rates_block(const BrickRatesArgs &A, const SrcRecords<STAGED> &R,
+template <int S, bool XSPH, bool ETA0, bool FAST, bool STAGED, bool TABLE>
+__device__ __forceinline__ void rates_block(const BrickRatesArgs &A, const SrcRecords<STAGED, TABLE> &R,
                                             float mb, const uint4 *lgrp, int D, int d, int lane,
                                             const DestPre &pre, const float4 &vi, const float4 &st) {
     const unsigned mask = S > 1 ? __ballot_sync(0xffffffffu, d < D) : 0xffffffffu;
     if (d < D)
-        rates_dest<S, XSPH, ETA0, FAST, STAGED>(A, R, mb, lgrp + d, D, lane, pre, vi, st, mask);
-    if (D > (int)blockDim.x / S) rates_more<XSPH, ETA0, FAST, STAGED>(A, mb, blockDim.x / S);
-    if (*A.maxcnt > A.cap) rates_rest<XSPH, ETA0, STAGED>(A);
+        rates_dest<S, XSPH, ETA0, FAST, STAGED, TABLE>(A, R, mb, lgrp + d, D, lane, pre, vi, st, mask);
+    if (D > (int)blockDim.x / S) rates_more<XSPH, ETA0, FAST, STAGED, TABLE>(A, mb, blockDim.x / S);
+    if (*A.maxcnt > A.cap) rates_rest<XSPH, ETA0, STAGED, TABLE>(A);
 }
 
-template <int S, bool XSPH, bool STAGED>
+template <int S, bool XSPH, bool STAGED, bool TABLE>
 __global__ void __maxnreg__(XSPH ? 80 : 64) k_brates(const __grid_constant__ BrickRatesArgs A) {
     const int b = blockIdx.x;
     const int2 dh = A.d.bdst[b];        // destinations, first destination
@@ -1305,7 +1392,7 @@ __global__ void __maxnreg__(XSPH ? 80 : 64) k_brates(const __grid_constant__ Bri
     if (dh.x == 0) return;
     const unsigned off = A.gate != nullptr ? *A.gate : 0u;   // tested after the staging
     const int T = sh.x, D = dh.x;
-    const int2 *tab = A.s.bstage + sh.y;
+    const StageTab<TABLE> tab = stage_tab<TABLE>(A, sh);
     const uint4 *lgrp = reinterpret_cast<const uint4 *>(A.nbr) + (size_t)dh.y * (A.cap >> 3);
     const int lane = threadIdx.x % S, d = threadIdx.x / S;
     DestPre pre;
@@ -1322,24 +1409,24 @@ __global__ void __maxnreg__(XSPH ? 80 : 64) k_brates(const __grid_constant__ Bri
     const bool try_fast = STAGED && A.tait_state != 0 && A.eta2 == 0.f && T > 0;
     const float mref = try_fast ? A.s.pm[sh.z].w : 0.f;
     bool same = true;
-    if (STAGED) same = stage<true>(A.s, tab, T, A.g.cs_f, A.sm, !try_fast, halpha, mref);
+    if (STAGED) same = stage<true, TABLE>(A.s, tab, T, A.g.cs_f, A.sm, !try_fast, halpha, mref);
     const bool fast = __syncthreads_and(try_fast && same) != 0;
     if (STAGED && try_fast && !fast) {
-        stage_state(A.s, tab, T, A.sm.off_s, halpha);
+        stage_state<TABLE>(A.s, tab, T, A.sm.off_s, halpha);
         __syncthreads();
     }
     if (off != 0u) return;
-    const SrcRecords<STAGED> R = make_records<STAGED>(A.sm, A.s, A.g.cs_f, tab, T, halpha);
+    const SrcRecords<STAGED, TABLE> R = make_records<STAGED, TABLE>(A.sm, A.s, A.g.cs_f, tab, T, halpha);
     if (A.eta2 == 0.f) {
         if constexpr (STAGED) {
             if (fast) {
-                rates_block<S, XSPH, true, true, STAGED>(A, R, mref, lgrp, D, d, lane, pre, vi, st);
+                rates_block<S, XSPH, true, true, STAGED, TABLE>(A, R, mref, lgrp, D, d, lane, pre, vi, st);
                 return;
             }
         }
-        rates_block<S, XSPH, true, false, STAGED>(A, R, 0.f, lgrp, D, d, lane, pre, vi, st);
+        rates_block<S, XSPH, true, false, STAGED, TABLE>(A, R, 0.f, lgrp, D, d, lane, pre, vi, st);
     } else {
-        rates_block<S, XSPH, false, false, STAGED>(A, R, 0.f, lgrp, D, d, lane, pre, vi, st);
+        rates_block<S, XSPH, false, false, STAGED, TABLE>(A, R, 0.f, lgrp, D, d, lane, pre, vi, st);
     }
 }
 
@@ -1402,7 +1489,8 @@ __global__ void __launch_bounds__(128) k_brick_count(Grid g, BrickGeom bk, const
     if (lane == 0) {
         // every block: as a source this array is staged by the blocks that
         // hold destinations of any array
-        const int tb = T > 0 ? (int)atomicAdd(stats + 3, (unsigned)T) : 0;
+        const int tb = T > 0 ? (int)atomicAdd(reinterpret_cast<unsigned long long *>(stats + 4),
+                                              (unsigned long long)T) : 0;
         const int db = D > 0 ? (int)atomicAdd(stats + 2, (unsigned)D) : 0;
         atomicMax(stats, (unsigned)T);
         atomicMax(stats + 1, (unsigned)D);
@@ -1411,7 +1499,7 @@ __global__ void __launch_bounds__(128) k_brick_count(Grid g, BrickGeom bk, const
     }
 }
 
-// bstage null: an array that no pass stages (brick_fill) gets its destinations only
+// bstage null: the destinations only (brick_fill)
 __global__ void __launch_bounds__(128) k_brick_fill(Grid g, BrickGeom bk, const int *cstart,
                                                     const float *scx, const int4 *bsrc,
                                                     const int2 *brow, const int2 *bdst,
@@ -1507,7 +1595,7 @@ BrickSrcDev make_bsrc(const ArraySnap &S) {
     BrickSrcDev s;
     s.pm = S.pm; s.velh = S.velh; s.st = S.st; s.scx = S.scx;
     s.cstart = S.cstart; s.perm = S.perm;
-    s.bsrc = S.bsrc; s.brow = S.brow; s.bstage = S.bstage;
+    s.bsrc = S.bsrc; s.brow = S.brow; s.bstage = S.b_table ? S.bstage : nullptr;
     s.x = S.view.x; s.y = S.view.y; s.z = S.view.z;
     return s;
 }
@@ -1527,7 +1615,7 @@ BrickDstDev make_bdst(const ArraySnap &D) {
 // populous block rounded to warps, at most 320 with one lane (three blocks of
 // 64-register threads per SM) and 512 with more; a block with more columns
 // takes them in rounds.
-int brick_threads(const sph_ctx *ctx, const ArraySnap &D) {
+int brick_threads(const ArraySnap &D, int lanes) {
     // environment SPH_BRICK_MAX_THREADS: another ceiling (a multiple of 32
     // up to 512), to measure it
     static int ceiling = -1;
@@ -1536,7 +1624,6 @@ int brick_threads(const sph_ctx *ctx, const ArraySnap &D) {
         const int v = e ? atoi(e) : 0;
         ceiling = (v >= 64 && v <= kBrickMaxThreads && v % 32 == 0) ? v : 0;
     }
-    const int lanes = ctx->bricks.lanes;
     const int top = ceiling > 0 ? ceiling : (lanes == 1 ? 320 : kBrickMaxThreads);
     const int want = (std::max(D.b_dmax, 1) * lanes + 31) / 32 * 32;
     return std::min(std::max(want, 64), top);
@@ -1666,28 +1753,46 @@ int brick_count(sph_ctx *ctx, int a, unsigned *stats) {
 }
 
 // The destinations are filled for every array: a pass over another, sparser
-// source takes this array's blocks however populous they are.  The sources
-// only where the array can be staged (the fields of brow hold 16 bits each).
+// source takes this array's blocks however populous they are.  The table of
+// staged entries (bstage, some five entries per particle in 3D) is for arrays
+// that a block can stage (the fields of brow hold 16 bits each), with fewer
+// than 2^31 entries (32-bit indices) and where there is memory for it; without
+// it the passes find the entries from the rows (environment
+// SPH_BRICK_STAGE_TABLE=0: always, to test that on small sets).  That costs
+// time only: RK2 step of 1 M particles 915 -> 1126 us, of 64 000 157 -> 180.
 int brick_fill(sph_ctx *ctx, int a) {
     ArraySnap &A = ctx->arrays[a];
     const BrickGeom &bk = ctx->bricks;
-    const bool source = A.b_tmax < 65535;
+    static int wanted = -1;
+    if (wanted < 0) {
+        const char *e = getenv("SPH_BRICK_STAGE_TABLE");
+        wanted = (e && atoi(e) == 0) ? 0 : 1;
+    }
     if (A.n > A.bdest_cap || !A.bdest) {
         cudaFree(A.bdest);
         A.bdest = nullptr;
         SPH_CUDA(cudaMalloc(&A.bdest, sizeof(int2) * A.n));
         A.bdest_cap = A.n;
     }
-    if (source && (A.b_staged > A.bstage_cap || !A.bstage)) {
+    A.b_table = wanted && A.b_tmax < 65535 && A.b_staged < INT32_MAX;
+    if (A.b_table && (A.b_staged > A.bstage_cap || !A.bstage)) {
         cudaFree(A.bstage);
         A.bstage = nullptr;
-        const int64_t want = A.b_staged + A.b_staged / 8;   // the next builds' too
-        SPH_CUDA(cudaMalloc(&A.bstage, sizeof(int2) * std::max<int64_t>(want, 1)));
-        A.bstage_cap = want;
+        A.bstage_cap = 0;
+        // (an eighth more, for the next builds)
+        for (const int64_t want : {A.b_staged + A.b_staged / 8, A.b_staged}) {
+            if (cudaMalloc(&A.bstage, sizeof(int2) * std::max<int64_t>(want, 1)) == cudaSuccess) {
+                A.bstage_cap = want;
+                break;
+            }
+            A.bstage = nullptr;
+            cudaGetLastError();     // (not the build's error)
+        }
+        A.b_table = A.bstage != nullptr;
     }
     k_brick_fill<<<(unsigned)bk.nbricks, 128, 0, ctx->stream>>>(
-        ctx->grid, bk, A.cstart, A.scx, A.bsrc, A.brow, A.bdst, source ? A.bstage : nullptr,
-        A.bdest);
+        ctx->grid, bk, A.cstart, A.scx, A.bsrc, A.brow, A.bdst,
+        A.b_table ? A.bstage : nullptr, A.bdest);
     count_launch();
     SPH_LAUNCH_CHECK("k_brick_fill");
     return SPH_OK;
@@ -1749,20 +1854,24 @@ int brick_density(sph_ctx *ctx, int dst, int src, NbrList &L, bool build, bool w
     a.st_out = st_out;
     a.gate = ctx->gate;
     if (D.n == 0) return SPH_OK;
-    const int nt = brick_threads(ctx, D);
+    // (without a table of entries: one lane, whatever the parts)
+    const int lanes = S.b_table ? ctx->bricks.lanes : 1;
+    const int nt = brick_threads(D, lanes);
     const int blocks = (int)ctx->bricks.nbricks;
-    const int lanes = ctx->bricks.lanes;
-#define BDL2(K_, L_, S_)                                                                  \
+#define BDL2(K_, L_, S_, T_)                                                              \
     do {                                                                                  \
-        int rc_ = allow_smem(K_<L_, S_>, bytes);                                          \
+        int rc_ = allow_smem(K_<L_, S_, T_>, bytes);                                      \
         if (rc_) return rc_;                                                              \
-        K_<L_, S_><<<blocks, nt, bytes, ctx->stream>>>(a);                                \
+        K_<L_, S_, T_><<<blocks, nt, bytes, ctx->stream>>>(a);                            \
     } while (0)
-#define BDL1(K_, L_) do { if (staged) BDL2(K_, L_, true); else BDL2(K_, L_, false); } while (0)
-#define BDL(L_) do { if (build) BDL1(k_bbuild, L_); else BDL1(k_bdensity, L_); } while (0)
-    if (lanes == 1) BDL(1);
-    else if (lanes == 2) BDL(2);
-    else BDL(4);
+#define BDL1(K_, L_, T_)                                                                  \
+    do { if (staged) BDL2(K_, L_, true, T_); else BDL2(K_, L_, false, T_); } while (0)
+#define BDL(L_, T_)                                                                       \
+    do { if (build) BDL1(k_bbuild, L_, T_); else BDL1(k_bdensity, L_, T_); } while (0)
+    if (!S.b_table) BDL(1, false);
+    else if (lanes == 1) BDL(1, true);
+    else if (lanes == 2) BDL(2, true);
+    else BDL(4, true);
 #undef BDL
 #undef BDL1
 #undef BDL2
@@ -1813,27 +1922,27 @@ int brick_rates(sph_ctx *ctx, int dst, const sph_source_term &term, NbrList &L,
     a.gate = ctx->gate;
     if (D.n == 0) return SPH_OK;
     const bool xsph = (term.flags & SPH_TERM_XSPH) != 0;
-    const int nt = brick_threads(ctx, D);
+    // (without a table of entries: one lane, whatever the parts)
+    const int lanes = S.b_table ? ctx->bricks.lanes : 1;
+    const int nt = brick_threads(D, lanes);
     const int blocks = (int)ctx->bricks.nbricks;
-    const int lanes = ctx->bricks.lanes;
-#define BRL2(L_, X_)                                                                      \
+#define BRL3(L_, X_, S_, T_)                                                              \
     do {                                                                                  \
-        if (staged) {                                                                     \
-            int rc_ = allow_smem(k_brates<L_, X_, true>, bytes);                          \
-            if (rc_) return rc_;                                                          \
-            k_brates<L_, X_, true><<<blocks, nt, bytes, ctx->stream>>>(a);                \
-        } else {                                                                          \
-            int rc_ = allow_smem(k_brates<L_, X_, false>, bytes);                         \
-            if (rc_) return rc_;                                                          \
-            k_brates<L_, X_, false><<<blocks, nt, bytes, ctx->stream>>>(a);               \
-        }                                                                                 \
+        int rc_ = allow_smem(k_brates<L_, X_, S_, T_>, bytes);                            \
+        if (rc_) return rc_;                                                              \
+        k_brates<L_, X_, S_, T_><<<blocks, nt, bytes, ctx->stream>>>(a);                  \
     } while (0)
-#define BRL(L_) do { if (xsph) BRL2(L_, true); else BRL2(L_, false); } while (0)
-    if (lanes == 1) BRL(1);
-    else if (lanes == 2) BRL(2);
-    else BRL(4);
+#define BRL2(L_, X_, T_)                                                                  \
+    do { if (staged) BRL3(L_, X_, true, T_); else BRL3(L_, X_, false, T_); } while (0)
+#define BRL(L_, T_)                                                                       \
+    do { if (xsph) BRL2(L_, true, T_); else BRL2(L_, false, T_); } while (0)
+    if (!S.b_table) BRL(1, false);
+    else if (lanes == 1) BRL(1, true);
+    else if (lanes == 2) BRL(2, true);
+    else BRL(4, true);
 #undef BRL
 #undef BRL2
+#undef BRL3
     count_launch();
     SPH_LAUNCH_CHECK("k_brates");
     return SPH_OK;

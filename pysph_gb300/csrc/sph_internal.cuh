@@ -236,9 +236,10 @@ struct ArraySnap {
     int2 *bdst = nullptr, *brow = nullptr, *bstage = nullptr, *bdest = nullptr;
     int64_t brick_cap = 0, brow_cap = 0, bstage_cap = 0, bdest_cap = 0;
     // largest staged count and largest count of destinations of a block,
-    // staged particles of all blocks
+    // staged particles of all blocks; whether this build has their bstage
     int b_tmax = 0, b_dmax = 0;
     int64_t b_staged = 0;
+    bool b_table = false;
 };
 
 // Neighbour list of one (destination, source) pair of arrays: entry k of
@@ -465,8 +466,9 @@ int record_refresh(sph_ctx *ctx, int array, const sph_array_view *view);
 // brick-staged pair passes (bricks.cu)
 constexpr int kMaxBrickArrays = 16;
 // statistics of an array's brick tables: largest staged count and largest
-// count of destinations of a block, destinations and staged particles in all
-constexpr int kBrickStats = 4;
+// count of destinations of a block, destinations in all, (unused,) staged
+// particles in all (64 bits)
+constexpr int kBrickStats = 6;
 void brick_geometry(sph_ctx *ctx);
 int brick_count(sph_ctx *ctx, int a, unsigned *stats);
 int brick_fill(sph_ctx *ctx, int a);

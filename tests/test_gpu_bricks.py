@@ -350,3 +350,49 @@ def test_crowded_destination_with_a_sparse_source(n, monkeypatch):
         ax, ay = oracle.pair_sum("momentum", dp, sp, off, idx, 2,
                                  dict(alpha=0.5, beta=0.5, eta=0.1), nout=2)[:2]
         assert normwise(dst.get("ax"), ax) < TOL and normwise(dst.get("ay"), ay) < TOL
+
+
+_HASH_MASSES = r'''
+import sys, hashlib
+sys.path.insert(0, ".")
+import numpy as np, pysph_gb300
+from pysph_gb300 import workloads as W
+api = pysph_gb300.api()
+h = hashlib.sha256()
+def run(s, particles, dt, names):
+    for _ in range(3):
+        s.integrator.integrate(dt)
+    assert particles.cell_manager.brick_pass_count() > 0
+    for f in names:
+        h.update(particles.arrays[0].get(f).tobytes())
+for n in (1000, 13824):
+    props = W.cube_lattice(n, seed=41)
+    run(*W.setup_cube(api, props), 1e-4, ("x", "y", "z", "u", "v", "w", "rho", "p", "cs"))
+    props["m"] = np.where(props["x"] < 0.3, 1.02 * props["m"], props["m"])
+    run(*W.setup_cube(api, props), 1e-4, ("x", "y", "z", "u", "v", "w", "rho", "p", "cs"))
+drop = W.elliptical_drop(dx=0.03, c0=100.0)
+run(*W.setup_drop(api, drop, c0=100.0), 1e-5, ("x", "y", "u", "v", "rho", "p", "cs"))
+print(h.hexdigest())
+'''
+
+
+def _hash_masses(**env):
+    e = dict(os.environ, PYSPH_GB300_BRICKS="1", **env)
+    r = subprocess.run([sys.executable, "-c", _HASH_MASSES], cwd=ROOT, env=e, capture_output=True,
+                       text=True, timeout=600)
+    assert r.returncode == 0, r.stderr[-3000:]
+    return r.stdout.split()[-1]
+
+
+@pytest.mark.parametrize("env", [{}, {"PYSPH_GB300_SKIN": "0"}, {"SPH_LIST_CAP": "9"},
+                                 {"SPH_BRICK_UNSTAGED": "1"},
+                                 {"SPH_BRICK_UNSTAGED": "1", "SPH_LIST_CAP": "9",
+                                  "PYSPH_GB300_SKIN": "0"}],
+                         ids=["staged", "no-skin", "over-full", "global-records", "all"])
+def test_records_found_from_rows_give_the_same_bits(env):
+    """A build without the table of staged entries (too many of them, or no
+    memory for it) finds every record from the rows of cells: the same bits,
+    with one mass and with two, in 3D and 2D."""
+    _need_gpu()
+    rows = _hash_masses(SPH_BRICK_STAGE_TABLE="0", **env)
+    assert rows == _hash_masses(**env)
