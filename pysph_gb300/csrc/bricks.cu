@@ -1434,7 +1434,8 @@ __global__ void __maxnreg__(XSPH ? 80 : 64) k_brates(const __grid_constant__ Bri
 // tables of the blocks of one array (ArraySnap): first, a warp per block, the
 // staged rows, the counts, and the places of its entries (one atomic per
 // table; they differ from build to build, the results do not depend on
-// them), then, the tables allocated, the entries, four warps per block (42 us
+// them) and the list of the blocks that have any, then, the tables allocated,
+// the entries of those, four warps per block (42 us
 // at 1 M particles, once per full build; a warp per block took 20 us more at
 // 275 000)
 // ---------------------------------------------------------------------------
@@ -1461,51 +1462,69 @@ __device__ __forceinline__ int dest_row(const Grid &g, const BlockGeo &G, const 
 
 __global__ void __launch_bounds__(128) k_brick_count(Grid g, BrickGeom bk, const int *cstart,
                                                      int4 *bsrc, int2 *brow, int2 *bdst,
-                                                     unsigned *stats) {
+                                                     int *blist, unsigned *stats) {
     const int lane = threadIdx.x & 31;
     const int64_t b = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
     if (b >= bk.nbricks) return;
     const BlockGeo G = block_geo(g, bk, (int)b);
-    int T = 0, first = 0;
-    int2 *rows = brow + b * bk.nrmax;
+    // first slot and length of staged row r
+    auto row = [&](int r, int &lo) {
+        lo = 0;
+        if (r >= G.nr) return 0;
+        const int c = ((G.zs0 + r / G.ry) * g.ny + G.ys0 + r % G.ry) * g.nx + G.xs0;
+        lo = cstart[c];
+        return cstart[c + G.lx] - lo;
+    };
+    int len, lo, T = 0, D = 0, first = 0;
     for (int r0 = 0; r0 < G.nr; r0 += 32) {
-        const int r = r0 + lane;
-        int lo = 0, len = 0;
-        if (r < G.nr) {
-            const int c = ((G.zs0 + r / G.ry) * g.ny + G.ys0 + r % G.ry) * g.nx + G.xs0;
-            lo = cstart[c];
-            len = cstart[c + G.lx] - lo;
-        }
-        const int inc = warp_scan(len);
-        if (r < G.nr) rows[r] = make_int2(lo, (int)((unsigned)(T + inc - len) | ((unsigned)len << 16)));
+        len = row(r0 + lane, lo);
         const unsigned some = __ballot_sync(0xffffffffu, len > 0);
         if (T == 0 && some) first = __shfl_sync(0xffffffffu, lo, __ffs(some) - 1);
-        T += __shfl_sync(0xffffffffu, inc, 31);
+        T += __reduce_add_sync(0xffffffffu, len);
+    }
+    // an empty block (most of the box of a splash) keeps no rows: its cells'
+    // starts are all the same, so a row of any offset has nothing in it
+    if (T == 0) {
+        if (lane == 0) {
+            bsrc[b] = make_int4(0, 0, 0, 0);
+            bdst[b] = make_int2(0, 0);
+        }
+        return;
+    }
+    int2 *rows = brow + b * bk.nrmax;
+    int at = 0;
+    for (int r0 = 0; r0 < G.nr; r0 += 32) {
+        len = row(r0 + lane, lo);
+        const int inc = warp_scan(len);
+        if (r0 + lane < G.nr)
+            rows[r0 + lane] = make_int2(lo, (int)((unsigned)(at + inc - len) | ((unsigned)len << 16)));
+        at += __shfl_sync(0xffffffffu, inc, 31);
     }
     const int ndr = (G.y1 - G.y0) * (G.z1 - G.z0);
-    int D = 0, lo;
     for (int r0 = 0; r0 < ndr; r0 += 32)
         D += __reduce_add_sync(0xffffffffu, dest_row(g, G, cstart, r0 + lane, lo));
     if (lane == 0) {
         // every block: as a source this array is staged by the blocks that
         // hold destinations of any array
-        const int tb = T > 0 ? (int)atomicAdd(reinterpret_cast<unsigned long long *>(stats + 4),
-                                              (unsigned long long)T) : 0;
+        const int tb = (int)atomicAdd(reinterpret_cast<unsigned long long *>(stats + 4),
+                                      (unsigned long long)T);
         const int db = D > 0 ? (int)atomicAdd(stats + 2, (unsigned)D) : 0;
         atomicMax(stats, (unsigned)T);
         atomicMax(stats + 1, (unsigned)D);
         bsrc[b] = make_int4(T, tb, first, 0);
         bdst[b] = make_int2(D, db);
+        blist[atomicAdd(stats + 3, 1u)] = (int)b;
     }
 }
 
 // bstage null: the destinations only (brick_fill)
 __global__ void __launch_bounds__(128) k_brick_fill(Grid g, BrickGeom bk, const int *cstart,
-                                                    const float *scx, const int4 *bsrc,
+                                                    const float *scx, const int *blist,
+                                                    const int4 *bsrc,
                                                     const int2 *brow, const int2 *bdst,
                                                     int2 *bstage, int2 *bdest) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int b = blockIdx.x;
+    const int b = blist[blockIdx.x];
     const int D = bdst[b].x;
     const BlockGeo G = block_geo(g, bk, b);
     const int2 *rows = brow + (int64_t)b * bk.nrmax;
@@ -1650,6 +1669,17 @@ int allow_smem(Kern *k, size_t bytes) {
 
 }  // namespace
 
+// Most blocks of a box whose destinations get several lanes.  A small set that
+// fills its box has fewer (686 of 39 304 particles in 3D); one with a few
+// particles far off has more, nearly all empty, and each part of a brick is a
+// block to launch.  Step in us with lanes / one lane: 2D, 5 025 particles, four
+// lanes, 434 bricks 75.3 / 75.9, 967 79.7 / 78.3, 2 664 95.1 / 81.6, 43 000 444 /
+// 157; 3D, four lanes, 4 096 particles 567 bricks 102 / 107, 2 352 126 / 112,
+// 8 000 particles 1 049 bricks 112 / 116, 2 352 132 / 137, 4 440 159 / 138; two
+// lanes, 21 952 particles 2 701 bricks 129 / 139, 6 147 157 / 159, 11 713 190 /
+// 166.
+constexpr int64_t kLaneBlocks2 = 152 * 16, kLaneBlocks3 = 152 * 40;
+
 // Brick geometry of the current grid: edge lengths (cells) per stencil
 // half-width, chosen so a brick holds a few hundred destinations and its
 // staging ~5-8 times as many sources.
@@ -1708,6 +1738,9 @@ void brick_geometry(sph_ctx *ctx) {
     for (const ArraySnap &A : ctx->arrays) n = std::max(n, A.n);
     bk.lanes = force_lanes ? force_lanes
                            : (n < 12000 ? 4 : (g.kz > 0 && n < 40000 ? 2 : 1));
+    const int64_t whole = (int64_t)((g.nx + bk.bx - 1) / bk.bx) * ((g.ny + bk.by - 1) / bk.by) *
+                          ((g.nz + bk.bz - 1) / bk.bz);
+    if (!force_lanes && whole * bk.lanes > (g.kz > 0 ? kLaneBlocks3 : kLaneBlocks2)) bk.lanes = 1;
     bk.px = bk.lanes > 1 && bk.bx > 1 ? 2 : 1;
     bk.py = bk.lanes > 2 && bk.by > 1 ? 2 : 1;
     bk.pz = 1;
@@ -1730,10 +1763,13 @@ int brick_count(sph_ctx *ctx, int a, unsigned *stats) {
     if (bk.nbricks > A.brick_cap || !A.bsrc) {
         cudaFree(A.bsrc);
         cudaFree(A.bdst);
+        cudaFree(A.blist);
         A.bsrc = nullptr;
         A.bdst = nullptr;
+        A.blist = nullptr;
         SPH_CUDA(cudaMalloc(&A.bsrc, sizeof(int4) * bk.nbricks));
         SPH_CUDA(cudaMalloc(&A.bdst, sizeof(int2) * bk.nbricks));
+        SPH_CUDA(cudaMalloc(&A.blist, sizeof(int) * bk.nbricks));
         A.brick_cap = bk.nbricks;
     }
     const int64_t nrow = bk.nbricks * bk.nrmax;
@@ -1746,7 +1782,7 @@ int brick_count(sph_ctx *ctx, int a, unsigned *stats) {
     const int th = 128, per = th / 32;
     const int blocks = (int)((bk.nbricks + per - 1) / per);
     k_brick_count<<<blocks, th, 0, ctx->stream>>>(ctx->grid, bk, A.cstart, A.bsrc, A.brow, A.bdst,
-                                                  stats);
+                                                  A.blist, stats);
     count_launch();
     SPH_LAUNCH_CHECK("k_brick_count");
     return SPH_OK;
@@ -1790,8 +1826,8 @@ int brick_fill(sph_ctx *ctx, int a) {
         }
         A.b_table = A.bstage != nullptr;
     }
-    k_brick_fill<<<(unsigned)bk.nbricks, 128, 0, ctx->stream>>>(
-        ctx->grid, bk, A.cstart, A.scx, A.bsrc, A.brow, A.bdst,
+    k_brick_fill<<<(unsigned)A.b_blocks, 128, 0, ctx->stream>>>(
+        ctx->grid, bk, A.cstart, A.scx, A.blist, A.bsrc, A.brow, A.bdst,
         A.b_table ? A.bstage : nullptr, A.bdest);
     count_launch();
     SPH_LAUNCH_CHECK("k_brick_fill");

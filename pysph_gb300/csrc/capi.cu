@@ -109,6 +109,7 @@ int sph_ctx_destroy(sph_ctx *c) {
         cudaFree(A.nrm); cudaFree(A.tan);
         cudaFree(A.cstart); cudaFree(A.order); cudaFree(A.refcell); cudaFree(A.pm0); cudaFree(A.inv);
         cudaFree(A.bsrc);
+        cudaFree(A.blist);
         cudaFree(A.bdst);
         cudaFree(A.brow);
         cudaFree(A.bstage);

@@ -881,6 +881,7 @@ int nnps_build(sph_ctx *ctx, const sph_array_view *arrays, int narrays, double c
             const bool any = arrays[a].n > 0;
             A.b_tmax = any ? (int)q[0] : 0;
             A.b_dmax = any ? (int)q[1] : 0;
+            A.b_blocks = any ? (int)q[3] : 0;
             A.b_staged = any ? (int64_t)(q[4] | ((unsigned long long)q[5] << 32)) : 0;
             if (any) {
                 const int rc = brick_fill(ctx, a);

@@ -230,14 +230,16 @@ struct ArraySnap {
     // block the staged count, the index of its first bstage entry and the
     // first staged slot (bsrc), per staged row of cells its first slot and
     // staging offset | length << 16 (brow), per staged particle its slot and
-    // cell (bstage).  As destinations: per block their count and the index of
+    // cell (bstage); the blocks that stage any (blist).  As destinations: per block their count and the index of
     // the first bdest entry (bdst), per destination its slot and cell (bdest).
     int4 *bsrc = nullptr;
+    int *blist = nullptr;
     int2 *bdst = nullptr, *brow = nullptr, *bstage = nullptr, *bdest = nullptr;
     int64_t brick_cap = 0, brow_cap = 0, bstage_cap = 0, bdest_cap = 0;
     // largest staged count and largest count of destinations of a block,
-    // staged particles of all blocks; whether this build has their bstage
-    int b_tmax = 0, b_dmax = 0;
+    // blocks that stage any particle, staged particles of all blocks; whether
+    // this build has their bstage
+    int b_tmax = 0, b_dmax = 0, b_blocks = 0;
     int64_t b_staged = 0;
     bool b_table = false;
 };
@@ -466,8 +468,8 @@ int record_refresh(sph_ctx *ctx, int array, const sph_array_view *view);
 // brick-staged pair passes (bricks.cu)
 constexpr int kMaxBrickArrays = 16;
 // statistics of an array's brick tables: largest staged count and largest
-// count of destinations of a block, destinations in all, (unused,) staged
-// particles in all (64 bits)
+// count of destinations of a block, destinations in all, blocks that stage any
+// particle, staged particles in all (64 bits)
 constexpr int kBrickStats = 6;
 void brick_geometry(sph_ctx *ctx);
 int brick_count(sph_ctx *ctx, int a, unsigned *stats);

@@ -396,3 +396,54 @@ def test_records_found_from_rows_give_the_same_bits(env):
     _need_gpu()
     rows = _hash_masses(SPH_BRICK_STAGE_TABLE="0", **env)
     assert rows == _hash_masses(**env)
+
+
+def _with_far_particles(props, far):
+    """Four particles of a 2D set moved far out, one to each quadrant."""
+    out = {k: v.copy() for k, v in props.items()}
+    for j, (sx, sy) in enumerate(((1, 1), (-1, 1), (1, -1), (-1, -1))):
+        out["x"][7 * j], out["y"][7 * j] = sx * far * (1 + 0.01 * j), sy * far * (1 + 0.01 * j)
+        out["u"][7 * j] = out["v"][7 * j] = 0.0
+    return out
+
+
+def _best_us(f, passes=20, rounds=8):
+    import time
+    f()
+    best = float("inf")
+    for _ in range(rounds):
+        torch.cuda.synchronize()
+        t = time.perf_counter()
+        for _ in range(passes):
+            f()
+        torch.cuda.synchronize()
+        best = min(best, (time.perf_counter() - t) / passes * 1e6)
+    return best
+
+
+def test_a_box_of_empty_bricks(monkeypatch):
+    """Four particles far from a drop make a box of 43 000 bricks, nearly all
+    empty: the step is the oracle's, and the empty bricks cost less than the
+    rest of it (a build under three times, a step under four times that of the
+    drop by itself)."""
+    _need_gpu()
+    monkeypatch.setenv("PYSPH_GB300_BRICKS", "1")
+    drop = W.elliptical_drop(dx=0.025, c0=100.0)
+    build, step = [], []
+    for props in (drop, _with_far_particles(drop, 40.0)):
+        s, particles = W.setup_drop(API, props, c0=100.0)
+        s.integrator.integrate(1e-6)
+        assert particles.cell_manager.brick_pass_count() > 0
+        pa = particles.arrays[0]
+        prob = oracle.Problem({"fluid": props}, oracle.drop_ops(c0=100.0), dim=2)
+        prob.integrate_euler(1e-6)
+        ref = prob.arrays["fluid"]
+        for p in ("rho", "p"):
+            assert normwise(pa.get(p), ref[p]) < TOL, p
+        for p in ("u", "v"):
+            assert normwise(pa.get(p) - props[p], ref[p] - props[p]) < TOL, p
+        step.append(_best_us(lambda: s.integrator.integrate(1e-7)))
+        build.append(_best_us(lambda: particles.cell_manager.rebuild(check_jump=False)))
+    print("build us %s, step us %s" % (build, step))
+    assert build[1] < 3.0 * build[0]
+    assert step[1] < 4.0 * step[0]
