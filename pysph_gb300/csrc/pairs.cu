@@ -784,8 +784,7 @@ __global__ void __launch_bounds__(kPairBlock) k_features(const __grid_constant__
     }
 }
 
-// The same features with one warp per destination (no periodic axis or
-// symmetry plane).  A list of up to 32 entries, the ordinary case: lane k
+// The same features by warps (no periodic axis or symmetry plane).  A list of up to 32 entries, the ordinary case: lane k
 // takes entry k with its whole record, counts the smaller squared distances
 // of the warp's entries (four to a shared-memory load; of equal ones the
 // earlier entry, whose slot is the smaller, comes first) and writes that row.
@@ -847,22 +846,22 @@ struct FeatRow {
 
 // a destination by the sort of its chunks (all lanes, the same s)
 template <int KX>
-__device__ __noinline__ void features_sorted(const FeatureArgs &A, int64_t s) {
+__device__ __forceinline__ void features_sort(const FeatureArgs &A, int64_t s) {
     constexpr int NN = SPH_MLP_NNBR, NC = SPH_MLP_NCH;
     static_assert(NN == 32, "one lane per kept neighbour");
     const int lane = threadIdx.x & 31;
     DestPos d;
-    if (!load_dest(A.g, A.d, (int)s, d)) return;
+    const bool real = load_dest(A.g, A.d, (int)s, d);
     const SrcDev &S = A.s;
     const float csf = A.g.cs_f;
-    const int listed = S.ncnt[s];
     constexpr uint64_t none = ~0ull;
     uint64_t best = none;
     // offsets carried by neighbours found by the traversal (flag set)
     float crx = 0.f, cry = 0.f;
     bool carried = false;
-    {
+    if (real) {
         using C = Code<KX>;
+        const int listed = S.ncnt[s];
         const int m = min(listed, A.cap);
         auto candidate = [&](int k) {
             uint64_t key = none;
@@ -943,15 +942,35 @@ __device__ __noinline__ void features_sorted(const FeatureArgs &A, int64_t s) {
     if (A.out_f) row.store_f(A.out_f + at);
 }
 
+// One destination per warp, for sets whose lists are mostly longer than 32 (the
+// sort is a long chain: more warps in flight, and six blocks per SM, 40
+// registers, count more than the decoding that every lane repeats).  110 592
+// destinations in 3D 135 us; with up to eight destinations per warp and the
+// sort as a call 209.  20 081 in 2D, 50 neighbours, first lists over-full, 100
+// against 165.
+template <int KX>
+__global__ void __launch_bounds__(256, 6) k_features_long(const __grid_constant__ FeatureArgs A) {
+    const int64_t s = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    if (s >= A.d.n || gated_off(A.gate)) return;
+    features_sort<KX>(A, s);
+}
+
+// the same as a call, for the few longer lists of k_features_warp
+template <int KX>
+__device__ __noinline__ void features_sorted(const FeatureArgs &A, int64_t s) {
+    features_sort<KX>(A, s);
+}
+
 // Up to kFeatDests destinations per warp: lane i reads and decodes
 // destination i (once, not in every lane), then the warp takes them one after
 // the other, the next one's list entries on their way meanwhile.  Bound by
 // issue and by the latency of the dependent gathers: 60 us at 80 000
-// destinations in 2D with every list sorted and every lane decoding, 33 so.
+// destinations in 2D with every list sorted and every lane decoding, 30 so
+// (call of features() 50 -> 30).
 // As many per warp as fill the chip, so that a small simulation's chain stays
 // short.  With 1 / 2 / 4 / 8: 10 200 destinations 11.3 / 8.4 / 9.1 / 12.1 us,
-// 20 000 16.7 / 14.0 / 12.5 / 15.0, 41 000 28 / 22 / 19 / 21, 80 000 52 / 40 /
-// 34 / 33.
+// 20 000 16.7 / 14.0 / 12.5 / 15.0, 41 000 28 / 22 / 19 / 21, 80 000 42 / 33 /
+// 30 / 30, 196 000 124 / 85 / 69 / 65.
 constexpr int kFeatDests = 8;
 constexpr int64_t kFeatWarps = 152 * 40;     // resident on the chip
 
@@ -967,12 +986,13 @@ __global__ void __launch_bounds__(256, 5) k_features_warp(const __grid_constant_
     __shared__ Dest s_dest[8][kFeatDests];
     __shared__ uint4 s_key[8][8];
     __shared__ uint4 s_row[8][NN * NC / 8];
+    __shared__ unsigned s_longer[8];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int64_t s0 = (blockIdx.x * (int64_t)8 + wid) * A.per;
-    if (s0 >= A.d.n || gated_off(A.gate)) return;
+    if (gated_off(A.gate)) return;
     const SrcDev &S = A.s;
     const float csf = A.g.cs_f;
-    const int nd = (int)min((int64_t)A.per, A.d.n - s0);
+    const int nd = (int)max((int64_t)0, min((int64_t)A.per, A.d.n - s0));
     const int limit = min(32, A.cap);
     if (lane < nd) {
         DestPos d;
@@ -991,7 +1011,7 @@ __global__ void __launch_bounds__(256, 5) k_features_warp(const __grid_constant_
     uint4 *keys = s_key[wid];
     uint32_t *row = reinterpret_cast<uint32_t *>(s_row[wid]);
     const uint32_t *lst = S.nbr + s0 + (int64_t)lane * A.stride;
-    uint32_t e = lane < min(s_dest[wid][0].listed, limit) ? lst[0] : 0u;
+    uint32_t e = nd > 0 && lane < min(s_dest[wid][0].listed, limit) ? lst[0] : 0u;
     unsigned longer = 0;
 #pragma unroll 1
     for (int i = 0; i < nd; ++i) {
@@ -1053,7 +1073,22 @@ __global__ void __launch_bounds__(256, 5) k_features_warp(const __grid_constant_
         if (A.out_bf && lane < NN * NC / 8)
             reinterpret_cast<uint4 *>(A.out_bf + at)[lane] = s_row[wid][lane];
     }
-    for (; longer; longer &= longer - 1) features_sorted<KX>(A, s0 + (__ffs(longer) - 1));
+    // the longer lists of the block, dealt out to its warps (they come in clumps,
+    // and consecutive destinations are neighbours; every warp its own: 80 000
+    // particles at random, 18 neighbours, 46 us against 36)
+    if (lane == 0) s_longer[wid] = longer;
+    if (!__syncthreads_or(longer != 0)) return;
+    for (int w = 0, k = wid; w < 8; ++w) {
+        unsigned m = s_longer[w];
+        const int c = __popc(m);
+        for (; k < c; k += 8) {
+            // (the k-th set bit, past those this warp has dropped)
+            unsigned q = m;
+            for (int i = 0; i < k; ++i) q &= q - 1;
+            features_sorted<KX>(A, (blockIdx.x * (int64_t)8 + w) * A.per + (__ffs(q) - 1));
+        }
+        k -= c;
+    }
 }
 
 DestDev make_dest(const ArraySnap &D) {
@@ -1555,6 +1590,24 @@ int rates_pass(sph_ctx *ctx, int dst, const sph_source_term *terms, int nterms,
     return SPH_OK;
 }
 
+// Entries of a list in the most populous block of the source's build (its
+// particles per cell there times the cells of the list sphere): what an
+// ordinary list of the set holds.  0 where the build has no blocks.
+double expected_list(const sph_ctx *ctx, const ArraySnap &S) {
+    const Grid &g = ctx->grid;
+    const BrickGeom &bk = ctx->bricks;
+    if (!ctx->bricks_ready || S.b_tmax <= 0) return 0.0;
+    // (the grid's border of k cells is empty)
+    auto span = [](int edge, int parts, int n, int k) {
+        return (double)std::max(1, std::min((edge + parts - 1) / parts + 2 * k, n - 2 * k));
+    };
+    const double cells = span(bk.bx, bk.px, g.nx, g.kx) * span(bk.by, bk.py, g.ny, g.ky) *
+                         span(bk.bz, bk.pz, g.nz, g.kz);
+    const double r = (ctx->build_h * g.radius_scale + g.skin) * g.inv_cs;
+    const double sphere = g.kz > 0 ? 4.1887902 * r * r * r : (g.ky > 0 ? 3.1415927 * r * r : 2.0 * r);
+    return S.b_tmax / cells * sphere;
+}
+
 int features_pass(sph_ctx *ctx, int dst, int src, const sph_mlp_feature_params *prm,
                   uint16_t *out_bf, float *out_f) {
     if (!ctx->built) return set_error(SPH_ERR_STATE, "features: no neighbour build");
@@ -1589,15 +1642,27 @@ int features_pass(sph_ctx *ctx, int dst, int src, const sph_mlp_feature_params *
     if (D.n == 0) return SPH_OK;
     const int b = blocks_for(D.n);
     const bool ext = a.g.periodic || a.g.symmetric;
-    // one warp per destination (environment SPH_FEATURES_THREAD=1, read at
-    // every call: one thread per destination)
+    // several destinations per warp where lists of 32 and less are the rule, one
+    // where they are longer or nothing is known of them.  The line, us with
+    // several / with one: 80 000 particles at random, 21.6 entries expected 36 /
+    // 50, 24.2 44 / 53, 26.1 56 / 60, 30.4 82 / 70; 20 000 (25 is what the host
+    // takes) 21.2 26 / 26, 24.1 28 / 27, 25.3 34 / 28, 30.6 44 / 29; lattice of
+    // 80 381, h / spacing 1.3 31 / 50, 1.5 42 / 52.  Dense clumps too small to show
+    // in a block's mean show in the longest list that the host has seen (a third
+    // of the particles in clumps 78 / 60).
+    // Environment SPH_FEATURES_THREAD=1, read at every call: one thread per
+    // destination.
+    const double expect = expected_list(ctx, ctx->arrays[src]);
+    const bool short_lists = expect > 0.0 && expect <= 24.0 && L->seen_max <= 48;
     const char *env_thread = getenv("SPH_FEATURES_THREAD");
     const bool per_thread = env_thread && atoi(env_thread) > 0;
     a.per = (int)std::min<int64_t>(kFeatDests, 1 + D.n / kFeatWarps);
     const int bw = (int)((D.n + 8 * a.per - 1) / (8 * a.per));
+    const int bl = (int)((D.n + 7) / 8);
 #define FLAUNCH(K) (ext ? k_features<K, true><<<b, kPairBlock, 0, ctx->stream>>>(a) \
                     : per_thread ? k_features<K, false><<<b, kPairBlock, 0, ctx->stream>>>(a) \
-                                 : k_features_warp<K><<<bw, 256, 0, ctx->stream>>>(a))
+                    : short_lists ? k_features_warp<K><<<bw, 256, 0, ctx->stream>>>(a) \
+                                  : k_features_long<K><<<bl, 256, 0, ctx->stream>>>(a))
     switch (code_variant(ctx)) {
         case 1: FLAUNCH(1); break;
         case 2: FLAUNCH(2); break;

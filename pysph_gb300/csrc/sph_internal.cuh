@@ -752,10 +752,10 @@ __device__ __forceinline__ void for_neighbours(const Grid &g, const SrcDev &S, c
             const int lo = some ? __ldg(cst + c0 + rlo) : 0;
             const int hi = some ? __ldg(cst + c0 + rhi + 1) : 0;
             const float wshift = (float)(wrap * g.nx);
-            const int len = S_ > 1 ? __reduce_max_sync(mask, hi - lo) : hi - lo;
-            for (int t = 0; t < len; t += S_) {
+            const int end = S_ > 1 ? lo + __reduce_max_sync(mask, hi - lo) : hi;
+            for (int j0 = lo; j0 < end; j0 += S_) {
                 // (a lane past its row takes some source, not listed)
-                const int jt = lo + t + (S_ > 1 ? (int)(threadIdx.x % S_) : 0);
+                const int jt = j0 + (S_ > 1 ? (int)(threadIdx.x % S_) : 0);
                 const bool in = S_ == 1 || jt < hi;
                 const int j = in ? jt : 0;
                 const float4 pj = __ldg(S.pm + j);

@@ -404,3 +404,38 @@ def test_trained_network_beats_no_network():
     err_zero = float(((run(zero) - plain).abs() / plain).max())
     print("density error: trained %.3g, without the term %.3g" % (err_net, err_zero))
     assert err_net < 0.5 * err_zero
+
+
+@pytest.mark.parametrize("clumps", [0, 40])
+@pytest.mark.parametrize("n,dim,hfac", [(900, 2, 3.0), (9000, 2, 1.8), (9000, 3, 1.2), (60000, 3, 1.2),
+                                        (60000, 2, 1.2)])
+def test_feature_rows_of_long_lists(n, dim, hfac, clumps, monkeypatch):
+    """Sets whose lists are longer than 32 as a rule, in 2D and 3D, and sets
+    of short lists with clumps of long ones: the rows of one thread per
+    destination, with lists that overflow their first capacity and after a
+    build that knows the counts."""
+    _need_gpu()
+    side = int(round(n ** (1.0 / dim)))
+    dx = 1.0 / side
+    rng = np.random.default_rng(n + clumps)
+    g = dx * (np.arange(side) + 0.5)
+    pos = [c.ravel() + 0.2 * dx * rng.uniform(-1, 1, side ** dim) for c in np.meshgrid(*[g] * dim)]
+    n = pos[0].size
+    for k in range(clumps):
+        a = rng.integers(0, n - 50)
+        for c in pos:
+            c[a:a + 50] = c[a] + 0.3 * dx * rng.uniform(-1, 1, 50)
+    props = dict(zip("xyz", pos))
+    props.update(h=np.full(n, hfac * dx), m=np.full(n, dx ** dim), rho=np.ones(n),
+                 p=rng.uniform(0, 1, n), cs=np.full(n, 100.0), u=rng.normal(0, 1, n),
+                 v=rng.normal(0, 1, n))
+    pa = API.base.get_particle_array(name="fluid", type=API.base.ParticleType.Fluid, **props)
+    cm = API.base.Particles(arrays=[pa]).cell_manager
+    for known in (False, True):
+        if known:
+            cm.rebuild(check_jump=False)
+        rows = {}
+        for thread in ("1", "0"):
+            monkeypatch.setenv("SPH_FEATURES_THREAD", thread)
+            rows[thread] = L.features(cm, pa, L.Normalisation(100.0), raw=True).clone()
+        assert torch.equal(rows["1"], rows["0"])
