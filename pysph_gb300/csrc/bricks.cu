@@ -36,10 +36,10 @@
 // S = 2 or 4 neighbouring threads (lanes) share a destination, lane s takes
 // the list's groups s, s + S, ..., and the groups' sums are folded in the
 // list's order (shuffles), so the result is the same bit for bit; the bricks
-// are divided into parts (blocks of their own, with the brick's origin).  (Two
-// source masses: whether a block reads two records per pair or three is its
-// own matter, and a part may hold one mass where its brick holds two; the last
-// bit of the viscosity's sound speed then differs.)
+// are divided into parts (blocks of their own, with the brick's origin).  (Whether a
+// block reads two records per pair or three is its own matter: a part may hold
+// one source mass where its brick holds two, or fit the shared memory where its
+// brick does not.  The last bit of the viscosity's sound speed then differs.)
 //
 // The neighbour relation is the reference's: strict r^2 < (radius_scale
 // h)^2, decided in FP32 outside a +-1e-5 relative band around the threshold
@@ -1001,9 +1001,13 @@ __device__ __forceinline__ void density_dest(const BrickDensityArgs &A, const Sr
     }
 }
 
-// Destinations past one per column of the block (few: blocks are launched
-// with the threads of an ordinary brick), shared by four lanes each.  A call
-// of its own, so that the passes keep its registers out of their loops.
+// Destinations past one per column of the block: a thread each while more than a
+// quarter of the block's threads have one, the last ones shared by four lanes
+// each.  (A wide support has a thousand destinations and more in a brick: RK2
+// step of 49 091 particles in 2D, h / dx 4, 422 us, with four lanes for all of
+// them 685; h / dx 1.7, some 120 past the block's 320 threads, 84, with four
+// lanes up to half the block 92.)  A call of its own, so that the passes keep
+// its registers out of their loops.
 template <bool STAGED, bool TABLE>
 __device__ __noinline__ void density_more(const BrickDensityArgs &A, int first) {
     constexpr int S = 4;
@@ -1013,8 +1017,17 @@ __device__ __noinline__ void density_more(const BrickDensityArgs &A, int first) 
     const SrcRecords<STAGED, TABLE> R =
         make_records<STAGED, TABLE>(A.sm, A.s, A.g.cs_f, stage_tab<TABLE>(A, sh), sh.x, 0.f);
     const uint4 *lgrp = reinterpret_cast<const uint4 *>(A.nbr) + (size_t)dh.y * (A.cap >> 3);
-    const int lane = threadIdx.x % S;
-    for (int r0 = first; r0 < dh.x; r0 += blockDim.x / S) {
+    const int lane = threadIdx.x % S, nt = blockDim.x;
+    int r0 = first;
+    for (; dh.x - r0 > nt / 4; r0 += nt) {
+        const int d = r0 + threadIdx.x;
+        if (d >= dh.x) continue;
+        DestPre p;
+        dest_prefetch<1>(A.d, A.g.cs_f, A.d.bdest[dh.y + d], A.cnt + dh.y, lgrp, A.cap, dh.x, d, 0,
+                         p);
+        density_dest<1, STAGED, TABLE>(A, R, lgrp + d, dh.x, 0, p, 0xffffffffu);
+    }
+    for (; r0 < dh.x; r0 += nt / S) {
         const int d = r0 + threadIdx.x / S;
         const unsigned mask = __ballot_sync(0xffffffffu, d < dh.x);
         if (d >= dh.x) continue;
@@ -1360,8 +1373,18 @@ __device__ __noinline__ void rates_more(const BrickRatesArgs &A, float mb, int f
     const SrcRecords<STAGED, TABLE> R = make_records<STAGED, TABLE>(A.sm, A.s, A.g.cs_f, stage_tab<TABLE>(A, sh), sh.x,
                                                       0.5f * A.alpha);
     const uint4 *lgrp = reinterpret_cast<const uint4 *>(A.nbr) + (size_t)dh.y * (A.cap >> 3);
-    const int lane = threadIdx.x % S;
-    for (int r0 = first; r0 < dh.x; r0 += blockDim.x / S) {
+    const int lane = threadIdx.x % S, nt = blockDim.x;
+    int r0 = first;
+    for (; dh.x - r0 > nt / 4; r0 += nt) {
+        const int d = r0 + threadIdx.x;
+        if (d >= dh.x) continue;
+        DestPre p;
+        dest_prefetch<1>(A.d, A.g.cs_f, A.d.bdest[dh.y + d], A.cnt + dh.y, lgrp, A.cap, dh.x, d, 0,
+                         p);
+        rates_dest<1, XSPH, ETA0, FAST, STAGED, TABLE>(A, R, mb, lgrp + d, dh.x, 0, p,
+                                                       A.d.velh[p.s], A.d.st[p.s], 0xffffffffu);
+    }
+    for (; r0 < dh.x; r0 += nt / S) {
         const int d = r0 + threadIdx.x / S;
         const unsigned mask = __ballot_sync(0xffffffffu, d < dh.x);
         if (d >= dh.x) continue;

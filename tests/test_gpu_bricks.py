@@ -447,3 +447,52 @@ def test_a_box_of_empty_bricks(monkeypatch):
     print("build us %s, step us %s" % (build, step))
     assert build[1] < 3.0 * build[0]
     assert step[1] < 4.0 * step[0]
+
+
+_HASH_WIDE = r'''
+import sys, hashlib
+sys.path.insert(0, ".")
+import pysph_gb300
+from pysph_gb300 import workloads as W
+api = pysph_gb300.api()
+h = hashlib.sha256()
+def run(s, particles, dt, names):
+    for _ in range(2):
+        s.integrator.integrate(dt)
+    particles.cell_manager.rebuild(check_jump=False)
+    s.integrator.integrate(dt)
+    assert particles.cell_manager.brick_pass_count() > 0
+    for f in names:
+        h.update(particles.arrays[0].get(f).tobytes())
+for hdx in (1.7, 2.2, 4.0):
+    run(*W.setup_drop(api, W.elliptical_drop(dx=0.02, hdx=hdx, c0=100.0), c0=100.0), 1e-6,
+        ("x", "y", "u", "v", "rho", "p", "cs"))
+run(*W.setup_cube(api, W.cube_lattice(8000, hdx=2.0, seed=5)), 1e-5,
+    ("x", "y", "z", "u", "v", "w", "rho", "p", "cs"))
+print(h.hexdigest())
+'''
+
+
+_ONE = {"SPH_BRICK_LANES": "1"}
+
+
+@pytest.mark.parametrize("records,envs", [
+    ("1", [_ONE, dict(_ONE, SPH_BRICK_MAX_THREADS="64"), dict(_ONE, SPH_BRICK_MAX_THREADS="512")]),
+    ("0", [{}, _ONE, dict(_ONE, SPH_BRICK_MAX_THREADS="64"),
+           dict(_ONE, SPH_BRICK_MAX_THREADS="512"), {"SPH_BRICK_LANES": "2"}])],
+    ids=["threads", "threads-and-lanes"])
+def test_wide_supports_give_the_same_bits(records, envs):
+    """Bricks with more destinations than the block has threads -- a few more,
+    and several times as many -- in rounds of a thread each and of four lanes:
+    the same bits whatever the block's threads, and its lanes (with three
+    records per pair: a part of a brick can be small enough to stage, and so
+    read two, where the brick is not)."""
+    _need_gpu()
+    seen = set()
+    for env in envs:
+        e = dict(os.environ, PYSPH_GB300_BRICKS="1", SPH_BRICK_TWO_RECORDS=records, **env)
+        r = subprocess.run([sys.executable, "-c", _HASH_WIDE], cwd=ROOT, env=e,
+                           capture_output=True, text=True, timeout=600)
+        assert r.returncode == 0, r.stderr[-3000:]
+        seen.add(r.stdout.split()[-1])
+    assert len(seen) == 1
