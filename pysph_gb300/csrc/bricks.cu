@@ -1749,8 +1749,10 @@ void brick_geometry(sph_ctx *ctx) {
     // build.  Measured, rates + density in us at 1 / 2 / 4 lanes -- 3D: 4 096
     // particles 26.3 / 22.4 / 19.1, 8 000 28.9 / 23.8 / 22.3, 21 952 29.0 /
     // 26.6 / 35.6, 64 000 50.3 / 49.6 / 68.2; 2D: 5 025 18.2 / 17.8 / 15.9,
-    // 10 300 17.8 / 16.9 / 15.6, 20 106 17.9 / 18.4 / 22.4.  Environment SPH_BRICK_LANES forces the lanes (to measure them, and
-    // to test them at any size).
+    // 10 300 17.8 / 16.9 / 15.6, 20 106 17.9 / 18.4 / 22.4.  In 1D, whose lists are
+    // short, two: RK2 step of 4 000 with h / dx 2 77 / 77 / 92, with 3 93 / 80 /
+    // 94, with 6 119 / 104 / 104.  Environment SPH_BRICK_LANES forces the lanes (to
+    // measure them, and to test them at any size).
     static int force_lanes = -1;
     if (force_lanes < 0) {
         const char *l = getenv("SPH_BRICK_LANES");
@@ -1760,7 +1762,7 @@ void brick_geometry(sph_ctx *ctx) {
     int64_t n = 0;
     for (const ArraySnap &A : ctx->arrays) n = std::max(n, A.n);
     bk.lanes = force_lanes ? force_lanes
-                           : (n < 12000 ? 4 : (g.kz > 0 && n < 40000 ? 2 : 1));
+                           : (n < 12000 ? (g.ky > 0 || g.kz > 0 ? 4 : 2) : (g.kz > 0 && n < 40000 ? 2 : 1));
     const int64_t whole = (int64_t)((g.nx + bk.bx - 1) / bk.bx) * ((g.ny + bk.by - 1) / bk.by) *
                           ((g.nz + bk.bz - 1) / bk.bz);
     if (!force_lanes && whole * bk.lanes > (g.kz > 0 ? kLaneBlocks3 : kLaneBlocks2)) bk.lanes = 1;

@@ -496,3 +496,53 @@ def test_wide_supports_give_the_same_bits(records, envs):
         assert r.returncode == 0, r.stderr[-3000:]
         seen.add(r.stdout.split()[-1])
     assert len(seen) == 1
+
+
+_HASH_1D = r'''
+import sys, hashlib
+sys.path.insert(0, ".")
+import numpy as np, pysph_gb300
+api = pysph_gb300.api()
+base, sph, solver = api.base, api.sph, api.solver
+Fluid = base.ParticleType.Fluid
+h = hashlib.sha256()
+for n, hdx in ((1, 1.2), (50, 1.2), (700, 2.0), (4000, 3.0)):
+    x = (np.arange(n) + 0.5) / n
+    pa = base.get_particle_array(name="gas", type=Fluid, x=x, m=np.full(n, 1.0 / n),
+                                 h=np.full(n, hdx / n), rho=np.ones(n), u=0.1 * np.sin(20 * x),
+                                 cs=np.ones(n))
+    particles = base.Particles(arrays=[pa])
+    s = solver.Solver(dim=1, integrator_type=solver.RK2Integrator)
+    s.add_operation(solver.SPHOperation(sph.SPHRho.withargs(), on_types=[Fluid],
+                                        from_types=[Fluid], updates=["rho"], id="density"))
+    s.add_operation(solver.SPHOperation(sph.TaitEquation.withargs(co=1.0, ro=1.0),
+                                        on_types=[Fluid], updates=["p", "cs"], id="eos"))
+    s.add_operation(solver.SPHIntegration(sph.SPHPressureGradient.withargs(dim=1),
+                                          on_types=[Fluid], from_types=[Fluid], updates=["u"],
+                                          id="pgrad"))
+    s.add_operation(solver.SPHIntegration(
+        sph.MonaghanArtificialVsicosity.withargs(alpha=0.1, beta=0.0), on_types=[Fluid],
+        from_types=[Fluid], updates=["u", "v", "w"], id="avisc"))
+    s.add_operation_step([Fluid])
+    s.setup_integrator(particles)
+    for _ in range(4):
+        s.integrator.integrate(0.05 / n)
+    assert particles.cell_manager.brick_pass_count() > 0
+    for f in ("x", "u", "rho", "p", "cs"):
+        h.update(pa.get(f).tobytes())
+print(h.hexdigest())
+'''
+
+
+def test_lanes_in_1d_give_the_same_bits():
+    """1D sets, of one particle upwards: as they come, and with one, two and
+    four threads per destination."""
+    _need_gpu()
+    seen = set()
+    for env in ({}, {"SPH_BRICK_LANES": "1"}, {"SPH_BRICK_LANES": "2"}, {"SPH_BRICK_LANES": "4"}):
+        e = dict(os.environ, PYSPH_GB300_BRICKS="1", **env)
+        r = subprocess.run([sys.executable, "-c", _HASH_1D], cwd=ROOT, env=e,
+                           capture_output=True, text=True, timeout=600)
+        assert r.returncode == 0, r.stderr[-3000:]
+        seen.add(r.stdout.split()[-1])
+    assert len(seen) == 1
