@@ -1637,7 +1637,7 @@ BrickSrcDev make_bsrc(const ArraySnap &S) {
     BrickSrcDev s;
     s.pm = S.pm; s.velh = S.velh; s.st = S.st; s.scx = S.scx;
     s.cstart = S.cstart; s.perm = S.perm;
-    s.bsrc = S.bsrc; s.brow = S.brow; s.bstage = S.b_table ? S.bstage : nullptr;
+    s.bsrc = S.bsrc; s.brow = S.brow; s.bstage = S.bstage;
     s.x = S.view.x; s.y = S.view.y; s.z = S.view.z;
     return s;
 }
@@ -1785,25 +1785,21 @@ void brick_geometry(sph_ctx *ctx) {
 int brick_count(sph_ctx *ctx, int a, unsigned *stats) {
     ArraySnap &A = ctx->arrays[a];
     const BrickGeom &bk = ctx->bricks;
-    if (bk.nbricks > A.brick_cap || !A.bsrc) {
+    // one allocation for the four tables (a new simulation's first step pays for
+    // each), the widest entries first
+    const int64_t nb = bk.nbricks, nrow = nb * bk.nrmax;
+    const int64_t bytes = nb * (int64_t)(sizeof(int4) + sizeof(int2) + sizeof(int)) +
+                          nrow * (int64_t)sizeof(int2);
+    if (bytes > A.bcount_cap || !A.bsrc) {
         cudaFree(A.bsrc);
-        cudaFree(A.bdst);
-        cudaFree(A.blist);
         A.bsrc = nullptr;
-        A.bdst = nullptr;
-        A.blist = nullptr;
-        SPH_CUDA(cudaMalloc(&A.bsrc, sizeof(int4) * bk.nbricks));
-        SPH_CUDA(cudaMalloc(&A.bdst, sizeof(int2) * bk.nbricks));
-        SPH_CUDA(cudaMalloc(&A.blist, sizeof(int) * bk.nbricks));
-        A.brick_cap = bk.nbricks;
+        A.bcount_cap = 0;
+        SPH_CUDA(cudaMalloc((void **)&A.bsrc, bytes));
+        A.bcount_cap = bytes;
     }
-    const int64_t nrow = bk.nbricks * bk.nrmax;
-    if (nrow > A.brow_cap || !A.brow) {
-        cudaFree(A.brow);
-        A.brow = nullptr;
-        SPH_CUDA(cudaMalloc(&A.brow, sizeof(int2) * nrow));
-        A.brow_cap = nrow;
-    }
+    A.bdst = reinterpret_cast<int2 *>(A.bsrc + nb);
+    A.brow = A.bdst + nb;
+    A.blist = reinterpret_cast<int *>(A.brow + nrow);
     const int th = 128, per = th / 32;
     const int blocks = (int)((bk.nbricks + per - 1) / per);
     k_brick_count<<<blocks, th, 0, ctx->stream>>>(ctx->grid, bk, A.cstart, A.bsrc, A.brow, A.bdst,
@@ -1829,31 +1825,33 @@ int brick_fill(sph_ctx *ctx, int a) {
         const char *e = getenv("SPH_BRICK_STAGE_TABLE");
         wanted = (e && atoi(e) == 0) ? 0 : 1;
     }
-    if (A.n > A.bdest_cap || !A.bdest) {
+    // (one allocation, the destinations first)
+    A.b_table = wanted && A.b_tmax < 65535 && A.b_staged < INT32_MAX;
+    const int64_t least = A.n, exact = A.n + A.b_staged;
+    if ((A.b_table ? exact : least) > A.bfill_cap || !A.bdest) {
         cudaFree(A.bdest);
         A.bdest = nullptr;
-        SPH_CUDA(cudaMalloc(&A.bdest, sizeof(int2) * A.n));
-        A.bdest_cap = A.n;
-    }
-    A.b_table = wanted && A.b_tmax < 65535 && A.b_staged < INT32_MAX;
-    if (A.b_table && (A.b_staged > A.bstage_cap || !A.bstage)) {
-        cudaFree(A.bstage);
-        A.bstage = nullptr;
-        A.bstage_cap = 0;
-        // (an eighth more, for the next builds)
-        for (const int64_t want : {A.b_staged + A.b_staged / 8, A.b_staged}) {
-            if (cudaMalloc(&A.bstage, sizeof(int2) * std::max<int64_t>(want, 1)) == cudaSuccess) {
-                A.bstage_cap = want;
-                break;
+        A.bfill_cap = 0;
+        // (an eighth more of the staged entries, for the next builds)
+        for (const int64_t want : {exact + A.b_staged / 8, exact}) {
+            if (!A.b_table || A.bdest) break;
+            if (cudaMalloc((void **)&A.bdest, sizeof(int2) * want) == cudaSuccess) {
+                A.bfill_cap = want;
+            } else {
+                A.bdest = nullptr;
+                cudaGetLastError();     // (not the build's error)
             }
-            A.bstage = nullptr;
-            cudaGetLastError();     // (not the build's error)
         }
-        A.b_table = A.bstage != nullptr;
+        if (!A.bdest) {
+            A.b_table = false;
+            SPH_CUDA(cudaMalloc((void **)&A.bdest, sizeof(int2) * least));
+            A.bfill_cap = least;
+        }
     }
+    A.bstage = A.b_table ? A.bdest + A.n : nullptr;
     k_brick_fill<<<(unsigned)A.b_blocks, 128, 0, ctx->stream>>>(
         ctx->grid, bk, A.cstart, A.scx, A.blist, A.bsrc, A.brow, A.bdst,
-        A.b_table ? A.bstage : nullptr, A.bdest);
+        A.bstage, A.bdest);
     count_launch();
     SPH_LAUNCH_CHECK("k_brick_fill");
     return SPH_OK;

@@ -109,10 +109,6 @@ int sph_ctx_destroy(sph_ctx *c) {
         cudaFree(A.nrm); cudaFree(A.tan);
         cudaFree(A.cstart); cudaFree(A.order); cudaFree(A.refcell); cudaFree(A.pm0); cudaFree(A.inv);
         cudaFree(A.bsrc);
-        cudaFree(A.blist);
-        cudaFree(A.bdst);
-        cudaFree(A.brow);
-        cudaFree(A.bstage);
         cudaFree(A.bdest);
     }
     cudaFree(c->d_box); cudaFree(c->d_hmax); cudaFree(c->d_status);

@@ -235,7 +235,9 @@ struct ArraySnap {
     int4 *bsrc = nullptr;
     int *blist = nullptr;
     int2 *bdst = nullptr, *brow = nullptr, *bstage = nullptr, *bdest = nullptr;
-    int64_t brick_cap = 0, brow_cap = 0, bstage_cap = 0, bdest_cap = 0;
+    // (two allocations: at bsrc, bcount_cap bytes, with bdst, brow and blist; at
+    // bdest, bfill_cap entries, with bstage)
+    int64_t bcount_cap = 0, bfill_cap = 0;
     // largest staged count and largest count of destinations of a block,
     // blocks that stage any particle, staged particles of all blocks; whether
     // this build has their bstage
