@@ -439,3 +439,31 @@ def test_feature_rows_of_long_lists(n, dim, hfac, clumps, monkeypatch):
             monkeypatch.setenv("SPH_FEATURES_THREAD", thread)
             rows[thread] = L.features(cm, pa, L.Normalisation(100.0), raw=True).clone()
         assert torch.equal(rows["1"], rows["0"])
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("n", [1, 64, 1023, 1024, 1025, 2049, 39000])
+def test_third_layer_gradient_over_blocks(n, shift):
+    """dW3 = dy^T h2 and db3 = sum dy at the edges of the kernel's blocks (1024
+    rows in one chain) with h2 on and off the 16-byte grid.  Bound: a value
+    passes the roundings of its block's chain, min(n, 1024), one per block
+    after the first, and dy three (y - t, 1 / n, their product); each is at
+    most 2^-24 of the sum of the magnitudes so far."""
+    _need_gpu()
+    model, _ = _model(3)
+    xg, _ = _x(n, 4)
+    tg = torch.tensor(np.random.default_rng(5).normal(0, 1, (n, M.NOUT)), dtype=torch.float32,
+                      device="cuda")
+    y, cache = model.forward(xg, save=True)
+    room = torch.empty(n * M.NH + 8, dtype=torch.bfloat16, device="cuda")
+    h2 = room[shift:shift + n * M.NH].view(n, M.NH)
+    h2.copy_(cache["h2"])
+    g, _ = model.backward(xg, dict(cache, h2=h2), y, tg)
+    g = g.double().cpu().numpy()
+    dy = ((y.double() - tg.double()) / n).cpu().numpy()
+    h = cache["h2"].double().cpu().numpy()
+    roundings = min(n, 1024) + (n + 1023) // 1024 + 3
+    eps = roundings * 2.0 ** -24 / (1.0 - roundings * 2.0 ** -24)
+    w3, b3 = g[M.OFF_W3:M.OFF_B3].reshape(M.NOUT, M.NH), g[M.OFF_B3:M.NPARAM]
+    assert np.all(np.abs(w3 - dy.T @ h) <= eps * (np.abs(dy).T @ np.abs(h)))
+    assert np.all(np.abs(b3 - dy.sum(0)) <= eps * np.abs(dy).sum(0))
