@@ -546,3 +546,99 @@ def test_lanes_in_1d_give_the_same_bits():
         assert r.returncode == 0, r.stderr[-3000:]
         seen.add(r.stdout.split()[-1])
     assert len(seen) == 1
+
+
+@pytest.mark.parametrize("env", [{"SPH_BRICK_UNSTAGED": "1"}, {"SPH_LIST_CAP": "9"},
+                                 {"SPH_BRICK_UNSTAGED": "1", "SPH_LIST_CAP": "9"},
+                                 {"SPH_BRICK_TWO_RECORDS": "0"}],
+                         ids=["global-records", "over-full-lists", "both", "three-records"])
+def test_one_lane_fallback_paths_match_oracle(env):
+    """The fallback paths with a thread per destination, which larger sets
+    have (these small ones would get two and four)."""
+    _need_gpu()
+    e = dict(os.environ, PYSPH_GB300_BRICKS="1", SPH_BRICK_LANES="1", **env)
+    r = subprocess.run([sys.executable, "-c", _SUB], cwd=ROOT, env=e, capture_output=True,
+                       text=True, timeout=600)
+    assert r.returncode == 0 and "ok" in r.stdout, r.stderr[-3000:]
+
+
+@pytest.mark.parametrize("env", [{"SPH_LIST_CAP": "9"}, {"SPH_BRICK_UNSTAGED": "1"},
+                                 {"SPH_LIST_CAP": "9", "SPH_BRICK_UNSTAGED": "1"}],
+                         ids=["over-full-lists", "global-records", "both"])
+def test_lanes_give_the_same_bits_on_fallback_paths(env):
+    """One, two or four threads per destination agree bit for bit where lists
+    overflow and where records are read from global memory."""
+    _need_gpu()
+    seen = set()
+    for lanes in ("1", "2", "4"):
+        e = dict(os.environ, PYSPH_GB300_BRICKS="1", SPH_BRICK_LANES=lanes, **env)
+        r = subprocess.run([sys.executable, "-c", _HASH], cwd=ROOT, env=e, capture_output=True,
+                           text=True, timeout=600)
+        assert r.returncode == 0, r.stderr[-3000:]
+        seen.add(r.stdout.split()[-1])
+    assert len(seen) == 1
+
+
+_HASH_LISTS_3D = r'''
+import sys, hashlib
+sys.path.insert(0, ".")
+import numpy as np, pysph_gb300
+from pysph_gb300 import workloads as W
+api = pysph_gb300.api()
+base, sph, solver = api.base, api.sph, api.solver
+Fluid = base.ParticleType.Fluid
+h = hashlib.sha256()
+def run(s, particles, dt, names):
+    for _ in range(2):
+        s.integrator.integrate(dt)
+    for a in particles.arrays:
+        for f in names:
+            h.update((a.get(f) + 0.0).tobytes())
+def cube(props, split, variable_h):
+    m = np.arange(len(props["x"])) % 4 == 0
+    parts = [props] if not split else [{k: v[~m] for k, v in props.items()},
+                                       {k: v[m] for k, v in props.items()}]
+    arrays = [base.get_particle_array(name="f%d" % i, type=Fluid, **p) for i, p in enumerate(parts)]
+    particles = base.Particles(arrays=arrays, variable_h=variable_h)
+    s = solver.Solver(dim=3, integrator_type=solver.RK2Integrator)
+    s.add_operation(solver.SPHOperation(sph.SPHRho.withargs(), on_types=[Fluid],
+                                        from_types=[Fluid], updates=["rho"], id="density"))
+    s.add_operation(solver.SPHOperation(sph.TaitEquation.withargs(co=1.0, ro=1.0),
+                                        on_types=[Fluid], updates=["p", "cs"], id="eos"))
+    s.add_operation(solver.SPHIntegration(sph.SPHPressureGradient.withargs(dim=3),
+                                          on_types=[Fluid], from_types=[Fluid],
+                                          updates=["u", "v", "w"], id="pgrad"))
+    s.add_operation(solver.SPHIntegration(
+        sph.MonaghanArtificialVsicosity.withargs(alpha=0.1, beta=0.0), on_types=[Fluid],
+        from_types=[Fluid], updates=["u", "v", "w"], id="avisc"))
+    s.add_operation_step([Fluid])
+    s.setup_integrator(particles)
+    return s, particles
+names = ("x", "y", "z", "u", "v", "w", "rho", "p", "cs")
+for n in (64, 4913):
+    props = W.cube_lattice(n, seed=9, vel_std=0.1)
+    run(*cube(props, True, False), 1e-4, names)
+    run(*cube(W.jitter_h(props), False, True), 1e-4, names)
+drop = W.elliptical_drop(dx=0.06, c0=100.0)
+run(*W.setup_drop(api, W.jitter_h(drop), c0=100.0, variable_h=True), 1e-5, names)
+run(*W.setup_fluid_solver(api, W.circular_patch(dx=0.06)), 1e-5, names)
+strip = W.periodic_strip(dx=0.05, nx=31, ny=7, jitter=0.1)
+run(*W.setup_drop(api, strip, c0=10.0, periodic_domain=base.PeriodicDomain(0.0, 1.55)), 1e-4, names)
+print(h.hexdigest())
+'''
+
+
+@pytest.mark.parametrize("subdiv", [1, 2, 3])
+def test_list_lanes_give_the_same_bits_over_half_widths(subdiv):
+    """One, two, four or eight threads per destination of the list builds and
+    the list-streaming passes, with stencils of one to three cells, in 3D (two
+    arrays; variable h) and in 2D: bit for bit the same."""
+    _need_gpu()
+    seen = set()
+    for lanes in ("1", "2", "4", "8"):
+        e = dict(os.environ, SPH_PAIR_LANES=lanes, PYSPH_GB300_SUBDIV=str(subdiv))
+        r = subprocess.run([sys.executable, "-c", _HASH_LISTS_3D], cwd=ROOT, env=e,
+                           capture_output=True, text=True, timeout=600)
+        assert r.returncode == 0, r.stderr[-3000:]
+        seen.add(r.stdout.split()[-1])
+    assert len(seen) == 1
