@@ -1490,38 +1490,36 @@ __global__ void __launch_bounds__(128) k_brick_count(Grid g, BrickGeom bk, const
     const int64_t b = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5);
     if (b >= bk.nbricks) return;
     const BlockGeo G = block_geo(g, bk, (int)b);
-    // first slot and length of staged row r
-    auto row = [&](int r, int &lo) {
-        lo = 0;
-        if (r >= G.nr) return 0;
-        const int c = ((G.zs0 + r / G.ry) * g.ny + G.ys0 + r % G.ry) * g.nx + G.xs0;
-        lo = cstart[c];
-        return cstart[c + G.lx] - lo;
-    };
-    int len, lo, T = 0, D = 0, first = 0;
+    // an empty block (most of the box of a splash) keeps no rows, and rows before
+    // the first that has anything are zeros: the starts of an empty row's cells
+    // are all the same, so a row of any first slot has nothing in it
+    int2 *rows = brow + b * bk.nrmax;
+    int T = 0, D = 0, first = 0, lo;
     for (int r0 = 0; r0 < G.nr; r0 += 32) {
-        len = row(r0 + lane, lo);
+        const int r = r0 + lane;
+        int len = 0;
+        lo = 0;
+        if (r < G.nr) {
+            const int c = ((G.zs0 + r / G.ry) * g.ny + G.ys0 + r % G.ry) * g.nx + G.xs0;
+            lo = cstart[c];
+            len = cstart[c + G.lx] - lo;
+        }
         const unsigned some = __ballot_sync(0xffffffffu, len > 0);
-        if (T == 0 && some) first = __shfl_sync(0xffffffffu, lo, __ffs(some) - 1);
-        T += __reduce_add_sync(0xffffffffu, len);
+        if (T == 0) {
+            if (!some) continue;
+            first = __shfl_sync(0xffffffffu, lo, __ffs(some) - 1);
+            for (int q = lane; q < r0; q += 32) rows[q] = make_int2(0, 0);
+        }
+        const int inc = warp_scan(len);
+        if (r < G.nr) rows[r] = make_int2(lo, (int)((unsigned)(T + inc - len) | ((unsigned)len << 16)));
+        T += __shfl_sync(0xffffffffu, inc, 31);
     }
-    // an empty block (most of the box of a splash) keeps no rows: its cells'
-    // starts are all the same, so a row of any offset has nothing in it
     if (T == 0) {
         if (lane == 0) {
             bsrc[b] = make_int4(0, 0, 0, 0);
             bdst[b] = make_int2(0, 0);
         }
         return;
-    }
-    int2 *rows = brow + b * bk.nrmax;
-    int at = 0;
-    for (int r0 = 0; r0 < G.nr; r0 += 32) {
-        len = row(r0 + lane, lo);
-        const int inc = warp_scan(len);
-        if (r0 + lane < G.nr)
-            rows[r0 + lane] = make_int2(lo, (int)((unsigned)(at + inc - len) | ((unsigned)len << 16)));
-        at += __shfl_sync(0xffffffffu, inc, 31);
     }
     const int ndr = (G.y1 - G.y0) * (G.z1 - G.z0);
     for (int r0 = 0; r0 < ndr; r0 += 32)
@@ -1540,14 +1538,14 @@ __global__ void __launch_bounds__(128) k_brick_count(Grid g, BrickGeom bk, const
     }
 }
 
-// bstage null: the destinations only (brick_fill)
+// blist null: every block; bstage null: the destinations only (brick_fill)
 __global__ void __launch_bounds__(128) k_brick_fill(Grid g, BrickGeom bk, const int *cstart,
                                                     const float *scx, const int *blist,
                                                     const int4 *bsrc,
                                                     const int2 *brow, const int2 *bdst,
                                                     int2 *bstage, int2 *bdest) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const int b = blist[blockIdx.x];
+    const int b = blist != nullptr ? blist[blockIdx.x] : blockIdx.x;
     const int D = bdst[b].x;
     const BlockGeo G = block_geo(g, bk, b);
     const int2 *rows = brow + (int64_t)b * bk.nrmax;
@@ -1850,8 +1848,8 @@ int brick_fill(sph_ctx *ctx, int a) {
     }
     A.bstage = A.b_table ? A.bdest + A.n : nullptr;
     k_brick_fill<<<(unsigned)A.b_blocks, 128, 0, ctx->stream>>>(
-        ctx->grid, bk, A.cstart, A.scx, A.blist, A.bsrc, A.brow, A.bdst,
-        A.bstage, A.bdest);
+        ctx->grid, bk, A.cstart, A.scx, A.b_blocks < bk.nbricks ? A.blist : nullptr, A.bsrc, A.brow,
+        A.bdst, A.bstage, A.bdest);
     count_launch();
     SPH_LAUNCH_CHECK("k_brick_fill");
     return SPH_OK;

@@ -642,3 +642,48 @@ def test_list_lanes_give_the_same_bits_over_half_widths(subdiv):
         assert r.returncode == 0, r.stderr[-3000:]
         seen.add(r.stdout.split()[-1])
     assert len(seen) == 1
+
+
+_SPARSE_3D = r'''
+import sys, hashlib
+sys.path.insert(0, ".")
+import numpy as np, oracle, pysph_gb300
+from pysph_gb300 import workloads as W
+from tests.golden_util import normwise
+api = pysph_gb300.api()
+props = W.cube_lattice(4096, seed=6)
+rng = np.random.default_rng(8)
+for c in "xyz":                 # a tenth of the cube scattered over a box 3 wide
+    props[c][::10] = rng.uniform(-1.0, 2.0, props[c][::10].size)
+s, particles = W.setup_cube(api, props)
+s.integrator.integrate(1e-4)
+assert particles.cell_manager.brick_pass_count() >= 4
+pa = particles.arrays[0]
+prob = oracle.Problem({"fluid": props}, oracle.cube_ops(), dim=3)
+prob.integrate_rk2(1e-4)
+for p in ("rho", "p"):
+    assert normwise(pa.get(p), prob.arrays["fluid"][p]) < 1e-5, p
+for p in ("x", "u", "w"):
+    assert normwise(pa.get(p) - props[p], prob.arrays["fluid"][p] - props[p]) < 1e-5, p
+h = hashlib.sha256()
+for f in ("x", "y", "z", "u", "v", "w", "rho", "p", "cs"):
+    h.update(pa.get(f).tobytes())
+print(h.hexdigest())
+'''
+
+
+def test_blocks_of_few_occupied_rows():
+    """Bricks of which only some rows of cells, not the first ones, hold
+    anything, beside empty and full ones: the oracle's step, and the same
+    bits with the staged entries from their table and from the rows, with one
+    to four lanes."""
+    _need_gpu()
+    seen = set()
+    for env in ({}, {"SPH_BRICK_STAGE_TABLE": "0"}, {"SPH_BRICK_LANES": "1"},
+                {"SPH_BRICK_LANES": "2"}, {"SPH_BRICK_LANES": "4"}):
+        e = dict(os.environ, PYSPH_GB300_BRICKS="1", **env)
+        r = subprocess.run([sys.executable, "-c", _SPARSE_3D], cwd=ROOT, env=e,
+                           capture_output=True, text=True, timeout=600)
+        assert r.returncode == 0, r.stderr[-3000:]
+        seen.add(r.stdout.split()[-1])
+    assert len(seen) == 1
