@@ -56,19 +56,19 @@ STEP_ALG_BYTES = 694.0
 # FLOPs per neighbour pair: density 24, momentum 72 (FMA = 2)
 PAIR_FLOPS = {"RatesStage": 72.0, "DensityStage": 24.0, "ListStage": 12.0}
 FP32_NOMINAL_TFLOPS = 152 * 128 * 2 * 2.07e9 / 1e12
-# DRAM bytes per particle per launch (from the DRAM throughput and duration of
-# one ncu capture of the 1M-particle lattice, brick-staged passes at cell
+# DRAM bytes per particle per launch (dram__bytes_read.sum + dram__bytes_write.sum
+# of one ncu capture of the 1M-particle lattice, brick-staged passes at cell
 # subdivision 2); the traffic grows with the particle count, so it is scaled
 # by n
-NCU_TRAFFIC_PER_PARTICLE = {"DensityStage": 270.0, "RatesStage": 335.0}
+NCU_TRAFFIC_PER_PARTICLE = {"DensityStage": 268.3, "RatesStage": 329.5}
 # The unit that bounds each pair kernel in the same capture, as a fraction of
 # that unit's peak: the L1 / shared-memory pipe that serves the staged-record
 # reads, with instruction issue behind it
 NCU_LIMITER = {
-    "RatesStage": {"kernel": "k_brates", "unit": "L1 / shared-memory pipe", "frac": 0.783,
-                   "issue_frac": 0.601, "dram_frac": 0.197},
-    "DensityStage": {"kernel": "k_bdensity", "unit": "L1 / shared-memory pipe", "frac": 0.702,
-                     "issue_frac": 0.590, "dram_frac": 0.283},
+    "RatesStage": {"kernel": "k_brates", "unit": "L1 / shared-memory pipe", "frac": 0.786,
+                   "issue_frac": 0.603, "dram_frac": 0.196},
+    "DensityStage": {"kernel": "k_bdensity", "unit": "L1 / shared-memory pipe", "frac": 0.700,
+                     "issue_frac": 0.588, "dram_frac": 0.282},
 }
 
 

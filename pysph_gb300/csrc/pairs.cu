@@ -1124,6 +1124,8 @@ int blocks_for(int64_t n) {
 // pass of n destinations: as many of 8 and 4 as run in one wave (blocks: the
 // resident blocks per SM), else two while the pass is short, where a chain of
 // half the length still counts more than the instructions that are added.
+// (The wave is a little strict: 20 106 destinations are 3 % past one with
+// eight, and take four where the lists alone would be 2 us faster with eight.)
 // Measured (us per pass with 1 / 2 / 4 / 8):
 //   rates (4 blocks), variable h: 5 025 particles 44 / 26 / 17 / 13, 16 000
 //   44 / 27 / 18 / 25, 31 400 45 / 28 / 33 / 45, 100 000 89 / 76 / 89 / 119,
